@@ -30,6 +30,7 @@ constexpr int MAX_SLOTS = 8;
 constexpr int MAX_OUTS = 4;
 constexpr int MAX_N = 5;  // up to degree 4
 constexpr int LANE_ROW_SLOTS = 8;  // value rows the lane kernel's slot tables cover
+constexpr int LANE_MAX_OUT = 4;    // output components of a lane kernel launch
 
 enum ErrorBits : int {
   ERR_UNDECLARED_DEPENDENCY = 1,
@@ -85,6 +86,20 @@ struct CellTables {
   unsigned int val_rows;
   signed char lane_vslot[LANE_ROW_SLOTS];
   signed char lane_gslot[LANE_ROW_SLOTS];
+  // the same by (field, age), for a field's first component, and a block field's first output
+  // component: one constant-bank operand where a callback names its field and age
+  int lane_v[MAX_FIELDS][NAGE];
+  int lane_g[MAX_FIELDS][NAGE];
+  int lane_out[MAX_FIELDS];
+  // gradient terms along d enter the lane kernel's integral as (h_0 / h_d) g_d, on any box:
+  // h_0 / h_d = rsig / 2^63 * 2^rk; rpow2: a power of two (1 on cubes)
+  unsigned long long rsig[3];
+  int rk[3];
+  int rpow2[3];
+  // what the scales add to the exponents of the value terms and of the gradient terms along d,
+  // at a float's exponent position, EXP_BIAS more so that it is never negative
+  unsigned int hadd;
+  unsigned int radd[3];
 };
 
 template <int dim, int degree, typename number = double>
@@ -104,14 +119,19 @@ struct CellCtx {
   // exponents [row][cells per block]; null when the kernel contracts in the arithmetic type
   const long long* vals_fx = nullptr;
   const int* ex_in = nullptr;
-  int cpb = 0;
+  int cpb = 0;  // (the lane kernel's exponents are high words: E at bit 20)
   // Row layout: point q of the thread's cell sits at lc * nq + q, or at q * cpt + lc when cpt > 0
   // (the lane kernel, prismspf/gpu/cell_kernel_lanes.cuh). lean: the lane kernel's all-integer
-  // contractions (value terms stored unweighted, derivatives rounded by to_double_fast), with the
-  // point's index along each direction in qi.
+  // contractions, with the point's index along each direction in qi, its entry in pe and the
+  // entry step from it towards the other points of its lines in step; the submitted terms
+  // (nterm components of a value and dim gradient entries, unweighted) stay in registers.
   int cpt = 0;
   int lean = 0;
   int qi[3] = {0, 0, 0};
+  int pe = 0;
+  int step[3] = {0, 0, 0};
+  int nterm = 0;
+  number term[LANE_MAX_OUT * (1 + dim)];
   // value terms stored unweighted (a kernel integrating them in fixed point), on any layout
   int raw_values = 0;
 };
@@ -147,6 +167,21 @@ class FieldContainer {
 
   template <TensorRank Rank>
   PPF_HD Value<Rank> get_value(unsigned int field_index, DependencyType type) const {
+    if constexpr (lane_capable) {
+      if (ctx.lean) {
+        const int vs = lane_slot(ctx.tab->lane_v, field_index, type);
+        if (vs >= 0) {
+          const number* v0 = ctx.vals + vs * ctx.stride + ctx.pe;
+          if constexpr (Rank == TensorRank::Scalar || dim == 1) {
+            return ScalarValue(v0[0]);
+          } else {
+            Value<Rank> v;
+            for (int c = 0; c < int(dim); ++c) v[c] = v0[c * ctx.stride];
+            return v;
+          }
+        }
+      }
+    }
     const int row = row_of(field_index, type);
     if constexpr (Rank == TensorRank::Scalar || dim == 1) {
       return ScalarValue(row < 0 ? number(0) : nodal(row, ctx.q));
@@ -164,8 +199,22 @@ class FieldContainer {
 
   template <TensorRank Rank>
   PPF_HD Gradient<Rank> get_gradient(unsigned int field_index, DependencyType type) const {
-    const int row = row_of(field_index, type);
     Gradient<Rank> g;
+    if constexpr (lane_capable) {
+      if (ctx.lean) {
+        const int gs = lane_slot(ctx.tab->lane_g, field_index, type);
+        if (gs >= 0) {
+          if constexpr (Rank == TensorRank::Scalar) {
+            for (int d = 0; d < int(dim); ++d) g[d] = lane_deriv(gs, d);
+          } else {
+            for (int c = 0; c < int(dim); ++c)
+              for (int d = 0; d < int(dim); ++d) g[c][d] = lane_deriv(gs + c, d);
+          }
+          return g;
+        }
+      }
+    }
+    const int row = row_of(field_index, type);
     if (row < 0) return g;
     if constexpr (Rank == TensorRank::Scalar) {
       for (int d = 0; d < int(dim); ++d) g[d] = deriv(row, d);
@@ -320,22 +369,39 @@ class FieldContainer {
 
   // --- submissions --------------------------------------------------------------------
   PPF_HD void set_value_term(unsigned int field_index, const ScalarValue& val) {
+    if (ctx.lean) {
+      const int o = lane_component(field_index);
+      if (o >= 0) set_term(o, 0, val.v);
+      return;
+    }
     const int o = out_row(field_index);
     if (o < 0) return;
-    ctx.outs[o * ctx.stride + slot()] = (ctx.lean || ctx.raw_values) ? val.v : val.v * ctx.tab->jxw[ctx.q];
+    ctx.outs[o * ctx.stride + slot()] = ctx.raw_values ? val.v : val.v * ctx.tab->jxw[ctx.q];
     ctx.submitted |= 1 << (2 * ctx.tab->out_of[field_index]);
   }
 
   PPF_HD void set_value_term(unsigned int field_index, const dealii::Tensor<1, dim, ScalarValue>& val) {
+    if (ctx.lean) {
+      const int o = lane_component(field_index);
+      if (o >= 0)
+        for (int c = 0; c < int(dim); ++c) set_term(o, c, 0, val[c].v);
+      return;
+    }
     const int o = out_row(field_index);
     if (o < 0) return;
     for (int c = 0; c < int(dim); ++c)
       ctx.outs[(o + c * (1 + dim)) * ctx.stride + slot()] =
-          (ctx.lean || ctx.raw_values) ? val[c].v : val[c].v * ctx.tab->jxw[ctx.q];
+          ctx.raw_values ? val[c].v : val[c].v * ctx.tab->jxw[ctx.q];
     ctx.submitted |= 1 << (2 * ctx.tab->out_of[field_index]);
   }
 
   PPF_HD void set_gradient_term(unsigned int field_index, const dealii::Tensor<1, dim, ScalarValue>& g) {
+    if (ctx.lean) {
+      const int o = lane_component(field_index);
+      if (o >= 0)
+        for (int d = 0; d < int(dim); ++d) set_term(o, 1 + d, g[d].v);
+      return;
+    }
     const int o = out_row(field_index);
     if (o < 0) return;
     // gradients are stored unscaled: the integration weights (jdt) carry JxW / h_d
@@ -344,6 +410,13 @@ class FieldContainer {
   }
 
   PPF_HD void set_gradient_term(unsigned int field_index, const dealii::Tensor<2, dim, ScalarValue>& g) {
+    if (ctx.lean) {
+      const int o = lane_component(field_index);
+      if (o >= 0)
+        for (int c = 0; c < int(dim); ++c)
+          for (int d = 0; d < int(dim); ++d) set_term(o, c, 1 + d, g[c][d].v);
+      return;
+    }
     const int o = out_row(field_index);
     if (o < 0) return;
     for (int c = 0; c < int(dim); ++c)
@@ -358,6 +431,69 @@ class FieldContainer {
 
  private:
   Ctx& ctx;
+
+  static constexpr bool lane_capable = std::is_same<number, double>::value && degree <= 2;
+
+  // slot of a (field, age) in one of the lane kernel's tables, -1 without one
+  PPF_HD static int lane_slot(const int (&slots)[gpu::MAX_FIELDS][gpu::NAGE], unsigned int field_index,
+                              DependencyType type) {
+    const int age = gpu::age_of(type);
+    return field_index < unsigned(gpu::MAX_FIELDS) && age >= 0 ? slots[field_index][age] : -1;
+  }
+
+  // first output component of a block field in the lane kernel
+  PPF_HD int lane_component(unsigned int field_index) const {
+    const int o = field_index < unsigned(gpu::MAX_FIELDS) ? ctx.tab->lane_out[field_index] : -1;
+    if (o < 0) {
+#ifdef __CUDA_ARCH__
+      atomicOr(ctx.err, int(gpu::ERR_UNDECLARED_SUBMISSION));
+#endif
+    }
+    return o;
+  }
+
+  // entry i (0 value, 1 + d gradient) of scalar component o, or of component c of the vector
+  // field starting at o. The registers are named by constants: a launch with one component (one
+  // vector field) has its only possible o, the others select.
+  PPF_HD void set_term(int o, int i, number v) {
+    if (ctx.nterm == 1) {
+      ctx.term[i] = v;
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < gpu::LANE_MAX_OUT; ++k)
+      if (k < ctx.nterm && k == o) ctx.term[k * (1 + int(dim)) + i] = v;
+  }
+  PPF_HD void set_term(int o, int c, int i, number v) {
+    if (ctx.nterm == int(dim)) {
+      ctx.term[c * (1 + int(dim)) + i] = v;
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < gpu::LANE_MAX_OUT; ++k)
+      if (k < ctx.nterm && k == o + c) ctx.term[k * (1 + int(dim)) + i] = v;
+  }
+
+  // the lane kernel's derivative along d of the row in gradient slot gs: the exact line sum of the
+  // fixed-point values, taken from this point outwards (own value, its neighbour m, the far end f:
+  // the end rows of a Q2 line are +-(4 (m - own) + (own - f)), its middle row f - m), rounded once
+  // with 1/h_d folded in; NaN for a cell holding a non-finite value. (The three rows as one formula
+  // without the branch, which is uniform in a warp, measured slower.)
+  PPF_HD number lane_deriv(int gs, int d) const {
+    const long long* u = ctx.vals_fx + gs * ctx.stride + ctx.pe;
+    const int E = int((unsigned int)ctx.ex_in[gs * ctx.cpb + ctx.lc] >> 20);
+    const int st = ctx.step[d];
+    long long s;
+    if (n > 2 && ctx.qi[d] == 1) {
+      s = u[st] - u[-st];
+    } else {
+      const long long own = u[0];
+      s = n == 2 ? u[st] - own : ((u[st] - own) << 2) + (own - u[2 * st]);
+    }
+    return gpu::fx::to_double_cut(s, E - 1023 - gpu::fx::LANE_TOP_VALUES + ctx.tab->dk[d], ctx.tab->dsig[d],
+                                  ctx.tab->dpow2[d] == 0, E >= gpu::fx::EXP_WIDE, E >= gpu::fx::EXP_NONFINITE,
+                                  ctx.qi[d] == int(degree) ? 0x80000000u : 0u);
+  }
 
   // offset of point p of this thread's cell within a row
   PPF_HD int pt(int p) const { return ctx.cpt ? p * ctx.cpt + ctx.lc : ctx.lc * int(dofs_per_component) + p; }
@@ -394,10 +530,10 @@ class FieldContainer {
         // value rebuilt from the fixed-point copy (exact to 2^-58 of the cell's largest value)
         const int vs = ctx.tab->lane_vslot[row];
         if (vs >= 0) return ctx.vals[vs * ctx.stride + pt(q)];
-        const int E = ctx.ex_in[row * ctx.cpb + ctx.lc];
-        const long long x = ctx.vals_fx[ctx.tab->lane_gslot[row] * ctx.stride + pt(q)];
-        const double v = gpu::fx::to_double_fast(x, E - 1023 - gpu::fx::TOP_VALUES, 1ull << 63, false);
-        return E == gpu::fx::EXP_NONFINITE ? gpu::fx::quiet_nan() : v;
+        const int gs = ctx.tab->lane_gslot[row];
+        const int E = int((unsigned int)ctx.ex_in[gs * ctx.cpb + ctx.lc] >> 20);
+        return gpu::fx::to_double_cut(ctx.vals_fx[gs * ctx.stride + pt(q)], E - 1023 - gpu::fx::LANE_TOP_VALUES,
+                                      1ull << 63, false, E >= gpu::fx::EXP_WIDE, E >= gpu::fx::EXP_NONFINITE);
       }
     }
     return ctx.vals[row * ctx.stride + pt(q)];
@@ -415,29 +551,7 @@ class FieldContainer {
     int stride_d = 1;
     for (int e = 0; e < d; ++e) stride_d *= n;
     if constexpr (std::is_same<number, double>::value && degree <= 2) {
-      if (ctx.lean && ((ctx.tab->fx_rows >> row) & 1u)) {
-        // the lane kernel (rows read as gradients have a fixed-point copy; the test is uniform):
-        // the line's fixed-point values at a point stride of cpt, the exact sum for this point's
-        // position qd on the line, rounded once with 1/h_d folded in; NaN for a cell holding a
-        // non-finite value (block exponent 2047)
-        const int qd = ctx.qi[d];
-        const int E = ctx.ex_in[row * ctx.cpb + ctx.lc];
-        const int sq = stride_d * ctx.cpt;
-        const long long* u =
-            ctx.vals_fx + ctx.tab->lane_gslot[row] * ctx.stride + (ctx.q - qd * stride_d) * ctx.cpt + ctx.lc;
-        long long s;
-        if constexpr (n == 2) {
-          s = u[sq] - u[0];
-        } else {
-          const long long u0 = u[0], u2 = u[2 * sq];
-          const long long a = u2 - u0;
-          const long long b = (u0 + u2 - (u[sq] << 1)) << 1;
-          s = qd == 1 ? a : (qd == 0 ? a - b : a + b);
-        }
-        const double g = gpu::fx::to_double_fast(s, E - 1023 - gpu::fx::TOP_VALUES + ctx.tab->dk[d],
-                                                 ctx.tab->dsig[d], ctx.tab->dpow2[d] == 0);
-        return E == gpu::fx::EXP_NONFINITE ? gpu::fx::quiet_nan() : g;
-      }
+      if (ctx.lean && ((ctx.tab->fx_rows >> row) & 1u)) return lane_deriv(ctx.tab->lane_gslot[row], d);
     }
     const int qd = (ctx.q / stride_d) % n;
     const int base = row * ctx.stride + ctx.lc * int(dofs_per_component) + (ctx.q - qd * stride_d);

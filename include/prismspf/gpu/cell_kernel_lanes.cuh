@@ -1,5 +1,5 @@
-// Lane kernel: the cell loop of an FP64 Q1/Q2 operator on cubic cells with every contraction in
-// exact 64-bit integers, laid out so that one lane of a warp is one cell.
+// Lane kernel: the cell loop of an FP64 Q1/Q2 operator with every contraction in exact 64-bit
+// integers, laid out so that one lane of a warp is one cell.
 //
 // The same per-cell work as cell_kernel (MFOperator::compute_local_operator,
 // src/solvers/mf_operator.cc:34-80, with FieldContainer::reinit_and_eval /
@@ -13,26 +13,35 @@
 //     [point][cell], so every access is a contiguous warp row, a point's position on its lines
 //     is uniform across the warp, and the per-cell block exponents are shared-memory atomics on
 //     32 distinct words, one per thread and row;
-//   * derivatives: exact integer line sums of the nodal values' fixed-point copies, rounded
-//     once by to_double_fast (prismspf/gpu/fixed_point.cuh) with 1/h_d folded in;
-//   * integration: the submitted value term (as h v) and gradient terms of a cell and output
-//     component share one block exponent; every node's integral is the exact integer sum
-//     2^vw(q) X(q) + sum_d 2^wo_d(q) L_d(q) (L_d the Gauss-Lobatto line integral of the
-//     gradient terms along d, the last direction's taken from the thread's own points; 2^vw and
-//     2^wo the integer quadrature weights) rounded once with the scale detJ / (h W^dim): no FP64
-//     instruction outside the user's callback. On GB300 the FP64 pipe retires about two
-//     operations per SM per clock and every FP64 conversion runs on it too, so the integer path
-//     (issue slots) replaces 9-10 FP64 operations per point;
-//   * four block barriers per tile: nodal values and exponents, fixed-point copies, submitted
-//     terms and exponents, their fixed-point copies. The value-row exponents alternate between
-//     two buffers so that clearing the next tile's needs no extra barrier;
-//   * the cell tables and the flat row lists are kernel parameters (constant-bank loads); every
-//     output component is integrated (rows the callback leaves stay zero), so no branch depends
-//     on which terms were submitted; lanes past the last cell recompute the last cell and skip
-//     its scatter.
-// Accuracy: every derivative and every node's integral is one rounding of an exact sum of
-// values quantised to 2^-58 (derivatives) or 2^-52 (integration) of the largest magnitude of
-// their cell and row, as in the other integer-contraction kernels.
+//   * derivatives: exact integer line sums of the nodal values' fixed-point copies, taken from the
+//     point outwards and rounded once with 1/h_d folded in (FieldContainer::lane_deriv);
+//   * integration: the submitted value term (as h_0 v) and gradient terms (as (h_0 / h_d) g_d) of a
+//     cell and output component share one block exponent; with the integer quadrature weights
+//     (1, 1 or 1, 4, 1 per direction) divided out of its node, an integral is the exact sum
+//     x + sum_d L_d, L_d = +-(4 (own + m) - (own + f)) at the ends of a Q2 line and g_0 - g_2 in its
+//     middle: no weight is multiplied in, 25 is the largest coefficient sum, and the terms keep 57
+//     bits below the cell's largest one. It is rounded once with the scale detJ / (h_0 W^dim) and
+//     the node's weight as an exponent. No FP64 instruction outside the user's callback: on GB300
+//     the FP64 pipe retires about two operations per SM per clock and every FP64 conversion runs
+//     on it too, so the integer path (issue slots) replaces 9-10 FP64 operations per point;
+//   * the terms a callback submits stay in registers: with one output component from the callback
+//     through the exponent barrier to the integration (only the gradient rows other threads read
+//     pass through shared memory), with several until they are stored;
+//   * four block barriers per tile: nodal values and exponents, fixed-point copies, the terms'
+//     exponents, their fixed-point copies. The exponents alternate between two buffers so that
+//     resetting the next tile's needs no extra barrier;
+//   * the cell tables and the flat row lists are kernel parameters (constant-bank loads), with the
+//     slots by (field, age) so that a getter's look-up is one operand; every output component is
+//     integrated (rows the callback leaves stay zero), so no branch depends on which terms were
+//     submitted; lanes past the last cell recompute the last cell and skip its scatter.
+// Accuracy: every derivative and every node's integral is one rounding of an exact sum of values
+// cut to 2^-59 (derivatives) or 2^-57 (integration) of the largest magnitude of their cell and row.
+//
+// What bounds it: instruction issue (58-61 % of the slots, the ALU pipe 50-57 % busy, the FP64 pipe
+// 31-55 %; DRAM 4 %). Cahn-Hilliard 64^3 Q2, per launch of the c and the mu block: 130 and 157 us at
+// 444 instructions a point, against 208 and 213 us at 690 with rounded instead of cut conversions,
+// weights as 64-bit shifts and the terms through shared memory, and 243 and 293 us for cell_kernel.
+// Stretched cells (64 x 60 x 52): 105 and 128 us against 188 and 226 us for cell_kernel.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -60,14 +69,13 @@ struct LaneShape {
 };
 constexpr int LANE_CPT = 32;  // cells per tile
 
-// fixed-point top of the integration: |X| <= 2^53 and |L_d| <= 8 * 2^53 keep the weighted sum
-// below 2^53 (2^6 + 3 * 2^4 * 8) < 2^62
+// fixed-point top of the integration where terms are rounded (the ensemble's tiles): |X| <= 2^53
+// and |L_d| <= 8 * 2^53 keep the weighted sum below 2^53 (2^6 + 3 * 2^4 * 8) < 2^62
 constexpr int LANE_TOP_TERMS = 52;
 
 // An operator may ask for a register budget (`cell_lane_min_blocks`, resident blocks per SM);
-// the default aims at about 48 registers a thread (Cahn-Hilliard Q2 3-D: 4 blocks of 288 threads
-// at 46 registers measured 0.210 ms per launch against 0.218 ms for 5 blocks at 38 registers,
-// which the shared memory would allow)
+// the default aims at about 48 registers a thread (Cahn-Hilliard Q2 3-D, c block: 4 blocks of 288
+// threads at 56 registers measured 130 us a launch against 143 us for 5 blocks and 146 us for 3)
 template <class PDE, int threads, class = void>
 struct CellLaneMinBlocks {
   static constexpr int value = 65536 / (threads * 48) > 0 ? (65536 / (threads * 48) < 32 ? 65536 / (threads * 48) : 32) : 1;
@@ -77,14 +85,26 @@ struct CellLaneMinBlocks<PDE, threads, std::void_t<decltype(PDE::cell_lane_min_b
   static constexpr int value = PDE::cell_lane_min_blocks;
 };
 
+// The output components (bit c: c components in a block) an operator's lane kernels are compiled
+// for: `cell_lane_components`, by default 1 to 4
+template <class PDE, class = void>
+struct CellLaneComponents {
+  static constexpr unsigned int value = 2u | 4u | 8u | 16u;
+};
+template <class PDE>
+struct CellLaneComponents<PDE, std::void_t<decltype(PDE::cell_lane_components)>> {
+  static constexpr unsigned int value = PDE::cell_lane_components;
+};
+
 // shared memory of a tile: the double copies of the nv value rows, the fixed-point copies of the
-// ng gradient rows, the submitted terms (nout components of 1 + dim rows), then the block
-// exponents (two buffers of nrows_in rows, one of nout)
+// ng gradient rows, the gradient terms of the nout components (one component keeps its value and
+// last-direction terms in registers: dim - 1 rows; several keep 1 + dim rows each), then the block
+// exponents of the gradient rows and of the components (two buffers each)
 template <int dim, int degree>
-__host__ __device__ constexpr size_t lane_smem_bytes(int nv, int ng, int nrows_in, int nout) {
+__host__ __device__ constexpr size_t lane_smem_bytes(int nv, int ng, int nout) {
   using S = LaneShape<dim, degree>;
-  return (size_t)S::nq * LANE_CPT * 8 * (size_t)(nv + ng + nout * (1 + dim)) +
-         4 * (size_t)LANE_CPT * (size_t)(2 * nrows_in + nout);
+  return (size_t)S::nq * LANE_CPT * 8 * (size_t)(nv + ng + (nout == 1 ? dim - 1 : nout * (1 + dim))) +
+         4 * (size_t)LANE_CPT * (size_t)(2 * ng + 2 * nout);
 }
 
 // Gauss-Lobatto line integral of the terms g at the line's node j (line_integral of
@@ -102,11 +122,25 @@ __device__ __forceinline__ long long lane_line_integral(int j, long long g0, lon
   }
 }
 
+// t plus the line integral over its node's integer weight (1 at the ends, 4 in the middle of a Q2
+// line), from the point's own term outwards: own, its neighbour m and the far end f for an end of
+// the line, the line's first and last term as m and f for its middle
+template <int n>
+__device__ __forceinline__ long long lane_add_integral(int j, long long t, long long own, long long m, long long f) {
+  if constexpr (n == 2) {
+    return j == 0 ? t - own - m : t + own + m;
+  } else {
+    if (j == 1) return t + m - f;
+    if (j == 0) return t - ((own + m) << 2) + own + f;
+    return t + ((own + m) << 2) - own - f;
+  }
+}
+
 // The rows of one launch as flat lists (built on the host from the launch record): input rows
 // (one per component of each dependency slot) and output components (one per component of each
-// block field, with its value row and dim gradient rows).
+// block field).
 constexpr int LANE_MAX_IN = 6;
-constexpr int LANE_MAX_OUT = 3;
+constexpr int LANE_MAX_OUT = pg::LANE_MAX_OUT;
 struct LaneRows {
   int nin;
   int nout;
@@ -116,13 +150,19 @@ struct LaneRows {
   const double* in_base[LANE_MAX_IN];    // vector of the row's slot
   const int* in_cmap[LANE_MAX_IN];       // constraint map for a constrained read, else null
   unsigned int in_off[LANE_MAX_IN];      // component offset c * N
+  int in_v[LANE_MAX_IN], in_g[LANE_MAX_IN];  // the row's double and fixed-point copy, -1 without one
   double* out_acc[LANE_MAX_OUT];         // accumulator of the output's field
   const int* out_cmap[LANE_MAX_OUT];     // condensation map, else null
   unsigned int out_off[LANE_MAX_OUT];    // component offset c * N
   int out_row[LANE_MAX_OUT];             // value row of the component (dim gradient rows follow)
 };
 
-template <class PDE, int dim, int degree, int MODE, int MINB>
+// the high word of |v|, whose bits above 20 are the biased exponent: ordered like |v|
+__device__ __forceinline__ unsigned int lane_abs_hi(double v) { return (unsigned int)__double2hiint(v) & 0x7fffffffu; }
+
+// NC: output components of the launch. One component keeps the terms of the thread's n points in
+// registers between the callback and the integration; several pass them through shared memory.
+template <class PDE, int dim, int degree, int MODE, int NC, int MINB>
 __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
     cell_kernel_lanes(const __grid_constant__ CellLaunch P, const __grid_constant__ PDE pde,
                       const __grid_constant__ pg::CellTables<dim, degree, double> T,
@@ -134,28 +174,32 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   constexpr int n = S::n, nq = S::nq, cols = S::cols, k = degree, CPT = LANE_CPT;
   constexpr int ROW = nq * CPT;   // entries of one row
   constexpr int JS = cols * CPT;  // entry stride between a thread's points
-  constexpr int TOPT = LANE_TOP_TERMS;
+  constexpr int TOPT = fx::LANE_TOP_INTEGRAL;
+  constexpr int TC = 1 + dim;     // terms of a component
+  constexpr bool REGS = NC == 1;
+  constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20, FLOOR_OUT = (fx::EXP_FLOOR + fx::EXP_BIAS) << 20;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // the tables are a kernel parameter: read-only constant-bank loads, uniform where their index is
   const Tab* tab = &T;
   double* vals = reinterpret_cast<double*>(smem_raw);               // [nv][q][cell]
   long long* vfx = reinterpret_cast<long long*>(vals + R.nv * ROW);  // [ng][q][cell]
-  double* outs = reinterpret_cast<double*>(vfx + R.ng * ROW);       // [out rows][q][cell]
-  const int nrows_out = R.nout * (1 + dim);
-  int* ex_in = reinterpret_cast<int*>(outs + nrows_out * ROW);       // [2][nin][cell]
-  int* ex_out = ex_in + 2 * R.nin * CPT;                             // [nout][cell]
+  long long* outs = vfx + R.ng * ROW;                               // terms [row][q][cell]
+  // block exponents of the gradient rows and (EXP_BIAS more) of the components, as high words
+  unsigned int* ex_in = reinterpret_cast<unsigned int*>(outs + (REGS ? dim - 1 : NC * TC) * ROW);  // [2][ng][cell]
+  unsigned int* ex_out = ex_in + 2 * R.ng * CPT;                    // [2][NC][cell]
 
   const int t = threadIdx.x;
   const int lc = t & 31;
-  const int w = t >> 5;          // point of the first dim-1 directions
+  const int w = __shfl_sync(0xffffffffu, t >> 5, 0);  // point of the first dim-1 directions (uniform)
   const int p0 = w * CPT + lc;   // entry of the thread's first point; point j at p0 + j * JS
   const int qa = w % n;
   const int qb = dim > 2 ? w / n : 0;
-  const unsigned int fx_rows = tab->fx_rows;  // input rows read as gradients (fixed-point copies)
+  // entry steps from the thread's points along the first directions (back from a line's last point)
+  const int step0 = qa == k ? -CPT : CPT;
+  const int step1 = qb == k ? -n * CPT : n * CPT;
   const int hpow2 = tab->hpow2, hk = tab->hk;
   const unsigned long long hsig = tab->hsig;
-  // both exponent buffers: 0 for rows with a fixed-point copy, -1 for rows read as values only
-  for (int i = t; i < 2 * R.nin * CPT; i += S::threads) ex_in[i] = ((fx_rows >> ((i / CPT) % R.nin)) & 1u) ? 0 : -1;
+  for (int i = t; i < 2 * (R.ng + NC) * CPT; i += S::threads) ex_in[i] = i < 2 * R.ng * CPT ? FLOOR : FLOOR_OUT;
   const unsigned int nn0 = (unsigned int)P.nn[0], nn1 = (unsigned int)P.nn[1];
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;  // lattice stride of the last direction
   const unsigned int ncells = (unsigned int)P.ncells;
@@ -164,8 +208,10 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
 
   int par = 0;
   for (unsigned int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, par ^= 1) {
-    int* exi = ex_in + par * R.nin * CPT;
-    int* exn = ex_in + (par ^ 1) * R.nin * CPT;
+    unsigned int* exi = ex_in + par * R.ng * CPT;
+    unsigned int* exn = ex_in + (par ^ 1) * R.ng * CPT;
+    unsigned int* exo = ex_out + par * NC * CPT;
+    unsigned int* exon = ex_out + (par ^ 1) * NC * CPT;
     // lanes past the last cell redo the last cell and skip its scatter
     const unsigned int cell_t = tile * CPT + lc;
     const bool active = cell_t < ncells;
@@ -190,63 +236,67 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
 #pragma unroll
     for (int r = 0; r < LANE_MAX_IN; ++r) {
       if (r < R.nin) {
-        const double* base = R.in_base[r];
-        int e = 0;
+        const double* base = R.in_base[r] + R.in_off[r];
+        double v[n];
+        if (R.in_cmap[r]) {
+          const int* cm = R.in_cmap[r] + R.in_off[r];
 #pragma unroll
-        for (int j = 0; j < n; ++j) {
-          const unsigned int idx = node0 + (unsigned int)j * lstride + R.in_off[r];
-          double v;
-          if (R.in_cmap[r]) {
-            const int m = __ldg(R.in_cmap[r] + idx);
+          for (int j = 0; j < n; ++j) {
+            const unsigned int idx = node0 + (unsigned int)j * lstride;
+            const int m = __ldg(cm + idx);
             const double own = __ldg(base + idx);
-            v = m == (int)idx ? own : (m >= 0 ? __ldg(base + m) : 0.0);
-          } else {
-            v = __ldg(base + idx);
+            v[j] = m == (int)(idx + R.in_off[r]) ? own : (m >= 0 ? __ldg(R.in_base[r] + m) : 0.0);
           }
-          const int vs = tab->lane_vslot[r], gs = tab->lane_gslot[r];
-          if (vs >= 0) vals[vs * ROW + p0 + j * JS] = v;
-          // a gradient row's double stays in its fixed-point slot until converted in place
-          if (gs >= 0) vfx[gs * ROW + p0 + j * JS] = __double_as_longlong(v);
-          e = max(e, fx::exponent(v));
+        } else {
+#pragma unroll
+          for (int j = 0; j < n; ++j) v[j] = __ldg(base + (node0 + (unsigned int)j * lstride));
         }
-        if ((fx_rows >> r) & 1u) atomicMax(&exi[r * CPT + lc], e);
+        const int vs = R.in_v[r], gs = R.in_g[r];
+        if (vs >= 0) {
+#pragma unroll
+          for (int j = 0; j < n; ++j) vals[vs * ROW + p0 + j * JS] = v[j];
+        }
+        if (gs >= 0) {
+          unsigned int m = 0;
+#pragma unroll
+          for (int j = 0; j < n; ++j) {
+            // a gradient row's double stays in its fixed-point slot until converted in place
+            vfx[gs * ROW + p0 + j * JS] = __double_as_longlong(v[j]);
+            m = max(m, lane_abs_hi(v[j]));
+          }
+          atomicMax(&exi[gs * CPT + lc], m);
+        }
       }
     }
     __syncthreads();  // nodal values and their block exponents complete
 
-    // fixed-point copies; clear the submitted terms, their exponents and the next tile's
-    // value-row exponents
+    // fixed-point copies; reset the next tile's exponents
 #pragma unroll
-    for (int r = 0; r < LANE_MAX_IN; ++r) {
-      if (r < R.nin && ((fx_rows >> r) & 1u)) {
+    for (int g = 0; g < LANE_MAX_IN; ++g) {
+      if (g < R.ng) {
         // (a cell holding a non-finite value gets meaningless copies: every result read from them
         // is replaced by NaN)
-        const int E = exi[r * CPT + lc];
-        long long* x = vfx + tab->lane_gslot[r] * ROW + p0;
+        const unsigned int E = fx::high_exponent((int)(exi[g * CPT + lc] >> 20));
+        long long* x = vfx + g * ROW + p0;
 #pragma unroll
-        for (int j = 0; j < n; ++j) x[j * JS] = fx::to_fixed_fast<fx::TOP_VALUES>(__longlong_as_double(x[j * JS]), E);
+        for (int j = 0; j < n; ++j) x[j * JS] = fx::to_fixed_cut<fx::LANE_TOP_VALUES>(__longlong_as_double(x[j * JS]), E);
       }
     }
-#pragma unroll
-    for (int o = 0; o < LANE_MAX_OUT; ++o)
-      if (o < R.nout)
-#pragma unroll
-        for (int i = 0; i <= dim; ++i)
-#pragma unroll
-          for (int j = 0; j < n; ++j) outs[(R.out_row[o] + i) * ROW + p0 + j * JS] = 0.0;
-    for (int i = t; i < R.nin * CPT; i += S::threads) exn[i] = ((fx_rows >> (i / CPT)) & 1u) ? 0 : -1;
-    for (int i = t; i < R.nout * CPT; i += S::threads) ex_out[i] = 0;
+    for (int g = w; g < R.ng; g += cols) exn[g * CPT + lc] = FLOOR;
+    for (int o = w; o < NC; o += cols) exon[o * CPT + lc] = FLOOR_OUT;
     __syncthreads();  // fixed-point copies visible
 
     // the user callback at each of the thread's points
     const SimulationTimer& timer = P.timer_dev ? *P.timer_dev : P.timer;
-    // (one copy of the callback's code: unrolling the points measured slower)
-#pragma unroll 1
-    for (int j = 0; j < n; ++j) {
+    double term[REGS ? n * TC : 1];
+    unsigned int em[NC * TC];  // largest magnitude of each term over the thread's points
+#pragma unroll
+    for (int i = 0; i < NC * TC; ++i) em[i] = 0;
+    auto point = [&](int j, double* keep) {
       pg::CellCtx<dim, degree, double> ctx;
       ctx.tab = tab;
       ctx.vals = vals;
-      ctx.outs = outs;
+      ctx.outs = nullptr;
       ctx.stride = ROW;
       ctx.lc = lc;
       ctx.q = w + j * cols;
@@ -256,88 +306,150 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
       ctx.err = P.err;
       ctx.submitted = 0;
       ctx.vals_fx = vfx;
-      ctx.ex_in = exi;
+      ctx.ex_in = reinterpret_cast<const int*>(exi);
       ctx.cpb = CPT;
       ctx.cpt = CPT;
       ctx.lean = 1;
       ctx.qi[0] = qa;
       ctx.qi[1] = dim > 2 ? qb : j;
       ctx.qi[2] = dim > 2 ? j : 0;
+      ctx.pe = p0 + j * JS;
+      ctx.step[0] = step0;
+      ctx.step[1] = dim > 2 ? step1 : (j == k ? -JS : JS);
+      ctx.step[2] = dim > 2 ? (j == k ? -JS : JS) : 0;
+      ctx.nterm = NC;
+#pragma unroll
+      for (int i = 0; i < NC * TC; ++i) ctx.term[i] = 0.0;
       FieldContainer<dim, degree, double> fc(ctx);
       if constexpr (MODE == MODE_LHS) pde.compute_lhs(fc, timer, P.block_id);
       else pde.compute_rhs(fc, timer, P.block_id);
-    }
-    // block exponents of every output component's terms (rows the callback left are zero): the
-    // value term enters as h v (one binade more when h is not a power of two)
 #pragma unroll
-    for (int o = 0; o < LANE_MAX_OUT; ++o) {
-      if (o < R.nout) {
-        const int rv = R.out_row[o];
-        int e = 0;
+      for (int i = 0; i < NC * TC; ++i) em[i] = max(em[i], lane_abs_hi(ctx.term[i]));
+      if constexpr (REGS) {
 #pragma unroll
-        for (int j = 0; j < n; ++j) {
-          const int ev = fx::exponent(outs[rv * ROW + p0 + j * JS]);
-          const int eh = ev + hk + (hpow2 ? 0 : 1);
-          e = max(e, ev == 0 ? 0 : (ev == fx::EXP_NONFINITE || eh >= fx::EXP_NONFINITE ? fx::EXP_NONFINITE : max(eh, 0)));
+        for (int i = 0; i < TC; ++i) keep[i] = ctx.term[i];
+      } else {
 #pragma unroll
-          for (int d = 0; d < dim; ++d) e = max(e, fx::exponent(outs[(rv + 1 + d) * ROW + p0 + j * JS]));
-        }
-        atomicMax(&ex_out[o * CPT + lc], e);
+        for (int i = 0; i < NC * TC; ++i) outs[i * ROW + p0 + j * JS] = __double_as_longlong(ctx.term[i]);
       }
+    };
+    if constexpr (REGS) {
+#pragma unroll
+      for (int j = 0; j < n; ++j) point(j, term + j * TC);
+    } else {
+      // (one copy of the callback's code)
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) point(j, nullptr);
+    }
+    // block exponents of every output component's terms (those the callback left are zero): the
+    // value term enters as h v, the gradient terms as (h_0 / h_d) g
+#pragma unroll
+    for (int o = 0; o < NC; ++o) {
+      unsigned int e = em[o * TC] + tab->hadd, raw = em[o * TC];
+#pragma unroll
+      for (int d = 0; d < dim; ++d) {
+        e = max(e, em[o * TC + 1 + d] + tab->radd[d]);
+        raw = max(raw, em[o * TC + 1 + d]);
+      }
+      atomicMax(&exo[o * CPT + lc], raw >= 0x7ff00000u ? 0xfff00000u : e);
     }
     __syncthreads();  // submitted terms and their block exponents complete
 
-    // the submitted terms in place to fixed point
+    // the submitted terms to fixed point (with a non-finite term the copies are meaningless and the
+    // integral is replaced by NaN)
+    auto fixed_value = [&](double v, int E) {
+      return hpow2 ? fx::to_fixed_cut<TOPT>(v, fx::high_exponent(E - hk))
+                   : fx::to_fixed_cut_scaled<TOPT>(v, fx::high_exponent(E), hsig, hk);
+    };
+    auto fixed_gradient = [&](double g, int d, int E) {
+      if (d == 0) return fx::to_fixed_cut<TOPT>(g, fx::high_exponent(E));
+      return tab->rpow2[d] ? fx::to_fixed_cut<TOPT>(g, fx::high_exponent(E - tab->rk[d]))
+                           : fx::to_fixed_cut_scaled<TOPT>(g, fx::high_exponent(E), tab->rsig[d], tab->rk[d]);
+    };
+    // one node's integral from its component's value term x and line integrals, and its scatter
+    // (distribute_local_to_global through the constraint map)
+    const int sab = (n > 2 && qa == 1 ? 2 : 0) + (n > 2 && qb == 1 ? 2 : 0);
+    auto scatter = [&](int o, int j, int E, long long Tx) {
+      const int vw = sab + (n > 2 && j == 1 ? 2 : 0);
+      const double r = fx::to_double_cut(Tx, E - 1023 - TOPT + tab->ik[0] + vw, tab->isig[0], true,
+                                         E >= fx::EXP_WIDE, E >= fx::EXP_NONFINITE);
+      const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
+      const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
+      if (active && target >= 0) atomicAdd(R.out_acc[o] + target, r);
+    };
+    if constexpr (REGS) {
+      const int E = (int)(exo[lc] >> 20) - fx::EXP_BIAS;
+      long long X[n], G[dim][n];
 #pragma unroll
-    for (int o = 0; o < LANE_MAX_OUT; ++o) {
-      if (o < R.nout) {
-        const int rv = R.out_row[o];
-        // (with E = 2047 the copies are meaningless and the integral is replaced by NaN)
-        const int E = ex_out[o * CPT + lc];
-        long long* ox = reinterpret_cast<long long*>(outs);
+      for (int j = 0; j < n; ++j) {
+        X[j] = fixed_value(term[j * TC], E);
 #pragma unroll
-        for (int j = 0; j < n; ++j) {
-          const int e0 = rv * ROW + p0 + j * JS;
-          const double v = outs[e0];
-          ox[e0] = hpow2 ? fx::to_fixed_fast<TOPT>(v, E - hk) : fx::to_fixed_scaled<TOPT>(v, E, hsig, hk);
-#pragma unroll
-          for (int d = 0; d < dim; ++d) ox[e0 + (1 + d) * ROW] = fx::to_fixed_fast<TOPT>(outs[e0 + (1 + d) * ROW], E);
+        for (int d = 0; d < dim; ++d) {
+          G[d][j] = fixed_gradient(term[j * TC + 1 + d], d, E);
+          if (d < dim - 1) outs[d * ROW + p0 + j * JS] = G[d][j];
         }
       }
-    }
-    __syncthreads();  // fixed-point terms visible
-
-    // integrate and scatter (distribute_local_to_global through the constraint map)
-    const long long* ox = reinterpret_cast<const long long*>(outs);
+      __syncthreads();  // fixed-point terms visible
+      // the first directions' lines, the position on them uniform across the warp
 #pragma unroll
-    for (int o = 0; o < LANE_MAX_OUT; ++o) {
-      if (o < R.nout) {
-        const int rv = R.out_row[o];
-        const int E = ex_out[o * CPT + lc];
-        // the last direction's line is the thread's own points
-        const long long* gl = ox + (rv + dim) * ROW + p0;
-        const long long z0 = gl[0], z1 = gl[JS], z2 = n > 2 ? gl[2 * JS] : 0ll;
+      for (int d = 0; d < dim - 1; ++d) {
+        const long long* g = outs + d * ROW + p0;
+        const int st = d == 0 ? step0 : step1, id = d == 0 ? qa : qb;
+        if (n > 2 && id == 1) {
+#pragma unroll
+          for (int j = 0; j < n; ++j) X[j] = lane_add_integral<n>(1, X[j], 0, g[j * JS - st], g[j * JS + st]);
+        } else if (id == 0) {
+#pragma unroll
+          for (int j = 0; j < n; ++j)
+            X[j] = lane_add_integral<n>(0, X[j], G[d][j], g[j * JS + st], n > 2 ? g[j * JS + 2 * st] : 0ll);
+        } else {
+#pragma unroll
+          for (int j = 0; j < n; ++j)
+            X[j] = lane_add_integral<n>(k, X[j], G[d][j], g[j * JS + st], n > 2 ? g[j * JS + 2 * st] : 0ll);
+        }
+      }
+      // the last direction's line is the thread's own points
+      const long long* z = G[dim - 1];
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        if (n > 2 && j == 1) X[j] = lane_add_integral<n>(1, X[j], 0, z[0], z[n - 1]);
+        else X[j] = lane_add_integral<n>(j, X[j], z[j], z[j == 0 ? 1 : n - 2], z[j == 0 ? n - 1 : 0]);
+        scatter(0, j, E, X[j]);
+      }
+    } else {
+#pragma unroll
+      for (int o = 0; o < NC; ++o) {
+        const int E = (int)(exo[o * CPT + lc] >> 20) - fx::EXP_BIAS;
+#pragma unroll
+        for (int i = 0; i < TC; ++i) {
+          long long* x = outs + (o * TC + i) * ROW + p0;
+#pragma unroll
+          for (int j = 0; j < n; ++j) {
+            const double v = __longlong_as_double(x[j * JS]);
+            x[j * JS] = i == 0 ? fixed_value(v, E) : fixed_gradient(v, i - 1, E);
+          }
+        }
+      }
+      __syncthreads();  // fixed-point terms visible
+#pragma unroll
+      for (int o = 0; o < NC; ++o) {
+        const int E = (int)(exo[o * CPT + lc] >> 20) - fx::EXP_BIAS;
+        const long long* x = outs + o * TC * ROW + p0;
+        const long long* z = x + dim * ROW;  // the last direction's line is the thread's own points
+        const long long z0 = z[0], z1 = z[JS], z2 = n > 2 ? z[2 * JS] : 0ll;
 #pragma unroll
         for (int j = 0; j < n; ++j) {
-          const int q = w + j * cols;
-          const int e0 = rv * ROW + p0 + j * JS;
-          // this point's integration weights: powers of two from the tables
-          long long Tx = (long long)((unsigned long long)ox[e0] << tab->vw_sh[q]);
+          long long Tx = x[j * JS];
 #pragma unroll
           for (int d = 0; d < dim - 1; ++d) {
-            const int sd = d == 0 ? 1 : n;
-            const int id = d == 0 ? qa : qb;
-            const long long* g = ox + (rv + 1 + d) * ROW + (q - id * sd) * CPT + lc;
-            const long long L = lane_line_integral<n>(id, g[0], g[sd * CPT], n > 2 ? g[2 * sd * CPT] : 0ll);
-            Tx += (long long)((unsigned long long)L << tab->wo_sh[d][q]);
+            const long long* g = x + (1 + d) * ROW + j * JS;
+            const int st = d == 0 ? step0 : step1, id = d == 0 ? qa : qb;
+            if (n > 2 && id == 1) Tx = lane_add_integral<n>(1, Tx, 0, g[-st], g[st]);
+            else Tx = lane_add_integral<n>(id, Tx, g[0], g[st], n > 2 ? g[2 * st] : 0ll);
           }
-          const long long Lz = lane_line_integral<n>(j, z0, z1, z2);
-          Tx += (long long)((unsigned long long)Lz << tab->wo_sh[dim - 1][q]);
-          const double rr = fx::to_double_fast(Tx, E - 1023 - TOPT + tab->ik[0], tab->isig[0], true);
-          const double r = E == fx::EXP_NONFINITE ? fx::quiet_nan() : rr;
-          const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
-          const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
-          if (active && target >= 0) atomicAdd(R.out_acc[o] + target, r);
+          if (n > 2 && j == 1) Tx = lane_add_integral<n>(1, Tx, 0, z0, z2);
+          else Tx = lane_add_integral<n>(j, Tx, j == 0 ? z0 : (n > 2 ? z2 : z1), j == 0 || n > 2 ? z1 : z0, j == 0 ? z2 : z0);
+          scatter(o, j, E, Tx);
         }
       }
     }
@@ -512,11 +624,11 @@ inline bool lane_rows(const CellLaunch& P, int dim, LaneRows* R) {
   return row == P.nrows_out;
 }
 
-template <class PDE, int dim, int degree, int mode, int MINB>
+template <class PDE, int dim, int degree, int mode, int NC, int MINB>
 cudaError_t launch_lanes(const CellLaunch& P, const LaneRows& R, const void* obj, cudaStream_t s) {
   using S = LaneShape<dim, degree>;
-  auto kern = cell_kernel_lanes<PDE, dim, degree, mode, MINB>;
-  const size_t smem = lane_smem_bytes<dim, degree>(R.nv, R.ng, R.nin, R.nout);
+  auto kern = cell_kernel_lanes<PDE, dim, degree, mode, NC, MINB>;
+  const size_t smem = lane_smem_bytes<dim, degree>(R.nv, R.ng, NC);
   constexpr int MAX_DEVICES = 64;
   static size_t attr_smem_of[MAX_DEVICES] = {};
   static int occ_of[MAX_DEVICES] = {};
@@ -607,8 +719,21 @@ cudaError_t launch_cell_kernel_lanes_impl(const CellLaunch& P, const void* obj, 
   const unsigned int mask = (1u << R.nin) - 1u;
   R.nv = __builtin_popcount(tab->val_rows & mask);
   R.ng = __builtin_popcount(tab->fx_rows & mask);
-  if (lane_smem_bytes<dim, degree>(R.nv, R.ng, R.nin, R.nout) > 232448) return cudaErrorNotSupported;
-  return launch_lanes<PDE, dim, degree, mode, MINB>(P, R, obj, s);
+  for (int r = 0; r < R.nin; ++r) {
+    R.in_v[r] = tab->lane_vslot[r];
+    R.in_g[r] = tab->lane_gslot[r];
+  }
+  if (lane_smem_bytes<dim, degree>(R.nv, R.ng, R.nout) > 232448) return cudaErrorNotSupported;
+  constexpr unsigned int C = CellLaneComponents<PDE>::value;
+  if constexpr (C & 2u)
+    if (R.nout == 1) return launch_lanes<PDE, dim, degree, mode, 1, MINB>(P, R, obj, s);
+  if constexpr (C & 4u)
+    if (R.nout == 2) return launch_lanes<PDE, dim, degree, mode, 2, MINB>(P, R, obj, s);
+  if constexpr (C & 8u)
+    if (R.nout == 3) return launch_lanes<PDE, dim, degree, mode, 3, MINB>(P, R, obj, s);
+  if constexpr (C & 16u)
+    if (R.nout == 4) return launch_lanes<PDE, dim, degree, mode, 4, MINB>(P, R, obj, s);
+  return cudaErrorNotSupported;
 }
 
 }  // namespace ppf

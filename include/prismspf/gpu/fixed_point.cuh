@@ -68,6 +68,8 @@ PPF_FX double double_of(unsigned long long b) {
 #endif
 }
 
+PPF_FX double quiet_nan() { return double_of(0x7ff8000000000000ull); }
+
 PPF_FX int clz64(unsigned long long a) {
 #ifdef __CUDA_ARCH__
   return __clzll((long long)a);
@@ -195,6 +197,116 @@ PPF_FX double to_double_fast(long long x, int lsb, unsigned long long sig, bool 
   return double_of(ok ? bits : edge);
 }
 
+// The conversions of the lane kernel's rows. They differ from to_fixed_fast / to_double_fast in what
+// their callers guarantee: block exponents are at least EXP_FLOOR (rows start their exponent there),
+// and the scales of an operator are within 2^+-MAX_SCALE (the tables leave the lane kernel off
+// otherwise), so that no result falls below the normal range and zeros need no test of their own.
+constexpr int EXP_FLOOR = 192;
+// fixed-point tops of the lane kernel: |3 u + 4 v + w| <= 8 * 2^60 keeps a derivative's line sum
+// below 2^63, and |x + sum_d L_d| <= (1 + 3 * 8) 2^58 a node's integral over its weight
+constexpr int LANE_TOP_VALUES = 59;
+constexpr int LANE_TOP_INTEGRAL = 57;
+constexpr int MAX_SCALE = 60;
+constexpr int EXP_BIAS = 64;    // of the exponents of scaled terms
+constexpr int EXP_WIDE = 1900;  // block exponents from here on may give results beyond the range
+
+// a >> r for any r >= 0 (zero from 64 up)
+PPF_FX unsigned long long shr64(unsigned long long a, unsigned int r) {
+#ifdef __CUDA_ARCH__
+  unsigned long long o;
+  asm("shr.u64 %0, %1, %2;" : "=l"(o) : "l"(a), "r"(r));  // clamps shifts above 63
+  return o;
+#else
+  return r > 63u ? 0ull : a >> r;
+#endif
+}
+// high word of (hi:lo) << r and low word of (hi:lo) >> r, 0 <= r < 32
+PPF_FX unsigned int funnel_l(unsigned int lo, unsigned int hi, unsigned int r) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, r);
+#else
+  return (unsigned int)(((((unsigned long long)hi << 32) | lo) << r) >> 32);
+#endif
+}
+PPF_FX unsigned int funnel_r(unsigned int lo, unsigned int hi, unsigned int r) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_r(lo, hi, r);
+#else
+  return (unsigned int)((((unsigned long long)hi << 32) | lo) >> r);
+#endif
+}
+PPF_FX unsigned long long join(unsigned int lo, unsigned int hi) { return ((unsigned long long)hi << 32) | lo; }
+PPF_FX long long with_sign(unsigned long long a, unsigned int sign_word) {
+  return (int)sign_word < 0 ? (long long)(0ull - a) : (long long)a;
+}
+
+// v * 2^(1023 + TOP - E) rounded towards zero, for exponent(v) <= E and E >= EXP_FLOOR: less than
+// one unit off, what to_fixed with a top one lower is at most off (half of its unit, twice as large).
+// Zeros and values far below the block's largest give 0. `Ehi` is E in a high word's exponent
+// position with the bits below it set, so that E - exponent(v) is one subtraction and shift.
+template <int TOP>
+PPF_FX long long to_fixed_cut(double v, unsigned int Ehi) {
+  static_assert(TOP >= 52 && TOP <= 60, "fixed-point top out of range");
+  const unsigned long long b = bits_of(v);
+  const unsigned int hi = (unsigned int)(b >> 32), lo = (unsigned int)b;
+  const unsigned int mhi = (hi & 0xfffffu) | 0x100000u;
+  const unsigned long long m = join(lo << (TOP - 52), funnel_l(lo, mhi, TOP - 52));
+  return with_sign(shr64(m, (Ehi - (hi & 0x7fffffffu)) >> 20), hi);
+}
+PPF_FX unsigned int high_exponent(int E) { return ((unsigned int)E << 20) | 0xfffffu; }
+
+// v * sigma * 2^(k + 1023 + TOP - E) rounded towards zero, sigma = sig / 2^63 in [1, 2), for
+// exponent(v) + k + 1 <= E and E >= EXP_FLOOR
+template <int TOP>
+PPF_FX long long to_fixed_cut_scaled(double v, unsigned int Ehi, unsigned long long sig, int k) {
+  static_assert(TOP >= 52 && TOP <= 60, "fixed-point top out of range");
+  const unsigned long long b = bits_of(v);
+  const unsigned int hi = (unsigned int)(b >> 32);
+  const unsigned long long P = mulhi64(((b & 0xfffffffffffffull) | (1ull << 52)) << 11, sig);
+  // (E - k is at least exponent(v) + 1)
+  return with_sign(shr64(P, ((Ehi - ((unsigned int)k << 20) - (hi & 0x7fffffffu)) >> 20) + (62u - TOP)), hi);
+}
+
+// the general case of to_double_cut: any |x| = a < 2^63, exponents beyond the normal range (an
+// infinity or a NaN), a quiet NaN when `bad`
+PPF_FX double to_double_any(unsigned long long a, unsigned int sign, int lsb, bool bad) {
+  if (bad) return quiet_nan();
+  if (a == 0) return 0.0;
+  const int lz = clz64(a);  // at least 1
+  const unsigned long long r = ((a << (lz - 1)) + 0x200ull) >> 10;
+  const int be1 = 1085 + lsb - lz;
+  const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)(be1 < 2046 ? be1 : 2046) << 20);
+  return double_of(join((unsigned int)r, hi | sign));
+}
+
+// (+-x) * 2^lsb, or (+-x) * 2^lsb * sigma when `scaled` (from the product's floor to a multiple of
+// 2^(lsb + 1)), |x| < 2^63, rounded to nearest (ties away from zero), with x negated when `flip` is
+// the sign bit's mask (else 0); a quiet NaN when `bad`. The caller's E and scales keep the result
+// above the subnormal range, and below infinity unless `wide`. The common case (more than 32
+// significant bits) takes 32-bit shifts and adds only, the rest to_double_any: selects in place of
+// that branch measured slower (Cahn-Hilliard 64^3 Q2: 142 against 130 us a launch).
+PPF_FX double to_double_cut(long long x, int lsb, unsigned long long sig, bool scaled, bool wide, bool bad,
+                            unsigned int flip = 0u) {
+  unsigned long long a = x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x;
+  if (scaled) {
+    a = mulhi64(a, sig);  // floor(|x| * sigma / 2) < 2^63
+    ++lsb;
+  }
+  const unsigned int sign = ((unsigned int)((unsigned long long)x >> 32) ^ flip) & 0x80000000u;
+  const unsigned int ahi = (unsigned int)(a >> 32), alo = (unsigned int)a;
+  if (ahi == 0 || wide) return to_double_any(a, sign, lsb, bad);
+#ifdef __CUDA_ARCH__
+  const int sh = __clz((int)ahi) - 1;
+#else
+  const int sh = clz64(a) - 1;
+#endif
+  // leading one to bit 62, half a unit of the last kept bit added, 53 bits (2^53 on a carry) kept
+  const unsigned long long t = join(alo << sh, funnel_l(alo, ahi, (unsigned int)sh)) + 0x200ull;
+  const unsigned int thi = (unsigned int)(t >> 32);
+  const unsigned int hi = (thi >> 10) + ((unsigned int)(1084 + lsb - sh) << 20);
+  return double_of(join(funnel_r((unsigned int)t, thi, 10), hi | sign));
+}
+
 // Gauss-Lobatto line contractions on the unit interval, exact in integers.
 // Derivative at node qd of the line values u: sum_j D[qd][j] u_j with D = {-1, 1 / -1, 1} (Q1)
 // or {-3, 4, -1 / -1, 0, 1 / 1, -4, 3} (Q2); for Q2 with a = u2 - u0 and b = 2 (u0 - 2 u1 + u2)
@@ -246,8 +358,6 @@ struct FastDiv {
 #endif
   }
 };
-
-PPF_FX double quiet_nan() { return double_of(0x7ff8000000000000ull); }
 
 // a scale factor s > 0 as s = sigma * 2^k, sigma in [1, 2) held as sigma * 2^63
 struct Scale {

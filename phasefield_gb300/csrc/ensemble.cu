@@ -125,7 +125,7 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
   ctx.submitted = 0;
   // integer integration of the value and gradient terms where the tables allow it (square cells):
   // the lane kernel's arithmetic (prismspf/gpu/cell_kernel_lanes.cuh) on this layout
-  const bool fxi = P.fx && tab->fx_lanes;
+  const bool fxi = P.fx && tab->fx_cubic;
   if (P.fx) {
     ctx.vals_fx = vals_fx;
     ctx.ex_in = ex_in;

@@ -61,10 +61,10 @@ struct BlockPlan {
   signed char out_row0[pg::MAX_OUTS];
   // integer contractions (FP64 Q1/Q2): on in the tables; arithmetic chosen for this plan
   // (-1 until the first plain launch times the modes; 1 integer derivatives + FP64
-  // integration, 2 both in integers, 3 FP64 derivatives + integer integration, 4 the lane kernel:
-  // every contraction in integers, cubic cells only)
+  // integration, 2 both in integers, 3 FP64 derivatives + integer integration, 4 and 5 the lane
+  // kernel: every contraction in integers, on cubic and on stretched cells)
   bool fx = false;
-  bool fx_lanes = false;
+  int fx_lanes = 0;                // the plan's lane kernel mode (4, 5 or 0 for none)
   int fx_mode = -1;
   int fx_timed = 0;                // online timing of the multigrid outer operator
   cudaEvent_t fx_ev[16] = {};
@@ -86,7 +86,7 @@ struct MGLevel {
   void* inv_diag = nullptr;     // len, level precision
   void* tables = nullptr;       // CellTables for the LHS (level precision)
   std::vector<unsigned char> h_tables;  // host copy (the lane kernel takes it as a kernel parameter)
-  bool fx_lanes = false;        // FP64 level whose tables allow the lane kernel
+  int fx_lanes = 0;             // the FP64 level's lane kernel mode (4, 5 or 0 for none)
   void* acc = nullptr;          // accumulator
   void* x = nullptr;            // level solution
   void* b = nullptr;            // level defect (right-hand side)
@@ -108,7 +108,7 @@ struct MGLevel {
   void* t1 = nullptr;
   void* cvt = nullptr;          // precision-conversion buffer (coarsest level of a mixed hierarchy)
   // contraction mode of the level's FP64 operator (integer contractions, FP64 Q1/Q2): its first
-  // plain LHS launches run modes 1, 2, 3 (and 4 where the lane kernel applies) twice under CUDA
+  // plain LHS launches run modes 1, 2, 3 (and the lane kernel where it applies) twice under CUDA
   // events, then the fastest stays
   int fx_mode = -1;
   int fx_timed = 0;

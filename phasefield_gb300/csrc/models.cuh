@@ -24,6 +24,7 @@ using namespace prismspf;
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct AllenCahn {
+  static constexpr unsigned int cell_lane_components = 2u | 4u;  // n; mg_n and f_tot
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number m_well;
@@ -53,6 +54,7 @@ struct AllenCahn {
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct CahnHilliard {
+  static constexpr unsigned int cell_lane_components = 2u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   // Q2 3-D: 32 registers and 8 resident blocks per SM measured 2.7 % faster than the free
@@ -93,6 +95,7 @@ constexpr int ESHELBY_MAX_INCLUSIONS = 64;
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct Eshelby {
+  static constexpr unsigned int cell_lane_components = 1u << dim;
   using ScalarValue = dealii::VectorizedArray<number>;
   using VectorGrad = dealii::Tensor<2, dim, ScalarValue>;
   // register budget of the FP32 operator (the multigrid smoothing levels)
@@ -155,6 +158,7 @@ struct Eshelby {
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct CoupledACCH {
+  static constexpr unsigned int cell_lane_components = 4u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number Mc;
@@ -281,6 +285,7 @@ PPF_HD ACCHPoint<number> acch_point(number c, number n) {
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct CoupledACCHTangent {
+  static constexpr unsigned int cell_lane_components = 4u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number Mc, Mn, Kn;
@@ -314,6 +319,7 @@ struct CoupledACCHTangent {
 
 template <unsigned int dim, unsigned int degree, typename number>
 struct CoupledACCHAdjoint {
+  static constexpr unsigned int cell_lane_components = 16u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number Mc, Mn, Kn;
@@ -362,6 +368,7 @@ namespace ppf {
 // and the post-processing block 2 of the explicit application.
 template <unsigned int dim, unsigned int degree, typename number>
 struct AllenCahnImplicit {
+  static constexpr unsigned int cell_lane_components = 2u | 4u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number m_well;
@@ -404,6 +411,7 @@ struct AllenCahnImplicit {
 // (block 0) and the post-processing block 2.
 template <unsigned int dim, unsigned int degree, typename number>
 struct CahnHilliardImplicit {
+  static constexpr unsigned int cell_lane_components = 2u | 4u;
   using ScalarValue = dealii::VectorizedArray<number>;
   using ScalarGrad = dealii::Tensor<1, dim, ScalarValue>;
   number McV;

@@ -126,7 +126,9 @@ GLRule gauss_lobatto(int n) {
 // PPF_FP64_CONTRACTIONS=1 asks for the FP64 contractions.
 template <int dim, int degree>
 static void fixed_point_tables(pg::CellTables<dim, degree, double>& t, const GLRule& g, const double* h, double detJ,
-                               unsigned int fx_rows, unsigned int val_rows) {
+                               const signed char slot_of[pg::MAX_FIELDS][pg::NAGE], const signed char* slot_comp0,
+                               const signed char* out_of, const signed char* out_row0, unsigned int fx_rows,
+                               unsigned int val_rows) {
   constexpr int n = degree + 1, nq = pg::CellTables<dim, degree, double>::nq;
   t.fx = 0;
   t.fx_rows = fx_rows;
@@ -134,6 +136,20 @@ static void fixed_point_tables(pg::CellTables<dim, degree, double>& t, const GLR
   for (int r = 0, nv = 0, ng = 0; r < pg::LANE_ROW_SLOTS; ++r) {
     t.lane_vslot[r] = (signed char)(((val_rows >> r) & 1u) ? nv++ : -1);
     t.lane_gslot[r] = (signed char)(((fx_rows >> r) & 1u) ? ng++ : -1);
+  }
+  std::memset(t.lane_v, -1, sizeof(t.lane_v));
+  std::memset(t.lane_g, -1, sizeof(t.lane_g));
+  std::memset(t.lane_out, -1, sizeof(t.lane_out));
+  for (int f = 0; f < pg::MAX_FIELDS; ++f) {
+    for (int a = 0; a < pg::NAGE; ++a) {
+      const int s = slot_of[f][a];
+      const int row = s >= 0 ? slot_comp0[s] : pg::LANE_ROW_SLOTS;
+      if (row < pg::LANE_ROW_SLOTS) {
+        t.lane_v[f][a] = t.lane_vslot[row];
+        t.lane_g[f][a] = t.lane_gslot[row];
+      }
+    }
+    if (out_of[f] >= 0) t.lane_out[f] = out_row0[(int)out_of[f]] / (1 + dim);
   }
   if (degree > 2) return;
   const char* env = std::getenv("PPF_FP64_CONTRACTIONS");
@@ -193,8 +209,20 @@ static void fixed_point_tables(pg::CellTables<dim, degree, double>& t, const GLR
   t.hsig = hs.sig;
   t.hk = hs.k;
   t.hpow2 = hs.sig == (1ull << 63) ? 1 : 0;
-  // the lane kernel integrates every direction with one scale (cubic cells)
-  t.fx_lanes = t.fx_cubic;
+  // the lane kernel integrates every direction with direction 0's scale: gradient terms along d
+  // enter as (h_0 / h_d) g
+  bool in_range = std::abs(t.hk) <= pg::fx::MAX_SCALE;
+  for (int d = 0; d < 3; ++d) {
+    const pg::fx::Scale rs = pg::fx::make_scale(d < dim ? h[0] / h[d] : 1.0);
+    t.rsig[d] = rs.sig;
+    t.rk[d] = rs.k;
+    t.rpow2[d] = rs.sig == (1ull << 63) ? 1 : 0;
+    in_range = in_range && std::abs(t.dk[d]) <= pg::fx::MAX_SCALE && std::abs(t.ik[d]) <= pg::fx::MAX_SCALE &&
+               std::abs(t.rk[d]) <= pg::fx::MAX_SCALE;
+  }
+  t.hadd = (unsigned int)(t.hk + (t.hpow2 ? 0 : 1) + pg::fx::EXP_BIAS) << 20;
+  for (int d = 0; d < 3; ++d) t.radd[d] = (unsigned int)(t.rk[d] + (t.rpow2[d] ? 0 : 1) + pg::fx::EXP_BIAS) << 20;
+  t.fx_lanes = in_range ? 1 : 0;
   t.fx = 1;
 }
 template <int dim, int degree>
@@ -242,7 +270,7 @@ static std::vector<unsigned char> tables_impl(const double* lo, const double* h,
   }
   for (int i = 0; i < n; ++i) t.gl_x[i] = g.x[i];
   t.vol = detJ;
-  fixed_point_tables<dim, degree>(t, g, h, detJ, fx_rows, val_rows);
+  fixed_point_tables<dim, degree>(t, g, h, detJ, slot_of, slot_comp0, out_of, out_row0, fx_rows, val_rows);
   std::memcpy(t.slot_of, slot_of, sizeof(t.slot_of));
   std::memcpy(t.slot_comp0, slot_comp0, sizeof(t.slot_comp0));
   std::memcpy(t.out_of, out_of, sizeof(t.out_of));
@@ -310,33 +338,36 @@ static bool tables_fx(const std::vector<unsigned char>& tab, int dim, int degree
   return false;
 }
 template <int dim, int degree>
-static bool tables_lanes_impl(const unsigned char* tab) {
+static int tables_lanes_impl(const unsigned char* tab) {
   const auto* t = reinterpret_cast<const pg::CellTables<dim, degree, double>*>(tab);
-  return t->fx != 0 && t->fx_lanes != 0;
+  return t->fx == 0 || t->fx_lanes == 0 ? 0 : (t->fx_cubic ? 4 : 5);
 }
-// whether the tables allow the lane kernel (integer contractions on cubic cells)
-bool tables_lanes(const std::vector<unsigned char>& tab, int dim, int degree) {
-  if (tab.empty()) return false;
+// the tables' lane kernel mode: 4 on cubic cells, 5 on stretched ones, 0 without integer contractions
+int tables_lanes(const std::vector<unsigned char>& tab, int dim, int degree) {
+  if (tab.empty()) return 0;
   const unsigned char* t = tab.data();
   PPF_DD_SWITCH(tables_lanes_impl, t)
-  return false;
+  return 0;
 }
 
-// the launch-record fields of a contraction mode (1-4, see BlockPlan::fx_mode)
+// the launch-record fields of a contraction mode (1-5, see BlockPlan::fx_mode)
 void set_fx_mode(CellLaunch& L, int m) {
   L.fx_deriv = m != 3;
   L.fx_int = m == 2 || m == 3;
-  L.fx_lanes = m == 4;
+  L.fx_lanes = m >= 4;
 }
 
-// PPF_CONTRACTION_MODE: a fixed contraction mode (1-4), or 0 when unset; mode 4 falls back to
-// mode 1 where the lane kernel does not apply
-int env_fx_mode(bool lanes_ok) {
+// PPF_CONTRACTION_MODE: a fixed contraction mode (1-5), or 0 when unset; modes 4 and 5 fall back to
+// mode 1 where theirs is not the operator's lane kernel mode
+int env_fx_mode(int lanes) {
   const char* env = std::getenv("PPF_CONTRACTION_MODE");
-  if (!(env && env[0] >= '1' && env[0] <= '4' && env[1] == 0)) return 0;
+  if (!(env && env[0] >= '1' && env[0] <= '5' && env[1] == 0)) return 0;
   const int m = env[0] - '0';
-  return m == 4 && !lanes_ok ? 1 : m;
+  return m >= 4 && m != lanes ? 1 : m;
 }
+
+// the i-th mode an operator's timing tries (0, 1, ..): 1 to 3, then its lane kernel mode
+int timed_fx_mode(int i, int lanes) { return i < 3 ? 1 + i : lanes; }
 
 std::vector<unsigned char> build_cell_tables(int dim, int degree, int precision, const double* lo, const double* h,
                                              const signed char slot_of[pg::MAX_FIELDS][pg::NAGE],
@@ -743,7 +774,7 @@ int launch_cell(ppf_handle h, int b, int which, const double* const* src, bool p
       // right-hand side of a linear or Newton block (once per solve) takes the lane kernel
       // where it applies, else mode 1
       if (which == 0 && B.desc.solve_type != PPF_EXPLICIT && !env_fx_mode(P.fx_lanes)) {
-        P.fx_mode = P.fx_lanes ? 4 : 1;
+        P.fx_mode = P.fx_lanes ? P.fx_lanes : 1;
       } else {
         const int rc = choose_fx_mode(h, P, mode, L, smem);
         if (rc) return rc;
@@ -758,10 +789,10 @@ int launch_cell(ppf_handle h, int b, int which, const double* const* src, bool p
 // each in fixed point (issue slots) or in FP64 (the FP64 pipe). Which split is cheapest depends
 // on how much FP64 work the callback itself does, so the first plain launch of a plan times
 // modes 1 (integer derivatives, FP64 integration), 2 (both integer), 3 (FP64 derivatives,
-// integer integration) and, on cubic cells, 4 (the lane kernel), twice each, back to back into
+// integer integration) and the lane kernel (4 on cubic cells, 5 on others), twice each, back to back into
 // the block's accumulators (which every caller has just zeroed, and which are zeroed again
-// afterwards), and keeps the fastest. PPF_CONTRACTION_MODE=1-4 fixes the mode; a plan first
-// launched inside a graph capture takes mode 4 where it applies, else mode 1.
+// afterwards), and keeps the fastest. PPF_CONTRACTION_MODE=1-5 fixes the mode; a plan first
+// launched inside a graph capture takes the lane kernel where it applies, else mode 1.
 static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch& L, size_t smem) {
   if (const int m = env_fx_mode(P.fx_lanes)) {
     P.fx_mode = m;
@@ -771,7 +802,7 @@ static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
   if (h->capturing || cs != cudaStreamCaptureStatusNone) {
-    P.fx_mode = P.fx_lanes ? 4 : 1;
+    P.fx_mode = P.fx_lanes ? P.fx_lanes : 1;
     return PPF_OK;
   }
   const int nm = P.fx_lanes ? 4 : 3;
@@ -782,7 +813,7 @@ static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch
   CellLaunch T = L;
   if (e == cudaSuccess) e = cudaEventRecord(ev[0], h->stream);
   for (int r = 0; r < NT && e == cudaSuccess; ++r) {
-    set_fx_mode(T, 1 + r % nm);
+    set_fx_mode(T, timed_fx_mode(r % nm, P.fx_lanes));
     e = h->custom_launch ? (cudaError_t)h->custom_launch(h->dim, h->k, mode, 0, &T, h->model_obj.data(), smem,
                                                          (void*)h->stream)
                          : h->model->launch(h->dim, h->k, mode, 0, T, h->model_obj.data(), smem, h->stream);
@@ -803,7 +834,7 @@ static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch
   int m = 0;
   for (int i = 1; i < nm; ++i)
     if (best[i] < best[m]) m = i;
-  P.fx_mode = 1 + m;
+  P.fx_mode = timed_fx_mode(m, P.fx_lanes);
   return PPF_OK;
 }
 

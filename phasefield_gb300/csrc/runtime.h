@@ -38,11 +38,14 @@ std::vector<unsigned char> build_cell_tables(int dim, int degree, int precision,
                                              const signed char* slot_comp0, const signed char* out_of,
                                              const signed char* out_row0, unsigned int fx_rows = 0xffffffffu,
                                              unsigned int val_rows = 0xffffffffu);
-// whether FP64 tables allow the lane kernel (integer contractions, cubic cells)
-bool tables_lanes(const std::vector<unsigned char>& tab, int dim, int degree);
-// the launch-record fields of contraction mode m (1-4)
+// the lane kernel mode of FP64 tables: 4 on cubic cells, 5 on stretched ones, 0 where it does not apply
+int tables_lanes(const std::vector<unsigned char>& tab, int dim, int degree);
+// the launch-record fields of contraction mode m (1-5)
 void set_fx_mode(CellLaunch& L, int m);
-// PPF_CONTRACTION_MODE (1-4, mode 4 only where the lane kernel applies, else 1), 0 when unset
-int env_fx_mode(bool lanes_ok);
+// PPF_CONTRACTION_MODE (1-5; 4 and 5 only where they are the operator's lane kernel mode `lanes`,
+// else 1), 0 when unset
+int env_fx_mode(int lanes);
+// the i-th mode an operator's timing tries (3 of them, or 4 with a lane kernel mode)
+int timed_fx_mode(int i, int lanes);
 
 }  // namespace ppf
