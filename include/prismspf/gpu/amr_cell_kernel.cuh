@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
   int* ex_in = reinterpret_cast<int*>(vals_fx + P.nrows_in * S::threads);
   bool fx_on = false;
   unsigned int fx_rows = 0;
+  chain_release();
+  chain_wait();
   if constexpr (FXC) {
     unsigned int dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
@@ -123,16 +125,16 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
               if (sd.constrained_read) {
                 const int m = __ldg(sd.cmap + idx);
                 if (m == (int)idx) {
-                  v = __ldg(ptr + idx);
+                  v = ptr[idx];
                 } else if (m >= AMR_HANG_BASE) {
                   const int r = m - AMR_HANG_BASE;
                   for (int e = __ldg(A.h_ptr + r); e < __ldg(A.h_ptr + r + 1); ++e) {
                     const long long mi = base + __ldg(A.h_idx + e);
-                    if (__ldg(sd.cmap + mi) == (int)mi) v += number(__ldg(A.h_w + e)) * __ldg(ptr + mi);
+                    if (__ldg(sd.cmap + mi) == (int)mi) v += number(__ldg(A.h_w + e)) * ptr[mi];
                   }
                 }
               } else {
-                v = __ldg(ptr + idx);
+                v = ptr[idx];
               }
             }
             vals[(row + c) * S::threads + t] = v;
@@ -252,8 +254,7 @@ cudaError_t launch_amr_cell_kernel(const AmrCellLaunch& A, const void* obj, size
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, S::threads, smem, s>>>(A, *reinterpret_cast<const PDE*>(obj));
-  return cudaGetLastError();
+  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, A, *reinterpret_cast<const PDE*>(obj));
 }
 
 }  // namespace ppf

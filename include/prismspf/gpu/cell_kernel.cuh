@@ -66,6 +66,31 @@ using prismspf::FieldContainer;
 using prismspf::SimulationTimer;
 namespace pg = prismspf::gpu;
 
+// Programmatic dependent launch (launch_chained): a kernel launched
+// this way may start while the kernel before it on its stream still runs. chain_wait returns
+// when that kernel has completed and its writes are visible; nothing another kernel writes may be
+// touched before it. chain_release lets the next kernel of the chain start (it waits in its own
+// chain_wait); every kernel of a chain waits, so completion is transitive along the stream. Both
+// do nothing in a kernel that was launched plainly.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// launches a kernel that begins with chain_wait as a dependent of the one before it on the stream
+template <class... K, class... A>
+cudaError_t launch_chained(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...);
+}
+
 enum CellMode { MODE_RHS = 0, MODE_LHS = 1, MODE_DIAG = 2 };
 
 struct SlotDesc {
@@ -244,6 +269,8 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
   int* ex_out = ex_in + P.nrows_in * cpb;
   bool fx_on = false, fx_int = false;  // fx_on: fixed-point derivatives
   unsigned int tab_fx_rows = 0;
+  chain_release();
+  chain_wait();  // (the allocation-free step's tables come from the kernel before)
   if constexpr (FXC) {
     unsigned int dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
@@ -318,10 +345,10 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
                   // the value load issues with the map load: almost every entry is free, so
                   // the dependent second load is only paid on constrained entries
                   const int m = __ldg(sd.cmap + idx);
-                  const number own = __ldg(ptr + idx);
-                  v = m == (int)idx ? own : (m >= 0 ? __ldg(ptr + m) : number(0));
+                  const number own = ptr[idx];
+                  v = m == (int)idx ? own : (m >= 0 ? ptr[m] : number(0));
                 } else {
-                  v = __ldg(ptr + idx);
+                  v = ptr[idx];
                 }
               }
               vals[(row + c) * S::threads + t] = v;

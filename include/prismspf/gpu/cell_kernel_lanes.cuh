@@ -20,7 +20,7 @@
 //     (1, 1 or 1, 4, 1 per direction) divided out of its node, an integral is the exact sum
 //     x + sum_d L_d, L_d = +-(4 (own + m) - (own + f)) at the ends of a Q2 line and g_0 - g_2 in its
 //     middle: no weight is multiplied in, 25 is the largest coefficient sum, and the terms keep 57
-//     bits below the cell's largest one. It is rounded once with the scale detJ / (h_0 W^dim) and
+//     bits (59 on Q1 cells) below the cell's largest one. It is rounded once with the scale detJ / (h_0 W^dim) and
 //     the node's weight as an exponent. No FP64 instruction outside the user's callback: on GB300
 //     the FP64 pipe retires about two operations per SM per clock and every FP64 conversion runs
 //     on it too, so the integer path (issue slots) replaces 9-10 FP64 operations per point;
@@ -35,7 +35,7 @@
 //     integrated (rows the callback leaves stay zero), so no branch depends on which terms were
 //     submitted; lanes past the last cell recompute the last cell and skip its scatter.
 // Accuracy: every derivative and every node's integral is one rounding of an exact sum of values
-// cut to 2^-59 (derivatives) or 2^-57 (integration) of the largest magnitude of their cell and row.
+// cut to 2^-59 (derivatives) or 2^-57 (integration, 2^-59 on Q1 cells) of the largest magnitude of their cell and row.
 //
 // What bounds it: instruction issue (58-61 % of the slots, the ALU pipe 50-57 % busy, the FP64 pipe
 // 31-55 %; DRAM 4 %). Cahn-Hilliard 64^3 Q2, per launch of the c and the mu block: 130 and 157 us at
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   constexpr int n = S::n, nq = S::nq, cols = S::cols, k = degree, CPT = LANE_CPT;
   constexpr int ROW = nq * CPT;   // entries of one row
   constexpr int JS = cols * CPT;  // entry stride between a thread's points
-  constexpr int TOPT = fx::LANE_TOP_INTEGRAL;
+  constexpr int TOPT = n == 2 ? fx::LANE_TOP_INTEGRAL_Q1 : fx::LANE_TOP_INTEGRAL;
   constexpr int TC = 1 + dim;     // terms of a component
   constexpr bool REGS = NC == 1;
   constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20, FLOOR_OUT = (fx::EXP_FLOOR + fx::EXP_BIAS) << 20;
@@ -204,6 +204,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;  // lattice stride of the last direction
   const unsigned int ncells = (unsigned int)P.ncells;
   const unsigned int ntiles = (ncells + CPT - 1) / CPT;
+  chain_release();
+  chain_wait();
   __syncthreads();  // exponent buffers set
 
   int par = 0;
@@ -244,12 +246,12 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
           for (int j = 0; j < n; ++j) {
             const unsigned int idx = node0 + (unsigned int)j * lstride;
             const int m = __ldg(cm + idx);
-            const double own = __ldg(base + idx);
-            v[j] = m == (int)(idx + R.in_off[r]) ? own : (m >= 0 ? __ldg(R.in_base[r] + m) : 0.0);
+            const double own = base[idx];
+            v[j] = m == (int)(idx + R.in_off[r]) ? own : (m >= 0 ? R.in_base[r][m] : 0.0);
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < n; ++j) v[j] = __ldg(base + (node0 + (unsigned int)j * lstride));
+          for (int j = 0; j < n; ++j) v[j] = base[node0 + (unsigned int)j * lstride];
         }
         const int vs = R.in_v[r], gs = R.in_g[r];
         if (vs >= 0) {
@@ -491,6 +493,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;
   const unsigned int ncells = (unsigned int)P.ncells;
   const unsigned int ntiles = (ncells + CPT - 1) / CPT;
+  chain_release();
+  chain_wait();
 
   for (unsigned int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned int cell_t = tile * CPT + lc;
@@ -521,10 +525,10 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
           float v;
           if (R.in_cmap[r]) {
             const int m = __ldg(R.in_cmap[r] + idx);
-            const float own = __ldg(base + idx);
-            v = m == (int)idx ? own : (m >= 0 ? __ldg(base + m) : 0.f);
+            const float own = base[idx];
+            v = m == (int)idx ? own : (m >= 0 ? base[m] : 0.f);
           } else {
-            v = __ldg(base + idx);
+            v = base[idx];
           }
           vals[r * ROW + p0 + j * JS] = v;
         }
@@ -655,10 +659,8 @@ cudaError_t launch_lanes(const CellLaunch& P, const LaneRows& R, const void* obj
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, S::threads, smem, s>>>(P, *reinterpret_cast<const PDE*>(obj),
-                                                *reinterpret_cast<const pg::CellTables<dim, degree, double>*>(P.tables_host),
-                                                R);
-  return cudaGetLastError();
+  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj),
+                        *reinterpret_cast<const pg::CellTables<dim, degree, double>*>(P.tables_host), R);
 }
 
 template <class PDE, int dim, int degree, int MINB>
@@ -692,10 +694,8 @@ cudaError_t launch_lanes_f32(const CellLaunch& P, const LaneRows& R, const void*
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, S::threads, smem, s>>>(P, *reinterpret_cast<const PDE*>(obj),
-                                                *reinterpret_cast<const pg::CellTables<dim, degree, float>*>(P.tables_host),
-                                                R);
-  return cudaGetLastError();
+  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj),
+                        *reinterpret_cast<const pg::CellTables<dim, degree, float>*>(P.tables_host), R);
 }
 
 // the FP32 lane kernel for an FP32 Q1/Q2 left-hand side, or cudaErrorNotSupported

@@ -130,6 +130,8 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
   namespace fx = pg::fx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Tab* tab = reinterpret_cast<Tab*>(smem_raw);
+  chain_release();
+  chain_wait();
   {
     const int nwords = (int)(sizeof(Tab) / 4);
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);
@@ -209,10 +211,10 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
               const unsigned int idx = node + (unsigned int)c * N;
               if (sd.constrained_read) {
                 const int m = __ldg(sd.cmap + idx);
-                const double own = __ldg(ptr + idx);
-                v = m == (int)idx ? own : (m >= 0 ? __ldg(ptr + m) : 0.0);
+                const double own = ptr[idx];
+                v = m == (int)idx ? own : (m >= 0 ? ptr[m] : 0.0);
               } else {
-                v = __ldg(ptr + idx);
+                v = ptr[idx];
               }
             }
             const int r = row + c;
@@ -347,8 +349,7 @@ cudaError_t launch_cell_kernel_warp_impl(const CellLaunch& P, const void* obj, s
   long long grid = (long long)sms * occ;
   if (grid > blocks_needed) grid = blocks_needed;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, W::threads, smem, s>>>(P, *reinterpret_cast<const PDE*>(obj));
-  return cudaGetLastError();
+  return launch_chained(kern, dim3((unsigned)grid), dim3(W::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj));
 }
 
 }  // namespace ppf

@@ -203,8 +203,10 @@ PPF_FX double to_double_fast(long long x, int lsb, unsigned long long sig, bool 
 // otherwise), so that no result falls below the normal range and zeros need no test of their own.
 constexpr int EXP_FLOOR = 192;
 // fixed-point tops of the lane kernel: |3 u + 4 v + w| <= 8 * 2^60 keeps a derivative's line sum
-// below 2^63, and |x + sum_d L_d| <= (1 + 3 * 8) 2^58 a node's integral over its weight
+// below 2^63; so does |x + sum_d L_d|, a node's integral over its weight, which is at most
+// (1 + 3 * 2) 2^60 on Q1 cells and (1 + 3 * 8) 2^58 on Q2 cells
 constexpr int LANE_TOP_VALUES = 59;
+constexpr int LANE_TOP_INTEGRAL_Q1 = 59;
 constexpr int LANE_TOP_INTEGRAL = 57;
 constexpr int MAX_SCALE = 60;
 constexpr int EXP_BIAS = 64;    // of the exponents of scaled terms

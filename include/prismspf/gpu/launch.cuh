@@ -50,8 +50,7 @@ cudaError_t launch_cell_kernel_impl(const CellLaunch& P, const void* obj, size_t
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, S::threads, smem, s>>>(P, *reinterpret_cast<const PDE*>(obj));
-  return cudaGetLastError();
+  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj));
 }
 
 // An operator may run its FP64 Q1/Q2 left-hand side on the warp-resident kernel

@@ -49,7 +49,7 @@ struct AmrState {
 namespace {
 
 // value of a free or Dirichlet row after the explicit update
-__device__ __forceinline__ double amr_final_value(const double* __restrict__ acc, const double* __restrict__ invm,
+__device__ __forceinline__ double amr_final_value(const double* acc, const double* __restrict__ invm,
                                                   const int* __restrict__ cmap, const double* __restrict__ dvals,
                                                   long long gi, long long i) {
   const int cm = cmap ? cmap[gi] : (int)gi;
@@ -60,11 +60,13 @@ __device__ __forceinline__ double amr_final_value(const double* __restrict__ acc
 // accumulator, Dirichlet rows take their values, hanging rows the interpolant of their masters'
 // final values (computed here from the masters' accumulators, so one launch does all rows; the
 // reference's invM is 0 on hanging rows and distribute() sets them)
-__global__ void amr_finalize_kernel(double* __restrict__ u, const double* __restrict__ acc,
-                                    const double* __restrict__ invm, const int* __restrict__ cmap,
-                                    const double* __restrict__ dvals, const int* __restrict__ h_ptr,
-                                    const int* __restrict__ h_idx, const double* __restrict__ h_w, long long N,
-                                    int* err) {
+__global__ void amr_finalize_kernel(double* u, const double* acc, double* clear, const double* __restrict__ invm,
+                                    const int* __restrict__ cmap, const double* dvals, const int* __restrict__ h_ptr,
+                                    const int* __restrict__ h_idx, const double* __restrict__ h_w, long long N, int* err,
+                                    prismspf::SimulationTimer* timer, double dt) {
+  chain_release();
+  chain_wait();
+  if (timer && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) timer->increment(dt);
   const long long base = blockIdx.y * N;
   int bad = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
@@ -83,6 +85,7 @@ __global__ void amr_finalize_kernel(double* __restrict__ u, const double* __rest
     }
     bad |= !isfinite(v);
     u[gi] = v;
+    if (clear) clear[gi] = 0.0;
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, int(pg::ERR_NONFINITE));
 }
@@ -362,12 +365,12 @@ static int distribute(ppf_handle h, FieldState& F, double* v) {
 
 int amr_apply_constraints(ppf_handle h, FieldState& F, double* v) { return distribute(h, F, v); }
 
-int amr_finalize_explicit(ppf_handle h, FieldState& F) {
+int amr_finalize_explicit(ppf_handle h, FieldState& F, double* clear, prismspf::SimulationTimer* timer) {
   AmrState& S = *h->amr;
   dim3 grid(grid_for(h->N), F.ncomp);
-  amr_finalize_kernel<<<grid, 256, 0, h->stream>>>(F.cur, F.acc, h->d_invm, F.constrained ? F.cmap : nullptr, F.dvals,
-                                                   S.d_h_ptr, S.d_h_idx, S.d_h_w, h->N, h->d_err);
-  PPF_CUDA(h, cudaGetLastError());
+  PPF_CUDA(h, launch_chained(amr_finalize_kernel, grid, dim3(256), 0, h->stream, F.cur, F.acc, clear, h->d_invm,
+                             F.constrained ? F.cmap : nullptr, F.dvals, S.d_h_ptr, S.d_h_idx, S.d_h_w, h->N, h->d_err,
+                             timer, h->dt));
   h->all_launches++;
   return PPF_OK;
 }
@@ -544,8 +547,7 @@ static int adapt(ppf_handle h) {
       else F.old[a - 1] = nv;
     }
     if (rc) break;
-    cudaFree(F.acc);
-    F.acc = nullptr;
+    free_acc(F);
     F.len = len;
     if (cudaMalloc(&F.acc, sizeof(double) * len) != cudaSuccess) rc = fail(h, PPF_ERR_CUDA, "out of device memory");
   }
@@ -676,7 +678,7 @@ int ppf_set_adaptivity(ppf_handle h, const ppf_adaptivity* a) {
       cudaFree(F.old[k]);
       F.old[k] = nullptr;
     }
-    cudaFree(F.acc);
+    free_acc(F);
     F.len = F.ncomp * h->N;
     PPF_CUDA(h, cudaMalloc(&F.cur, sizeof(double) * F.len));
     PPF_CUDA(h, cudaMemsetAsync(F.cur, 0, sizeof(double) * F.len, h->stream));

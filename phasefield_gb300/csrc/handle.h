@@ -24,6 +24,10 @@ struct FieldState {
   double* cur = nullptr;
   double* old[4] = {nullptr, nullptr, nullptr, nullptr};
   double* acc = nullptr;
+  // Explicit solves alternate between two accumulators: the finalize kernel that reads one clears
+  // the other for the next solve, in place of a launch of its own. acc_clean: acc is all zero.
+  double* acc2 = nullptr;
+  bool acc_clean = false;
   int* cmap = nullptr;
   double* dvals = nullptr;
   std::vector<int> h_cmap;
@@ -211,6 +215,8 @@ struct ppf_handle_s {
   long long graph_state_version = -1; // state buffers the increment graph was captured on
   // CUDA graph of the explicit increment loop
   prismspf::SimulationTimer* d_timer = nullptr;
+  std::vector<double*> graph_acc;  // each field's accumulator at the start of the graph
+  bool advance_timer = false;      // (while capturing) the next finalize launch advances d_timer
   cudaGraphExec_t run_graph = nullptr;
   cudaStream_t graph_stream = nullptr;
   int graph_period = 0;
@@ -240,6 +246,10 @@ inline int fail(ppf_handle h, int code, const std::string& msg) {
   } while (0)
 
 unsigned grid_for(long long n);
+// makes F.acc all zero (a memset unless it already is) / the second accumulator of explicit solves
+int clear_acc(ppf_handle h, FieldState& F);
+int ensure_acc2(ppf_handle h, FieldState& F);
+void free_acc(FieldState& F);
 int check_err(ppf_handle h);
 double* state_ptr(ppf_handle h, int f, int age);
 // records a kernel launch for the statistics; brackets cell launches with events when timing
@@ -254,7 +264,7 @@ struct AdjointState;
 void free_adjoint(AdjointState* A);
 // adaptive meshes (amr.cu)
 int amr_launch_cell(ppf_handle h, int b, int which, const CellLaunch& L);
-int amr_finalize_explicit(ppf_handle h, FieldState& F);
+int amr_finalize_explicit(ppf_handle h, FieldState& F, double* clear, prismspf::SimulationTimer* timer);
 int amr_remesh_if_due(ppf_handle h);
 unsigned amr_next_remesh(ppf_handle h, unsigned inc);
 int amr_permute_io(ppf_handle h, int f, double* host, const double* dev_src, double* dev_dst, int ordering,

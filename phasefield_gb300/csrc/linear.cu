@@ -1007,6 +1007,7 @@ int linear_solve(ppf_handle h, int b) {
   auto outer_apply = [&](const double* src, double* dst, bool plain) -> int {
     const double* srcs[PPF_MAX_FIELDS] = {src};
     PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * n, h->stream));
+    F.acc_clean = false;
     if (h->amr) {
       int rc = launch_cell(h, b, 1, srcs, plain);
       if (rc) return rc;
@@ -1098,6 +1099,7 @@ int linear_solve(ppf_handle h, int b) {
   // rhs = S * compute_rhs
   {
     PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * n, h->stream));
+    F.acc_clean = false;
     if (B.plan[0].valid && B.plan[0].nslots >= 0) {
       int rc = launch_cell(h, b, 0, nullptr);
       if (rc) return rc;

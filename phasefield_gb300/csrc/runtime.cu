@@ -403,24 +403,44 @@ size_t cell_smem(int dim, int degree, int precision, int nrows_in, int nrows_out
 // u = invM (.) acc with constraints: masters/free rows scale their own accumulator, periodic
 // images copy their master's result, Dirichlet rows take their value.
 // With u2 set (a queued run streaming the field out) the result is written there as well, so the
-// copy to the host reads a buffer the following increments do not touch.
-__global__ void finalize_explicit_kernel(double* __restrict__ u, const double* __restrict__ acc,
-                                         const double* __restrict__ invm, const int* __restrict__ cmap,
-                                         const double* __restrict__ dvals, long long N, int* err,
-                                         double* __restrict__ u2) {
+// copy to the host reads a buffer the following increments do not touch. `clear` (the other
+// accumulator of the field, which nothing reads any more) is zeroed for the next solve, and `timer`
+// (in a captured increment, after its last block) advanced: work that took a memset and a launch of
+// their own (128^2 Q1 Allen-Cahn: 12.9 us an increment before, with four launches).
+// Bound by memory: 36 bytes a node plus 8 for `clear`; four rows in flight a thread.
+__global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const double* acc, double* clear,
+                                                                const double* __restrict__ invm,
+                                                                const int* __restrict__ cmap, const double* dvals,
+                                                                long long N, int* err, double* u2,
+                                                                prismspf::SimulationTimer* timer, double dt) {
+  constexpr int U = 4;
+  chain_release();
+  chain_wait();
   const int c = blockIdx.y;
   const long long base = c * N;
+  const long long step = (long long)gridDim.x * blockDim.x;
   int bad = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    const long long gi = base + i;
-    const int cm = cmap ? cmap[gi] : (int)gi;
-    double v;
-    if (cm >= 0) v = invm[cm - base] * acc[cm];
-    else v = dvals[-1 - cm];
-    bad |= !isfinite(v);
-    u[gi] = v;
-    if (u2) u2[gi] = v;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < N; i0 += U * step) {
+    int cm[U];
+    double v[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const long long i = i0 + k * step;
+      cm[k] = i < N ? (cmap ? cmap[base + i] : (int)(base + i)) : (int)base;
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) v[k] = cm[k] >= 0 ? invm[cm[k] - base] * acc[cm[k]] : dvals[-1 - cm[k]];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const long long i = i0 + k * step;
+      if (i >= N) continue;
+      bad |= !isfinite(v[k]);
+      u[base + i] = v[k];
+      if (u2) u2[base + i] = v[k];
+      if (clear) clear[base + i] = 0.0;
+    }
   }
+  if (timer && blockIdx.x == 0 && c == 0 && threadIdx.x == 0) timer->increment(dt);
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, int(pg::ERR_NONFINITE));
 }
 
@@ -873,19 +893,55 @@ int stream_field_out(ppf_handle h, FieldState& F, const double* src, bool staged
 int finish_streamed_outputs(ppf_handle h);
 static int ensure_out_stage(ppf_handle h, FieldState& F);
 
+int clear_acc(ppf_handle h, FieldState& F) {
+  if (!F.acc_clean) PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
+  F.acc_clean = true;
+  return PPF_OK;
+}
+
+int ensure_acc2(ppf_handle h, FieldState& F) {
+  if (!F.acc2) PPF_CUDA(h, cudaMalloc(&F.acc2, sizeof(double) * F.len));
+  return PPF_OK;
+}
+
+void free_acc(FieldState& F) {
+  cudaFree(F.acc);
+  cudaFree(F.acc2);
+  F.acc = F.acc2 = nullptr;
+  F.acc_clean = false;
+}
+
 static int explicit_solve(ppf_handle h, int b) {
   BlockState& B = h->blocks[b];
+  // a caller's own capture (not the increment graph, whose period returns the accumulators to where
+  // they were) may replay this solve on its own: it clears its accumulator itself and keeps it
+  bool alternate = true;
+  if (!h->capturing) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
+    alternate = cs == cudaStreamCaptureStatusNone;
+  }
   for (int i = 0; i < B.desc.n_fields; ++i) {
     FieldState& F = h->fields[B.desc.field_indices[i]];
-    PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
+    int rc = alternate ? ensure_acc2(h, F) : PPF_OK;
+    if (!alternate) F.acc_clean = false;
+    if (!rc) rc = clear_acc(h, F);
+    if (rc) return rc;
+    F.acc_clean = false;
   }
   int rc = launch_cell(h, b, 0, nullptr);
   if (rc) return rc;
   for (int i = 0; i < B.desc.n_fields; ++i) {
     FieldState& F = h->fields[B.desc.field_indices[i]];
+    double* clear = alternate ? F.acc2 : nullptr;
+    prismspf::SimulationTimer* timer = h->advance_timer && i + 1 == B.desc.n_fields ? h->d_timer : nullptr;
     if (h->amr) {
-      rc = amr_finalize_explicit(h, F);
+      rc = amr_finalize_explicit(h, F, clear, timer);
       if (rc) return rc;
+      if (alternate) {
+        std::swap(F.acc, F.acc2);
+        F.acc_clean = true;
+      }
       continue;
     }
     // a queued run streaming this field out: the finalize writes the output staging buffer too
@@ -896,11 +952,15 @@ static int explicit_solve(ppf_handle h, int b) {
       if (rc) return rc;
       PPF_CUDA(h, cudaStreamWaitEvent(h->stream, F.out_free, 0));
     }
-    dim3 grid(grid_for(h->N), F.ncomp);
-    finalize_explicit_kernel<<<grid, 256, 0, h->stream>>>(F.cur, F.acc, h->d_invm, F.constrained ? F.cmap : nullptr,
-                                                          F.dvals, h->N, h->d_err, staged ? F.out_stage : nullptr);
-    PPF_CUDA(h, cudaGetLastError());
+    dim3 grid(grid_for((h->N + 3) / 4), F.ncomp);
+    PPF_CUDA(h, launch_chained(finalize_explicit_kernel, grid, dim3(256), 0, h->stream, F.cur, F.acc, clear, h->d_invm,
+                               F.constrained ? F.cmap : nullptr, F.dvals, h->N, h->d_err,
+                               staged ? F.out_stage : nullptr, timer, h->dt));
     h->all_launches++;
+    if (alternate) {
+      std::swap(F.acc, F.acc2);
+      F.acc_clean = true;
+    }
     if (F.stream_out) {
       // the field is final: copy it out on the copy stream while the later blocks compute
       rc = stream_field_out(h, F, staged ? F.out_stage : F.cur, staged);
@@ -1040,11 +1100,24 @@ static void end_increment(ppf_handle h) {
   h->timer.increment(h->dt);
 }
 
+// the block whose finalize launch ends an increment of the graph (-1: none does)
+static int last_explicit_block(ppf_handle h) {
+  int last = -1;
+  for (int b = 0; b < (int)h->blocks.size(); ++b) {
+    const ppf_block_desc& d = h->blocks[b].desc;
+    if (d.solve_type == PPF_EXPLICIT && d.solve_timing != PPF_POSTPROCESS && d.solve_timing != PPF_NUCLEATION_RATE) last = b;
+  }
+  return last;
+}
+
 static int solve_increment(ppf_handle h, int output_every) {
   const unsigned inc = h->timer.get_increment();
   const bool is_output = output_every > 0 && inc % (unsigned)output_every == 0;
+  const int last = h->capturing ? last_explicit_block(h) : -1;
   for (size_t b = 0; b < h->blocks.size(); ++b) {
+    h->advance_timer = (int)b == last;
     int rc = increment_block(h, (int)b, is_output);
+    h->advance_timer = false;
     if (rc) return rc;
   }
   if (h->amr) {
@@ -1295,7 +1368,7 @@ void ppf_destroy(ppf_handle h) {
   for (auto& F : h->fields) {
     cudaFree(F.cur);
     for (int a = 0; a < 4; ++a) cudaFree(F.old[a]);
-    cudaFree(F.acc);
+    free_acc(F);
     cudaFree(F.cmap);
     cudaFree(F.dvals);
   }
@@ -1501,7 +1574,8 @@ static int rotation_period(ppf_handle h) {
     }
     p = p / a * q;
   }
-  return p;
+  // an even number of increments brings the alternating accumulators back as well
+  return p % 2 ? 2 * p : p;
 }
 
 static int capture_graph(ppf_handle h) {
@@ -1513,13 +1587,21 @@ static int capture_graph(ppf_handle h) {
   const int period = rotation_period(h);
   const prismspf::SimulationTimer saved = h->timer;
   const long long launches0 = h->all_launches;
+  const int last = last_explicit_block(h);
+  h->graph_acc.clear();
+  for (auto& F : h->fields) {
+    int rc = ensure_acc2(h, F);
+    if (!rc) rc = clear_acc(h, F);
+    if (rc) return rc;
+    h->graph_acc.push_back(F.acc);
+  }
   cudaGraph_t g;
   PPF_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   h->capturing = true;
   int rc = PPF_OK;
   for (int i = 0; i < period && !rc; ++i) {
     rc = solve_increment(h, 0);
-    if (!rc) {
+    if (!rc && last < 0) {
       advance_timer_kernel<<<1, 1, 0, h->stream>>>(h->d_timer, h->dt);
       h->all_launches++;
     }
@@ -1577,6 +1659,16 @@ static int run_increments(ppf_handle h, unsigned int n_increments, int output_ev
         }
         PPF_CUDA(h, cudaMemcpyAsync(h->d_timer, &h->timer, sizeof(prismspf::SimulationTimer), cudaMemcpyHostToDevice,
                                     h->stream));
+        // the accumulators the graph starts from, all zero
+        for (size_t f = 0; f < h->fields.size(); ++f) {
+          FieldState& F = h->fields[f];
+          if (F.acc != h->graph_acc[f]) {
+            std::swap(F.acc, F.acc2);
+            F.acc_clean = false;
+          }
+          const int rc = clear_acc(h, F);
+          if (rc) return rc;
+        }
         const unsigned reps = remaining / period;
         for (unsigned r = 0; r < reps; ++r) PPF_CUDA(h, cudaGraphLaunch(h->run_graph, h->stream));
         for (unsigned k = 0; k < reps * (unsigned)period; ++k) h->timer.increment(h->dt);
@@ -1659,6 +1751,7 @@ int ppf_apply_device(ppf_handle h, int b, int which, const double* d_src, double
     FieldState& F = h->fields[B.desc.field_indices[i]];
     srcs[i] = d_src ? d_src + off : nullptr;
     PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
+    F.acc_clean = false;
     off += F.len;
   }
   int rc = launch_cell(h, b, which, srcs);
