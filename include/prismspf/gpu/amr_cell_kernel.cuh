@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
       for (int s = 0; s < pg::MAX_SLOTS; ++s) {
         if (s < P.nslots) {
           const SlotDesc& sd = P.slots[s];
-          const number* ptr = static_cast<const number*>(sd.ptr);
+          const number* ptr = global_ptr(static_cast<const number*>(sd.ptr));
           for (int c = 0; c < sd.ncomp; ++c) {
             number v = number(0);
             if (active) {

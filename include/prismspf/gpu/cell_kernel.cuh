@@ -75,6 +75,14 @@ namespace pg = prismspf::gpu;
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A pointer out of a launch record, told to be one to global memory: its plain loads may then move
+// across shared-memory stores, as __ldg's do.
+template <class T>
+__device__ __forceinline__ T* global_ptr(T* p) {
+  __builtin_assume(__isGlobal(p));
+  return p;
+}
+
 // launches a kernel that begins with chain_wait as a dependent of the one before it on the stream
 template <class... K, class... A>
 cudaError_t launch_chained(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
         if (s < P.nslots) {
           const SlotDesc& sd = P.slots[s];
           if (!(MODE == MODE_DIAG && sd.is_src)) {
-            const number* ptr = static_cast<const number*>(sd.ptr);
+            const number* ptr = global_ptr(static_cast<const number*>(sd.ptr));
             for (int c = 0; c < sd.ncomp; ++c) {
               number v = number(0);
               if (active) {

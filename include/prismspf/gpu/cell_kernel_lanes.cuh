@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
 #pragma unroll
     for (int r = 0; r < LANE_MAX_IN; ++r) {
       if (r < R.nin) {
-        const double* base = R.in_base[r] + R.in_off[r];
+        const double* base = global_ptr(R.in_base[r] + R.in_off[r]);
         double v[n];
         if (R.in_cmap[r]) {
           const int* cm = R.in_cmap[r] + R.in_off[r];
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
             const unsigned int idx = node0 + (unsigned int)j * lstride;
             const int m = __ldg(cm + idx);
             const double own = base[idx];
-            v[j] = m == (int)(idx + R.in_off[r]) ? own : (m >= 0 ? R.in_base[r][m] : 0.0);
+            v[j] = m == (int)(idx + R.in_off[r]) ? own : (m >= 0 ? global_ptr(R.in_base[r] + m)[0] : 0.0);
           }
         } else {
 #pragma unroll
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
                                          E >= fx::EXP_WIDE, E >= fx::EXP_NONFINITE);
       const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
       const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
-      if (active && target >= 0) atomicAdd(R.out_acc[o] + target, r);
+      if (active && target >= 0) atomicAdd(global_ptr(R.out_acc[o] + target), r);
     };
     if constexpr (REGS) {
       const int E = (int)(exo[lc] >> 20) - fx::EXP_BIAS;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
 #pragma unroll
     for (int r = 0; r < LANE_MAX_IN; ++r) {
       if (r < R.nin) {
-        const float* base = reinterpret_cast<const float*>(R.in_base[r]);
+        const float* base = global_ptr(reinterpret_cast<const float*>(R.in_base[r]));
 #pragma unroll
         for (int j = 0; j < n; ++j) {
           const unsigned int idx = node0 + (unsigned int)j * lstride + R.in_off[r];
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
           }
           const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
           const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
-          if (active && target >= 0) atomicAdd(reinterpret_cast<float*>(R.out_acc[o]) + target, r);
+          if (active && target >= 0) atomicAdd(global_ptr(reinterpret_cast<float*>(R.out_acc[o]) + target), r);
         }
       }
     }

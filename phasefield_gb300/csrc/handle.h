@@ -91,7 +91,8 @@ struct MGLevel {
   void* tables = nullptr;       // CellTables for the LHS (level precision)
   std::vector<unsigned char> h_tables;  // host copy (the lane kernel takes it as a kernel parameter)
   int fx_lanes = 0;             // the FP64 level's lane kernel mode (4, 5 or 0 for none)
-  void* acc = nullptr;          // accumulator
+  void* acc = nullptr;          // accumulator of the next product, all zero
+  void* acc2 = nullptr;         // the last product's: what reads one clears the other, and they swap
   void* x = nullptr;            // level solution
   void* b = nullptr;            // level defect (right-hand side)
   void* r = nullptr;            // residual / work
@@ -99,6 +100,7 @@ struct MGLevel {
   void* w1 = nullptr;
   double lambda_max = 0.0;      // Chebyshev interval
   double lambda_min = 0.0;
+  double pattern_mean = -1.0;   // mean of the eigenvalue estimate's start pattern over the free rows
   bool eig_done = false;
   // separable transfer to the next finer level: per axis CSR of the 1-D prolongation
   // (fine index -> coarse entries) and of its transpose (coarse index -> fine entries)
@@ -108,9 +110,6 @@ struct MGLevel {
   int* r_ptr[3] = {nullptr, nullptr, nullptr};
   int* r_col[3] = {nullptr, nullptr, nullptr};
   void* r_val[3] = {nullptr, nullptr, nullptr};
-  void* t0 = nullptr;           // transfer work buffers (fine-sized)
-  void* t1 = nullptr;
-  void* cvt = nullptr;          // precision-conversion buffer (coarsest level of a mixed hierarchy)
   // contraction mode of the level's FP64 operator (integer contractions, FP64 Q1/Q2): its first
   // plain LHS launches run modes 1, 2, 3 (and the lane kernel where it applies) twice under CUDA
   // events, then the fastest stays
@@ -135,7 +134,11 @@ struct LinearState {
   double* q = nullptr;
   double* z = nullptr;
   double* inv_diag = nullptr;   // fine FP64 inverse diagonal (Chebyshev preconditioner)
-  double* partial = nullptr;    // dot-product partial sums
+  double* partial = nullptr;    // partial sums of reductions and their block counters
+  double* scal = nullptr;       // Krylov scalars on the device
+  size_t scal_len = 0;
+  double* h_scal = nullptr;     // residual norms on their way to the host (pinned)
+  cudaEvent_t scal_ev[4] = {};
   double cheb_lmax = 0.0, cheb_lmin = 0.0;
   bool cheb_eig_done = false;
   int last_iterations = 0;

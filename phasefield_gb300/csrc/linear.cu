@@ -47,131 +47,307 @@ __global__ void convert_kernel(long long n, const Tin* __restrict__ x, Tout* __r
     y[i] = Tout(x[i]);
 }
 
-template <typename T>
-__global__ void mul_kernel(long long n, const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    y[i] = a[i] * b[i];
+// Sum of one double per thread over the grid: per-block tree sums, summed in block order by the
+// block that finishes last (the same sum whichever that is), so a reduction is part of the launch
+// that makes its terms. True in the last block's thread 0, with the sum in *total.
+__device__ bool grid_sum(double v, double* partial, unsigned int* counter, double* total) {
+  __shared__ double s[256];
+  __shared__ bool last;
+  const unsigned nb = gridDim.x * gridDim.y, b = blockIdx.y * gridDim.x + blockIdx.x;
+  s[threadIdx.x] = v;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    partial[b] = s[0];
+    __threadfence();
+    last = atomicAdd(counter, 1u) == nb - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double acc = 0.0;
+  for (unsigned i = threadIdx.x; i < nb; i += blockDim.x) acc += __ldcg(partial + i);
+  __syncthreads();
+  s[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return false;
+  *total = s[0];
+  *counter = 0;
+  return true;
 }
 
-// per-block partial sums of x.y in FP64 (deterministic two-stage reduction)
+// out = x.y in FP64
 template <typename T>
-__global__ void dot_partial_kernel(long long n, const T* __restrict__ x, const T* __restrict__ y, double* partial) {
-  __shared__ double s[256];
-  double acc = 0.0;
+__global__ void __launch_bounds__(256) dot_kernel(long long n, const T* x, const T* y, double* partial,
+                                                  unsigned int* counter, double* out) {
+  chain_release();
+  chain_wait();
+  double acc = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     acc += double(x[i]) * double(y[i]);
-  s[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+  if (grid_sum(acc, partial, counter, &total)) *out = total;
 }
 
-__global__ void dot_final_kernel(int nb, double* partial) {
-  __shared__ double s[256];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) acc += partial[i];
-  s[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[nb] = s[0];
-}
+// The kernels below read a product's accumulator and clear the level's other one (`clear`) for the
+// next product. (Clearing the same accumulator in place needs no second one, but storing to the rows
+// the cells' atomic adds have just left took five times as long: 73 instead of 13 us on 48^3 Q2
+// vectors.)
 
-// dst = scale (.) acc on free rows, zero on constrained rows (per node scale, component blocks)
+// dst = scale (.) acc on free rows, zero on constrained rows (per node scale, component blocks);
+// with `out` also out = w.dst
 template <typename T>
-__global__ void level_finalize_kernel(T* __restrict__ dst, const T* __restrict__ acc, const T* __restrict__ scale,
-                                      const int* __restrict__ cmap, long long N) {
+__global__ void __launch_bounds__(256) level_finalize_kernel(T* dst, const T* acc, T* clear, const T* __restrict__ scale,
+                                                             const int* __restrict__ cmap, long long N, const T* w,
+                                                             double* partial, unsigned int* counter, double* out) {
+  chain_release();
+  chain_wait();
   const long long base = blockIdx.y * N;
+  double sum = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
     const bool free_row = !cmap || cmap[gi] == (int)gi;
-    dst[gi] = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    const T v = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    if (clear) clear[gi] = T(0);
+    dst[gi] = v;
+    if (out) sum += double(w[gi]) * double(v);
   }
+  if (out && grid_sum(sum, partial, counter, &total)) *out = total;
 }
 
 // inverse diagonal: d = scale (.) acc, zero entries -> 1, inverted
 template <typename T>
-__global__ void inv_diag_kernel(T* __restrict__ inv, const T* __restrict__ acc, const T* __restrict__ scale, long long N) {
+__global__ void inv_diag_kernel(T* inv, const T* acc, T* clear, const T* __restrict__ scale, long long N) {
+  chain_release();
+  chain_wait();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
     T d = scale ? acc[gi] * scale[i] : acc[gi];
+    clear[gi] = T(0);
     if (d == T(0)) d = T(1);
     inv[gi] = T(1) / d;
   }
 }
 
-// periodic images add into their master, then images and Dirichlet rows are zeroed
+// One axis of a transfer between two levels as CSR rows (output index -> input entries)
 template <typename T>
-__global__ void condense_add_kernel(long long len, T* v, const int* __restrict__ cmap) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x) {
-    const int m = cmap[i];
-    if (m >= 0 && m != (int)i) atomicAdd(v + m, v[i]);
-  }
-}
+struct AxisRows {
+  const int* ptr;
+  const int* col;
+  const T* val;
+};
 template <typename T>
-__global__ void zero_constrained_kernel(long long len, T* v, const int* __restrict__ cmap) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x)
-    if (cmap[i] != (int)i) v[i] = T(0);
-}
-// images take their master's value (AffineConstraints::distribute with homogeneous rows)
-template <typename T>
-__global__ void copy_masters_kernel(long long len, T* v, const int* __restrict__ cmap) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x) {
-    const int m = cmap[i];
-    if (m != (int)i) v[i] = m >= 0 ? v[m] : T(0);
-  }
-}
+struct Transfer {
+  AxisRows<T> axis[3];
+  int nout[3], nin[3];   // lattice extents of the output and the input level
+  int periodic[3];
+  int dim;
+  long long Nout, Nin;
+};
 
-// one 1-D sparse operator along `axis`: out(i) = sum_k val[k] in(i with axis index col[k])
-template <typename T>
-__global__ void axis_csr_kernel(const T* __restrict__ in, T* __restrict__ out, int o0, int o1, int o2, int axis,
-                                int in_axis_len, const int* __restrict__ ptr, const int* __restrict__ col,
-                                const T* __restrict__ val) {
-  const long long total = (long long)o0 * o1 * o2;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int i0 = (int)(idx % o0);
-    const int i1 = (int)((idx / o0) % o1);
-    const int i2 = (int)(idx / ((long long)o0 * o1));
-    const int row = axis == 0 ? i0 : (axis == 1 ? i1 : i2);
-    const int d0 = axis == 0 ? in_axis_len : o0;
-    const int d1 = axis == 1 ? in_axis_len : o1;
-    T s = T(0);
-    for (int k = ptr[row]; k < ptr[row + 1]; ++k) {
-      const int c = col[k];
-      const long long j = axis == 0 ? ((long long)i2 * d1 + i1) * d0 + c
-                        : axis == 1 ? ((long long)i2 * d1 + c) * d0 + i0
-                                    : ((long long)c * d1 + i1) * d0 + i0;
-      s += val[k] * in[j];
+// the tensor product of one CSR row per axis applied to `in` (FP entries of type Ti)
+template <typename T, typename Ti>
+__device__ __forceinline__ T transfer_row(const Transfer<T>& A, const Ti* in, int i0, int i1, int i2) {
+  T s2 = T(0);
+  const int b2 = A.dim > 2 ? A.axis[2].ptr[i2] : 0, e2 = A.dim > 2 ? A.axis[2].ptr[i2 + 1] : 1;
+  const int b1 = A.axis[1].ptr[i1], e1 = A.axis[1].ptr[i1 + 1];
+  const int b0 = A.axis[0].ptr[i0], e0 = A.axis[0].ptr[i0 + 1];
+  for (int k2 = b2; k2 < e2; ++k2) {
+    const int c2 = A.dim > 2 ? A.axis[2].col[k2] : 0;
+    T s1 = T(0);
+    for (int k1 = b1; k1 < e1; ++k1) {
+      const Ti* row = in + ((long long)c2 * A.nin[1] + A.axis[1].col[k1]) * A.nin[0];
+      T s0 = T(0);
+      for (int k0 = b0; k0 < e0; ++k0) s0 += A.axis[0].val[k0] * T(row[A.axis[0].col[k0]]);
+      s1 += A.axis[1].val[k1] * s0;
     }
-    out[idx] = s;
+    s2 += A.dim > 2 ? A.axis[2].val[k2] * s1 : s1;
+  }
+  return s2;
+}
+
+// x += P e from the coarse correction e (type Tc): all axes in one pass (at most 27 entries a row,
+// 8 on average for Q2 3-D, read from L1/L2, instead of dim passes over fine-sized work vectors);
+// images take their master's row, Dirichlet rows nothing
+template <typename T, typename Tc>
+__global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_constant__ Transfer<T> A, T* x, const Tc* e,
+                                                             const int* __restrict__ cmap) {
+  chain_release();
+  chain_wait();
+  const long long base = blockIdx.y * A.Nout;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
+    const int m = cmap ? cmap[base + i] : (int)(base + i);
+    if (m < 0) continue;
+    const unsigned node = (unsigned)(m - base);
+    const unsigned r = node / (unsigned)A.nout[0];
+    const int i0 = (int)(node - r * (unsigned)A.nout[0]);
+    const int i2 = (int)(r / (unsigned)A.nout[1]);
+    const int i1 = (int)(r - (unsigned)i2 * (unsigned)A.nout[1]);
+    x[base + i] += transfer_row<T, Tc>(A, e + blockIdx.y * A.Nin, i0, i1, i2);
   }
 }
 
-// Chebyshev update: u = c1 u + c2 P (b - Ax); x += u
+// b = P^T r on the coarse level (stored as Tc): all axes in one pass; a periodic node sums its
+// images' rows as well, constrained rows are zero
+template <typename T, typename Tc>
+__global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ Transfer<T> A, Tc* b, const T* r,
+                                                       const int* __restrict__ cmap) {
+  chain_release();
+  chain_wait();
+  const long long base = blockIdx.y * A.Nout;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
+    T s = T(0);
+    if (!cmap || cmap[base + i] == (int)(base + i)) {
+      const unsigned node = (unsigned)i;
+      const unsigned q = node / (unsigned)A.nout[0];
+      const int i0 = (int)(node - q * (unsigned)A.nout[0]);
+      const int i2 = (int)(q / (unsigned)A.nout[1]);
+      const int i1 = (int)(q - (unsigned)i2 * (unsigned)A.nout[1]);
+      const int m0 = A.periodic[0] && i0 == 0, m1 = A.periodic[1] && i1 == 0, m2 = A.periodic[2] && i2 == 0;
+      for (int e2 = 0; e2 <= m2; ++e2)
+        for (int e1 = 0; e1 <= m1; ++e1)
+          for (int e0 = 0; e0 <= m0; ++e0)
+            s += transfer_row<T, T>(A, r + blockIdx.y * A.Nin, e0 ? A.nout[0] - 1 : i0, e1 ? A.nout[1] - 1 : i1,
+                                    e2 ? A.nout[2] - 1 : i2);
+    }
+    b[base + i] = Tc(s);
+  }
+}
+
+// First Chebyshev step from x = 0: x = u = c2 P b
 template <typename T>
-__global__ void cheb_update_kernel(long long n, T* __restrict__ x, T* __restrict__ u, const T* __restrict__ b,
-                                   const T* __restrict__ Ax, const T* __restrict__ pinv, double c1, double c2) {
+__global__ void __launch_bounds__(256) cheb_start_kernel(long long n, T* x, T* u, const T* b,
+                                                         const T* pinv, double c2) {
+  chain_release();
+  chain_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const T r = Ax ? b[i] - Ax[i] : b[i];
-    const T ui = T(c1) * u[i] + T(c2) * pinv[i] * r;
+    const T ui = T(c2) * pinv[i] * b[i];
     u[i] = ui;
-    x[i] += ui;
+    x[i] = ui;
   }
 }
 
-// CG kernels (FP64)
-__global__ void cg_update_xr_kernel(long long n, double alpha, const double* __restrict__ p,
-                                    const double* __restrict__ q, double* __restrict__ x, double* __restrict__ r) {
+// A Chebyshev step from the raw product: Ax = scale (.) acc on free rows; u = c1 u + c2 P (b - Ax);
+// x += u (one pass instead of a memset, a finalize and an update launch with Ax in between: 20 % of
+// the mixed-precision iterations' kernel time)
+template <typename T>
+__global__ void __launch_bounds__(256) cheb_step_kernel(T* x, T* u, const T* b, const T* acc, T* clear,
+                                                        const T* __restrict__ scale,
+                                                        const int* __restrict__ cmap, const T* pinv, double c1,
+                                                        double c2, long long N) {
+  chain_release();
+  chain_wait();
+  const long long base = blockIdx.y * N;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+    const long long gi = base + i;
+    const bool free_row = !cmap || cmap[gi] == (int)gi;
+    const T Ax = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    clear[gi] = T(0);
+    const T r = b[gi] - Ax;
+    const T ui = c1 == 0.0 ? T(c2) * pinv[gi] * r : T(c1) * u[gi] + T(c2) * pinv[gi] * r;
+    u[gi] = ui;
+    x[gi] += ui;
+  }
+}
+
+// r = b - scale (.) acc (constrained rows: b)
+template <typename T>
+__global__ void __launch_bounds__(256) residual_kernel(T* r, const T* b, const T* acc, T* clear,
+                                                       const T* __restrict__ scale,
+                                                       const int* __restrict__ cmap, long long N) {
+  chain_release();
+  chain_wait();
+  const long long base = blockIdx.y * N;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+    const long long gi = base + i;
+    const bool free_row = !cmap || cmap[gi] == (int)gi;
+    const T Ax = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    clear[gi] = T(0);
+    r[gi] = b[gi] - Ax;
+  }
+}
+
+// Krylov scalars on the device (LinearState::scal), so that an iteration needs no value on the host
+// but the residual norm its caller tests
+enum Scalar { SC_RZ = 0 /* two, alternating */, SC_PQ = 2, SC_RR = 3, SC_DONE = 4, SC_TMP = 5, SC_EIG = 8 };
+
+// CG: x += alpha p, r -= alpha q with alpha = rz / pq, and rr = r.r; sc[SC_DONE] is set once
+// sqrt(rr) < tol, after which the kernel does nothing (iterations queued past convergence)
+__global__ void __launch_bounds__(256) cg_update_kernel(long long n, double* sc, int rz, const double* p, const double* q,
+                                                        double* x, double* r, double tol, double* partial,
+                                                        unsigned int* counter) {
+  chain_release();
+  chain_wait();
+  if (sc[SC_DONE] != 0.0) return;
+  const double alpha = sc[SC_RZ + rz] / sc[SC_PQ];
+  double acc = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     x[i] += alpha * p[i];
-    r[i] -= alpha * q[i];
+    const double ri = r[i] - alpha * q[i];
+    r[i] = ri;
+    acc += ri * ri;
+  }
+  if (grid_sum(acc, partial, counter, &total)) {
+    sc[SC_RR] = total;
+    if (sqrt(total) < tol) sc[SC_DONE] = 1.0;
+  }
+}
+
+// p = z + beta p with beta = rz_new / rz (first: p = z)
+__global__ void __launch_bounds__(256) cg_direction_kernel(long long n, const double* sc, int rz, int first,
+                                                           const double* z, double* p) {
+  chain_release();
+  chain_wait();
+  const double beta = first ? 0.0 : sc[SC_RZ + rz] / sc[SC_RZ + 1 - rz];
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    p[i] = first ? z[i] : z[i] + beta * p[i];
+}
+
+// The eigenvalue estimate's CG: r -= alpha q, z = P r with the sums r.r and r.z of step `it`
+// (start: z = P r, p = z and the sums of r alone); e holds per step pq, rr, rz
+template <typename T>
+__global__ void __launch_bounds__(256) eig_update_kernel(long long n, double* e, int it, const T* q, T* r, T* z, T* p,
+                                                         const T* pinv, double* partial, unsigned int* counter) {
+  chain_release();
+  chain_wait();
+  const bool start = it < 0;
+  const double alpha = start ? 0.0 : e[3 * it + 2] / e[3 * it + 3];
+  double rr = 0.0, rz = 0.0, total;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const T ri = start ? r[i] : T(-alpha * double(q[i]) + double(r[i]));
+    const T zi = pinv[i] * ri;
+    r[i] = ri;
+    z[i] = zi;
+    if (start) p[i] = zi;
+    rr += double(ri) * double(ri);
+    rz += double(ri) * double(zi);
+  }
+  // e: rr_0, rz_0 at 1, 2; step it: pq at 3 it + 3, rr at 3 it + 4, rz at 3 it + 5
+  if (grid_sum(rr, partial, counter, &total)) e[3 * it + 4] = total;
+  __syncthreads();
+  if (grid_sum(rz, partial + 1024, counter + 1, &total)) e[3 * it + 5] = total;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) eig_direction_kernel(long long n, const double* e, int it, const T* z, T* p) {
+  chain_release();
+  chain_wait();
+  const double beta = e[3 * it + 5] / e[3 * it + 2];
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    p[i] = T(double(z[i]) + beta * double(p[i]));
+}
+
+// the Dirichlet values of the constrained rows, zero elsewhere (the inhomogeneous lift's vector)
+__global__ void lift_values_kernel(double* g, const int* __restrict__ cmap, const double* dvals, long long len) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x) {
+    const int m = cmap[i];
+    g[i] = m < 0 ? dvals[-1 - m] : 0.0;
   }
 }
 
@@ -186,15 +362,45 @@ static void by_precision(int precision, F&& f) {
   else f(double(0));
 }
 
-static int dot(ppf_handle h, LinearState& L, int precision, long long n, const void* x, const void* y, double* out) {
-  const unsigned nb = std::min<long long>(1024, (n + 255) / 256) > 0 ? (unsigned)std::min<long long>(1024, (n + 255) / 256) : 1;
-  if (precision)
-    dot_partial_kernel<float><<<nb, 256, 0, h->stream>>>(n, (const float*)x, (const float*)y, L.partial);
-  else
-    dot_partial_kernel<double><<<nb, 256, 0, h->stream>>>(n, (const double*)x, (const double*)y, L.partial);
-  dot_final_kernel<<<1, 256, 0, h->stream>>>((int)nb, L.partial);
-  h->all_launches += 2;
-  PPF_CUDA(h, cudaMemcpyAsync(out, L.partial + nb, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+// blocks of a reduction over n entries (at most 1024 partial sums)
+static unsigned dot_blocks(long long n) { return (unsigned)std::max<long long>(1, std::min<long long>(1024, (n + 255) / 256)); }
+
+static unsigned int* counters(LinearState& L) { return reinterpret_cast<unsigned int*>(L.partial + 2048); }
+
+// work space of the reductions and the Krylov scalars, on the device and in pinned host memory
+static int ensure_scalars(ppf_handle h, LinearState& L) {
+  const size_t len = SC_EIG + 8 + 3 * (size_t)L.params.eig_cg_iterations;
+  if (L.scal && len > L.scal_len) {  // (parameters set again before a block's first linear solve)
+    PPF_CUDA(h, cudaFree(L.scal));
+    L.scal = nullptr;
+  }
+  if (!L.scal) {
+    PPF_CUDA(h, cudaMalloc(&L.scal, sizeof(double) * len));
+    PPF_CUDA(h, cudaMemset(L.scal, 0, sizeof(double) * len));
+    L.scal_len = len;
+  }
+  if (L.partial) return PPF_OK;
+  PPF_CUDA(h, cudaMalloc(&L.partial, sizeof(double) * 2056));
+  PPF_CUDA(h, cudaMemset(L.partial, 0, sizeof(double) * 2056));
+  PPF_CUDA(h, cudaMallocHost(&L.h_scal, sizeof(double) * 4));
+  for (auto& ev : L.scal_ev) PPF_CUDA(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  return PPF_OK;
+}
+
+// sc = x.y on the device
+template <typename T>
+static int dot_device(ppf_handle h, LinearState& L, long long n, const T* x, const T* y, double* out) {
+  PPF_CUDA(h, launch_chained(dot_kernel<T>, dim3(dot_blocks(n)), dim3(256), 0, h->stream, n, x, y, L.partial, counters(L), out));
+  h->all_launches++;
+  return PPF_OK;
+}
+
+// x.y on the host (waits for the stream)
+static int dot(ppf_handle h, LinearState& L, int, long long n, const void* x, const void* y, double* out) {
+  int rc = ensure_scalars(h, L);
+  if (!rc) rc = dot_device<double>(h, L, n, (const double*)x, (const double*)y, L.scal + SC_TMP);
+  if (rc) return rc;
+  PPF_CUDA(h, cudaMemcpyAsync(out, L.scal + SC_TMP, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   PPF_CUDA(h, cudaStreamSynchronize(h->stream));
   return PPF_OK;
 }
@@ -463,8 +669,7 @@ static int level_cell_launch(ppf_handle h, BlockState& B, MGLevel& lv, int mode,
   }
   const size_t smem = cell_smem(h->dim, h->k, lv.precision, P.nrows_in, P.nrows_out);
   const void* obj = lv.precision ? h->model_obj_f32.data() : h->model_obj.data();
-  PPF_CUDA(h, cudaMemsetAsync(lv.acc, 0, lv.len * esize(lv.precision), h->stream));
-  if (slot >= 0) PPF_CUDA(h, cudaEventRecord(lv.fx_ev[2 * slot], h->stream));  // after the memset
+  // (the level's accumulator is all zero: the kernel that read the other one cleared it)
   const int rc = timed_cell_launch(h, lv.precision, mode, L, obj, smem);
   if (rc) return rc;
   return online_mode_end(h, lv.fx_mode, lv.fx_timed, lv.fx_ev, slot, lv.fx_lanes);
@@ -472,38 +677,41 @@ static int level_cell_launch(ppf_handle h, BlockState& B, MGLevel& lv, int mode,
 
 static bool scaled(const LinearState& L) { return L.params.tolerance_type != 0; }
 
-// dst = S A src on level lv (S = invM^1/2 or identity)
-static int level_apply(ppf_handle h, BlockState& B, MGLevel& lv, const void* src, void* dst, bool plain_read = false) {
-  int rc = level_cell_launch(h, B, lv, MODE_LHS, src, plain_read);
+template <typename T>
+static const T* level_scale(const LinearState& L, const MGLevel& lv) {
+  return scaled(L) ? (const T*)lv.invm_sqrt : nullptr;
+}
+static const int* level_map(const MGLevel& lv) { return lv.constrained ? lv.cmap : nullptr; }
+static dim3 level_grid(ppf_handle h, const BlockState& B, const MGLevel& lv) {
+  return dim3(grid_for(lv.N), h->fields[B.desc.field_indices[0]].ncomp);
+}
+
+// dst = S A src on level lv (S = invM^1/2 or identity); with `out` also out = src.dst
+template <typename T>
+static int level_apply(ppf_handle h, BlockState& B, MGLevel& lv, const T* src, T* dst, double* out = nullptr) {
+  int rc = level_cell_launch(h, B, lv, MODE_LHS, src, false);
   if (rc) return rc;
-  dim3 grid(grid_for(lv.N), h->fields[B.desc.field_indices[0]].ncomp);
-  const int* cm = lv.constrained ? lv.cmap : nullptr;
-  const bool sc = scaled(B.lin);
-  if (lv.precision)
-    level_finalize_kernel<float><<<grid, 256, 0, h->stream>>>((float*)dst, (const float*)lv.acc,
-                                                              sc ? (const float*)lv.invm_sqrt : nullptr, cm, lv.N);
-  else
-    level_finalize_kernel<double><<<grid, 256, 0, h->stream>>>((double*)dst, (const double*)lv.acc,
-                                                               sc ? (const double*)lv.invm_sqrt : nullptr, cm, lv.N);
+  dim3 grid = level_grid(h, B, lv);
+  if (out) grid.x = std::min(grid.x, 1024u / grid.y);
+  PPF_CUDA(h, launch_chained(level_finalize_kernel<T>, grid, dim3(256), 0, h->stream, dst, (const T*)lv.acc, (T*)lv.acc2,
+                             level_scale<T>(B.lin, lv), level_map(lv), lv.N, src, B.lin.partial, counters(B.lin), out));
+  std::swap(lv.acc, lv.acc2);
   h->all_launches++;
-  PPF_CUDA(h, cudaGetLastError());
   return PPF_OK;
 }
 
-static int level_diagonal(ppf_handle h, BlockState& B, MGLevel& lv) {
+template <typename T>
+static int level_diagonal_t(ppf_handle h, BlockState& B, MGLevel& lv) {
   int rc = level_cell_launch(h, B, lv, MODE_DIAG, lv.x, false);
   if (rc) return rc;
-  dim3 grid(grid_for(lv.N), h->fields[B.desc.field_indices[0]].ncomp);
-  const bool sc = scaled(B.lin);
-  if (lv.precision)
-    inv_diag_kernel<float><<<grid, 256, 0, h->stream>>>((float*)lv.inv_diag, (const float*)lv.acc,
-                                                        sc ? (const float*)lv.invm_sqrt : nullptr, lv.N);
-  else
-    inv_diag_kernel<double><<<grid, 256, 0, h->stream>>>((double*)lv.inv_diag, (const double*)lv.acc,
-                                                         sc ? (const double*)lv.invm_sqrt : nullptr, lv.N);
+  PPF_CUDA(h, launch_chained(inv_diag_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.inv_diag,
+                             (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), lv.N));
+  std::swap(lv.acc, lv.acc2);
   h->all_launches++;
-  PPF_CUDA(h, cudaGetLastError());
   return PPF_OK;
+}
+static int level_diagonal(ppf_handle h, BlockState& B, MGLevel& lv) {
+  return lv.precision ? level_diagonal_t<float>(h, B, lv) : level_diagonal_t<double>(h, B, lv);
 }
 
 // largest eigenvalue of the symmetric tridiagonal (diag a, off-diagonal b) by bisection
@@ -537,62 +745,56 @@ static double tridiag_max_eig(const std::vector<double>& a, const std::vector<do
 }
 
 // Lanczos estimate of the largest eigenvalue of P A (P = inverse diagonal) on level lv:
-// eig_cg_iterations CG steps on A x = pattern from x = 0 (uses lv.x, lv.b, lv.r, lv.w0, lv.w1)
+// eig_cg_iterations CG steps on A x = pattern from x = 0 (uses lv.b, lv.r, lv.w0, lv.w1). The steps
+// are queued without waiting for their scalars, which come to the host once at the end.
 template <typename T>
 static int estimate_eigenvalues(ppf_handle h, BlockState& B, MGLevel& lv) {
   LinearState& L = B.lin;
-  const int prec = lv.precision;
-  {
+  const long long n = lv.len;
+  int rc = ensure_scalars(h, L);
+  if (rc) return rc;
+  if (!(lv.pattern_mean >= 0.0)) {
     unsigned long long* d_sums = reinterpret_cast<unsigned long long*>(L.partial);
     PPF_CUDA(h, cudaMemsetAsync(d_sums, 0, 2 * sizeof(unsigned long long), h->stream));
     pattern_sum_kernel<<<grid_for(lv.len), 256, 0, h->stream>>>(lv.cmap, lv.len, d_sums);
     unsigned long long sums[2];
     PPF_CUDA(h, cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, h->stream));
     PPF_CUDA(h, cudaStreamSynchronize(h->stream));
-    const double mean = double(sums[0]) / double(std::max<unsigned long long>(1, sums[1]));
-    pattern_kernel<T><<<grid_for(lv.len), 256, 0, h->stream>>>((T*)lv.b, lv.cmap, lv.len, mean);
-    h->all_launches += 2;
-    PPF_CUDA(h, cudaGetLastError());
+    lv.pattern_mean = double(sums[0]) / double(std::max<unsigned long long>(1, sums[1]));
+    h->all_launches++;
   }
-  T* x = (T*)lv.x;
   T* r = (T*)lv.r;
   T* z = (T*)lv.w0;
   T* p = (T*)lv.w1;
-  PPF_CUDA(h, cudaMemsetAsync(x, 0, sizeof(T) * lv.len, h->stream));
-  PPF_CUDA(h, cudaMemcpyAsync(r, lv.b, sizeof(T) * lv.len, cudaMemcpyDeviceToDevice, h->stream));
-  const long long n = lv.len;
-  mul_kernel<T><<<grid_for(n), 256, 0, h->stream>>>(n, (const T*)lv.inv_diag, r, z);
-  PPF_CUDA(h, cudaMemcpyAsync(p, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, h->stream));
-  double rz;
-  int rc = dot(h, L, prec, n, r, z, &rz);
-  if (rc) return rc;
-  double r0;
-  rc = dot(h, L, prec, n, r, r, &r0);
-  if (rc) return rc;
+  T* q = (T*)lv.b;
+  double* e = L.scal + SC_EIG;
+  pattern_kernel<T><<<grid_for(n), 256, 0, h->stream>>>(r, lv.cmap, n, lv.pattern_mean);
+  PPF_CUDA(h, cudaGetLastError());
+  PPF_CUDA(h, launch_chained(eig_update_kernel<T>, dim3(dot_blocks(n)), dim3(256), 0, h->stream, n, e, -1, q, r, z, p,
+                             (const T*)lv.inv_diag, L.partial, counters(L)));
+  h->all_launches += 2;
+  const int steps = L.params.eig_cg_iterations;
+  for (int it = 0; it < steps; ++it) {
+    rc = level_apply<T>(h, B, lv, p, q, e + 3 * it + 3);
+    if (rc) return rc;
+    PPF_CUDA(h, launch_chained(eig_update_kernel<T>, dim3(dot_blocks(n)), dim3(256), 0, h->stream, n, e, it, q, r, z, p,
+                               (const T*)lv.inv_diag, L.partial, counters(L)));
+    PPF_CUDA(h, launch_chained(eig_direction_kernel<T>, dim3(grid_for(n)), dim3(256), 0, h->stream, n, e, it, z, p));
+    h->all_launches += 2;
+  }
+  std::vector<double> he(3 * steps + 6);
+  PPF_CUDA(h, cudaMemcpyAsync(he.data(), e, sizeof(double) * (3 * steps + 3), cudaMemcpyDeviceToHost, h->stream));
+  PPF_CUDA(h, cudaStreamSynchronize(h->stream));
+  const double r0 = he[1];
+  double rz = he[2];
   std::vector<double> alphas, betas;
-  for (int it = 0; it < L.params.eig_cg_iterations; ++it) {
-    rc = level_apply(h, B, lv, p, lv.b);  // b reused as q = A p (pattern no longer needed)
-    if (rc) return rc;
-    double pq;
-    rc = dot(h, L, prec, n, p, lv.b, &pq);
-    if (rc) return rc;
+  for (int it = 0; it < steps; ++it) {
+    const double pq = he[3 * it + 3], rr = he[3 * it + 4], rz_new = he[3 * it + 5];
     if (pq <= 0.0 || !std::isfinite(pq)) break;
-    const double alpha = rz / pq;
-    axpby(h, prec, n, alpha, p, 1.0, x);
-    axpby(h, prec, n, -alpha, lv.b, 1.0, r);
-    alphas.push_back(alpha);
-    double rr;
-    rc = dot(h, L, prec, n, r, r, &rr);
-    if (rc) return rc;
+    alphas.push_back(rz / pq);
     if (std::sqrt(rr) < 1e-10 * std::sqrt(r0)) break;
-    mul_kernel<T><<<grid_for(n), 256, 0, h->stream>>>(n, (const T*)lv.inv_diag, r, z);
-    double rz_new;
-    rc = dot(h, L, prec, n, r, z, &rz_new);
-    if (rc) return rc;
-    const double beta = rz_new / rz;
+    betas.push_back(rz_new / rz);
     rz = rz_new;
-    betas.push_back(beta);
-    axpby(h, prec, n, 1.0, z, beta, p);
   }
   // Lanczos matrix of the CG coefficients
   const int m = (int)alphas.size();
@@ -608,26 +810,15 @@ static int estimate_eigenvalues(ppf_handle h, BlockState& B, MGLevel& lv) {
   return PPF_OK;
 }
 
-// Chebyshev smoother on level lv: x <- x + p(P A)(P (b - A x)); zero_start: x := 0 first
+// Chebyshev smoother on level lv: x <- x + p(P A)(P (b - A x)); zero_start: from x = 0
 template <typename T>
-static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start) {
+static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start, const T* b, T* x) {
   const double theta = 0.5 * (lv.lambda_max + lv.lambda_min);
   const double delta = 0.5 * (lv.lambda_max - lv.lambda_min);
   const double sigma = theta / delta;
-  const long long n = lv.len;
-  T* x = (T*)lv.x;
   T* u = (T*)lv.w0;
-  T* Ax = (T*)lv.r;
-  if (zero_start) PPF_CUDA(h, cudaMemsetAsync(x, 0, sizeof(T) * n, h->stream));
-  PPF_CUDA(h, cudaMemsetAsync(u, 0, sizeof(T) * n, h->stream));
   double rho_prev = 1.0 / sigma;
   for (int k = 0; k < B.lin.params.smoother_degree; ++k) {
-    const T* ax = nullptr;
-    if (!(zero_start && k == 0)) {
-      int rc = level_apply(h, B, lv, x, Ax);
-      if (rc) return rc;
-      ax = Ax;
-    }
     double c1, c2;
     if (k == 0) {
       c1 = 0.0;
@@ -638,89 +829,76 @@ static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start) 
       c2 = 2.0 * rho / delta;
       rho_prev = rho;
     }
-    cheb_update_kernel<T><<<grid_for(n), 256, 0, h->stream>>>(n, x, u, (const T*)lv.b, ax, (const T*)lv.inv_diag, c1, c2);
+    if (zero_start && k == 0) {
+      PPF_CUDA(h, launch_chained(cheb_start_kernel<T>, dim3(grid_for(lv.len)), dim3(256), 0, h->stream, lv.len, x, u, b,
+                                 (const T*)lv.inv_diag, c2));
+    } else {
+      int rc = level_cell_launch(h, B, lv, MODE_LHS, x, false);
+      if (rc) return rc;
+      PPF_CUDA(h, launch_chained(cheb_step_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, x, u, b,
+                                 (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), level_map(lv),
+                                 (const T*)lv.inv_diag, c1, c2, lv.N));
+      std::swap(lv.acc, lv.acc2);
+    }
     h->all_launches++;
   }
-  PPF_CUDA(h, cudaGetLastError());
   return PPF_OK;
 }
 
-static int smooth(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start) {
-  if (lv.precision) return chebyshev<float>(h, B, lv, zero_start);
-  return chebyshev<double>(h, B, lv, zero_start);
-}
-
-// separable transfer between level c (coarse) and c+1 (fine), in precision `prec`
+// the transfer between level c and the next finer one f, output on f (prolongation) or on c
 template <typename T>
-static void transfer(ppf_handle h, MGLevel& cl, MGLevel& fl, const T* in, T* out, bool prolongate, int ncomp) {
-  const int dim = h->dim;
-  for (int comp = 0; comp < ncomp; ++comp) {
-    const T* src = in + comp * (prolongate ? cl.N : fl.N);
-    T* dst = out + comp * (prolongate ? fl.N : cl.N);
-    int cur[3] = {1, 1, 1};
-    for (int d = 0; d < 3; ++d) cur[d] = prolongate ? cl.nn[d] : fl.nn[d];
-    const T* a = src;
-    for (int d = 0; d < dim; ++d) {
-      int nxt[3] = {cur[0], cur[1], cur[2]};
-      nxt[d] = prolongate ? fl.nn[d] : cl.nn[d];
-      T* b = (d == dim - 1) ? dst : (T*)((d % 2 == 0) ? fl.t0 : fl.t1);
-      const int* ptr = prolongate ? cl.p_ptr[d] : cl.r_ptr[d];
-      const int* col = prolongate ? cl.p_col[d] : cl.r_col[d];
-      const T* val = (const T*)(prolongate ? cl.p_val[d] : cl.r_val[d]);
-      const long long total = (long long)nxt[0] * nxt[1] * nxt[2];
-      axis_csr_kernel<T><<<grid_for(total), 256, 0, h->stream>>>(a, b, nxt[0], nxt[1], nxt[2], d, cur[d], ptr, col, val);
-      h->all_launches++;
-      a = b;
-      cur[d] = nxt[d];
-    }
+static Transfer<T> transfer(ppf_handle h, const MGLevel& c, const MGLevel& f, bool prolongate) {
+  Transfer<T> A;
+  std::memset(&A, 0, sizeof(A));
+  const MGLevel& out = prolongate ? f : c;
+  const MGLevel& in = prolongate ? c : f;
+  A.dim = h->dim;
+  for (int d = 0; d < 3; ++d) {
+    A.nout[d] = out.nn[d];
+    A.nin[d] = in.nn[d];
+    A.periodic[d] = d < h->dim ? h->mesh.periodic[d] : 0;
+    A.axis[d].ptr = prolongate ? c.p_ptr[d] : c.r_ptr[d];
+    A.axis[d].col = prolongate ? c.p_col[d] : c.r_col[d];
+    A.axis[d].val = (const T*)(prolongate ? c.p_val[d] : c.r_val[d]);
   }
+  A.Nout = out.N;
+  A.Nin = in.N;
+  return A;
 }
 
-// V-cycle on level l: lv.b holds the defect, lv.x receives the correction
-static int vcycle(ppf_handle h, BlockState& B, int l) {
+static int vcycle(ppf_handle h, BlockState& B, int l, const void* b, void* x);
+
+// V-cycle on level l (entries T) with the defect b; x receives the correction. Tc: the entries of
+// the next coarser level.
+template <typename T, typename Tc>
+static int vcycle_level(ppf_handle h, BlockState& B, int l, const T* b, T* x) {
   auto& lvs = B.lin.levels;
   MGLevel& lv = lvs[l];
-  const int ncomp = h->fields[B.desc.field_indices[0]].ncomp;
-  if (l == 0) return smooth(h, B, lv, true);  // coarse: the smoother as coarse solver
-  int rc = smooth(h, B, lv, true);
-  if (rc) return rc;
-  // residual t = b - A x into lv.r
-  rc = level_apply(h, B, lv, lv.x, lv.r);
-  if (rc) return rc;
-  axpby(h, lv.precision, lv.len, 1.0, lv.b, -1.0, lv.r);
+  int rc = chebyshev<T>(h, B, lv, true, b, x);
+  if (rc || l == 0) return rc;  // coarse: the smoother as coarse solver
   MGLevel& cl = lvs[l - 1];
-  // restrict in the fine precision; the coarse level may hold another precision
-  void* cb = (cl.precision == lv.precision) ? cl.b : cl.cvt;
-  if (lv.precision) transfer<float>(h, cl, lv, (const float*)lv.r, (float*)cb, false, ncomp);
-  else transfer<double>(h, cl, lv, (const double*)lv.r, (double*)cb, false, ncomp);
-  if (cl.constrained) {
-    if (lv.precision) {
-      condense_add_kernel<float><<<grid_for(cl.len), 256, 0, h->stream>>>(cl.len, (float*)cb, cl.cmap);
-      zero_constrained_kernel<float><<<grid_for(cl.len), 256, 0, h->stream>>>(cl.len, (float*)cb, cl.cmap);
-    } else {
-      condense_add_kernel<double><<<grid_for(cl.len), 256, 0, h->stream>>>(cl.len, (double*)cb, cl.cmap);
-      zero_constrained_kernel<double><<<grid_for(cl.len), 256, 0, h->stream>>>(cl.len, (double*)cb, cl.cmap);
-    }
-    h->all_launches += 2;
-  }
-  if (cb != cl.b) convert(h, lv.precision, cl.precision, cl.len, cb, cl.b);
-  rc = vcycle(h, B, l - 1);
+  rc = level_cell_launch(h, B, lv, MODE_LHS, x, false);
   if (rc) return rc;
-  // prolongate-add the coarse correction
-  const void* cx = cl.x;
-  if (cl.precision != lv.precision) {
-    convert(h, cl.precision, lv.precision, cl.len, cl.x, cl.cvt);
-    cx = cl.cvt;
-  }
-  if (lv.precision) transfer<float>(h, cl, lv, (const float*)cx, (float*)lv.r, true, ncomp);
-  else transfer<double>(h, cl, lv, (const double*)cx, (double*)lv.r, true, ncomp);
-  if (lv.constrained) {
-    if (lv.precision) copy_masters_kernel<float><<<grid_for(lv.len), 256, 0, h->stream>>>(lv.len, (float*)lv.r, lv.cmap);
-    else copy_masters_kernel<double><<<grid_for(lv.len), 256, 0, h->stream>>>(lv.len, (double*)lv.r, lv.cmap);
-    h->all_launches++;
-  }
-  axpby(h, lv.precision, lv.len, 1.0, lv.r, 1.0, lv.x);
-  return smooth(h, B, lv, false);
+  PPF_CUDA(h, launch_chained(residual_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.r, b,
+                             (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), level_map(lv), lv.N));
+  std::swap(lv.acc, lv.acc2);
+  PPF_CUDA(h, launch_chained(restrict_kernel<T, Tc>, level_grid(h, B, cl), dim3(256), 0, h->stream,
+                             transfer<T>(h, cl, lv, false), (Tc*)cl.b, (const T*)lv.r, level_map(cl)));
+  h->all_launches += 2;
+  rc = vcycle(h, B, l - 1, cl.b, cl.x);
+  if (rc) return rc;
+  PPF_CUDA(h, launch_chained(prolongate_add_kernel<T, Tc>, level_grid(h, B, lv), dim3(256), 0, h->stream,
+                             transfer<T>(h, cl, lv, true), x, (const Tc*)cl.x, level_map(lv)));
+  h->all_launches++;
+  return chebyshev<T>(h, B, lv, false, b, x);
+}
+
+static int vcycle(ppf_handle h, BlockState& B, int l, const void* b, void* x) {
+  const int prec = B.lin.levels[l].precision;
+  const int coarse = l > 0 ? B.lin.levels[l - 1].precision : prec;
+  if (prec && coarse) return vcycle_level<float, float>(h, B, l, (const float*)b, (float*)x);
+  if (prec) return vcycle_level<float, double>(h, B, l, (const float*)b, (float*)x);
+  return vcycle_level<double, double>(h, B, l, (const double*)b, (double*)x);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -755,7 +933,7 @@ static int init_linear(ppf_handle h, int b) {
   PPF_CUDA(h, cudaMalloc(&L.p, sizeof(double) * len));
   PPF_CUDA(h, cudaMalloc(&L.q, sizeof(double) * len));
   PPF_CUDA(h, cudaMalloc(&L.z, sizeof(double) * len));
-  PPF_CUDA(h, cudaMalloc(&L.partial, sizeof(double) * 1100));
+  if (const int rc = ensure_scalars(h, L)) return rc;
   // levels: coarsest refinement R - depth + 1 .. R (depth 1 = the fine level only)
   const int R = h->mesh.global_refinement;
   int depth = L.params.preconditioner == 2 ? std::max(1, L.params.mg_depth) : 1;
@@ -853,7 +1031,7 @@ static int init_linear(ppf_handle h, int b) {
     PPF_CUDA(h, cudaMemcpy(lv.tables, tab.data(), tab.size(), cudaMemcpyHostToDevice));
     lv.fx_lanes = lv.precision == 0 ? tables_lanes(tab, h->dim, h->k) : 0;
     lv.h_tables = std::move(tab);
-    for (void** p : {&lv.inv_diag, &lv.acc, &lv.x, &lv.b, &lv.r, &lv.w0, &lv.w1}) {
+    for (void** p : {&lv.inv_diag, &lv.acc, &lv.acc2, &lv.x, &lv.b, &lv.r, &lv.w0, &lv.w1}) {
       rc = alloc_real(h, p, lv.len, lv.precision);
       if (rc) return rc;
     }
@@ -875,13 +1053,6 @@ static int init_linear(ppf_handle h, int b) {
       if (!rc) rc = upload_vec<int>(h, (void**)&cl.r_ptr[d], tptr);
       if (!rc) rc = upload_vec<int>(h, (void**)&cl.r_col[d], tcol);
       if (!rc) rc = upload_real(h, &cl.r_val[d], tval, tp);
-      if (rc) return rc;
-    }
-    int rc = alloc_real(h, &fl.t0, fl.N, tp);
-    if (!rc) rc = alloc_real(h, &fl.t1, fl.N, tp);
-    if (rc) return rc;
-    if (cl.precision != tp) {  // conversion buffer of coarse size in the transfer precision
-      rc = alloc_real(h, &cl.cvt, cl.len, tp);
       if (rc) return rc;
     }
   }
@@ -912,11 +1083,15 @@ static int precondition(ppf_handle h, BlockState& B, const double* r, double* z)
     return PPF_OK;
   }
   MGLevel& fine = L.levels.back();
-  // the fine level's defect/solution vectors carry the V-cycle (or the Chebyshev smoother)
-  convert(h, 0, fine.precision, n, r, fine.b);
-  int rc = L.params.preconditioner == 1 ? smooth(h, B, fine, true) : vcycle(h, B, (int)L.levels.size() - 1);
+  const int top = (int)L.levels.size() - 1;
+  if (!fine.precision)
+    return L.params.preconditioner == 1 ? chebyshev<double>(h, B, fine, true, r, z) : vcycle(h, B, top, r, z);
+  // an FP32 fine level's own vectors carry the V-cycle
+  convert(h, 0, 1, n, r, fine.b);
+  int rc = L.params.preconditioner == 1 ? chebyshev<float>(h, B, fine, true, (const float*)fine.b, (float*)fine.x)
+                                        : vcycle(h, B, top, fine.b, fine.x);
   if (rc) return rc;
-  convert(h, fine.precision, 0, n, fine.x, z);
+  convert(h, 1, 0, n, fine.x, z);
   return PPF_OK;
 }
 
@@ -947,7 +1122,18 @@ static int precondition_graphed(ppf_handle h, BlockState& B, const double* r, do
     L.pc_nograph = true;
     return precondition(h, B, r, z);
   }
+  std::vector<void*> acc0;
+  for (auto& lv : L.levels) acc0.push_back(lv.acc);
   int rc = precondition(h, B, r, z);
+  // a replay starts where the capture did: a level left on its other accumulator (an odd number of
+  // products, the coarsest level's) clears the first one and returns to it
+  for (size_t l = 0; l < L.levels.size() && !rc; ++l) {
+    MGLevel& lv = L.levels[l];
+    if (lv.acc == acc0[l]) continue;
+    std::swap(lv.acc, lv.acc2);
+    if (cudaMemsetAsync(lv.acc, 0, lv.len * esize(lv.precision), h->stream) != cudaSuccess)
+      rc = fail(h, PPF_ERR_CUDA, "preconditioner capture");
+  }
   cudaGraph_t graph = nullptr;
   const cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
   if (rc) {
@@ -963,6 +1149,51 @@ static int precondition_graphed(ppf_handle h, BlockState& B, const double* r, do
   PPF_CUDA(h, cudaGraphLaunch(L.pc_graph, h->stream));
   h->all_launches++;
   return PPF_OK;
+}
+
+// CG on A x = b from the residual r of the iterate x (SolverCG): M(r, z) applies the preconditioner,
+// A(p, q, pq) the operator with pq = p.q on the device. alpha, beta and the convergence test stay on
+// the device; the host reads each residual norm, one iteration behind the work it has queued where
+// the preconditioner is cheap, so that it never waits with an empty stream (a V-cycle is longer than
+// that wait, and queueing one past convergence would cost more). What runs past convergence changes
+// neither x nor r.
+template <class Mf, class Af>
+static int conjugate_gradients(ppf_handle h, LinearState& L, long long n, double* x, double* r, double* z, double* p,
+                               double* q, double tol, Mf&& M, Af&& A, int* its, double* res, bool* converged) {
+  const int lag = L.params.preconditioner == 2 ? 0 : 1;
+  const bool plain = L.params.preconditioner == 0;  // z is r itself
+  double* sc = L.scal;
+  int rc = PPF_OK;
+  PPF_CUDA(h, cudaMemsetAsync(sc, 0, sizeof(double) * SC_EIG, h->stream));
+  const int max_it = L.params.max_iterations;
+  for (int it = 0;; ++it) {
+    // it: iterations queued so far; `seen` is the newest whose residual the host reads now
+    const int seen = it == max_it ? it : it - lag;
+    for (int s = it == max_it ? std::max(1, it - lag) : seen; s >= 1 && s <= seen; ++s) {
+      PPF_CUDA(h, cudaEventSynchronize(L.scal_ev[s & 3]));
+      *res = std::sqrt(L.h_scal[s & 3]);
+      *its = s;
+      if (!std::isfinite(*res)) return fail(h, PPF_ERR_NAN, "non-finite residual in the linear solve");
+      if (*res < tol) {
+        *converged = true;
+        return PPF_OK;
+      }
+    }
+    if (it == max_it) return PPF_OK;
+    const int rz = it & 1;
+    const double* zz = plain ? r : z;
+    if (!plain && (rc = M(r, z))) return rc;
+    if ((rc = dot_device<double>(h, L, n, r, zz, sc + SC_RZ + rz))) return rc;
+    PPF_CUDA(h, launch_chained(cg_direction_kernel, dim3(grid_for(n)), dim3(256), 0, h->stream, n, (const double*)sc, rz,
+                               it == 0 ? 1 : 0, zz, p));
+    if ((rc = A(p, q, sc + SC_PQ))) return rc;
+    PPF_CUDA(h, launch_chained(cg_update_kernel, dim3(dot_blocks(n)), dim3(256), 0, h->stream, n, sc, rz,
+                               (const double*)p, (const double*)q, x, r, tol, L.partial, counters(L)));
+    h->all_launches += 2;
+    const int s = it + 1;
+    PPF_CUDA(h, cudaMemcpyAsync(L.h_scal + (s & 3), sc + SC_RR, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    PPF_CUDA(h, cudaEventRecord(L.scal_ev[s & 3], h->stream));
+  }
 }
 
 int linear_solve(ppf_handle h, int b) {
@@ -989,7 +1220,7 @@ int linear_solve(ppf_handle h, int b) {
         PPF_CUDA(h, cudaMalloc(v, sizeof(double) * len));
       }
       PPF_CUDA(h, cudaMemsetAsync(L.x_hom, 0, sizeof(double) * len, h->stream));
-      if (!L.partial) PPF_CUDA(h, cudaMalloc(&L.partial, sizeof(double) * 1100));
+      if (const int rc = ensure_scalars(h, L)) return rc;
       L.mesh_version = h->mesh_version;
       L.initialized = true;
     }
@@ -1004,19 +1235,27 @@ int linear_solve(ppf_handle h, int b) {
   const long long n = F.len;
   // FP64 outer operator on the problem lattice (the handle's FP64 LHS plan), also when the
   // fine multigrid level runs in FP32
-  auto outer_apply = [&](const double* src, double* dst, bool plain) -> int {
+  // (with `out` also out = src.dst)
+  auto finalize = [&](double* dst, const double* w, double* out) -> int {
+    dim3 grid(grid_for(h->N), F.ncomp);
+    if (out) grid.x = std::min(grid.x, 1024u / grid.y);
+    if (const int rc = ensure_acc2(h, F)) return rc;
+    PPF_CUDA(h, launch_chained(level_finalize_kernel<double>, grid, dim3(256), 0, h->stream, dst, (const double*)F.acc,
+                               F.acc2, scaled(L) ? h->d_invm_sqrt : nullptr, F.constrained ? F.cmap : nullptr, h->N, w,
+                               L.partial, counters(L), out));
+    h->all_launches++;
+    std::swap(F.acc, F.acc2);
+    F.acc_clean = true;
+    return PPF_OK;
+  };
+  auto outer_apply = [&](const double* src, double* dst, bool plain, double* out) -> int {
     const double* srcs[PPF_MAX_FIELDS] = {src};
-    PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * n, h->stream));
+    int rc = clear_acc(h, F);
+    if (rc) return rc;
     F.acc_clean = false;
     if (h->amr) {
-      int rc = launch_cell(h, b, 1, srcs, plain);
-      if (rc) return rc;
-      dim3 grid(grid_for(h->N), F.ncomp);
-      level_finalize_kernel<double><<<grid, 256, 0, h->stream>>>(dst, F.acc, scaled(L) ? h->d_invm_sqrt : nullptr,
-                                                                 F.constrained ? F.cmap : nullptr, h->N);
-      h->all_launches++;
-      PPF_CUDA(h, cudaGetLastError());
-      return PPF_OK;
+      rc = launch_cell(h, b, 1, srcs, plain);
+      return rc ? rc : finalize(dst, src, out);
     }
     CellLaunch Lc;
     std::memset(&Lc, 0, sizeof(Lc));
@@ -1064,16 +1303,10 @@ int linear_solve(ppf_handle h, int b) {
       set_fx_mode(Lc, m);
     }
     const size_t smem = cell_smem(h->dim, h->k, 0, P.nrows_in, P.nrows_out);
-    int rc = timed_cell_launch(h, 0, MODE_LHS, Lc, h->model_obj.data(), smem);
+    rc = timed_cell_launch(h, 0, MODE_LHS, Lc, h->model_obj.data(), smem);
     if (rc) return rc;
     rc = online_mode_end(h, P.fx_mode, P.fx_timed, P.fx_ev, slot, P.fx_lanes);
-    if (rc) return rc;
-    dim3 grid(grid_for(h->N), F.ncomp);
-    level_finalize_kernel<double><<<grid, 256, 0, h->stream>>>(dst, F.acc, scaled(L) ? h->d_invm_sqrt : nullptr,
-                                                               F.constrained ? F.cmap : nullptr, h->N);
-    h->all_launches++;
-    PPF_CUDA(h, cudaGetLastError());
-    return PPF_OK;
+    return rc ? rc : finalize(dst, src, out);
   };
   // phase timers (host wall clock; each phase ends on a stream synchronisation)
   auto now = [] { return std::chrono::steady_clock::now(); };
@@ -1098,29 +1331,33 @@ int linear_solve(ppf_handle h, int b) {
   const auto t_setup = now();
   // rhs = S * compute_rhs
   {
-    PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * n, h->stream));
+    int rc = clear_acc(h, F);
+    if (rc) return rc;
     F.acc_clean = false;
     if (B.plan[0].valid && B.plan[0].nslots >= 0) {
-      int rc = launch_cell(h, b, 0, nullptr);
+      rc = launch_cell(h, b, 0, nullptr);
       if (rc) return rc;
     }
-    dim3 grid(grid_for(h->N), F.ncomp);
-    level_finalize_kernel<double><<<grid, 256, 0, h->stream>>>(L.rhs, F.acc, scaled(L) ? h->d_invm_sqrt : nullptr,
-                                                               F.constrained ? F.cmap : nullptr, h->N);
-    h->all_launches++;
+    rc = finalize(L.rhs, nullptr, nullptr);
+    if (rc) return rc;
   }
   // inhomogeneous Dirichlet values g and rhs -= S A_plain g
-  PPF_CUDA(h, cudaMemsetAsync(L.g, 0, sizeof(double) * n, h->stream));
   bool has_inhom = false;
   for (double v : F.h_dvals) has_inhom |= v != 0.0;
   if (has_inhom) {
-    std::vector<double> gh(n, 0.0);
-    for (long long i = 0; i < n; ++i)
-      if (F.h_cmap[i] < 0) gh[i] = F.h_dvals[-1 - F.h_cmap[i]];
-    if (h->amr) amr_fill_hanging(h, F.ncomp, gh.data());  // hanging nodes on Dirichlet faces
-    PPF_CUDA(h, cudaMemcpyAsync(L.g, gh.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-    PPF_CUDA(h, cudaStreamSynchronize(h->stream));
-    int rc = outer_apply(L.g, L.q, true);
+    if (h->amr) {
+      std::vector<double> gh(n, 0.0);
+      for (long long i = 0; i < n; ++i)
+        if (F.h_cmap[i] < 0) gh[i] = F.h_dvals[-1 - F.h_cmap[i]];
+      amr_fill_hanging(h, F.ncomp, gh.data());  // hanging nodes on Dirichlet faces
+      PPF_CUDA(h, cudaMemcpyAsync(L.g, gh.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
+      PPF_CUDA(h, cudaStreamSynchronize(h->stream));
+    } else {
+      lift_values_kernel<<<grid_for(n), 256, 0, h->stream>>>(L.g, F.cmap, F.dvals, n);
+      PPF_CUDA(h, cudaGetLastError());
+      h->all_launches++;
+    }
+    int rc = outer_apply(L.g, L.q, true, nullptr);
     if (rc) return rc;
     axpby(h, 0, n, -1.0, L.q, 1.0, L.rhs);
   }
@@ -1129,7 +1366,7 @@ int linear_solve(ppf_handle h, int b) {
   // CG on S A x = rhs from the previous homogeneous solution (SolverCG)
   double* x = L.x_hom;
   const double tol = L.params.tolerance * normalization(h, L);
-  int rc = outer_apply(x, L.q, false);
+  int rc = outer_apply(x, L.q, false, nullptr);
   if (rc) return rc;
   PPF_CUDA(h, cudaMemcpyAsync(L.r, L.rhs, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
   axpby(h, 0, n, -1.0, L.q, 1.0, L.r);
@@ -1140,39 +1377,10 @@ int linear_solve(ppf_handle h, int b) {
   int it = 0;
   bool converged = res < tol;
   if (!converged) {
-    rc = precondition_graphed(h, B, L.r, L.z);
+    rc = conjugate_gradients(
+        h, L, n, x, L.r, L.z, L.p, L.q, tol, [&](const double* in, double* out) { return precondition_graphed(h, B, in, out); },
+        [&](const double* in, double* out, double* pq) { return outer_apply(in, out, false, pq); }, &it, &res, &converged);
     if (rc) return rc;
-    PPF_CUDA(h, cudaMemcpyAsync(L.p, L.z, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
-    double rz;
-    rc = dot(h, L, 0, n, L.r, L.z, &rz);
-    if (rc) return rc;
-    while (it < L.params.max_iterations) {
-      rc = outer_apply(L.p, L.q, false);
-      if (rc) return rc;
-      double pq;
-      rc = dot(h, L, 0, n, L.p, L.q, &pq);
-      if (rc) return rc;
-      const double alpha = rz / pq;
-      cg_update_xr_kernel<<<grid_for(n), 256, 0, h->stream>>>(n, alpha, L.p, L.q, x, L.r);
-      h->all_launches++;
-      ++it;
-      rc = dot(h, L, 0, n, L.r, L.r, &rr);
-      if (rc) return rc;
-      res = std::sqrt(rr);
-      if (!std::isfinite(res)) return fail(h, PPF_ERR_NAN, "non-finite residual in the linear solve");
-      if (res < tol) {
-        converged = true;
-        break;
-      }
-      rc = precondition_graphed(h, B, L.r, L.z);
-      if (rc) return rc;
-      double rz_new;
-      rc = dot(h, L, 0, n, L.r, L.z, &rz_new);
-      if (rc) return rc;
-      const double beta = rz_new / rz;
-      rz = rz_new;
-      axpby(h, 0, n, 1.0, L.z, beta, L.p);
-    }
   }
   PPF_CUDA(h, cudaStreamSynchronize(h->stream));
   const auto t_end = now();
@@ -1187,7 +1395,7 @@ int linear_solve(ppf_handle h, int b) {
   L.last_rhs_norm = std::sqrt(bb);
   // solution = x_hom + g, then constraints
   PPF_CUDA(h, cudaMemcpyAsync(F.cur, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
-  axpby(h, 0, n, 1.0, L.g, 1.0, F.cur);
+  if (has_inhom) axpby(h, 0, n, 1.0, L.g, 1.0, F.cur);
   rc = ppf_apply_constraints(h, f);
   if (rc) return rc;
   rc = check_err(h);
@@ -1235,34 +1443,14 @@ static int block_krylov(ppf_handle h, int b, const double* rhs, double* x, doubl
   int it = 0;
   *conv = res < tol;
   if (!*conv && L.params.solver_type == 0) {
-    double* z = v[2];
-    double* p = v[3];
-    if ((rc = M(r, z))) return rc;
-    PPF_CUDA(h, cudaMemcpyAsync(p, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
-    double rz;
-    if ((rc = dot(h, L, 0, n, r, z, &rz))) return rc;
-    while (it < L.params.max_iterations) {
-      if ((rc = A(p, q))) return rc;
-      double pq;
-      if ((rc = dot(h, L, 0, n, p, q, &pq))) return rc;
-      const double alpha = rz / pq;
-      cg_update_xr_kernel<<<grid_for(n), 256, 0, h->stream>>>(n, alpha, p, q, x, r);
-      h->all_launches++;
-      ++it;
-      if ((rc = dot(h, L, 0, n, r, r, &rr))) return rc;
-      res = std::sqrt(rr);
-      if (!std::isfinite(res)) return fail(h, PPF_ERR_NAN, "non-finite residual in the linear solve");
-      if (res < tol) {
-        *conv = true;
-        break;
-      }
-      if ((rc = M(r, z))) return rc;
-      double rz_new;
-      if ((rc = dot(h, L, 0, n, r, z, &rz_new))) return rc;
-      const double beta = rz_new / rz;
-      rz = rz_new;
-      axpby(h, 0, n, 1.0, z, beta, p);
-    }
+    rc = conjugate_gradients(
+        h, L, n, x, r, v[2], v[3], q, tol, M,
+        [&](const double* in, double* out, double* pq) -> int {
+          const int e = A(in, out);
+          return e ? e : dot_device<double>(h, L, n, in, out, pq);
+        },
+        &it, &res, conv);
+    if (rc) return rc;
   } else if (!*conv) {
     // BiCGStab (van der Vorst), right-preconditioned, with the half-step convergence check
     double* rbar = v[2];
@@ -1384,7 +1572,7 @@ int newton_solve(ppf_handle h, int b) {
     for (double*& p : L.kv) PPF_CUDA(h, cudaMalloc(&p, sizeof(double) * n));
     cudaFree(L.rhs);  // a Newton block's rhs vector holds its block residual
     PPF_CUDA(h, cudaMalloc(&L.rhs, sizeof(double) * n));
-    if (!L.partial) PPF_CUDA(h, cudaMalloc(&L.partial, sizeof(double) * 1100));
+    if (const int rc = ensure_scalars(h, L)) return rc;
     L.block_len = n;
   }
   double* R = L.rhs;
@@ -1438,7 +1626,10 @@ int newton_solve(ppf_handle h, int b) {
 
 void free_linear(LinearState& L) {
   drop_pc_graph(L);
-  for (double* p : {L.rhs, L.g, L.x_hom, L.r, L.p, L.q, L.z, L.inv_diag, L.partial, L.newton_update}) cudaFree(p);
+  for (double* p : {L.rhs, L.g, L.x_hom, L.r, L.p, L.q, L.z, L.inv_diag, L.partial, L.scal, L.newton_update}) cudaFree(p);
+  cudaFreeHost(L.h_scal);
+  for (auto& ev : L.scal_ev)
+    if (ev) cudaEventDestroy(ev);
   for (double*& p : L.kv) {
     cudaFree(p);
     p = nullptr;
@@ -1449,7 +1640,7 @@ void free_linear(LinearState& L) {
     for (auto& ev : lv.fx_ev)
       if (ev) cudaEventDestroy(ev);
     cudaFree(lv.cmap);
-    for (void* p : {lv.invm_sqrt, lv.inv_diag, lv.tables, lv.acc, lv.x, lv.b, lv.r, lv.w0, lv.w1, lv.t0, lv.t1, lv.cvt})
+    for (void* p : {lv.invm_sqrt, lv.inv_diag, lv.tables, lv.acc, lv.acc2, lv.x, lv.b, lv.r, lv.w0, lv.w1})
       cudaFree(p);
     for (int d = 0; d < 3; ++d) {
       cudaFree(lv.p_ptr[d]);

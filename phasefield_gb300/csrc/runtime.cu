@@ -445,9 +445,12 @@ __global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const
 }
 
 // dst = scale (.) acc on unconstrained rows, 0 on constrained rows (MFOperator::compute_operator
-// leaves constrained rows of dst untouched after zeroing, then scales).
-__global__ void finalize_apply_kernel(double* __restrict__ dst, const double* __restrict__ acc,
-                                      const double* __restrict__ scale, const int* __restrict__ cmap, long long N) {
+// leaves constrained rows of dst untouched after zeroing, then scales); `clear`, the field's other
+// accumulator, is zeroed for the next product.
+__global__ void finalize_apply_kernel(double* dst, const double* acc, double* clear, const double* __restrict__ scale,
+                                      const int* __restrict__ cmap, long long N) {
+  chain_release();
+  chain_wait();
   const int c = blockIdx.y;
   const long long base = c * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
@@ -455,6 +458,7 @@ __global__ void finalize_apply_kernel(double* __restrict__ dst, const double* __
     const int cm = cmap ? cmap[gi] : (int)gi;
     double v = 0.0;
     if (cm == (int)gi) v = scale ? acc[gi] * scale[i] : acc[gi];
+    if (clear) clear[gi] = 0.0;
     dst[gi] = v;
   }
 }
@@ -893,8 +897,20 @@ int stream_field_out(ppf_handle h, FieldState& F, const double* src, bool staged
 int finish_streamed_outputs(ppf_handle h);
 static int ensure_out_stage(ppf_handle h, FieldState& F);
 
+// Whether a launch sequence may leave its field on its other accumulator: not in a caller's own
+// capture, which may be replayed by itself (the increment graph's period returns to where it began)
+static int alternating(ppf_handle h, bool* yes) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!h->capturing) PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
+  *yes = cs == cudaStreamCaptureStatusNone;
+  return PPF_OK;
+}
+
+// (a caller's own capture clears in any case)
 int clear_acc(ppf_handle h, FieldState& F) {
-  if (!F.acc_clean) PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
+  bool alternate = true;
+  if (const int rc = alternating(h, &alternate)) return rc;
+  if (!F.acc_clean || !alternate) PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
   F.acc_clean = true;
   return PPF_OK;
 }
@@ -913,18 +929,11 @@ void free_acc(FieldState& F) {
 
 static int explicit_solve(ppf_handle h, int b) {
   BlockState& B = h->blocks[b];
-  // a caller's own capture (not the increment graph, whose period returns the accumulators to where
-  // they were) may replay this solve on its own: it clears its accumulator itself and keeps it
   bool alternate = true;
-  if (!h->capturing) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
-    alternate = cs == cudaStreamCaptureStatusNone;
-  }
+  if (const int rc = alternating(h, &alternate)) return rc;
   for (int i = 0; i < B.desc.n_fields; ++i) {
     FieldState& F = h->fields[B.desc.field_indices[i]];
     int rc = alternate ? ensure_acc2(h, F) : PPF_OK;
-    if (!alternate) F.acc_clean = false;
     if (!rc) rc = clear_acc(h, F);
     if (rc) return rc;
     F.acc_clean = false;
@@ -1747,23 +1756,32 @@ int ppf_apply_device(ppf_handle h, int b, int which, const double* d_src, double
   BlockState& B = h->blocks[b];
   const double* srcs[PPF_MAX_FIELDS] = {};
   long long off = 0;
+  bool alternate = true;
+  int rc = alternating(h, &alternate);
+  if (rc) return rc;
   for (int i = 0; i < B.desc.n_fields; ++i) {
     FieldState& F = h->fields[B.desc.field_indices[i]];
     srcs[i] = d_src ? d_src + off : nullptr;
-    PPF_CUDA(h, cudaMemsetAsync(F.acc, 0, sizeof(double) * F.len, h->stream));
+    rc = alternate ? ensure_acc2(h, F) : PPF_OK;
+    if (!rc) rc = clear_acc(h, F);
+    if (rc) return rc;
     F.acc_clean = false;
     off += F.len;
   }
-  int rc = launch_cell(h, b, which, srcs);
+  rc = launch_cell(h, b, which, srcs);
   if (rc) return rc;
   off = 0;
   for (int i = 0; i < B.desc.n_fields; ++i) {
     FieldState& F = h->fields[B.desc.field_indices[i]];
     const double* sc = scale == 1 ? h->d_invm : (scale == 2 ? h->d_invm_sqrt : nullptr);
     dim3 grid(grid_for(h->N), F.ncomp);
-    finalize_apply_kernel<<<grid, 256, 0, h->stream>>>(d_dst + off, F.acc, sc, F.constrained ? F.cmap : nullptr, h->N);
-    PPF_CUDA(h, cudaGetLastError());
+    PPF_CUDA(h, launch_chained(finalize_apply_kernel, grid, dim3(256), 0, h->stream, d_dst + off, (const double*)F.acc,
+                               alternate ? F.acc2 : nullptr, sc, F.constrained ? F.cmap : nullptr, h->N));
     h->all_launches++;
+    if (alternate) {
+      std::swap(F.acc, F.acc2);
+      F.acc_clean = true;
+    }
     off += F.len;
   }
   return PPF_OK;
