@@ -19,6 +19,7 @@
 #include <prismspf/gpu/fixed_point.cuh>
 
 #include <type_traits>
+#include <utility>
 
 PRISMS_PF_BEGIN_NAMESPACE
 
@@ -37,6 +38,17 @@ enum ErrorBits : int {
   ERR_UNDECLARED_SUBMISSION = 2,
   ERR_NONFINITE = 4,
 };
+
+// f(0), f(1), .. f(N - 1) with the index as a constant: loops over components that must end up in
+// registers whatever the unroller makes of them
+template <int... I, class F>
+PPF_HD void each_of(std::integer_sequence<int, I...>, F&& f) {
+  (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, class F>
+PPF_HD void each(F&& f) {
+  each_of(std::make_integer_sequence<int, N>{}, f);
+}
 
 PPF_HD constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }
 
@@ -130,8 +142,13 @@ struct CellCtx {
   int qi[3] = {0, 0, 0};
   int pe = 0;
   int step[3] = {0, 0, 0};
+  // (nterm > 0: the terms stay in registers)
   int nterm = 0;
   number term[LANE_MAX_OUT * (1 + dim)];
+  // diagonal probe (prismspf/gpu/cell_diagonal.cuh): the rows of probe_rows hold one at cell node
+  // `probe` and zero elsewhere
+  int probe = -1;
+  unsigned int probe_rows = 0;
   // value terms stored unweighted (a kernel integrating them in fixed point), on any layout
   int raw_values = 0;
 };
@@ -204,23 +221,22 @@ class FieldContainer {
       if (ctx.lean) {
         const int gs = lane_slot(ctx.tab->lane_g, field_index, type);
         if (gs >= 0) {
-          if constexpr (Rank == TensorRank::Scalar) {
-            for (int d = 0; d < int(dim); ++d) g[d] = lane_deriv(gs, d);
-          } else {
-            for (int c = 0; c < int(dim); ++c)
-              for (int d = 0; d < int(dim); ++d) g[c][d] = lane_deriv(gs + c, d);
-          }
+          if constexpr (Rank == TensorRank::Scalar)
+            gpu::each<int(dim)>([&](auto d) { g[d] = lane_deriv(gs, d); });
+          else
+            gpu::each<int(dim * dim)>([&](auto i) { g[i / int(dim)][i % int(dim)] = lane_deriv(gs + i / int(dim), i % int(dim)); });
           return g;
         }
       }
     }
     const int row = row_of(field_index, type);
     if (row < 0) return g;
+    // (a lane kernel's row without a fixed-point copy comes here too: plain_deriv)
     if constexpr (Rank == TensorRank::Scalar) {
-      for (int d = 0; d < int(dim); ++d) g[d] = deriv(row, d);
+      for (int d = 0; d < int(dim); ++d) g[d] = plain_deriv(row, d);
     } else {
       for (int c = 0; c < int(dim); ++c)
-        for (int d = 0; d < int(dim); ++d) g[c][d] = deriv(row + c, d);
+        for (int d = 0; d < int(dim); ++d) g[c][d] = plain_deriv(row + c, d);
     }
     return g;
   }
@@ -236,14 +252,15 @@ class FieldContainer {
                                                                              DependencyType type) const {
     const Gradient<Rank> g = get_gradient<Rank>(field_index, type);
     dealii::SymmetricTensor<2, dim, ScalarValue> s;
-    for (int i = 0; i < int(dim); ++i) {
-      s.a[i][i] = g[i][i];
-      for (int j = i + 1; j < int(dim); ++j) {
-        ScalarValue v = number(0.5) * (g[i][j] + g[j][i]);
+    gpu::each<int(dim * dim)>([&](auto k) {
+      constexpr int i = k / int(dim), j = k % int(dim);
+      if constexpr (i == j) s.a[i][i] = g[i][i];
+      if constexpr (i < j) {
+        const ScalarValue v(gpu::fx::half_of((g[i][j] + g[j][i]).v));
         s.a[i][j] = v;
         s.a[j][i] = v;
       }
-    }
+    });
     return s;
   }
 
@@ -258,7 +275,7 @@ class FieldContainer {
     const int row = row_of(field_index, type);
     ScalarValue s(number(0));
     if (row < 0) return s;
-    for (int d = 0; d < int(dim); ++d) s += deriv(row + d, d);
+    gpu::each<int(dim)>([&](auto d) { s += deriv(row + d, d); });
     return s;
   }
 
@@ -369,7 +386,7 @@ class FieldContainer {
 
   // --- submissions --------------------------------------------------------------------
   PPF_HD void set_value_term(unsigned int field_index, const ScalarValue& val) {
-    if (ctx.lean) {
+    if (ctx.nterm) {
       const int o = lane_component(field_index);
       if (o >= 0) set_term(o, 0, val.v);
       return;
@@ -381,10 +398,12 @@ class FieldContainer {
   }
 
   PPF_HD void set_value_term(unsigned int field_index, const dealii::Tensor<1, dim, ScalarValue>& val) {
-    if (ctx.lean) {
+    if (ctx.nterm) {
       const int o = lane_component(field_index);
-      if (o >= 0)
+      if (o >= 0) {
+#pragma unroll
         for (int c = 0; c < int(dim); ++c) set_term(o, c, 0, val[c].v);
+      }
       return;
     }
     const int o = out_row(field_index);
@@ -396,7 +415,7 @@ class FieldContainer {
   }
 
   PPF_HD void set_gradient_term(unsigned int field_index, const dealii::Tensor<1, dim, ScalarValue>& g) {
-    if (ctx.lean) {
+    if (ctx.nterm) {
       const int o = lane_component(field_index);
       if (o >= 0)
         for (int d = 0; d < int(dim); ++d) set_term(o, 1 + d, g[d].v);
@@ -410,11 +429,10 @@ class FieldContainer {
   }
 
   PPF_HD void set_gradient_term(unsigned int field_index, const dealii::Tensor<2, dim, ScalarValue>& g) {
-    if (ctx.lean) {
+    if (ctx.nterm) {
       const int o = lane_component(field_index);
       if (o >= 0)
-        for (int c = 0; c < int(dim); ++c)
-          for (int d = 0; d < int(dim); ++d) set_term(o, c, 1 + d, g[c][d].v);
+        gpu::each<int(dim * dim)>([&](auto i) { set_term(o, i / int(dim), 1 + i % int(dim), g[i / int(dim)][i % int(dim)].v); });
       return;
     }
     const int o = out_row(field_index);
@@ -523,7 +541,10 @@ class FieldContainer {
     return ctx.tab->out_row0[o];
   }
 
+  PPF_HD bool probed(int row) const { return ctx.probe >= 0 && ((ctx.probe_rows >> row) & 1u); }
+
   PPF_HD number nodal(int row, int q) const {
+    if (probed(row)) return q == ctx.probe ? number(1) : number(0);
     if constexpr (std::is_same<number, double>::value && degree <= 2) {
       if (ctx.lean) {
         // the lane kernel: the row's double copy, or for a row read only as a gradient its
@@ -548,12 +569,21 @@ class FieldContainer {
 
   // first derivative along direction d at this thread's quadrature point
   PPF_HD number deriv(int row, int d) const {
-    int stride_d = 1;
-    for (int e = 0; e < d; ++e) stride_d *= n;
-    if constexpr (std::is_same<number, double>::value && degree <= 2) {
+    if constexpr (lane_capable) {
       if (ctx.lean && ((ctx.tab->fx_rows >> row) & 1u)) return lane_deriv(ctx.tab->lane_gslot[row], d);
     }
+    return plain_deriv(row, d);
+  }
+
+  // the same of a row that is not one of a lane kernel's fixed-point rows
+  PPF_HD number plain_deriv(int row, int d) const {
+    int stride_d = 1;
+    for (int e = 0; e < d; ++e) stride_d *= n;
     const int qd = (ctx.q / stride_d) % n;
+    if (probed(row)) {
+      const int id = (ctx.probe / stride_d) % n;
+      return ctx.q - qd * stride_d == ctx.probe - id * stride_d ? ctx.tab->Dh[d][qd][id] : number(0);
+    }
     const int base = row * ctx.stride + ctx.lc * int(dofs_per_component) + (ctx.q - qd * stride_d);
     if constexpr (std::is_same<number, double>::value && degree <= 2) {
       if (ctx.vals_fx && !ctx.lean) {
@@ -592,6 +622,12 @@ class FieldContainer {
     for (int k = 0; k < d; ++k) sd *= n;
     for (int k = 0; k < e; ++k) se *= n;
     const int qd = (ctx.q / sd) % n, qe = (ctx.q / se) % n;
+    if (probed(row)) {
+      const int id = (ctx.probe / sd) % n, ie = (ctx.probe / se) % n;
+      if (d == e) return ctx.q - qd * sd == ctx.probe - id * sd ? ctx.tab->D2h[d][qd][id] : number(0);
+      return ctx.q - qd * sd - qe * se == ctx.probe - id * sd - ie * se ? ctx.tab->Dh[d][qd][id] * ctx.tab->Dh[e][qe][ie]
+                                                                       : number(0);
+    }
     const int vr = vrow(row);
     if (vr < 0) {
       // the lane kernel keeps no double copy of a row declared without values or Hessians

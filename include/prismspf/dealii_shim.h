@@ -210,7 +210,14 @@ struct SymmetricTensor<2, dim, T> {
   struct CRow { const T* r; PPF_HD const T& operator[](unsigned int j) const { return r[j]; } };
   PPF_HD Row operator[](unsigned int i) { return Row{a[i]}; }
   PPF_HD CRow operator[](unsigned int i) const { return CRow{a[i]}; }
-  PPF_HD operator Tensor<2, dim, T>() const { Tensor<2, dim, T> t; for (int i = 0; i < dim; ++i) for (int j = 0; j < dim; ++j) t[i][j] = a[i][j]; return t; }
+  PPF_HD operator Tensor<2, dim, T>() const {
+    Tensor<2, dim, T> t;
+#pragma unroll
+    for (int i = 0; i < dim; ++i)
+#pragma unroll
+      for (int j = 0; j < dim; ++j) t[i][j] = a[i][j];
+    return t;
+  }
   PPF_HD T norm() const { using std::sqrt; T s = a[0][0] * a[0][0]; for (int i = 0; i < dim; ++i) for (int j = 0; j < dim; ++j) if (i || j) s = s + a[i][j] * a[i][j]; return sqrt(s); }
 };
 template <int dim, typename T> PPF_HD T trace(const SymmetricTensor<2, dim, T>& A) { T s = A.a[0][0]; for (int i = 1; i < dim; ++i) s = s + A.a[i][i]; return s; }

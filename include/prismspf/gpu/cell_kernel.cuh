@@ -4,8 +4,7 @@
 // Restates the per-cell work of MFOperator::compute_local_operator
 // (src/solvers/mf_operator.cc:34-80) with FieldContainer::reinit_and_eval /
 // integrate_and_distribute (include/prismspf/core/field_container.h:794-882) as one GPU
-// kernel, plus the diagonal probe of MFOperator::compute_local_field_diagonal
-// (src/solvers/mf_operator.cc:147-218):
+// kernel:
 //   * DoF vectors are stored in lattice order (x fastest) with periodic images kept, so the
 //     nodes of cell (cx,cy,cz) are a dense (k+1)^dim box of the lattice: the gather needs no
 //     index map. Constraint maps are int32 arrays over the same index space:
@@ -19,9 +18,7 @@
 //   * distribute_local_to_global: rows constrained to a master add into the master,
 //     Dirichlet rows are dropped; contributions of neighbouring cells meet through
 //     atomicAdd into a zeroed accumulator (the finalize kernels apply invM and constraints).
-//   * MODE_DIAG replaces the SRC dependency of each block field by unit probes on one cell
-//     node at a time (identity in every component, as the reference submits
-//     identity<Rank>()) and keeps the integrated entry at the probed node.
+//   * MODE_DIAG is the diagonal probe's own kernel (prismspf/gpu/cell_diagonal.cuh).
 //   * FP64 Q1/Q2 launches contract exactly in 64-bit integers (prismspf/gpu/fixed_point.cuh):
 //     rows read as gradients get a fixed-point copy with a per-cell block exponent, the
 //     derivatives are integer line sums rounded once, and with fx_int the submitted gradient
@@ -141,7 +138,24 @@ struct CellLaunch {
   // of `tables` (tables_host) as a kernel parameter
   int fx_lanes;
   const void* tables_host;
+  // cell index -> coordinates: multiply-high divisors of nc[0] and nc[1] (filled by the launchers: a
+  // thread that makes its own spends two 64-bit divisions before its first load)
+  unsigned int div_m[2], div_l[2];
+  __device__ __forceinline__ unsigned int div(unsigned int v, int d) const {
+    return (__umulhi(v, div_m[d]) + v) >> div_l[d];
+  }
 };
+
+inline CellLaunch with_divisors(const CellLaunch& L) {
+  CellLaunch P = L;
+  for (int d = 0; d < 2; ++d) {
+    pg::fx::FastDiv f;
+    f.init((unsigned int)P.nc[d]);
+    P.div_m[d] = f.m;
+    P.div_l[d] = f.l;
+  }
+  return P;
+}
 
 template <int dim, int degree>
 struct CellShape {
@@ -271,7 +285,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
   number* outs = vals + P.nrows_in * S::threads;
   __shared__ int sflags;
   // integer contractions: enabled by the launch's tables, and only with the shared memory for them
-  constexpr bool FXC = cell_fx_capable<dim, degree, number>() && MODE != MODE_DIAG;
+  constexpr bool FXC = cell_fx_capable<dim, degree, number>();
   long long* vals_fx = reinterpret_cast<long long*>(outs + P.nrows_out * S::threads);
   int* ex_in = reinterpret_cast<int*>(vals_fx + P.nrows_in * S::threads);
   int* ex_out = ex_in + P.nrows_in * cpb;
@@ -289,10 +303,6 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
     fx_on = fx_ok && P.fx_deriv != 0;
     if constexpr (FXINT) fx_int = fx_ok && P.fx_int != 0;
   }
-  // cell coordinates by multiply-high division (cell indices stay below 2^31: DoF indices are int)
-  pg::fx::FastDiv div0, div1;
-  div0.init((unsigned int)P.nc[0]);
-  div1.init((unsigned int)P.nc[1]);
 
   // stage the tables once per resident block
   {
@@ -317,12 +327,13 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
     long long node = 0;
     if (active) {
       const unsigned int cl = (unsigned int)cell;
-      const unsigned int q0 = div0.div(cl);
-      cx = (int)(cl - q0 * div0.d);
+      // (multiply-high division: cell indices stay below 2^31, DoF indices being int)
+      const unsigned int q0 = P.div(cl, 0);
+      cx = (int)(cl - q0 * (unsigned int)P.nc[0]);
       if (dim == 2) cy = (int)q0;
       if (dim > 2) {
-        const unsigned int q1 = div1.div(q0);
-        cy = (int)(q0 - q1 * div1.d);
+        const unsigned int q1 = P.div(q0, 1);
+        cy = (int)(q0 - q1 * (unsigned int)P.nc[1]);
         cz = (int)q1;
       }
       node = ((long long)(k * cz + qc) * P.nn[1] + (k * cy + qb)) * P.nn[0] + (k * cx + qa);
@@ -335,15 +346,14 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
     }
     __syncthreads();  // tables staged; previous tile finished with vals/outs/sflags
 
-    // gather (read_dof_values_plain, or read_dof_values for constrained src); in MODE_DIAG
-    // the SRC rows are written by the probe loop below
+    // gather (read_dof_values_plain, or read_dof_values for constrained src)
     {
       int row = 0;
 #pragma unroll
       for (int s = 0; s < pg::MAX_SLOTS; ++s) {
         if (s < P.nslots) {
           const SlotDesc& sd = P.slots[s];
-          if (!(MODE == MODE_DIAG && sd.is_src)) {
+          {
             const number* ptr = global_ptr(static_cast<const number*>(sd.ptr));
             for (int c = 0; c < sd.ncomp; ++c) {
               number v = number(0);
@@ -370,7 +380,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
       }
     }
 
-    if constexpr (MODE != MODE_DIAG) {
+    {
       if constexpr (FXC) {
         if (fx_on) {
           __syncthreads();  // block exponents of the value rows complete
@@ -473,69 +483,6 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
                 if (target >= 0) atomicAdd(static_cast<number*>(od.acc) + target, r);
               }
             }
-          }
-        }
-      }
-    } else {
-      // diagonal by unit probes: for each SRC slot (one per block field) and each cell node i
-#pragma unroll 1
-      for (int s = 0; s < P.nslots; ++s) {
-        const SlotDesc& sd = P.slots[s];
-        if (!sd.is_src) continue;
-        int row = 0;
-        for (int s2 = 0; s2 < s; ++s2) row += P.slots[s2].ncomp;
-        const int o = sd.out_index;
-        const OutDesc& od = P.outs[o];
-        const int row0 = tab->out_row0[o];
-        number mine[3] = {number(0), number(0), number(0)};
-#pragma unroll 1
-        for (int i = 0; i < nq; ++i) {
-          // submit zero to every SRC slot, identity at node i of this one
-          int rr = 0;
-          for (int s2 = 0; s2 < P.nslots; ++s2) {
-            if (P.slots[s2].is_src)
-              for (int c = 0; c < P.slots[s2].ncomp; ++c)
-                vals[(rr + c) * S::threads + t] = (s2 == s && q == i) ? number(1) : number(0);
-            rr += P.slots[s2].ncomp;
-          }
-          if (t == 0) sflags = 0;
-          for (int r = 0; r < P.nrows_out; ++r) outs[r * S::threads + t] = number(0);
-          __syncthreads();
-          pg::CellCtx<dim, degree, number> ctx;
-          ctx.tab = tab;
-          ctx.vals = vals;
-          ctx.outs = outs;
-          ctx.stride = S::threads;
-          ctx.lc = lc;
-          ctx.q = q;
-          ctx.cell[0] = cx;
-          ctx.cell[1] = cy;
-          ctx.cell[2] = cz;
-          ctx.err = P.err;
-          ctx.submitted = 0;
-          if (active) {
-            FieldContainer<dim, degree, number> fc(ctx);
-            const SimulationTimer timer = P.timer_dev ? *P.timer_dev : P.timer;
-            pde.compute_lhs(fc, timer, P.block_id);
-            if (ctx.submitted) atomicOr(&sflags, ctx.submitted);
-          }
-          __syncthreads();
-          const int flags = sflags;
-          if (active && q == i) {
-            const bool has_v = flags & (1 << (2 * o));
-            const bool has_g = flags & (2 << (2 * o));
-            for (int c = 0; c < sd.ncomp; ++c)
-              mine[c] = integrate_row<dim, degree, number>(tab, outs, row0 + c * (1 + dim), has_v, has_g, t, lc, q,
-                                                           qa, qb, qc);
-          }
-          __syncthreads();
-          (void)row;
-        }
-        if (active) {
-          for (int c = 0; c < sd.ncomp; ++c) {
-            const long long idx = node + c * P.N;
-            const int target = od.cmap ? od.cmap[idx] : (int)idx;
-            if (target >= 0) atomicAdd(static_cast<number*>(od.acc) + target, mine[c]);
           }
         }
       }

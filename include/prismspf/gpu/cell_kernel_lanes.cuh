@@ -85,6 +85,17 @@ struct CellLaneMinBlocks<PDE, threads, std::void_t<decltype(PDE::cell_lane_min_b
   static constexpr int value = PDE::cell_lane_min_blocks;
 };
 
+// ... of a launch with NC output components: with several, shared memory admits fewer blocks than the
+// register budget would (3 components on Q2 3-D: 104 KB, 2 blocks), and the registers they leave free
+// go to the callback (the 48^3 Q2 elasticity product: 296 us at 56 registers, spilling, 248 us at 87)
+template <class PDE, int dim, int degree, int NC>
+constexpr int lane_min_blocks() {
+  using S = LaneShape<dim, degree>;
+  constexpr int regs = CellLaneMinBlocks<PDE, S::threads>::value;
+  constexpr int smem = 232448 / (S::nq * LANE_CPT * 8 * (NC == 1 ? 1 : NC * (2 + dim)));
+  return NC == 1 || regs < smem ? regs : (smem > 0 ? smem : 1);
+}
+
 // The output components (bit c: c components in a block) an operator's lane kernels are compiled
 // for: `cell_lane_components`, by default 1 to 4
 template <class PDE, class = void>
@@ -712,7 +723,6 @@ cudaError_t launch_cell_kernel_lanes_f32_impl(const CellLaunch& P, const void* o
 // limits (the caller then takes the thread-block kernel)
 template <class PDE, int dim, int degree, int mode>
 cudaError_t launch_cell_kernel_lanes_impl(const CellLaunch& P, const void* obj, cudaStream_t s) {
-  constexpr int MINB = CellLaneMinBlocks<PDE, LaneShape<dim, degree>::threads>::value;
   LaneRows R;
   if (!P.tables_host || !lane_rows(P, dim, &R)) return cudaErrorNotSupported;
   const auto* tab = static_cast<const pg::CellTables<dim, degree, double>*>(P.tables_host);
@@ -726,13 +736,13 @@ cudaError_t launch_cell_kernel_lanes_impl(const CellLaunch& P, const void* obj, 
   if (lane_smem_bytes<dim, degree>(R.nv, R.ng, R.nout) > 232448) return cudaErrorNotSupported;
   constexpr unsigned int C = CellLaneComponents<PDE>::value;
   if constexpr (C & 2u)
-    if (R.nout == 1) return launch_lanes<PDE, dim, degree, mode, 1, MINB>(P, R, obj, s);
+    if (R.nout == 1) return launch_lanes<PDE, dim, degree, mode, 1, lane_min_blocks<PDE, dim, degree, 1>()>(P, R, obj, s);
   if constexpr (C & 4u)
-    if (R.nout == 2) return launch_lanes<PDE, dim, degree, mode, 2, MINB>(P, R, obj, s);
+    if (R.nout == 2) return launch_lanes<PDE, dim, degree, mode, 2, lane_min_blocks<PDE, dim, degree, 2>()>(P, R, obj, s);
   if constexpr (C & 8u)
-    if (R.nout == 3) return launch_lanes<PDE, dim, degree, mode, 3, MINB>(P, R, obj, s);
+    if (R.nout == 3) return launch_lanes<PDE, dim, degree, mode, 3, lane_min_blocks<PDE, dim, degree, 3>()>(P, R, obj, s);
   if constexpr (C & 16u)
-    if (R.nout == 4) return launch_lanes<PDE, dim, degree, mode, 4, MINB>(P, R, obj, s);
+    if (R.nout == 4) return launch_lanes<PDE, dim, degree, mode, 4, lane_min_blocks<PDE, dim, degree, 4>()>(P, R, obj, s);
   return cudaErrorNotSupported;
 }
 

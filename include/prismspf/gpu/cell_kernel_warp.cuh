@@ -162,9 +162,6 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
   const int qc = dim > 2 ? q / (n * n) : 0;
   const bool lane_ok = lane < W::lanes;
   const bool writer = q == 0 && lc < cpw;  // writes the cell's exponents
-  pg::fx::FastDiv div0, div1;
-  div0.init((unsigned int)P.nc[0]);
-  div1.init((unsigned int)P.nc[1]);
   const unsigned int nn0 = (unsigned int)P.nn[0], nn1 = (unsigned int)P.nn[1];
   const unsigned int N = (unsigned int)P.N;
   const unsigned int ncells = (unsigned int)P.ncells;
@@ -177,12 +174,12 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
     int cx = 0, cy = 0, cz = 0;
     unsigned int node = 0;
     if (active) {
-      const unsigned int q0 = div0.div(cell);
-      cx = (int)(cell - q0 * div0.d);
+      const unsigned int q0 = P.div(cell, 0);
+      cx = (int)(cell - q0 * (unsigned int)P.nc[0]);
       if (dim == 2) cy = (int)q0;
       if (dim > 2) {
-        const unsigned int q1 = div1.div(q0);
-        cy = (int)(q0 - q1 * div1.d);
+        const unsigned int q1 = P.div(q0, 1);
+        cy = (int)(q0 - q1 * (unsigned int)P.nc[1]);
         cz = (int)q1;
       }
       node = ((unsigned int)(k * cz + qc) * nn1 + (unsigned int)(k * cy + qb)) * nn0 + (unsigned int)(k * cx + qa);
@@ -204,7 +201,7 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
       for (int s = 0; s < pg::MAX_SLOTS; ++s) {
         if (s < P.nslots) {
           const SlotDesc& sd = P.slots[s];
-          const double* ptr = static_cast<const double*>(sd.ptr);
+          const double* ptr = global_ptr(static_cast<const double*>(sd.ptr));
           for (int c = 0; c < sd.ncomp; ++c) {
             double v = 0.0;
             if (active) {
@@ -349,7 +346,8 @@ cudaError_t launch_cell_kernel_warp_impl(const CellLaunch& P, const void* obj, s
   long long grid = (long long)sms * occ;
   if (grid > blocks_needed) grid = blocks_needed;
   if (grid < 1) grid = 1;
-  return launch_chained(kern, dim3((unsigned)grid), dim3(W::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj));
+  return launch_chained(kern, dim3((unsigned)grid), dim3(W::threads), smem, s, with_divisors(P),
+                        *reinterpret_cast<const PDE*>(obj));
 }
 
 }  // namespace ppf

@@ -86,6 +86,22 @@ PPF_FX unsigned long long mulhi64(unsigned long long a, unsigned long long b) {
 #endif
 }
 
+// 0.5 v and a + b for a == b, exact, by the exponent field where the operands are normal numbers away
+// from the ends of the range: a few integer instructions, where each would occupy GB300's FP64 pipe
+// for as long as sixty of them
+PPF_FX double half_of(double v) {
+  const unsigned long long b = bits_of(v);
+  const unsigned int e = (unsigned int)(b >> 52) & 0x7ffu;
+  return e - 2u < 2045u ? double_of(b - (1ull << 52)) : 0.5 * v;
+}
+PPF_FX float half_of(float v) { return 0.5f * v; }
+PPF_FX double sum_of_equals(double a, double b) {
+  const unsigned long long x = bits_of(a);
+  const unsigned int e = (unsigned int)(x >> 52) & 0x7ffu;
+  return x == bits_of(b) && e - 1u < 2045u ? double_of(x + (1ull << 52)) : a + b;
+}
+PPF_FX float sum_of_equals(float a, float b) { return a + b; }
+
 // biased exponent of v (0 for zeros and subnormals, 2047 for infinities and NaNs)
 PPF_FX int exponent(double v) { return (int)((bits_of(v) >> 52) & 0x7ff); }
 

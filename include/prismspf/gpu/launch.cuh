@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include <prismspf/gpu/amr_cell_kernel.cuh>
+#include <prismspf/gpu/cell_diagonal.cuh>
 #include <prismspf/gpu/cell_kernel.cuh>
 #include <prismspf/gpu/cell_kernel_lanes.cuh>
 #include <prismspf/gpu/cell_kernel_warp.cuh>
@@ -50,7 +51,8 @@ cudaError_t launch_cell_kernel_impl(const CellLaunch& P, const void* obj, size_t
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, P, *reinterpret_cast<const PDE*>(obj));
+  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, with_divisors(P),
+                        *reinterpret_cast<const PDE*>(obj));
 }
 
 // An operator may run its FP64 Q1/Q2 left-hand side on the warp-resident kernel
@@ -88,6 +90,9 @@ inline bool use_warp_cell_kernel() {
 // for it (contraction modes 2 and 3 of FP64 Q1/Q2 operators)
 template <class PDE, int dim, int degree, int mode, typename number>
 cudaError_t launch_cell_kernel(const CellLaunch& P, const void* obj, size_t smem, cudaStream_t s) {
+  if constexpr (mode == MODE_DIAG) {
+    return launch_cell_diagonal<PDE, dim, degree, number>(P, obj, s);
+  } else {
   if constexpr (std::is_same<number, float>::value && degree <= 2 && mode == MODE_LHS) {
     // FP32 left-hand sides (mixed-precision smoothing levels) on the lane layout when asked
     if (P.fx_lanes) {
@@ -95,7 +100,7 @@ cudaError_t launch_cell_kernel(const CellLaunch& P, const void* obj, size_t smem
       if (e != cudaErrorNotSupported) return e;
     }
   }
-  if constexpr (cell_fx_capable<dim, degree, number>() && mode != MODE_DIAG) {
+  if constexpr (cell_fx_capable<dim, degree, number>()) {
     if (P.fx_lanes) {
       // the lane kernel when its rows and tile fit (and the host tables came with the launch),
       // else integer derivatives on the thread-block tiles
@@ -110,6 +115,7 @@ cudaError_t launch_cell_kernel(const CellLaunch& P, const void* obj, size_t smem
     if (P.fx_int) return launch_cell_kernel_impl<PDE, dim, degree, mode, number, true>(P, obj, smem, s);
   }
   return launch_cell_kernel_impl<PDE, dim, degree, mode, number, false>(P, obj, smem, s);
+  }
 }
 
 // The adaptive-mesh kernel for a mode without the MODE_AMR flag; `rec` is an AmrCellLaunch.

@@ -5,6 +5,7 @@
 
 #include <prismspf/config.h>
 #include <prismspf/dealii_shim.h>
+#include <prismspf/gpu/fixed_point.cuh>
 
 #include <type_traits>
 
@@ -37,6 +38,12 @@ PPF_HD bool stiffness_zero(const C& c) {
   if constexpr (std::is_arithmetic<C>::value) return zero_bits(c);
   else return zero_bits(c.v);
 }
+// a + b of a symmetric pair of entries, usually the same value twice
+template <typename T>
+PPF_HD T pair_sum(const T& a, const T& b) {
+  if constexpr (std::is_same<T, dealii::VectorizedArray<double>>::value) return T(gpu::fx::sum_of_equals(a.v, b.v));
+  else return a + b;
+}
 // whether a Voigt stiffness couples normal and shear strains nowhere and each shear strain only
 // to its own stress (orthotropic axes along the mesh: cubic and isotropic materials included)
 template <int nv, typename C>
@@ -62,16 +69,21 @@ PPF_HD void compute_stress(const dealii::Tensor<2, voigt_tensor_size<dim>, C>& e
   constexpr int nv = voigt_tensor_size<dim>;
   constexpr int nn = nv == 6 ? 3 : (nv == 3 ? 2 : 1);
   if (detail::orthotropic<nv, C>(elasticity_tensor)) {
+#pragma unroll
     for (int i = 0; i < nn; ++i) {
       T s = elasticity_tensor[i][0] * strain[0];
+#pragma unroll
       for (int j = 1; j < nn; ++j) s = s + elasticity_tensor[i][j] * strain[j];
       stress[i] = s;
     }
+#pragma unroll
     for (int i = nn; i < nv; ++i) stress[i] = elasticity_tensor[i][i] * strain[i];
     return;
   }
+#pragma unroll
   for (int i = 0; i < nv; ++i) {
     T s = elasticity_tensor[i][0] * strain[0];
+#pragma unroll
     for (int j = 1; j < nv; ++j) s = s + elasticity_tensor[i][j] * strain[j];
     stress[i] = s;
   }
@@ -87,9 +99,9 @@ PPF_HD void compute_stress(const dealii::Tensor<2, voigt_tensor_size<dim>, C>& e
     eps[0] = strain[0][0];
     eps[1] = strain[1][1];
     eps[2] = strain[2][2];
-    eps[3] = strain[1][2] + strain[2][1];
-    eps[4] = strain[0][2] + strain[2][0];
-    eps[5] = strain[0][1] + strain[1][0];
+    eps[3] = detail::pair_sum(strain[1][2], strain[2][1]);
+    eps[4] = detail::pair_sum(strain[0][2], strain[2][0]);
+    eps[5] = detail::pair_sum(strain[0][1], strain[1][0]);
     compute_stress<dim, T, C>(elasticity_tensor, eps, sig);
     stress[0][0] = sig[0];
     stress[1][1] = sig[1];
@@ -103,7 +115,7 @@ PPF_HD void compute_stress(const dealii::Tensor<2, voigt_tensor_size<dim>, C>& e
   } else if constexpr (dim == 2) {
     eps[0] = strain[0][0];
     eps[1] = strain[1][1];
-    eps[2] = strain[0][1] + strain[1][0];
+    eps[2] = detail::pair_sum(strain[0][1], strain[1][0]);
     compute_stress<dim, T, C>(elasticity_tensor, eps, sig);
     stress[0][0] = sig[0];
     stress[1][1] = sig[1];

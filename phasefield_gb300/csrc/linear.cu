@@ -96,15 +96,16 @@ __global__ void __launch_bounds__(256) dot_kernel(long long n, const T* x, const
 }
 
 // The kernels below read a product's accumulator and clear the level's other one (`clear`) for the
-// next product. (Clearing the same accumulator in place needs no second one, but storing to the rows
+// next product. The scatter adds nothing to constrained rows (images are condensed onto their
+// masters, Dirichlet rows dropped), so a product's constrained rows are zero without a look-up in the
+// constraint map. (Clearing the same accumulator in place needs no second one, but storing to the rows
 // the cells' atomic adds have just left took five times as long: 73 instead of 13 us on 48^3 Q2
 // vectors.)
 
-// dst = scale (.) acc on free rows, zero on constrained rows (per node scale, component blocks);
-// with `out` also out = w.dst
+// dst = scale (.) acc (per node scale, component blocks); with `out` also out = w.dst
 template <typename T>
 __global__ void __launch_bounds__(256) level_finalize_kernel(T* dst, const T* acc, T* clear, const T* __restrict__ scale,
-                                                             const int* __restrict__ cmap, long long N, const T* w,
+                                                             long long N, const T* w,
                                                              double* partial, unsigned int* counter, double* out) {
   chain_release();
   chain_wait();
@@ -112,8 +113,7 @@ __global__ void __launch_bounds__(256) level_finalize_kernel(T* dst, const T* ac
   double sum = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
-    const bool free_row = !cmap || cmap[gi] == (int)gi;
-    const T v = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    const T v = scale ? acc[gi] * scale[i] : acc[gi];
     if (clear) clear[gi] = T(0);
     dst[gi] = v;
     if (out) sum += double(w[gi]) * double(v);
@@ -150,6 +150,8 @@ struct Transfer {
   int periodic[3];
   int dim;
   long long Nout, Nin;
+  pg::fx::FastDiv fd[2];  // multiply-high divisors of nout[0] and nout[1]
+  __device__ __forceinline__ unsigned div(unsigned v, int d) const { return fd[d].div(v); }
 };
 
 // the tensor product of one CSR row per axis applied to `in` (FP entries of type Ti)
@@ -173,10 +175,112 @@ __device__ __forceinline__ T transfer_row(const Transfer<T>& A, const Ti* in, in
   return s2;
 }
 
+// Degrees 1 and 2, whose nodes nest, in closed form. A fine row of an axis is its coarse node, or
+// Q1 {1/2, 1/2}, Q2 {3/8, 3/4, -1/8} and its mirror image on the coarse cell's nodes; a coarse row
+// of the transpose Q1 {1/2, 1, 1/2}, Q2 {3/4, 1, 3/4} at a cell's middle node and
+// {-1/8, 0, 3/8, 1, 3/8, 0, -1/8} at a vertex, on the fine nodes around it.
+struct FineTaps {
+  int c0, n;  // first coarse node and number of taps
+  float w[3];
+};
+template <int degree>
+__device__ __forceinline__ FineTaps fine_taps(int i) {
+  FineTaps t;
+  t.n = 1;
+  t.w[0] = 1.f;
+  t.w[1] = t.w[2] = 0.f;
+  t.c0 = i >> 1;
+  if constexpr (degree == 1) {
+    if (i & 1) {
+      t.n = 2;
+      t.w[0] = t.w[1] = 0.5f;
+    }
+  } else {
+    if (i & 1) {
+      const bool first = (i & 3) == 1;
+      t.n = 3;
+      t.c0 = (i >> 2) * 2;
+      t.w[0] = first ? 0.375f : -0.125f;
+      t.w[1] = 0.75f;
+      t.w[2] = first ? -0.125f : 0.375f;
+    }
+  }
+  return t;
+}
+// weight of fine node 2 i + o in coarse row i (o from -3 to 3)
+template <int degree>
+__device__ __forceinline__ float coarse_weight(int i, int o) {
+  const int a = o < 0 ? -o : o;
+  if (a == 0) return 1.f;
+  if (degree == 1) return a == 1 ? 0.5f : 0.f;
+  if (i & 1) return a == 1 ? 0.75f : 0.f;
+  return a == 1 ? 0.375f : (a == 3 ? -0.125f : 0.f);
+}
+
+// the row (i0, i1, i2) of the prolongation applied to e
+template <typename T, typename Tc, int degree>
+__device__ __forceinline__ T prolong_row(const Transfer<T>& A, const Tc* e, int i0, int i1, int i2) {
+  if constexpr (degree > 2) {
+    return transfer_row<T, Tc>(A, e, i0, i1, i2);
+  } else {
+    const FineTaps t0 = fine_taps<degree>(i0), t1 = fine_taps<degree>(i1), t2 = fine_taps<degree>(i2);
+    T s2 = T(0);
+    for (int k2 = 0; k2 < t2.n; ++k2) {
+      T s1 = T(0);
+      for (int k1 = 0; k1 < t1.n; ++k1) {
+        const Tc* row = e + ((long long)(t2.c0 + k2) * A.nin[1] + (t1.c0 + k1)) * A.nin[0] + t0.c0;
+        T s0 = T(t0.w[0]) * T(row[0]);
+        if (t0.n > 1) s0 += T(t0.w[1]) * T(row[1]);
+        if (t0.n > 2) s0 += T(t0.w[2]) * T(row[2]);
+        s1 += T(k1 == 0 ? t1.w[0] : (k1 == 1 ? t1.w[1] : t1.w[2])) * s0;
+      }
+      s2 += T(k2 == 0 ? t2.w[0] : (k2 == 1 ? t2.w[1] : t2.w[2])) * s1;
+    }
+    return s2;
+  }
+}
+
+// the coarse row (i0, i1, i2) of the restriction applied to r
+template <typename T, int degree>
+__device__ __forceinline__ T restrict_row(const Transfer<T>& A, const T* r, int i0, int i1, int i2) {
+  if constexpr (degree > 2) {
+    return transfer_row<T, T>(A, r, i0, i1, i2);
+  } else {
+    constexpr int H = degree == 1 ? 1 : 3;
+    const int h0 = degree == 2 && (i0 & 1) ? 1 : H, h1 = degree == 2 && (i1 & 1) ? 1 : H;
+    const int h2 = A.dim < 3 ? 0 : (degree == 2 && (i2 & 1) ? 1 : H);
+    T s2 = T(0);
+    for (int o2 = -h2; o2 <= h2; ++o2) {
+      const T w2 = T(coarse_weight<degree>(i2, o2));
+      const int f2 = 2 * i2 + o2;
+      if (w2 == T(0) || f2 < 0 || f2 >= A.nin[2]) continue;
+      T s1 = T(0);
+      for (int o1 = -h1; o1 <= h1; ++o1) {
+        const T w1 = T(coarse_weight<degree>(i1, o1));
+        const int f1 = 2 * i1 + o1;
+        if (w1 == T(0) || f1 < 0 || f1 >= A.nin[1]) continue;
+        const T* row = r + ((long long)f2 * A.nin[1] + f1) * A.nin[0] + 2 * i0;
+        T s0 = row[0];
+        const T e1 = T(coarse_weight<degree>(i0, 1));
+        if (i0 > 0) s0 += e1 * row[-1];
+        if (2 * i0 + 1 < A.nin[0]) s0 += e1 * row[1];
+        if (h0 == 3) {
+          const T e3 = T(coarse_weight<degree>(i0, 3));
+          if (i0 > 1) s0 += e3 * row[-3];
+          if (2 * i0 + 3 < A.nin[0]) s0 += e3 * row[3];
+        }
+        s1 += w1 * s0;
+      }
+      s2 += w2 * s1;
+    }
+    return s2;
+  }
+}
+
 // x += P e from the coarse correction e (type Tc): all axes in one pass (at most 27 entries a row,
-// 8 on average for Q2 3-D, read from L1/L2, instead of dim passes over fine-sized work vectors);
-// images take their master's row, Dirichlet rows nothing
-template <typename T, typename Tc>
+// 8 on average for Q2 3-D, read from L1/L2), where one launch per component and axis went through
+// fine-sized work vectors; images take their master's row, Dirichlet rows nothing
+template <typename T, typename Tc, int degree>
 __global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_constant__ Transfer<T> A, T* x, const Tc* e,
                                                              const int* __restrict__ cmap) {
   chain_release();
@@ -186,17 +290,17 @@ __global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_consta
     const int m = cmap ? cmap[base + i] : (int)(base + i);
     if (m < 0) continue;
     const unsigned node = (unsigned)(m - base);
-    const unsigned r = node / (unsigned)A.nout[0];
+    const unsigned r = A.div(node, 0);
     const int i0 = (int)(node - r * (unsigned)A.nout[0]);
-    const int i2 = (int)(r / (unsigned)A.nout[1]);
+    const int i2 = (int)A.div(r, 1);
     const int i1 = (int)(r - (unsigned)i2 * (unsigned)A.nout[1]);
-    x[base + i] += transfer_row<T, Tc>(A, e + blockIdx.y * A.Nin, i0, i1, i2);
+    x[base + i] += prolong_row<T, Tc, degree>(A, e + blockIdx.y * A.Nin, i0, i1, i2);
   }
 }
 
 // b = P^T r on the coarse level (stored as Tc): all axes in one pass; a periodic node sums its
 // images' rows as well, constrained rows are zero
-template <typename T, typename Tc>
+template <typename T, typename Tc, int degree>
 __global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ Transfer<T> A, Tc* b, const T* r,
                                                        const int* __restrict__ cmap) {
   chain_release();
@@ -206,16 +310,16 @@ __global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ T
     T s = T(0);
     if (!cmap || cmap[base + i] == (int)(base + i)) {
       const unsigned node = (unsigned)i;
-      const unsigned q = node / (unsigned)A.nout[0];
+      const unsigned q = A.div(node, 0);
       const int i0 = (int)(node - q * (unsigned)A.nout[0]);
-      const int i2 = (int)(q / (unsigned)A.nout[1]);
+      const int i2 = (int)A.div(q, 1);
       const int i1 = (int)(q - (unsigned)i2 * (unsigned)A.nout[1]);
       const int m0 = A.periodic[0] && i0 == 0, m1 = A.periodic[1] && i1 == 0, m2 = A.periodic[2] && i2 == 0;
       for (int e2 = 0; e2 <= m2; ++e2)
         for (int e1 = 0; e1 <= m1; ++e1)
           for (int e0 = 0; e0 <= m0; ++e0)
-            s += transfer_row<T, T>(A, r + blockIdx.y * A.Nin, e0 ? A.nout[0] - 1 : i0, e1 ? A.nout[1] - 1 : i1,
-                                    e2 ? A.nout[2] - 1 : i2);
+            s += restrict_row<T, degree>(A, r + blockIdx.y * A.Nin, e0 ? A.nout[0] - 1 : i0, e1 ? A.nout[1] - 1 : i1,
+                                         e2 ? A.nout[2] - 1 : i2);
     }
     b[base + i] = Tc(s);
   }
@@ -234,21 +338,19 @@ __global__ void __launch_bounds__(256) cheb_start_kernel(long long n, T* x, T* u
   }
 }
 
-// A Chebyshev step from the raw product: Ax = scale (.) acc on free rows; u = c1 u + c2 P (b - Ax);
+// A Chebyshev step from the raw product: Ax = scale (.) acc; u = c1 u + c2 P (b - Ax);
 // x += u (one pass instead of a memset, a finalize and an update launch with Ax in between: 20 % of
 // the mixed-precision iterations' kernel time)
 template <typename T>
 __global__ void __launch_bounds__(256) cheb_step_kernel(T* x, T* u, const T* b, const T* acc, T* clear,
-                                                        const T* __restrict__ scale,
-                                                        const int* __restrict__ cmap, const T* pinv, double c1,
+                                                        const T* __restrict__ scale, const T* pinv, double c1,
                                                         double c2, long long N) {
   chain_release();
   chain_wait();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
-    const bool free_row = !cmap || cmap[gi] == (int)gi;
-    const T Ax = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    const T Ax = scale ? acc[gi] * scale[i] : acc[gi];
     clear[gi] = T(0);
     const T r = b[gi] - Ax;
     const T ui = c1 == 0.0 ? T(c2) * pinv[gi] * r : T(c1) * u[gi] + T(c2) * pinv[gi] * r;
@@ -257,18 +359,16 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(T* x, T* u, const T* b, 
   }
 }
 
-// r = b - scale (.) acc (constrained rows: b)
+// r = b - scale (.) acc
 template <typename T>
 __global__ void __launch_bounds__(256) residual_kernel(T* r, const T* b, const T* acc, T* clear,
-                                                       const T* __restrict__ scale,
-                                                       const int* __restrict__ cmap, long long N) {
+                                                       const T* __restrict__ scale, long long N) {
   chain_release();
   chain_wait();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
-    const bool free_row = !cmap || cmap[gi] == (int)gi;
-    const T Ax = free_row ? (scale ? acc[gi] * scale[i] : acc[gi]) : T(0);
+    const T Ax = scale ? acc[gi] * scale[i] : acc[gi];
     clear[gi] = T(0);
     r[gi] = b[gi] - Ax;
   }
@@ -694,7 +794,7 @@ static int level_apply(ppf_handle h, BlockState& B, MGLevel& lv, const T* src, T
   dim3 grid = level_grid(h, B, lv);
   if (out) grid.x = std::min(grid.x, 1024u / grid.y);
   PPF_CUDA(h, launch_chained(level_finalize_kernel<T>, grid, dim3(256), 0, h->stream, dst, (const T*)lv.acc, (T*)lv.acc2,
-                             level_scale<T>(B.lin, lv), level_map(lv), lv.N, src, B.lin.partial, counters(B.lin), out));
+                             level_scale<T>(B.lin, lv), lv.N, src, B.lin.partial, counters(B.lin), out));
   std::swap(lv.acc, lv.acc2);
   h->all_launches++;
   return PPF_OK;
@@ -836,7 +936,7 @@ static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start, 
       int rc = level_cell_launch(h, B, lv, MODE_LHS, x, false);
       if (rc) return rc;
       PPF_CUDA(h, launch_chained(cheb_step_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, x, u, b,
-                                 (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), level_map(lv),
+                                 (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv),
                                  (const T*)lv.inv_diag, c1, c2, lv.N));
       std::swap(lv.acc, lv.acc2);
     }
@@ -863,6 +963,7 @@ static Transfer<T> transfer(ppf_handle h, const MGLevel& c, const MGLevel& f, bo
   }
   A.Nout = out.N;
   A.Nin = in.N;
+  for (int d = 0; d < 2; ++d) A.fd[d].init((unsigned)out.nn[d]);
   return A;
 }
 
@@ -880,14 +981,17 @@ static int vcycle_level(ppf_handle h, BlockState& B, int l, const T* b, T* x) {
   rc = level_cell_launch(h, B, lv, MODE_LHS, x, false);
   if (rc) return rc;
   PPF_CUDA(h, launch_chained(residual_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.r, b,
-                             (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), level_map(lv), lv.N));
+                             (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), lv.N));
   std::swap(lv.acc, lv.acc2);
-  PPF_CUDA(h, launch_chained(restrict_kernel<T, Tc>, level_grid(h, B, cl), dim3(256), 0, h->stream,
+  auto restriction = h->k == 1 ? restrict_kernel<T, Tc, 1> : (h->k == 2 ? restrict_kernel<T, Tc, 2> : restrict_kernel<T, Tc, 3>);
+  PPF_CUDA(h, launch_chained(restriction, level_grid(h, B, cl), dim3(256), 0, h->stream,
                              transfer<T>(h, cl, lv, false), (Tc*)cl.b, (const T*)lv.r, level_map(cl)));
   h->all_launches += 2;
   rc = vcycle(h, B, l - 1, cl.b, cl.x);
   if (rc) return rc;
-  PPF_CUDA(h, launch_chained(prolongate_add_kernel<T, Tc>, level_grid(h, B, lv), dim3(256), 0, h->stream,
+  auto prolongation = h->k == 1 ? prolongate_add_kernel<T, Tc, 1>
+                                : (h->k == 2 ? prolongate_add_kernel<T, Tc, 2> : prolongate_add_kernel<T, Tc, 3>);
+  PPF_CUDA(h, launch_chained(prolongation, level_grid(h, B, lv), dim3(256), 0, h->stream,
                              transfer<T>(h, cl, lv, true), x, (const Tc*)cl.x, level_map(lv)));
   h->all_launches++;
   return chebyshev<T>(h, B, lv, false, b, x);
@@ -1241,7 +1345,7 @@ int linear_solve(ppf_handle h, int b) {
     if (out) grid.x = std::min(grid.x, 1024u / grid.y);
     if (const int rc = ensure_acc2(h, F)) return rc;
     PPF_CUDA(h, launch_chained(level_finalize_kernel<double>, grid, dim3(256), 0, h->stream, dst, (const double*)F.acc,
-                               F.acc2, scaled(L) ? h->d_invm_sqrt : nullptr, F.constrained ? F.cmap : nullptr, h->N, w,
+                               F.acc2, scaled(L) ? h->d_invm_sqrt : nullptr, h->N, w,
                                L.partial, counters(L), out));
     h->all_launches++;
     std::swap(F.acc, F.acc2);

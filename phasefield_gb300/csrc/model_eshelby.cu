@@ -25,6 +25,7 @@ size_t make_dim(const double* c, int nc, void* out, size_t cap, std::string* err
   }
   for (int i = 0; i < o.n_incl; ++i)
     for (int k = 0; k < 4; ++k) o.incl[i][k] = number(c[39 + 4 * i + k]);
+  o.set_reach();
   if (sizeof(o) > cap) return 0;
   std::memcpy(out, &o, sizeof(o));
   return sizeof(o);

@@ -308,6 +308,7 @@ static std::vector<unsigned char> tables_impl_f32(const double* lo, const double
   std::memcpy(t.slot_comp0, a.slot_comp0, sizeof(t.slot_comp0));
   std::memcpy(t.out_of, a.out_of, sizeof(t.out_of));
   std::memcpy(t.out_row0, a.out_row0, sizeof(t.out_row0));
+  std::memcpy(t.lane_out, a.lane_out, sizeof(t.lane_out));
   std::vector<unsigned char> out(sizeof(T32));
   std::memcpy(out.data(), &t, sizeof(T32));
   return out;
@@ -446,18 +447,17 @@ __global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const
 
 // dst = scale (.) acc on unconstrained rows, 0 on constrained rows (MFOperator::compute_operator
 // leaves constrained rows of dst untouched after zeroing, then scales); `clear`, the field's other
-// accumulator, is zeroed for the next product.
+// accumulator, is zeroed for the next product. The scatter adds nothing to constrained rows (images
+// are condensed onto their masters, Dirichlet rows dropped), so they need no look-up: 0 scales to 0.
 __global__ void finalize_apply_kernel(double* dst, const double* acc, double* clear, const double* __restrict__ scale,
-                                      const int* __restrict__ cmap, long long N) {
+                                      long long N) {
   chain_release();
   chain_wait();
   const int c = blockIdx.y;
   const long long base = c * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
-    const int cm = cmap ? cmap[gi] : (int)gi;
-    double v = 0.0;
-    if (cm == (int)gi) v = scale ? acc[gi] * scale[i] : acc[gi];
+    const double v = scale ? acc[gi] * scale[i] : acc[gi];
     if (clear) clear[gi] = 0.0;
     dst[gi] = v;
   }
@@ -1776,7 +1776,7 @@ int ppf_apply_device(ppf_handle h, int b, int which, const double* d_src, double
     const double* sc = scale == 1 ? h->d_invm : (scale == 2 ? h->d_invm_sqrt : nullptr);
     dim3 grid(grid_for(h->N), F.ncomp);
     PPF_CUDA(h, launch_chained(finalize_apply_kernel, grid, dim3(256), 0, h->stream, d_dst + off, (const double*)F.acc,
-                               alternate ? F.acc2 : nullptr, sc, F.constrained ? F.cmap : nullptr, h->N));
+                               alternate ? F.acc2 : nullptr, sc, h->N));
     h->all_launches++;
     if (alternate) {
       std::swap(F.acc, F.acc2);
