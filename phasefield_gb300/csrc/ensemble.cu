@@ -10,13 +10,19 @@
 //     third one (read one step earlier, so no block of this launch touches it). The three
 //     accumulators rotate; a launch depends only on the previous launch having finished.
 //   * one persistent launch for every instance and both degrees: a global list of cell tiles
-//     (instance, first cell) is walked grid-stride; a tile of a Q1 instance runs the Q1 body,
-//     of a Q2 instance the Q2 body (block-uniform branch), with the instance's parameters
-//     (m_well, kappa) and its cell tables, built once on the host with the engine's table
-//     builder for the instance's mesh spacing, copied into shared memory per tile (an integer
-//     copy: GB300's FP64 pipe is too narrow to recompute them per tile).
-//   * tile shapes (cells per tile for Q1 and for Q2) and the grid size are chosen by a
-//     project-written autotuner that times candidate shapes on the ensemble itself.
+//     (instance, first cell), the Q1 instances' first, of which each block takes a contiguous share of
+//     either degree, with the instance's parameters (m_well, kappa) and its cell tables, built once
+//     on the host with the engine's table builder for the instance's mesh spacing and copied into
+//     shared memory where a block's share moves on to another instance;
+//   * a tile is 32 cells on the lane kernel's layout and arithmetic (prismspf/gpu/cell_kernel_lanes.cuh:
+//     a lane a cell, every contraction in exact 64-bit integers, the terms in registers), n warps a
+//     tile and several tiles a block, so both degrees fill the same block of threads;
+//   * the warps of a block and the grid size are chosen by a project-written autotuner that times
+//     candidates on the ensemble itself.
+// FP64 contractions (PPF_FP64_CONTRACTIONS=1) run on one thread per point, tiles of up to 64 cells.
+// Bound by instruction issue and the callback's FP64 operations (9 a point). 48 instances of 32 to
+// 256 cells a side: 174 us a step (8 blocks of 6 warps an SM at 40 registers; 203 us with 2 blocks of
+// 18 warps at 56), against 273 us on one thread per point with the tables copied for each tile.
 // Natural boundary conditions (the ensemble workload has no constraints).
 #include <algorithm>
 #include <cmath>
@@ -56,7 +62,7 @@ struct EnsLaunch {
   long long total_len;
   double dt;
   const unsigned char* tables;  // per-instance CellTables<2, degree, double>
-  int fx;                       // integer derivatives (the tables enable them for Q1/Q2)
+  long long ntiles1;            // tiles of Q1 instances (the first of the list)
 };
 
 template <int degree, int CPB>
@@ -66,15 +72,7 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
   Tab* tab = reinterpret_cast<Tab*>(smem);
   double* vals = smem + (sizeof(Tab) + 7) / 8;
   double* outs = vals + CPB * nq;
-  long long* vals_fx = reinterpret_cast<long long*>(outs + 3 * CPB * nq);  // integer derivatives
-  int* ex_in = reinterpret_cast<int*>(vals_fx + CPB * nq);                 // per-cell block exponent
-  int* ex_out = ex_in + CPB;                                               // of the submitted terms
   const int t = threadIdx.x;
-  // last read before the previous tile's closing barrier
-  if (P.fx && t < CPB) {
-    ex_in[t] = 0;
-    ex_out[t] = 0;
-  }
   // stage the instance's tables (built on the host for its mesh spacing)
   {
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables + I.tab_off);
@@ -98,19 +96,10 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
     // gather: n = invM (.) acc of the previous step
     const double v = P.invm[I.off + node] * P.acc_in[I.off + node];
     vals[lc * nq + q] = v;
-    if (P.fx) atomicMax(&ex_in[lc], pg::fx::exponent(v));
   }
   if (in_tile)
     for (int r = 0; r < 3; ++r) outs[r * CPB * nq + lc * nq + q] = 0.0;
   __syncthreads();
-  if (P.fx) {
-    // fixed-point copy of the nodal values for exact integer derivatives (fixed_point.cuh)
-    if (active) {
-      const int E = ex_in[lc];
-      if (E != pg::fx::EXP_NONFINITE) vals_fx[lc * nq + q] = pg::fx::to_fixed(vals[lc * nq + q], E, pg::fx::TOP_VALUES);
-    }
-    __syncthreads();
-  }
   pg::CellCtx<2, degree, double> ctx;
   ctx.tab = tab;
   ctx.vals = vals;
@@ -123,64 +112,12 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
   ctx.cell[2] = 0;
   ctx.err = nullptr;
   ctx.submitted = 0;
-  // integer integration of the value and gradient terms where the tables allow it (square cells):
-  // the lane kernel's arithmetic (prismspf/gpu/cell_kernel_lanes.cuh) on this layout
-  const bool fxi = P.fx && tab->fx_cubic;
-  if (P.fx) {
-    ctx.vals_fx = vals_fx;
-    ctx.ex_in = ex_in;
-    ctx.cpb = CPB;
-    ctx.raw_values = fxi ? 1 : 0;
-  }
   if (active) {
     AllenCahn<2, degree, double> pde{I.m_well, I.kappa};
     FieldContainer<2, degree, double> fc(ctx);
     pde.compute_rhs(fc, SimulationTimer(P.dt, 0.0), 1u);
   }
   __syncthreads();
-  if (fxi) {
-    namespace fx = pg::fx;
-    constexpr int TOPT = LANE_TOP_TERMS;
-    const int S = CPB * nq;
-    const int p = lc * nq + q;
-    if (active) {
-      // block exponent of the cell's terms: the value term as h v, the two gradient terms
-      const int ev = fx::exponent(outs[p]);
-      const int eh = ev + tab->hk + (tab->hpow2 ? 0 : 1);
-      int e = ev == 0 ? 0 : (ev == fx::EXP_NONFINITE || eh >= fx::EXP_NONFINITE ? fx::EXP_NONFINITE : max(eh, 0));
-      e = max(e, fx::exponent(outs[S + p]));
-      e = max(e, fx::exponent(outs[2 * S + p]));
-      atomicMax(&ex_out[lc], e);
-    }
-    __syncthreads();
-    long long* ox = reinterpret_cast<long long*>(outs);
-    if (active) {
-      const int E = ex_out[lc];
-      const double v = outs[p];
-      ox[p] = tab->hpow2 ? fx::to_fixed_fast<TOPT>(v, E - tab->hk) : fx::to_fixed_scaled<TOPT>(v, E, tab->hsig, tab->hk);
-      ox[S + p] = fx::to_fixed_fast<TOPT>(outs[S + p], E);
-      ox[2 * S + p] = fx::to_fixed_fast<TOPT>(outs[2 * S + p], E);
-    }
-    __syncthreads();
-    if (active) {
-      const int E = ex_out[lc];
-      long long T = (long long)((unsigned long long)ox[p] << tab->vw_sh[q]);
-      {
-        const long long* g = ox + S + lc * nq + (q - qa);
-        const long long L = lane_line_integral<n>(qa, g[0], g[1], n > 2 ? g[2] : 0ll);
-        T += (long long)((unsigned long long)L << tab->wo_sh[0][q]);
-      }
-      {
-        const long long* g = ox + 2 * S + lc * nq + (q - qb * n);
-        const long long L = lane_line_integral<n>(qb, g[0], g[n], n > 2 ? g[2 * n] : 0ll);
-        T += (long long)((unsigned long long)L << tab->wo_sh[1][q]);
-      }
-      const double rr = fx::to_double_fast(T, E - 1023 - TOPT + tab->ik[0], tab->isig[0], true);
-      atomicAdd(P.acc_out + I.off + node, E == fx::EXP_NONFINITE ? fx::quiet_nan() : rr);
-    }
-    __syncthreads();
-    return;
-  }
   if (active) {
     double r = outs[lc * nq + q];
     {
@@ -200,6 +137,185 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
   __syncthreads();
 }
 
+// The lane layout. Shared memory of one tile: its instance's tables, the nodal values (double and
+// fixed-point), the gradient terms of the first direction, then the block exponents (two buffers of
+// one value row and one component).
+template <int degree>
+constexpr size_t ens_lane_tile_bytes() {
+  constexpr int nq = LaneShape<2, degree>::nq;
+  return (sizeof(pg::CellTables<2, degree, double>) + 15) / 16 * 16 + 8 * LANE_CPT * 3 * nq + 4 * LANE_CPT * 4;
+}
+
+// this block's tiles of one degree: WARPS / n tiles at a time, n warps each (cell_kernel_lanes with
+// one scalar row and one component)
+template <int degree, int WARPS>
+__device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long long tile0, long long ntiles) {
+  using S = LaneShape<2, degree>;
+  using Tab = pg::CellTables<2, degree, double>;
+  namespace fx = pg::fx;
+  constexpr int n = S::n, nq = S::nq, cols = S::cols, k = degree, CPT = LANE_CPT, per = WARPS / cols;
+  constexpr int ROW = nq * CPT, JS = cols * CPT;
+  constexpr int TOPT = n == 2 ? fx::LANE_TOP_INTEGRAL_Q1 : fx::LANE_TOP_INTEGRAL;
+  constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20, FLOOR_OUT = (fx::EXP_FLOOR + fx::EXP_BIAS) << 20;
+  const int lc = threadIdx.x & 31;
+  const int wi = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+  const int sub = wi / cols, w = wi - sub * cols;  // tile of the block's group, point of the first direction
+  unsigned char* base = smem + (size_t)sub * ens_lane_tile_bytes<degree>();
+  Tab* tab = reinterpret_cast<Tab*>(base);
+  double* vals = reinterpret_cast<double*>(base + (sizeof(Tab) + 15) / 16 * 16);
+  long long* vfx = reinterpret_cast<long long*>(vals + ROW);
+  long long* outs = vfx + ROW;
+  unsigned int* ex = reinterpret_cast<unsigned int*>(outs + ROW);  // [2][value row, component][cell]
+  const int p0 = w * CPT + lc;
+  const int step0 = w == k ? -CPT : CPT;
+  const long long steps = (ntiles + per - 1) / per;
+  const long long first = steps * blockIdx.x / gridDim.x, last = steps * (blockIdx.x + 1) / gridDim.x;
+  if (first == last) return;
+  for (int i = w * 32 + lc; i < 4 * CPT; i += cols * 32) ex[i] = (i / CPT) & 1 ? FLOOR_OUT : FLOOR;
+  __syncthreads();
+  int held = -1;  // the instance whose tables are in shared memory
+  int par = 0;
+  for (long long step = first; step < last; ++step, par ^= 1) {
+    // spare tiles of the last group redo the last tile and scatter nothing
+    const long long own = step * per + sub;
+    const long long tile = tile0 + (own < ntiles ? own : ntiles - 1);
+    const int inst = P.tile_inst[tile];
+    const EnsInstance& I = P.inst[inst];
+    if (inst != held) {  // (the tables were last read before the previous tile's last barrier)
+      const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables + I.tab_off);
+      unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
+      for (int i = w * 32 + lc; i < (int)(sizeof(Tab) / 4); i += cols * 32) dst[i] = src[i];
+      held = inst;
+    }
+    unsigned int* exi = ex + par * 2 * CPT;
+    unsigned int* exo = exi + CPT;
+    unsigned int* exn = ex + (par ^ 1) * 2 * CPT;
+    const unsigned int ncells = (unsigned int)I.nc[0] * (unsigned int)I.nc[1];
+    const unsigned int cell_t = (unsigned int)P.tile_cell0[tile] + lc;
+    const bool active = own < ntiles && cell_t < ncells;
+    const unsigned int cell = cell_t < ncells ? cell_t : ncells - 1;
+    const unsigned int nn0 = (unsigned int)I.nn[0];
+    const unsigned int cy = cell / (unsigned int)I.nc[0];
+    const unsigned int cx = cell - cy * (unsigned int)I.nc[0];
+    const long long node0 = I.off + (long long)(k * cy) * nn0 + (k * cx + w);
+    {
+      // gather: n = invM (.) acc of the previous step
+      double v[n];
+#pragma unroll
+      for (int j = 0; j < n; ++j) v[j] = P.invm[node0 + j * (long long)nn0] * P.acc_in[node0 + j * (long long)nn0];
+      unsigned int m = 0;
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        vals[p0 + j * JS] = v[j];
+        m = max(m, lane_abs_hi(v[j]));
+      }
+      atomicMax(&exi[lc], m);
+    }
+    __syncthreads();  // tables, nodal values and their block exponents complete
+    {
+      const unsigned int E = fx::high_exponent((int)(exi[lc] >> 20));
+#pragma unroll
+      for (int j = 0; j < n; ++j) vfx[p0 + j * JS] = fx::to_fixed_cut<fx::LANE_TOP_VALUES>(vals[p0 + j * JS], E);
+      if (w == 0) exn[lc] = FLOOR;
+      if (w == cols - 1) exn[CPT + lc] = FLOOR_OUT;
+    }
+    __syncthreads();  // fixed-point copies visible
+    AllenCahn<2, degree, double> pde{I.m_well, I.kappa};
+    const SimulationTimer timer(P.dt, 0.0);
+    double term[n][3];
+    unsigned int em[3] = {0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      pg::CellCtx<2, degree, double> ctx;
+      ctx.tab = tab;
+      ctx.vals = vals;
+      ctx.outs = nullptr;
+      ctx.stride = ROW;
+      ctx.lc = lc;
+      ctx.q = w + j * cols;
+      ctx.cell[0] = (int)cx;
+      ctx.cell[1] = (int)cy;
+      ctx.cell[2] = 0;
+      ctx.err = nullptr;
+      ctx.submitted = 0;
+      ctx.vals_fx = vfx;
+      ctx.ex_in = reinterpret_cast<const int*>(exi);
+      ctx.cpb = CPT;
+      ctx.cpt = CPT;
+      ctx.lean = 1;
+      ctx.qi[0] = w;
+      ctx.qi[1] = j;
+      ctx.pe = p0 + j * JS;
+      ctx.step[0] = step0;
+      ctx.step[1] = j == k ? -JS : JS;
+      ctx.nterm = 1;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) ctx.term[i] = 0.0;
+      FieldContainer<2, degree, double> fc(ctx);
+      pde.compute_rhs(fc, timer, 1u);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        term[j][i] = ctx.term[i];
+        em[i] = max(em[i], lane_abs_hi(ctx.term[i]));
+      }
+    }
+    {
+      const unsigned int raw = max(max(em[0], em[1]), em[2]);
+      const unsigned int e = max(max(em[0] + tab->hadd, em[1] + tab->radd[0]), em[2] + tab->radd[1]);
+      atomicMax(&exo[lc], raw >= 0x7ff00000u ? 0xfff00000u : e);
+    }
+    __syncthreads();  // the terms' block exponents complete
+    const int E = (int)(exo[lc] >> 20) - fx::EXP_BIAS;
+    const unsigned long long isig = tab->isig[0];
+    const int lsb = E - 1023 - TOPT + tab->ik[0];
+    long long X[n], Gx[n], Gy[n];
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      X[j] = tab->hpow2 ? fx::to_fixed_cut<TOPT>(term[j][0], fx::high_exponent(E - tab->hk))
+                        : fx::to_fixed_cut_scaled<TOPT>(term[j][0], fx::high_exponent(E), tab->hsig, tab->hk);
+      Gx[j] = fx::to_fixed_cut<TOPT>(term[j][1], fx::high_exponent(E));
+      Gy[j] = tab->rpow2[1] ? fx::to_fixed_cut<TOPT>(term[j][2], fx::high_exponent(E - tab->rk[1]))
+                            : fx::to_fixed_cut_scaled<TOPT>(term[j][2], fx::high_exponent(E), tab->rsig[1], tab->rk[1]);
+      outs[p0 + j * JS] = Gx[j];
+    }
+    __syncthreads();  // fixed-point terms visible
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      const long long* g = outs + p0 + j * JS;
+      if (n > 2 && w == 1) X[j] = lane_add_integral<n>(1, X[j], 0, g[-step0], g[step0]);
+      else X[j] = lane_add_integral<n>(w, X[j], Gx[j], g[step0], n > 2 ? g[2 * step0] : 0ll);
+    }
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      if (n > 2 && j == 1) X[j] = lane_add_integral<n>(1, X[j], 0, Gy[0], Gy[n - 1]);
+      else X[j] = lane_add_integral<n>(j, X[j], Gy[j], Gy[j == 0 ? 1 : n - 2], Gy[j == 0 ? n - 1 : 0]);
+      const int vw = (n > 2 && w == 1 ? 2 : 0) + (n > 2 && j == 1 ? 2 : 0);
+      const double r = fx::to_double_cut(X[j], lsb + vw, isig, true, E >= fx::EXP_WIDE, E >= fx::EXP_NONFINITE);
+      if (active) atomicAdd(P.acc_out + node0 + j * (long long)nn0, r);
+    }
+  }
+}
+
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 18 ? 2 : 48 / WARPS) ensemble_lane_kernel(const EnsLaunch P) {
+  extern __shared__ __align__(16) unsigned char ens_lane_smem[];
+  chain_release();
+  chain_wait();
+  // zero the third accumulator (read one step earlier, untouched by this launch)
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.total_len;
+       i += (long long)gridDim.x * blockDim.x)
+    P.acc_zero[i] = 0.0;
+  ens_lane_tiles<1, WARPS>(P, ens_lane_smem, 0, P.ntiles1);
+  __syncthreads();
+  ens_lane_tiles<2, WARPS>(P, ens_lane_smem, P.ntiles1, P.ntiles - P.ntiles1);
+}
+
+template <int WARPS>
+constexpr size_t ens_lane_smem_bytes() {
+  const size_t a = ens_lane_tile_bytes<1>() * (WARPS / 2), b = ens_lane_tile_bytes<2>() * (WARPS / 3);
+  return a > b ? a : b;
+}
+
 template <int CPB1, int CPB2, int THREADS>
 __global__ void __launch_bounds__(THREADS) ensemble_step_kernel(const EnsLaunch P) {
   extern __shared__ __align__(16) double ens_smem[];
@@ -217,9 +333,9 @@ __global__ void __launch_bounds__(THREADS) ensemble_step_kernel(const EnsLaunch 
 
 template <int CPB1, int CPB2>
 size_t ens_smem_bytes() {
-  // tables, values, three output rows, the fixed-point values and the per-cell exponents
-  const size_t t1 = (sizeof(pg::CellTables<2, 1, double>) + 7) / 8 * 8 + 8 * 5 * CPB1 * 4 + 8 * CPB1;
-  const size_t t2 = (sizeof(pg::CellTables<2, 2, double>) + 7) / 8 * 8 + 8 * 5 * CPB2 * 9 + 8 * CPB2;
+  // tables, values and three output rows
+  const size_t t1 = (sizeof(pg::CellTables<2, 1, double>) + 7) / 8 * 8 + 8 * 4 * CPB1 * 4;
+  const size_t t2 = (sizeof(pg::CellTables<2, 2, double>) + 7) / 8 * 8 + 8 * 4 * CPB2 * 9;
   return std::max(t1, t2) + 64;
 }
 
@@ -229,22 +345,27 @@ __global__ void ensemble_extract_kernel(double* out, const double* invm, const d
     out[i] = invm[i] * acc[i];
 }
 
-// tile-shape candidates: cells per tile for Q1 and for Q2, threads per block
+// tile-shape candidates: cells per tile for Q1 and for Q2, threads per block; on the lane layout
+// (32 cells a tile) 6, 12 or 18 warps a block
 struct Shape {
   int cpb1, cpb2, threads;
 };
 constexpr Shape SHAPES[] = {{64, 28, 256}, {32, 14, 128}, {16, 7, 64}};
+constexpr Shape LANE_SHAPES[] = {{LANE_CPT, LANE_CPT, 192}, {LANE_CPT, LANE_CPT, 384}, {LANE_CPT, LANE_CPT, 576}};
 constexpr int NSHAPES = 3;
+Shape shape_of(bool lanes, int s) { return lanes ? LANE_SHAPES[s] : SHAPES[s]; }
 
 typedef void (*EnsKernel)(const EnsLaunch);
-EnsKernel kernel_for(int s) {
+EnsKernel kernel_for(bool lanes, int s) {
+  if (lanes) return s == 0 ? ensemble_lane_kernel<6> : (s == 1 ? ensemble_lane_kernel<12> : ensemble_lane_kernel<18>);
   switch (s) {
     case 0: return ensemble_step_kernel<64, 28, 256>;
     case 1: return ensemble_step_kernel<32, 14, 128>;
     default: return ensemble_step_kernel<16, 7, 64>;
   }
 }
-size_t smem_for(int s) {
+size_t smem_for(bool lanes, int s) {
+  if (lanes) return s == 0 ? ens_lane_smem_bytes<6>() : (s == 1 ? ens_lane_smem_bytes<12>() : ens_lane_smem_bytes<18>());
   switch (s) {
     case 0: return ens_smem_bytes<64, 28>();
     case 1: return ens_smem_bytes<32, 14>();
@@ -265,7 +386,7 @@ struct ppf_ensemble_s {
   double* scratch = nullptr;
   int* tile_inst = nullptr;
   long long* tile_cell0 = nullptr;
-  long long ntiles = 0;
+  long long ntiles = 0, ntiles1 = 0;
   int shape = 0;
   int grid_mult = 4;
   int sms = 0;
@@ -280,7 +401,7 @@ struct ppf_ensemble_s {
   double gl_w[2][3];
   double gl_D[2][3][3];
   unsigned char* d_tables = nullptr;  // per-instance CellTables, 16-byte aligned
-  int fx = 0;                         // the instance tables enable integer derivatives
+  bool lanes = false;                 // every instance's tables allow the lane layout
 };
 
 namespace ppf {
@@ -299,7 +420,7 @@ int efail(ppf_ensemble e, int code, const std::string& m) {
 
 // tile list for the current shape
 int build_tiles(ppf_ensemble e) {
-  const Shape sh = SHAPES[e->shape];
+  const Shape sh = shape_of(e->lanes, e->shape);
   std::vector<int> ti;
   std::vector<long long> tc;
   for (int i = 0; i < e->n; ++i) {
@@ -311,15 +432,21 @@ int build_tiles(ppf_ensemble e) {
       tc.push_back(c);
     }
   }
-  // interleave instances so consecutive tiles (and thus the blocks of one wave) mix
-  // instances of both degrees
+  // on the lane layout the Q1 instances' tiles first, each instance's together; else interleave
+  // instances so consecutive tiles (and thus the blocks of one wave) mix instances of both degrees
   std::vector<size_t> order(ti.size());
   for (size_t k = 0; k < order.size(); ++k) order[k] = k;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
-    const long long ra = tc[a] / (e->h_inst[ti[a]].degree == 1 ? sh.cpb1 : sh.cpb2);
-    const long long rb = tc[b] / (e->h_inst[ti[b]].degree == 1 ? sh.cpb1 : sh.cpb2);
-    return ra < rb;
-  });
+  e->ntiles1 = 0;
+  for (int i : ti) e->ntiles1 += e->h_inst[i].degree == 1;
+  if (e->lanes)
+    std::stable_sort(order.begin(), order.end(),
+                     [&](size_t a, size_t b) { return e->h_inst[ti[a]].degree < e->h_inst[ti[b]].degree; });
+  else
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+      const long long ra = tc[a] / (e->h_inst[ti[a]].degree == 1 ? sh.cpb1 : sh.cpb2);
+      const long long rb = tc[b] / (e->h_inst[ti[b]].degree == 1 ? sh.cpb1 : sh.cpb2);
+      return ra < rb;
+    });
   std::vector<int> ti2(ti.size());
   std::vector<long long> tc2(tc.size());
   for (size_t k = 0; k < order.size(); ++k) {
@@ -354,16 +481,22 @@ EnsLaunch make_launch(ppf_ensemble e, long long step) {
   L.total_len = e->total;
   L.dt = e->dt;
   L.tables = e->d_tables;
-  L.fx = e->fx;
+  L.ntiles1 = e->ntiles1;
   return L;
 }
 
 int launch_step(ppf_ensemble e, long long step, cudaStream_t s) {
-  EnsKernel k = kernel_for(e->shape);
-  const size_t smem = smem_for(e->shape);
+  EnsKernel k = kernel_for(e->lanes, e->shape);
+  const size_t smem = smem_for(e->lanes, e->shape);
+  const Shape sh = shape_of(e->lanes, e->shape);
   long long grid = (long long)e->sms * e->grid_mult;
   grid = std::max<long long>(1, std::min(grid, e->ntiles));
-  k<<<(unsigned)grid, SHAPES[e->shape].threads, smem, s>>>(make_launch(e, step));
+  if (e->lanes) {
+    if (launch_chained(k, dim3((unsigned)grid), dim3(sh.threads), smem, s, make_launch(e, step)) != cudaSuccess)
+      return efail(e, PPF_ERR_CUDA, "ensemble step launch failed");
+    return PPF_OK;
+  }
+  k<<<(unsigned)grid, sh.threads, smem, s>>>(make_launch(e, step));
   return cudaGetLastError() == cudaSuccess ? PPF_OK : efail(e, PPF_ERR_CUDA, "ensemble step launch failed");
 }
 
@@ -424,9 +557,7 @@ int ppf_ensemble_create(int n_instances, const ppf_mesh_desc* meshes, const doub
         return PPF_ERR_UNSUPPORTED;
       }
       I.tab_off = (long long)tables.size();
-      const int tfx = I.degree == 1 ? reinterpret_cast<const pg::CellTables<2, 1, double>*>(tb.data())->fx
-                                    : reinterpret_cast<const pg::CellTables<2, 2, double>*>(tb.data())->fx;
-      e->fx = (i == 0 ? 1 : e->fx) & (tfx != 0 ? 1 : 0);
+      e->lanes = (i == 0 || e->lanes) && tables_lanes(tb, 2, I.degree) != 0;
       tables.insert(tables.end(), tb.begin(), tb.end());
       tables.resize((tables.size() + 15) / 16 * 16, 0);
     }
@@ -466,7 +597,9 @@ int ppf_ensemble_create(int n_instances, const ppf_mesh_desc* meshes, const doub
   }
   if (cudaMalloc(&e->scratch, sizeof(double) * off) != cudaSuccess) return bail(PPF_ERR_CUDA);
   for (int s = 0; s < NSHAPES; ++s)
-    cudaFuncSetAttribute(kernel_for(s), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for(s));
+    cudaFuncSetAttribute(kernel_for(e->lanes, s), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_for(e->lanes, s));
+  if (e->lanes) e->grid_mult = 8;  // 48 of an SM's warps
   if (build_tiles(e)) return bail(PPF_ERR_CUDA);
   *out = e;
   return PPF_OK;
