@@ -44,11 +44,30 @@ struct AdjointState {
 
 namespace {
 
-__global__ void scale_by_invm_kernel(double* __restrict__ out, const double* __restrict__ in,
-                                     const double* __restrict__ invm, long long N, int nf) {
-  const long long total = N * nf;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
-    out[i] = in[i] * invm[i % N];
+// out = invM (.) in per field; `clear` (nf N entries, may be null) zeroed for the launch that follows
+__global__ void scale_by_invm_kernel(double* out, const double* in, const double* __restrict__ invm, double* clear,
+                                     long long N) {
+  chain_release();
+  chain_wait();
+  const long long base = blockIdx.y * N;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+    out[base + i] = in[base + i] * invm[i];
+    if (clear) clear[base + i] = 0.0;
+  }
+}
+
+// sum of one field per block of threads (out[field]), in a fixed order
+__global__ void __launch_bounds__(1024) field_sum_kernel(const double* __restrict__ v, long long N, double* out) {
+  __shared__ double s[1024];
+  double acc = 0.0;
+  for (long long i = threadIdx.x; i < N; i += blockDim.x) acc += v[blockIdx.x * N + i];
+  s[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = s[0];
 }
 
 long long binom(int n, int k) {
@@ -89,18 +108,24 @@ Fields block_fields(ppf_handle h, int b) {
   return {&h->fields[d.field_indices[0]], &h->fields[d.field_indices[1]]};
 }
 
-// state (2N) -> old_1 of the block fields, one explicit solve, result -> dst (2N)
-int forward_step(ppf_handle h, AdjointState& A, const double* src, double* dst) {
+// One explicit solve from the state src (2N) to dst (2N, which may be src: the cell kernel has read the
+// state before the finalize kernels write it). The block fields' vectors stand on src and dst for the
+// solve instead of being copied to and from.
+int forward_step(ppf_handle h, AdjointState& A, double* src, double* dst) {
   Fields f = block_fields(h, A.block);
-  const size_t bytes = sizeof(double) * A.N;
-  PPF_CUDA(h, cudaMemcpyAsync(f.c->old[0], src, bytes, cudaMemcpyDeviceToDevice, h->stream));
-  PPF_CUDA(h, cudaMemcpyAsync(f.n->old[0], src + A.N, bytes, cudaMemcpyDeviceToDevice, h->stream));
-  int rc = explicit_solve_entry(h, A.block);
-  if (rc) return rc;
-  PPF_CUDA(h, cudaMemcpyAsync(dst, f.c->cur, bytes, cudaMemcpyDeviceToDevice, h->stream));
-  PPF_CUDA(h, cudaMemcpyAsync(dst + A.N, f.n->cur, bytes, cudaMemcpyDeviceToDevice, h->stream));
+  double* const old[2] = {f.c->old[0], f.n->old[0]};
+  double* const cur[2] = {f.c->cur, f.n->cur};
+  f.c->old[0] = src;
+  f.n->old[0] = src + A.N;
+  f.c->cur = dst;
+  f.n->cur = dst + A.N;
+  const int rc = explicit_solve_entry(h, A.block);
+  f.c->old[0] = old[0];
+  f.n->old[0] = old[1];
+  f.c->cur = cur[0];
+  f.n->cur = cur[1];
   A.forward_steps++;
-  return PPF_OK;
+  return rc;
 }
 
 // u_m from the snapshot of step a, stored in slot `dst`
@@ -108,7 +133,7 @@ int advance(ppf_handle h, AdjointState& A, int a, int m, int dst) {
   const int src = slot_of_step(A, a);
   if (src < 0) return fail(h, PPF_ERR_ARG, "internal: missing checkpoint");
   double* work = A.slot[A.S];
-  const double* cur = A.slot[src];
+  double* cur = A.slot[src];
   for (int k = a; k < m; ++k) {
     double* out = (k + 1 == m) ? A.slot[dst] : work;  // in place on the work slot is fine
     int rc = forward_step(h, A, cur, out);
@@ -152,7 +177,10 @@ int linearised_launch(ppf_handle h, AdjointState& A, const char* model, const vo
   L.timer = h->timer;
   L.block_id = 0;
   L.err = h->d_err;
-  L.fx_deriv = 1;  // integer derivatives where the tables allow them (FP64 Q1/Q2)
+  // integer derivatives where the tables allow them (FP64 Q1/Q2); the lane kernel, with 20 rows of
+  // shared memory for four fields in and four out, measured slower (128^2 Q2, 40 steps: 5.6 ms
+  // against 4.3 ms)
+  L.fx_deriv = 1;
   const size_t smem = cell_smem(h->dim, h->k, 0, L.nrows_in, L.nrows_out);
   cudaError_t e = ops->launch(h->dim, h->k, MODE_RHS, 0, L, obj, smem, h->stream);
   if (e != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("linearised kernel: ") + cudaGetErrorString(e));
@@ -165,8 +193,9 @@ int linearised_launch(ppf_handle h, AdjointState& A, const char* model, const vo
 int adjoint_step(ppf_handle h, AdjointState& A, int a) {
   const int s = slot_of_step(A, a);
   if (s < 0) return fail(h, PPF_ERR_ARG, "internal: adjoint step without its state");
-  scale_by_invm_kernel<<<grid_for(2 * A.N), 256, 0, h->stream>>>(A.w, A.lam, h->d_invm, A.N, 2);
-  PPF_CUDA(h, cudaMemsetAsync(A.lam_new, 0, sizeof(double) * 2 * A.N, h->stream));
+  PPF_CUDA(h, launch_chained(scale_by_invm_kernel, dim3(grid_for(A.N), 2), dim3(256), 0, h->stream, A.w,
+                             (const double*)A.lam, h->d_invm, A.lam_new, A.N));
+  h->all_launches++;
   double* outs[4] = {A.lam_new, A.lam_new + A.N, A.gpar, A.gpar + A.N};
   int rc = linearised_launch(h, A, "coupled_acch_adjoint", A.obj_adj.data(), A.slot[s], A.w, outs, 4);
   if (rc) return rc;
@@ -234,10 +263,12 @@ int setup(ppf_handle h, AdjointState& A, int b, int S) {
   A.block = b;
   A.S = std::max(1, S);
   A.N = h->N;
-  for (double* p : A.slot) cudaFree(p);
-  A.slot.assign(A.S + 1, nullptr);
+  // snapshot slots of earlier calls are kept
+  for (size_t i = A.S + 1; i < A.slot.size(); ++i) cudaFree(A.slot[i]);
+  A.slot.resize(A.S + 1, nullptr);
   A.slot_step.assign(A.S + 1, -1);
-  for (auto& p : A.slot) PPF_CUDA(h, cudaMalloc(&p, sizeof(double) * 2 * A.N));
+  for (auto& p : A.slot)
+    if (!p) PPF_CUDA(h, cudaMalloc(&p, sizeof(double) * 2 * A.N));
   if (!A.lam) {
     for (double** p : {&A.lam, &A.lam_new, &A.w, &A.gpar, &A.du, &A.dacc})
       PPF_CUDA(h, cudaMalloc(p, sizeof(double) * 2 * A.N));
@@ -333,18 +364,17 @@ int ppf_adjoint_backward(ppf_handle h, const double* dJ_duK, double* dJ_dparams,
   PPF_CUDA(h, cudaMemsetAsync(A.gpar, 0, sizeof(double) * 2 * A.N, h->stream));
   int rc = reverse(h, A, 0, A.K, A.S - 1);
   if (rc) return rc;
-  std::vector<double> g(2 * A.N);
-  PPF_CUDA(h, cudaMemcpyAsync(g.data(), A.gpar, sizeof(double) * 2 * A.N, cudaMemcpyDeviceToHost, h->stream));
+  // the parameter gradients: sums of the two density fields (into w, free by now)
+  double g[2] = {0.0, 0.0};
+  field_sum_kernel<<<2, 1024, 0, h->stream>>>(A.gpar, A.N, A.w);
+  PPF_CUDA(h, cudaGetLastError());
+  h->all_launches++;
+  PPF_CUDA(h, cudaMemcpyAsync(g, A.w, sizeof(g), cudaMemcpyDeviceToHost, h->stream));
   if (dJ_du0) PPF_CUDA(h, cudaMemcpyAsync(dJ_du0, A.lam, sizeof(double) * 2 * A.N, cudaMemcpyDeviceToHost, h->stream));
   PPF_CUDA(h, cudaStreamSynchronize(h->stream));
   if (dJ_dparams) {
-    double s0 = 0.0, s1 = 0.0;
-    for (long long i = 0; i < A.N; ++i) {
-      s0 += g[i];
-      s1 += g[A.N + i];
-    }
-    dJ_dparams[0] = s0;
-    dJ_dparams[1] = s1;
+    dJ_dparams[0] = g[0];
+    dJ_dparams[1] = g[1];
   }
   if (forward_steps) *forward_steps = A.forward_steps;
   // restore the first checkpoints so another backward pass could run; the state is kept
@@ -383,7 +413,9 @@ int ppf_tangent_linear(ppf_handle h, int b, int n_steps, const double* du0, cons
     double* outs[2] = {A.dacc, A.dacc + A.N};
     rc = linearised_launch(h, A, "coupled_acch_tangent", obj.data(), u, A.du, outs, 2);
     if (rc) return rc;
-    scale_by_invm_kernel<<<grid_for(2 * A.N), 256, 0, h->stream>>>(A.du, A.dacc, h->d_invm, A.N, 2);
+    PPF_CUDA(h, launch_chained(scale_by_invm_kernel, dim3(grid_for(A.N), 2), dim3(256), 0, h->stream, A.du,
+                               (const double*)A.dacc, h->d_invm, (double*)nullptr, A.N));
+    h->all_launches++;
     rc = forward_step(h, A, u, u);
     if (rc) return rc;
   }
