@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
   int* ex_in = reinterpret_cast<int*>(vals_fx + P.nrows_in * S::threads);
   bool fx_on = false;
   unsigned int fx_rows = 0;
-  chain_release();
   chain_wait();
+  chain_release();
   if constexpr (FXC) {
     unsigned int dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
@@ -92,10 +92,11 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
   const int qa = q % n;
   const int qb = dim > 1 ? (q / n) % n : 0;
   const int qc = dim > 2 ? q / (n * n) : 0;
-  const long long ntiles = (P.ncells + cpb - 1) / cpb;
+  const int cpt = P.cells_per_tile;
+  const long long ntiles = (P.ncells + cpt - 1) / cpt;
 
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long cell = tile * cpb + lc;
+    const long long cell = tile * cpt + lc;
     const bool active = cell < P.ncells;
     int4 info = make_int4(0, 0, 0, 0);
     long long dof = 0;
@@ -106,7 +107,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
     if constexpr (FXC) {
       // last read by the previous tile's callbacks; rows without a fixed-point copy keep -1
       if (fx_on)
-        for (int i = t; i < P.nrows_in * cpb; i += S::threads) ex_in[i] = ((fx_rows >> (i / cpb)) & 1u) ? 0 : -1;
+        for (int i = t; i < P.nrows_in * cpb; i += blockDim.x) ex_in[i] = ((fx_rows >> (i / cpb)) & 1u) ? 0 : -1;
     }
     __syncthreads();  // tables staged; previous tile finished with vals/outs/sflags
 
@@ -250,11 +251,14 @@ cudaError_t launch_amr_cell_kernel(const AmrCellLaunch& A, const void* obj, size
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
   }
-  const long long ntiles = (A.base.ncells + S::cpb - 1) / S::cpb;
+  AmrCellLaunch L = A;
+  const int cpt = L.base.cells_per_tile = cells_per_tile<dim, degree>(A.base.ncells, sms);
+  const long long ntiles = (A.base.ncells + cpt - 1) / cpt;
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, A, *reinterpret_cast<const PDE*>(obj));
+  return launch_chained(kern, dim3((unsigned)grid), dim3(cpt * S::nq), smem, s, L,
+                        *reinterpret_cast<const PDE*>(obj));
 }
 
 }  // namespace ppf

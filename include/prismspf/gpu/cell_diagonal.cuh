@@ -39,8 +39,8 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Tab* tab = reinterpret_cast<Tab*>(smem_raw);
   number* vals = reinterpret_cast<number*>(smem_raw + (sizeof(Tab) + 15) / 16 * 16);
-  chain_release();
   chain_wait();
+  chain_release();
   {
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);
     unsigned int* dst = reinterpret_cast<unsigned int*>(tab);

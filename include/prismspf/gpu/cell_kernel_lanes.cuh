@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;  // lattice stride of the last direction
   const unsigned int ncells = (unsigned int)P.ncells;
   const unsigned int ntiles = (ncells + CPT - 1) / CPT;
-  chain_release();
   chain_wait();
+  chain_release();
   __syncthreads();  // exponent buffers set
 
   int par = 0;
@@ -504,8 +504,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;
   const unsigned int ncells = (unsigned int)P.ncells;
   const unsigned int ntiles = (ncells + CPT - 1) / CPT;
-  chain_release();
   chain_wait();
+  chain_release();
 
   for (unsigned int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned int cell_t = tile * CPT + lc;

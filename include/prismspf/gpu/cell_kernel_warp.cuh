@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
   namespace fx = pg::fx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Tab* tab = reinterpret_cast<Tab*>(smem_raw);
-  chain_release();
   chain_wait();
+  chain_release();
   {
     const int nwords = (int)(sizeof(Tab) / 4);
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);

@@ -47,11 +47,13 @@ cudaError_t launch_cell_kernel_impl(const CellLaunch& P, const void* obj, size_t
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
   }
-  const long long ntiles = (P.ncells + S::cpb - 1) / S::cpb;
+  CellLaunch L = with_divisors(P);
+  const int cpt = L.cells_per_tile = cells_per_tile<dim, degree>(P.ncells, sms);
+  const long long ntiles = (P.ncells + cpt - 1) / cpt;
   long long grid = (long long)sms * occ;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
-  return launch_chained(kern, dim3((unsigned)grid), dim3(S::threads), smem, s, with_divisors(P),
+  return launch_chained(kern, dim3((unsigned)grid), dim3(cpt * S::nq), smem, s, L,
                         *reinterpret_cast<const PDE*>(obj));
 }
 

@@ -47,8 +47,8 @@ namespace {
 // out = invM (.) in per field; `clear` (nf N entries, may be null) zeroed for the launch that follows
 __global__ void scale_by_invm_kernel(double* out, const double* in, const double* __restrict__ invm, double* clear,
                                      long long N) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     out[base + i] = in[base + i] * invm[i];

@@ -64,8 +64,8 @@ __global__ void amr_finalize_kernel(double* u, const double* acc, double* clear,
                                     const int* __restrict__ cmap, const double* dvals, const int* __restrict__ h_ptr,
                                     const int* __restrict__ h_idx, const double* __restrict__ h_w, long long N, int* err,
                                     prismspf::SimulationTimer* timer, double dt) {
-  chain_release();
   chain_wait();
+  chain_release();
   if (timer && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) timer->increment(dt);
   const long long base = blockIdx.y * N;
   int bad = 0;

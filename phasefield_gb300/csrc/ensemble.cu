@@ -299,8 +299,8 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, WARPS == 18 ? 2 : 48 / WARPS) ensemble_lane_kernel(const EnsLaunch P) {
   extern __shared__ __align__(16) unsigned char ens_lane_smem[];
-  chain_release();
   chain_wait();
+  chain_release();
   // zero the third accumulator (read one step earlier, untouched by this launch)
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.total_len;
        i += (long long)gridDim.x * blockDim.x)

@@ -87,8 +87,8 @@ __device__ bool grid_sum(double v, double* partial, unsigned int* counter, doubl
 template <typename T>
 __global__ void __launch_bounds__(256) dot_kernel(long long n, const T* x, const T* y, double* partial,
                                                   unsigned int* counter, double* out) {
-  chain_release();
   chain_wait();
+  chain_release();
   double acc = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     acc += double(x[i]) * double(y[i]);
@@ -107,8 +107,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) level_finalize_kernel(T* dst, const T* acc, T* clear, const T* __restrict__ scale,
                                                              long long N, const T* w,
                                                              double* partial, unsigned int* counter, double* out) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * N;
   double sum = 0.0, total;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(256) level_finalize_kernel(T* dst, const T* ac
 // inverse diagonal: d = scale (.) acc, zero entries -> 1, inverted
 template <typename T>
 __global__ void inv_diag_kernel(T* inv, const T* acc, T* clear, const T* __restrict__ scale, long long N) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
@@ -283,8 +283,8 @@ __device__ __forceinline__ T restrict_row(const Transfer<T>& A, const T* r, int 
 template <typename T, typename Tc, int degree>
 __global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_constant__ Transfer<T> A, T* x, const Tc* e,
                                                              const int* __restrict__ cmap) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * A.Nout;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
     const int m = cmap ? cmap[base + i] : (int)(base + i);
@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_consta
 template <typename T, typename Tc, int degree>
 __global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ Transfer<T> A, Tc* b, const T* r,
                                                        const int* __restrict__ cmap) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * A.Nout;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
     T s = T(0);
@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ T
 template <typename T>
 __global__ void __launch_bounds__(256) cheb_start_kernel(long long n, T* x, T* u, const T* b,
                                                          const T* pinv, double c2) {
-  chain_release();
   chain_wait();
+  chain_release();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const T ui = T(c2) * pinv[i] * b[i];
     u[i] = ui;
@@ -345,8 +345,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) cheb_step_kernel(T* x, T* u, const T* b, const T* acc, T* clear,
                                                         const T* __restrict__ scale, const T* pinv, double c1,
                                                         double c2, long long N) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(256) cheb_step_kernel(T* x, T* u, const T* b, 
 template <typename T>
 __global__ void __launch_bounds__(256) residual_kernel(T* r, const T* b, const T* acc, T* clear,
                                                        const T* __restrict__ scale, long long N) {
-  chain_release();
   chain_wait();
+  chain_release();
   const long long base = blockIdx.y * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
     const long long gi = base + i;
@@ -383,8 +383,8 @@ enum Scalar { SC_RZ = 0 /* two, alternating */, SC_PQ = 2, SC_RR = 3, SC_DONE = 
 __global__ void __launch_bounds__(256) cg_update_kernel(long long n, double* sc, int rz, const double* p, const double* q,
                                                         double* x, double* r, double tol, double* partial,
                                                         unsigned int* counter) {
-  chain_release();
   chain_wait();
+  chain_release();
   if (sc[SC_DONE] != 0.0) return;
   const double alpha = sc[SC_RZ + rz] / sc[SC_PQ];
   double acc = 0.0, total;
@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(256) cg_update_kernel(long long n, double* sc,
 // p = z + beta p with beta = rz_new / rz (first: p = z)
 __global__ void __launch_bounds__(256) cg_direction_kernel(long long n, const double* sc, int rz, int first,
                                                            const double* z, double* p) {
-  chain_release();
   chain_wait();
+  chain_release();
   const double beta = first ? 0.0 : sc[SC_RZ + rz] / sc[SC_RZ + 1 - rz];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = first ? z[i] : z[i] + beta * p[i];
@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(256) cg_direction_kernel(long long n, const do
 template <typename T>
 __global__ void __launch_bounds__(256) eig_update_kernel(long long n, double* e, int it, const T* q, T* r, T* z, T* p,
                                                          const T* pinv, double* partial, unsigned int* counter) {
-  chain_release();
   chain_wait();
+  chain_release();
   const bool start = it < 0;
   const double alpha = start ? 0.0 : e[3 * it + 2] / e[3 * it + 3];
   double rr = 0.0, rz = 0.0, total;
@@ -436,8 +436,8 @@ __global__ void __launch_bounds__(256) eig_update_kernel(long long n, double* e,
 }
 template <typename T>
 __global__ void __launch_bounds__(256) eig_direction_kernel(long long n, const double* e, int it, const T* z, T* p) {
-  chain_release();
   chain_wait();
+  chain_release();
   const double beta = e[3 * it + 5] / e[3 * it + 2];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = T(double(z[i]) + beta * double(p[i]));

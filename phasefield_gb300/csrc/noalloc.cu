@@ -28,6 +28,7 @@
 // itself returns before its GPU work ends and so cannot report it.
 // ppf_allen_cahn_step_noalloc_status waits for a stream and reads that word (a copy into a
 // host int of the caller's stack, no allocation).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -60,11 +61,25 @@ struct alignas(16) TableBlob {
   unsigned char b[B];
 };
 
+// First launch of a step: the tables and the error word (block 0) and the cleared accumulator, in one
+// launch (the accumulator as a memset of its own and an unchained sequence took 20 us a step on a
+// 64^2 Q1 mesh, all of it launch latency)
 template <size_t B>
-__global__ void noalloc_stage_tables_kernel(const __grid_constant__ TableBlob<B> blob, unsigned char* dst,
-                                            int* err) {
-  for (int i = threadIdx.x; i < (int)B; i += blockDim.x) dst[i] = blob.b[i];
-  if (threadIdx.x == 0) *err = 0;
+__global__ void __launch_bounds__(256) noalloc_begin_kernel(const __grid_constant__ TableBlob<B> blob, unsigned char* dst,
+                                                            int* err, double* acc, int N) {
+  static_assert(B % 4 == 0, "tables are staged in words");
+  chain_wait();  // (the step before reads the accumulator and the tables)
+  chain_release();
+  if (blockIdx.x == 0) {
+    const unsigned int* src = reinterpret_cast<const unsigned int*>(blob.b);
+    for (int i = threadIdx.x; i < (int)(B / 4); i += blockDim.x) reinterpret_cast<unsigned int*>(dst)[i] = src[i];
+    if (threadIdx.x == 0) *err = 0;
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) acc[i] = 0.0;
+}
+
+unsigned noalloc_grid(long long N, int sms) {
+  return (unsigned)std::max<long long>(1, std::min<long long>((N + 255) / 256, (long long)sms * 8));
 }
 
 int noalloc_fail(int code, const char* msg) {
@@ -89,10 +104,11 @@ void gl_closed_form(int n, double* x, double* w) {
   }
 }
 
-// Builds the cell tables of block 1 and launches the kernel that writes them (and clears the
-// error word) into the scratch array; returns false when that launch fails.
+// Builds the cell tables of block 1 and launches the kernel that writes them into the scratch array
+// and clears the error word and the accumulator; returns false when that launch fails.
 template <int dim, int degree>
-bool stage_tables(const ppf_mesh_desc& m, const double* h, unsigned char* d_tables, int* d_err, cudaStream_t s) {
+bool stage_tables(const ppf_mesh_desc& m, const double* h, unsigned char* d_tables, int* d_err, double* acc,
+                  long long N, unsigned grid, cudaStream_t s) {
   using Tab = pg::CellTables<dim, degree>;
   static_assert(sizeof(Tab) <= NOALLOC_TABLE_BYTES, "cell tables exceed the scratch table region");
   static_assert(sizeof(Tab) <= 32000, "cell tables exceed the kernel-parameter limit");
@@ -158,50 +174,50 @@ bool stage_tables(const ppf_mesh_desc& m, const double* h, unsigned char* d_tabl
   t.slot_comp0[0] = 0;
   t.out_of[0] = 0;
   t.out_row0[0] = 0;
-  noalloc_stage_tables_kernel<sizeof(Tab)><<<1, 256, 0, s>>>(blob, d_tables, d_err);
-  return cudaGetLastError() == cudaSuccess;
+  return launch_chained(noalloc_begin_kernel<sizeof(Tab)>, dim3(grid), dim3(256), 0, s, blob, d_tables, d_err, acc,
+                        (int)N) == cudaSuccess;
 }
 
 bool stage_tables_dispatch(int dim, int degree, const ppf_mesh_desc& m, const double* h, unsigned char* d_tables,
-                           int* d_err, cudaStream_t s) {
+                           int* d_err, double* acc, long long N, unsigned grid, cudaStream_t s) {
   switch (dim * 10 + degree) {
-    case 21: return stage_tables<2, 1>(m, h, d_tables, d_err, s);
-    case 22: return stage_tables<2, 2>(m, h, d_tables, d_err, s);
-    case 23: return stage_tables<2, 3>(m, h, d_tables, d_err, s);
-    case 24: return stage_tables<2, 4>(m, h, d_tables, d_err, s);
-    case 31: return stage_tables<3, 1>(m, h, d_tables, d_err, s);
-    case 32: return stage_tables<3, 2>(m, h, d_tables, d_err, s);
-    case 33: return stage_tables<3, 3>(m, h, d_tables, d_err, s);
-    case 34: return stage_tables<3, 4>(m, h, d_tables, d_err, s);
+    case 21: return stage_tables<2, 1>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 22: return stage_tables<2, 2>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 23: return stage_tables<2, 3>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 24: return stage_tables<2, 4>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 31: return stage_tables<3, 1>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 32: return stage_tables<3, 2>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 33: return stage_tables<3, 3>(m, h, d_tables, d_err, acc, N, grid, s);
+    case 34: return stage_tables<3, 4>(m, h, d_tables, d_err, acc, N, grid, s);
     default: return false;
   }
 }
 
 struct LumpedMass1D {
-  double w[5];
+  double wh[3][5];  // GL weight x cell size per direction
   int k;
   int nc[3];
-  double h[3];
+  pg::fx::FastDiv fd[2];  // divisors of the lattice extents
 };
 
 // u_new = acc / m, with the lumped mass m of a natural-boundary uniform mesh evaluated from
 // the lattice indices: a product over directions of h_d times the GL weight of the node's
 // position in its cell, doubled where two cells share the node.
-__global__ void noalloc_finalize_kernel(double* __restrict__ u, const double* __restrict__ acc, const int nn0,
-                                        const int nn1, const long long N, const LumpedMass1D m, const int dim,
-                                        int* err) {
+__global__ void __launch_bounds__(256) noalloc_finalize_kernel(double* u, const double* acc, const int nn0, const int nn1,
+                                                               const int N, const LumpedMass1D m, const int dim,
+                                                               int* err) {
+  chain_wait();
+  chain_release();
   int bad = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    long long idx[3] = {i % nn0, (i / nn0) % nn1, i / ((long long)nn0 * nn1)};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    const unsigned r = m.fd[0].div((unsigned)i), z = m.fd[1].div(r);
+    const int idx[3] = {i - (int)r * nn0, (int)(r - z * (unsigned)nn1), (int)z};
     double mass = 1.0;
     for (int d = 0; d < dim; ++d) {
-      const long long I = idx[d];
-      const int a = (int)(I % m.k);
-      double w1;
-      if (a != 0) w1 = m.w[a];
-      else if (I == 0 || I == (long long)m.k * m.nc[d]) w1 = m.w[0];
-      else w1 = 2.0 * m.w[0];
-      mass *= w1 * m.h[d];
+      const int I = idx[d];
+      const int a = I % m.k;
+      const double w1 = a != 0 ? m.wh[d][a] : (I == 0 || I == m.k * m.nc[d] ? m.wh[d][0] : 2.0 * m.wh[d][0]);
+      mass = d == 0 ? w1 : mass * w1;
     }
     const double v = acc[i] / mass;
     bad |= !isfinite(v);
@@ -270,11 +286,9 @@ extern "C" int ppf_allen_cahn_step_noalloc(const ppf_mesh_desc* mesh, double m_w
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   AllenCahn<2, 1, double> pde{m_well, kappa};  // same layout for every dim/degree
-  // tables and the cleared error word, then the cleared accumulator
-  if (!stage_tables_dispatch(dim, degree, *mesh, h, d_tables, d_err, s))
+  const unsigned grid = noalloc_grid(N, g_sm_count[dev]);
+  if (!stage_tables_dispatch(dim, degree, *mesh, h, d_tables, d_err, acc, N, grid, s))
     return noalloc_fail(PPF_ERR_CUDA, "staging the cell tables failed");
-  if (cudaMemsetAsync(acc, 0, sizeof(double) * N, s) != cudaSuccess)
-    return noalloc_fail(PPF_ERR_CUDA, "clearing the accumulator failed");
 
   CellLaunch L;
   std::memset(&L, 0, sizeof(L));
@@ -301,17 +315,18 @@ extern "C" int ppf_allen_cahn_step_noalloc(const ppf_mesh_desc* mesh, double m_w
     return noalloc_fail(PPF_ERR_CUDA, "cell kernel launch failed");
 
   LumpedMass1D lm{};
-  double x[5];
-  gl_closed_form(degree + 1, x, lm.w);
+  double x[5], w[5];
+  gl_closed_form(degree + 1, x, w);
   lm.k = degree;
   for (int d = 0; d < 3; ++d) {
     lm.nc[d] = nc[d];
-    lm.h[d] = h[d];
+    for (int i = 0; i <= degree; ++i) lm.wh[d][i] = w[i] * h[d];
   }
-  long long grid = (N + 255) / 256;
-  if (grid > (long long)g_sm_count[dev] * 16) grid = (long long)g_sm_count[dev] * 16;
-  noalloc_finalize_kernel<<<(unsigned)grid, 256, 0, s>>>(d_n_new, acc, nn[0], nn[1], N, lm, dim, d_err);
-  if (cudaGetLastError() != cudaSuccess) return noalloc_fail(PPF_ERR_CUDA, "finalize kernel launch failed");
+  lm.fd[0].init((unsigned)nn[0]);
+  lm.fd[1].init((unsigned)nn[1]);
+  if (launch_chained(noalloc_finalize_kernel, dim3(grid), dim3(256), 0, s, d_n_new, (const double*)acc, nn[0], nn[1],
+                     (int)N, lm, dim, d_err) != cudaSuccess)
+    return noalloc_fail(PPF_ERR_CUDA, "finalize kernel launch failed");
   return PPF_OK;
 }
 

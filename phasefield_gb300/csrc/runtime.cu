@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const
                                                                 long long N, int* err, double* u2,
                                                                 prismspf::SimulationTimer* timer, double dt) {
   constexpr int U = 4;
-  chain_release();
   chain_wait();
+  chain_release();
   const int c = blockIdx.y;
   const long long base = c * N;
   const long long step = (long long)gridDim.x * blockDim.x;
@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const
 // are condensed onto their masters, Dirichlet rows dropped), so they need no look-up: 0 scales to 0.
 __global__ void finalize_apply_kernel(double* dst, const double* acc, double* clear, const double* __restrict__ scale,
                                       long long N) {
-  chain_release();
   chain_wait();
+  chain_release();
   const int c = blockIdx.y;
   const long long base = c * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
@@ -813,7 +813,7 @@ int launch_cell(ppf_handle h, int b, int which, const double* const* src, bool p
 // each in fixed point (issue slots) or in FP64 (the FP64 pipe). Which split is cheapest depends
 // on how much FP64 work the callback itself does, so the first plain launch of a plan times
 // modes 1 (integer derivatives, FP64 integration), 2 (both integer), 3 (FP64 derivatives,
-// integer integration) and the lane kernel (4 on cubic cells, 5 on others), twice each, back to back into
+// integer integration) and the lane kernel (4 on cubic cells, 5 on others) into
 // the block's accumulators (which every caller has just zeroed, and which are zeroed again
 // afterwards), and keeps the fastest. PPF_CONTRACTION_MODE=1-5 fixes the mode; a plan first
 // launched inside a graph capture takes the lane kernel where it applies, else mode 1.
@@ -830,18 +830,22 @@ static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch
     return PPF_OK;
   }
   const int nm = P.fx_lanes ? 4 : 3;
-  const int NT = 2 * nm;  // every mode, then again
+  // every mode once untimed (its code is loaded then), then twice timed: launches of a few
+  // microseconds several at a time, as the gap between two events is as long as they are
+  const int NT = 2 * nm;
+  const int burst = L.ncells > 200000 ? 1 : 6;
   cudaEvent_t ev[9] = {};
   cudaError_t e = cudaSuccess;
   for (int i = 0; i <= NT && e == cudaSuccess; ++i) e = cudaEventCreate(&ev[i]);
   CellLaunch T = L;
-  if (e == cudaSuccess) e = cudaEventRecord(ev[0], h->stream);
-  for (int r = 0; r < NT && e == cudaSuccess; ++r) {
-    set_fx_mode(T, timed_fx_mode(r % nm, P.fx_lanes));
-    e = h->custom_launch ? (cudaError_t)h->custom_launch(h->dim, h->k, mode, 0, &T, h->model_obj.data(), smem,
-                                                         (void*)h->stream)
-                         : h->model->launch(h->dim, h->k, mode, 0, T, h->model_obj.data(), smem, h->stream);
-    if (e == cudaSuccess) e = cudaEventRecord(ev[r + 1], h->stream);
+  for (int r = -nm; r < NT && e == cudaSuccess; ++r) {
+    if (r == 0) e = cudaEventRecord(ev[0], h->stream);
+    set_fx_mode(T, timed_fx_mode((r + nm) % nm, P.fx_lanes));
+    for (int k = 0; k < (r < 0 ? 1 : burst) && e == cudaSuccess; ++k)
+      e = h->custom_launch ? (cudaError_t)h->custom_launch(h->dim, h->k, mode, 0, &T, h->model_obj.data(), smem,
+                                                           (void*)h->stream)
+                           : h->model->launch(h->dim, h->k, mode, 0, T, h->model_obj.data(), smem, h->stream);
+    if (r >= 0 && e == cudaSuccess) e = cudaEventRecord(ev[r + 1], h->stream);
   }
   if (e == cudaSuccess) e = cudaEventSynchronize(ev[NT]);
   float best[4] = {1e30f, 1e30f, 1e30f, 1e30f};
@@ -1587,13 +1591,18 @@ static int rotation_period(ppf_handle h) {
   return p % 2 ? 2 * p : p;
 }
 
-static int capture_graph(ppf_handle h) {
+// One graph holds up to GRAPH_PERIODS rotation periods, as many as the run has left: kernels of one
+// graph are chained, successive graphs are not (48^2 Q1: 1.4 us a graph launch).
+constexpr int GRAPH_PERIODS = 8;
+
+static int capture_graph(ppf_handle h, unsigned remaining) {
   if (h->run_graph) {
     cudaGraphExecDestroy(h->run_graph);
     h->run_graph = nullptr;
   }
   if (!h->d_timer) PPF_CUDA(h, cudaMalloc(&h->d_timer, sizeof(prismspf::SimulationTimer)));
-  const int period = rotation_period(h);
+  const int base = rotation_period(h);
+  const int period = base * (int)std::max(1u, std::min((unsigned)GRAPH_PERIODS, remaining / (unsigned)base));
   const prismspf::SimulationTimer saved = h->timer;
   const long long launches0 = h->all_launches;
   const int last = last_explicit_block(h);
@@ -1624,7 +1633,7 @@ static int capture_graph(ppf_handle h) {
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
   h->graph_period = period;
-  h->graph_phase = h->rot_count % period;
+  h->graph_phase = h->rot_count % base;
   h->graph_launches = h->all_launches - launches0;
   h->all_launches = launches0;
   h->graph_stream = h->stream;
@@ -1660,10 +1669,12 @@ static int run_increments(ppf_handle h, unsigned int n_increments, int output_ev
           else if (due - 1 < last) last = (unsigned)(due - 1);
         }
       const unsigned remaining = last >= inc ? last - inc + 1 : 0;
-      if (remaining >= (unsigned)period) {
-        if (!h->run_graph || h->graph_stream != h->stream || h->graph_phase != h->rot_count % period ||
-            h->graph_mesh_version != h->mesh_version || h->graph_state_version != h->state_version) {
-          int rc = capture_graph(h);
+      const bool valid = h->run_graph && h->graph_stream == h->stream && h->graph_phase == h->rot_count % period &&
+                         h->graph_mesh_version == h->mesh_version && h->graph_state_version == h->state_version;
+      // (fewer increments than a captured graph holds run as plain launches)
+      if (remaining >= (unsigned)(valid ? h->graph_period : period)) {
+        if (!valid) {
+          int rc = capture_graph(h, remaining);
           if (rc) return rc;
         }
         PPF_CUDA(h, cudaMemcpyAsync(h->d_timer, &h->timer, sizeof(prismspf::SimulationTimer), cudaMemcpyHostToDevice,
@@ -1678,10 +1689,10 @@ static int run_increments(ppf_handle h, unsigned int n_increments, int output_ev
           const int rc = clear_acc(h, F);
           if (rc) return rc;
         }
-        const unsigned reps = remaining / period;
+        const unsigned held = (unsigned)h->graph_period, reps = remaining / held;
         for (unsigned r = 0; r < reps; ++r) PPF_CUDA(h, cudaGraphLaunch(h->run_graph, h->stream));
-        for (unsigned k = 0; k < reps * (unsigned)period; ++k) h->timer.increment(h->dt);
-        h->rot_count += (long long)reps * period;
+        for (unsigned k = 0; k < reps * held; ++k) h->timer.increment(h->dt);
+        h->rot_count += (long long)reps * held;
         h->all_launches += (long long)reps * h->graph_launches;
         h->cell_launches += 0;
         continue;
