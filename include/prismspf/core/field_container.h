@@ -149,8 +149,6 @@ struct CellCtx {
   // `probe` and zero elsewhere
   int probe = -1;
   unsigned int probe_rows = 0;
-  // value terms stored unweighted (a kernel integrating them in fixed point), on any layout
-  int raw_values = 0;
 };
 
 }  // namespace gpu
@@ -393,7 +391,7 @@ class FieldContainer {
     }
     const int o = out_row(field_index);
     if (o < 0) return;
-    ctx.outs[o * ctx.stride + slot()] = ctx.raw_values ? val.v : val.v * ctx.tab->jxw[ctx.q];
+    ctx.outs[o * ctx.stride + slot()] = val.v * ctx.tab->jxw[ctx.q];
     ctx.submitted |= 1 << (2 * ctx.tab->out_of[field_index]);
   }
 
@@ -409,8 +407,7 @@ class FieldContainer {
     const int o = out_row(field_index);
     if (o < 0) return;
     for (int c = 0; c < int(dim); ++c)
-      ctx.outs[(o + c * (1 + dim)) * ctx.stride + slot()] =
-          ctx.raw_values ? val[c].v : val[c].v * ctx.tab->jxw[ctx.q];
+      ctx.outs[(o + c * (1 + dim)) * ctx.stride + slot()] = val[c].v * ctx.tab->jxw[ctx.q];
     ctx.submitted |= 1 << (2 * ctx.tab->out_of[field_index]);
   }
 
@@ -599,7 +596,19 @@ class FieldContainer {
         // a row declared without gradients has no fixed-point copy (exponent -1)
       }
     }
-    // FP64 contraction over the nodal values
+    if constexpr (std::is_same<number, float>::value && degree <= 2) {
+      // the FP32 lane kernel: the own value (one load for all directions), then the others of the line
+      if (ctx.lean) {
+        const number* u = ctx.vals + row * ctx.stride + ctx.pe;
+        const number* Dr = ctx.tab->Dh[d][ctx.qi[d]];
+        const int st = ctx.step[d], i = ctx.qi[d];
+        if (n > 2 && i == 1) return fma(Dr[n - 1], u[st], fma(Dr[0], u[-st], Dr[1] * u[0]));
+        number s = fma(Dr[n > 2 ? 1 : 1 - i], u[st], Dr[i] * u[0]);
+        if (n > 2) s = fma(Dr[2 - i], u[2 * st], s);
+        return s;
+      }
+    }
+    // contraction over the nodal values
     const int q0 = ctx.q - qd * stride_d;
     const number* Dr = ctx.tab->Dh[d][qd];
     if (ctx.cpt) {
