@@ -227,6 +227,7 @@ struct ppf_handle_s {
   long long graph_launches = 0;
   long long rot_count = 0;
   bool capturing = false;
+  bool caller_captured = false;  // a caller has captured launches of this handle in a graph of its own
   // kernel timing
   bool timing = false;
   std::vector<cudaEvent_t> ev_pool;

@@ -902,15 +902,20 @@ int finish_streamed_outputs(ppf_handle h);
 static int ensure_out_stage(ppf_handle h, FieldState& F);
 
 // Whether a launch sequence may leave its field on its other accumulator: not in a caller's own
-// capture, which may be replayed by itself (the increment graph's period returns to where it began)
+// capture, nor after one on this handle: its replays, between any two calls, use the accumulator they
+// were captured with and leave it as it is, so every sequence then clears its own first. (The
+// increment graph's period returns to where it began.)
 static int alternating(ppf_handle h, bool* yes) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (!h->capturing) PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
-  *yes = cs == cudaStreamCaptureStatusNone;
+  if (!h->capturing) {
+    PPF_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) h->caller_captured = true;
+  }
+  *yes = h->capturing || !h->caller_captured;
   return PPF_OK;
 }
 
-// (a caller's own capture clears in any case)
+// (in and after a caller's own capture: clears in any case)
 int clear_acc(ppf_handle h, FieldState& F) {
   bool alternate = true;
   if (const int rc = alternating(h, &alternate)) return rc;
