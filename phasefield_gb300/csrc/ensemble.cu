@@ -10,8 +10,8 @@
 //     third one (read one step earlier, so no block of this launch touches it). The three
 //     accumulators rotate; a launch depends only on the previous launch having finished.
 //   * one persistent launch for every instance and both degrees: a global list of cell tiles
-//     (instance, first cell), the Q1 instances' first, of which each block takes a contiguous share of
-//     either degree, with the instance's parameters (m_well, kappa) and its cell tables, built once
+//     (instance, first cell), the Q1 instances' first, of which each block takes a contiguous share,
+//     with the instance's parameters (m_well, kappa) and its cell tables, built once
 //     on the host with the engine's table builder for the instance's mesh spacing and copied into
 //     shared memory where a block's share moves on to another instance;
 //   * a tile is 32 cells on the lane kernel's layout and arithmetic (prismspf/gpu/cell_kernel_lanes.cuh:
@@ -19,10 +19,10 @@
 //     tile and several tiles a block, so both degrees fill the same block of threads;
 //   * the warps of a block and the grid size are chosen by a project-written autotuner that times
 //     candidates on the ensemble itself.
-// FP64 contractions (PPF_FP64_CONTRACTIONS=1) run on one thread per point, tiles of up to 64 cells.
-// Bound by instruction issue and the callback's FP64 operations (9 a point). 48 instances of 32 to
-// 256 cells a side: 174 us a step (8 blocks of 6 warps an SM at 40 registers; 203 us with 2 blocks of
-// 18 warps at 56), against 273 us on one thread per point with the tables copied for each tile.
+// FP64 contractions (small ensembles, or PPF_FP64_CONTRACTIONS=1) run on one thread per point, tiles of
+// up to 64 cells. Bound by instruction issue and the callback's FP64 operations (9 a point). 48 instances
+// of 32 to 256 cells a side: 169 us a step (8 blocks of 6 warps an SM at 40 registers; 203 us with 2
+// blocks of 18 warps at 56), against 273 us on one thread per point with the tables copied for each tile.
 // Natural boundary conditions (the ensemble workload has no constraints).
 #include <algorithm>
 #include <cmath>
@@ -146,10 +146,17 @@ constexpr size_t ens_lane_tile_bytes() {
   return (sizeof(pg::CellTables<2, degree, double>) + 15) / 16 * 16 + 8 * LANE_CPT * 3 * nq + 4 * LANE_CPT * 4;
 }
 
-// this block's tiles of one degree: WARPS / n tiles at a time, n warps each (cell_kernel_lanes with
-// one scalar row and one component)
+// tile groups of a degree: WARPS / n tiles, n warps each
 template <int degree, int WARPS>
-__device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long long tile0, long long ntiles) {
+__host__ __device__ constexpr long long ens_groups(long long ntiles) {
+  return (ntiles + WARPS / (degree + 1) - 1) / (WARPS / (degree + 1));
+}
+
+// this block's groups [first, last) of one degree (cell_kernel_lanes with one scalar row and one
+// component). wait() comes before the first access to what earlier launches write.
+template <int degree, int WARPS, class Wait>
+__device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long long tile0, long long ntiles,
+                               long long first, long long last, Wait&& wait) {
   using S = LaneShape<2, degree>;
   using Tab = pg::CellTables<2, degree, double>;
   namespace fx = pg::fx;
@@ -168,9 +175,13 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
   unsigned int* ex = reinterpret_cast<unsigned int*>(outs + ROW);  // [2][value row, component][cell]
   const int p0 = w * CPT + lc;
   const int step0 = w == k ? -CPT : CPT;
-  const long long steps = (ntiles + per - 1) / per;
-  const long long first = steps * blockIdx.x / gridDim.x, last = steps * (blockIdx.x + 1) / gridDim.x;
-  if (first == last) return;
+  if (first >= last) return;
+  if (sub >= per) {  // a spare warp of a degree whose tiles do not fill the block: the barriers only
+    __syncthreads();
+    for (long long step = first; step < last; ++step)
+      for (int b = 0; b < 4; ++b) __syncthreads();
+    return;
+  }
   for (int i = w * 32 + lc; i < 4 * CPT; i += cols * 32) ex[i] = (i / CPT) & 1 ? FLOOR_OUT : FLOOR;
   __syncthreads();
   int held = -1;  // the instance whose tables are in shared memory
@@ -182,9 +193,11 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
     const int inst = P.tile_inst[tile];
     const EnsInstance& I = P.inst[inst];
     if (inst != held) {  // (the tables were last read before the previous tile's last barrier)
-      const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables + I.tab_off);
-      unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
-      for (int i = w * 32 + lc; i < (int)(sizeof(Tab) / 4); i += cols * 32) dst[i] = src[i];
+      // (both 16-byte aligned and padded to whole 16 bytes)
+      const uint4* src = reinterpret_cast<const uint4*>(P.tables + I.tab_off);
+      uint4* dst = reinterpret_cast<uint4*>(tab);
+#pragma unroll 4
+      for (int i = w * 32 + lc; i < (int)((sizeof(Tab) + 15) / 16); i += cols * 32) dst[i] = __ldg(src + i);
       held = inst;
     }
     unsigned int* exi = ex + par * 2 * CPT;
@@ -198,6 +211,7 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
     const unsigned int cy = cell / (unsigned int)I.nc[0];
     const unsigned int cx = cell - cy * (unsigned int)I.nc[0];
     const long long node0 = I.off + (long long)(k * cy) * nn0 + (k * cx + w);
+    wait();
     {
       // gather: n = invM (.) acc of the previous step
       double v[n];
@@ -297,17 +311,34 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
 }
 
 template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, WARPS == 18 ? 2 : 48 / WARPS) ensemble_lane_kernel(const EnsLaunch P) {
+__global__ void __launch_bounds__(32 * WARPS, 48 / WARPS) ensemble_lane_kernel(const EnsLaunch P) {
   extern __shared__ __align__(16) unsigned char ens_lane_smem[];
-  chain_wait();
-  chain_release();
-  // zero the third accumulator (read one step earlier, untouched by this launch)
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.total_len;
-       i += (long long)gridDim.x * blockDim.x)
-    P.acc_zero[i] = 0.0;
-  ens_lane_tiles<1, WARPS>(P, ens_lane_smem, 0, P.ntiles1);
-  __syncthreads();
-  ens_lane_tiles<2, WARPS>(P, ens_lane_smem, P.ntiles1, P.ntiles - P.ntiles1);
+  bool waited = false;
+  auto wait = [&]() {
+    if (waited) return;
+    waited = true;
+    chain_wait();
+    chain_release();
+    // zero the third accumulator (read one step earlier, untouched by this launch)
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.total_len;
+         i += (long long)gridDim.x * blockDim.x)
+      P.acc_zero[i] = 0.0;
+  };
+  // an equal share of all the work, the Q1 groups first: a thread has 2 points of a Q1 group, 3 of a
+  // Q2 group. Small ensembles have at most one group a block, where a share of either degree for every
+  // block ran two, one after the other; their step is latency, so the tile's look-ups and tables,
+  // which no launch writes, come before the wait for the previous step (100 steps of 8 instances of
+  // 16 to 32 cells a side: 1.32 ms before, 0.87 ms).
+  const long long g1 = ens_groups<1, WARPS>(P.ntiles1), g2 = ens_groups<2, WARPS>(P.ntiles - P.ntiles1);
+  auto group = [&](long long b) {
+    const long long u = (2 * g1 + 3 * g2) * b / gridDim.x;
+    return u < 2 * g1 ? u / 2 : g1 + (u - 2 * g1) / 3;
+  };
+  const long long first = group(blockIdx.x), last = group(blockIdx.x + 1);
+  ens_lane_tiles<1, WARPS>(P, ens_lane_smem, 0, P.ntiles1, first, last < g1 ? last : g1, wait);
+  if (first < g1 && last > g1) __syncthreads();
+  ens_lane_tiles<2, WARPS>(P, ens_lane_smem, P.ntiles1, P.ntiles - P.ntiles1, first > g1 ? first - g1 : 0, last - g1, wait);
+  wait();
 }
 
 template <int WARPS>
@@ -319,6 +350,8 @@ constexpr size_t ens_lane_smem_bytes() {
 template <int CPB1, int CPB2, int THREADS>
 __global__ void __launch_bounds__(THREADS) ensemble_step_kernel(const EnsLaunch P) {
   extern __shared__ __align__(16) double ens_smem[];
+  chain_wait();
+  chain_release();
   // zero the third accumulator (read one step earlier, untouched by this launch)
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < P.total_len;
        i += (long long)gridDim.x * blockDim.x)
@@ -346,18 +379,25 @@ __global__ void ensemble_extract_kernel(double* out, const double* invm, const d
 }
 
 // tile-shape candidates: cells per tile for Q1 and for Q2, threads per block; on the lane layout
-// (32 cells a tile) 6, 12 or 18 warps a block
+// (32 cells a tile) 6, 12 or 3 warps a block
 struct Shape {
   int cpb1, cpb2, threads;
 };
 constexpr Shape SHAPES[] = {{64, 28, 256}, {32, 14, 128}, {16, 7, 64}};
-constexpr Shape LANE_SHAPES[] = {{LANE_CPT, LANE_CPT, 192}, {LANE_CPT, LANE_CPT, 384}, {LANE_CPT, LANE_CPT, 576}};
+constexpr Shape LANE_SHAPES[] = {{LANE_CPT, LANE_CPT, 192}, {LANE_CPT, LANE_CPT, 384}, {LANE_CPT, LANE_CPT, 96}};
 constexpr int NSHAPES = 3;
+// The default by tiles of 32 cells an SM. Up to 3 a step is the latency of one tile, shortest with one
+// thread a point and FP64 sums, 128 threads a block (100 steps of 8 instances of 16 to 32 and 20 of
+// 16 to 32 cells a side: 0.57 and 0.96 ms, lane layout 0.83 and 1.19 ms; 16 of 24 to 48, just above:
+// 1.29 ms and 1.15 ms). Up to 32, blocks of 3 warps spread the tiles over the SMs (40 instances of 32
+// to 64: 2.4 ms, 2.6 ms with 6 warps); from there on 6 warps.
+constexpr long long POINT_TILES = 3, SPREAD_TILES = 32;
+constexpr int POINT_SHAPE = 1, SPREAD_SHAPE = 2;
 Shape shape_of(bool lanes, int s) { return lanes ? LANE_SHAPES[s] : SHAPES[s]; }
 
 typedef void (*EnsKernel)(const EnsLaunch);
 EnsKernel kernel_for(bool lanes, int s) {
-  if (lanes) return s == 0 ? ensemble_lane_kernel<6> : (s == 1 ? ensemble_lane_kernel<12> : ensemble_lane_kernel<18>);
+  if (lanes) return s == 0 ? ensemble_lane_kernel<6> : (s == 1 ? ensemble_lane_kernel<12> : ensemble_lane_kernel<3>);
   switch (s) {
     case 0: return ensemble_step_kernel<64, 28, 256>;
     case 1: return ensemble_step_kernel<32, 14, 128>;
@@ -365,7 +405,7 @@ EnsKernel kernel_for(bool lanes, int s) {
   }
 }
 size_t smem_for(bool lanes, int s) {
-  if (lanes) return s == 0 ? ens_lane_smem_bytes<6>() : (s == 1 ? ens_lane_smem_bytes<12>() : ens_lane_smem_bytes<18>());
+  if (lanes) return s == 0 ? ens_lane_smem_bytes<6>() : (s == 1 ? ens_lane_smem_bytes<12>() : ens_lane_smem_bytes<3>());
   switch (s) {
     case 0: return ens_smem_bytes<64, 28>();
     case 1: return ens_smem_bytes<32, 14>();
@@ -394,9 +434,9 @@ struct ppf_ensemble_s {
   long long step = 0;  // accumulator rotation counter
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;
-  cudaGraphExec_t graph = nullptr;
-  int graph_shape = -1, graph_grid = -1;
-  long long graph_phase = -1;
+  // the captured steps, by the accumulator rotation's phase they start from
+  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
+  int graph_shape[3] = {}, graph_grid[3] = {}, graph_steps[3] = {};
   std::string err;
   double gl_w[2][3];
   double gl_D[2][3][3];
@@ -406,6 +446,13 @@ struct ppf_ensemble_s {
 
 namespace ppf {
 namespace {
+
+void drop_graphs(ppf_ensemble e) {
+  for (auto& g : e->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
 
 int efail(ppf_ensemble e, int code, const std::string& m) {
   if (e) e->err = m;
@@ -453,10 +500,7 @@ int build_tiles(ppf_ensemble e) {
     ti2[k] = ti[order[k]];
     tc2[k] = tc[order[k]];
   }
-  if (e->graph) {  // the captured steps point at the previous tile list
-    cudaGraphExecDestroy(e->graph);
-    e->graph = nullptr;
-  }
+  drop_graphs(e);  // the captured steps point at the previous tile list
   cudaFree(e->tile_inst);
   cudaFree(e->tile_cell0);
   e->ntiles = (long long)ti2.size();
@@ -490,14 +534,17 @@ int launch_step(ppf_ensemble e, long long step, cudaStream_t s) {
   const size_t smem = smem_for(e->lanes, e->shape);
   const Shape sh = shape_of(e->lanes, e->shape);
   long long grid = (long long)e->sms * e->grid_mult;
-  grid = std::max<long long>(1, std::min(grid, e->ntiles));
+  long long work = e->ntiles;
   if (e->lanes) {
-    if (launch_chained(k, dim3((unsigned)grid), dim3(sh.threads), smem, s, make_launch(e, step)) != cudaSuccess)
-      return efail(e, PPF_ERR_CUDA, "ensemble step launch failed");
-    return PPF_OK;
+    const long long t1 = e->ntiles1, t2 = e->ntiles - t1;
+    work = e->shape == 0 ? ens_groups<1, 6>(t1) + ens_groups<2, 6>(t2)
+                         : (e->shape == 1 ? ens_groups<1, 12>(t1) + ens_groups<2, 12>(t2)
+                                          : ens_groups<1, 3>(t1) + ens_groups<2, 3>(t2));
   }
-  k<<<(unsigned)grid, sh.threads, smem, s>>>(make_launch(e, step));
-  return cudaGetLastError() == cudaSuccess ? PPF_OK : efail(e, PPF_ERR_CUDA, "ensemble step launch failed");
+  grid = std::max<long long>(1, std::min(grid, work));
+  if (launch_chained(k, dim3((unsigned)grid), dim3(sh.threads), smem, s, make_launch(e, step)) != cudaSuccess)
+    return efail(e, PPF_ERR_CUDA, "ensemble step launch failed");
+  return PPF_OK;
 }
 
 }  // namespace
@@ -596,10 +643,21 @@ int ppf_ensemble_create(int n_instances, const ppf_mesh_desc* meshes, const doub
     cudaMemset(e->acc[k], 0, sizeof(double) * off);
   }
   if (cudaMalloc(&e->scratch, sizeof(double) * off) != cudaSuccess) return bail(PPF_ERR_CUDA);
+  {
+    long long tiles = 0;
+    for (const EnsInstance& I : e->h_inst) tiles += ((long long)I.nc[0] * I.nc[1] + LANE_CPT - 1) / LANE_CPT;
+    if (tiles <= POINT_TILES * e->sms) {
+      e->lanes = false;
+      e->shape = POINT_SHAPE;
+    }
+    if (e->lanes) {
+      e->grid_mult = 8;  // 48 of an SM's warps with 6 a block
+      if (tiles <= SPREAD_TILES * e->sms) e->shape = SPREAD_SHAPE;
+    }
+  }
   for (int s = 0; s < NSHAPES; ++s)
     cudaFuncSetAttribute(kernel_for(e->lanes, s), cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem_for(e->lanes, s));
-  if (e->lanes) e->grid_mult = 8;  // 48 of an SM's warps
   if (build_tiles(e)) return bail(PPF_ERR_CUDA);
   *out = e;
   return PPF_OK;
@@ -608,7 +666,7 @@ int ppf_ensemble_create(int n_instances, const ppf_mesh_desc* meshes, const doub
 void ppf_ensemble_destroy(ppf_ensemble e) {
   if (!e) return;
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->graph) cudaGraphExecDestroy(e->graph);
+  drop_graphs(e);
   cudaFree(e->d_inst);
   cudaFree(e->d_tables);
   cudaFree(e->invm);
@@ -650,29 +708,33 @@ int ppf_ensemble_download(ppf_ensemble e, int i, double* host) {
 }
 
 // advance every instance by n_steps explicit steps: one launch per step; with use_graph the
-// steps are replayed from a captured graph of three steps (one accumulator rotation)
+// steps are replayed from a captured graph of up to eight accumulator rotations (three steps each:
+// launches inside a graph overlap, successive graphs do not)
 int ppf_ensemble_run(ppf_ensemble e, int n_steps, int use_graph) {
   if (!e || n_steps < 0) return PPF_ERR_ARG;
   int done = 0;
   if (use_graph) {
-    const long long phase = e->step % 3;
-    if (!e->graph || e->graph_shape != e->shape || e->graph_grid != e->grid_mult || e->graph_phase != phase) {
-      if (e->graph) cudaGraphExecDestroy(e->graph);
-      e->graph = nullptr;
+    const int phase = (int)(e->step % 3);
+    cudaGraphExec_t& exec = e->graph[phase];
+    if (!exec || e->graph_shape[phase] != e->shape || e->graph_grid[phase] != e->grid_mult) {
+      if (exec) cudaGraphExecDestroy(exec);
+      exec = nullptr;
+      const int held = 3 * std::max(1, std::min(8, n_steps / 3));
       cudaGraph_t g;
       ENS_CUDA(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < 3; ++k) launch_step(e, e->step + k, e->stream);
+      for (int k = 0; k < held; ++k) launch_step(e, e->step + k, e->stream);
       ENS_CUDA(e, cudaStreamEndCapture(e->stream, &g));
-      ENS_CUDA(e, cudaGraphInstantiate(&e->graph, g, 0));
+      ENS_CUDA(e, cudaGraphInstantiate(&exec, g, 0));
       cudaGraphDestroy(g);
-      e->graph_shape = e->shape;
-      e->graph_grid = e->grid_mult;
-      e->graph_phase = phase;
+      e->graph_shape[phase] = e->shape;
+      e->graph_grid[phase] = e->grid_mult;
+      e->graph_steps[phase] = held;
     }
-    while (n_steps - done >= 3) {
-      ENS_CUDA(e, cudaGraphLaunch(e->graph, e->stream));
-      done += 3;
-      e->step += 3;  // phase unchanged
+    const int held = e->graph_steps[phase];
+    while (n_steps - done >= held) {
+      ENS_CUDA(e, cudaGraphLaunch(exec, e->stream));
+      done += held;
+      e->step += held;  // phase unchanged
     }
   }
   for (; done < n_steps; ++done) {
@@ -745,10 +807,7 @@ int ppf_ensemble_synchronize(ppf_ensemble e) {
 int ppf_ensemble_set_stream(ppf_ensemble e, void* stream) {
   if (!e) return PPF_ERR_ARG;
   ENS_CUDA(e, cudaStreamSynchronize(e->stream));
-  if (e->graph) {
-    cudaGraphExecDestroy(e->graph);
-    e->graph = nullptr;
-  }
+  drop_graphs(e);
   e->stream = stream ? static_cast<cudaStream_t>(stream) : e->own_stream;
   return PPF_OK;
 }

@@ -128,8 +128,8 @@ struct Eshelby {
   // inclusions near a point only: one farther than its radius + 20 widths adds less than e^-40
   // (below FP64 resolution of the sum). FP32 rules most of those out, with a lower bound of the
   // distance that allows for its own rounding; the FP64 distance decides on the others. (64^3 Q2,
-  // 40 inclusions, the whole right-hand side: 11.2 ms with the test on FP64 distances, a division
-  // and a tanh an inclusion.)
+  // 40 inclusions, the whole right-hand side, bound by the FP64 pipe, 77 % busy: 6.3 ms, 11.2 ms with
+  // the test on FP64 distances, a division and a tanh an inclusion.)
   PPF_HD ScalarValue strain_magnitude(const dealii::Point<dim, ScalarValue>& p) const {
     if (n_incl == 0) {
       ScalarValue dist_from_inclusion = p.norm();

@@ -830,15 +830,18 @@ static int choose_fx_mode(ppf_handle h, BlockPlan& P, int mode, const CellLaunch
     return PPF_OK;
   }
   const int nm = P.fx_lanes ? 4 : 3;
-  // every mode once untimed (its code is loaded then), then twice timed: launches of a few
-  // microseconds several at a time, as the gap between two events is as long as they are
+  // every mode twice. A launch of a few microseconds is no longer than the gap between two events:
+  // below 200,000 points they are timed six at a time, after one untimed launch each that loads
+  // their code (single launches picked mode 1 for 128^2 Q1 Allen-Cahn, 11.6 us an increment where
+  // the lane kernel takes 9.5 us). Larger ones are not repeated: their first run would pay for it.
   const int NT = 2 * nm;
-  const int burst = L.ncells > 200000 ? 1 : 6;
+  const bool small = L.ncells * pg::ipow(h->k + 1, h->dim) < 200000;
+  const int burst = small ? 6 : 1;
   cudaEvent_t ev[9] = {};
   cudaError_t e = cudaSuccess;
   for (int i = 0; i <= NT && e == cudaSuccess; ++i) e = cudaEventCreate(&ev[i]);
   CellLaunch T = L;
-  for (int r = -nm; r < NT && e == cudaSuccess; ++r) {
+  for (int r = small ? -nm : 0; r < NT && e == cudaSuccess; ++r) {
     if (r == 0) e = cudaEventRecord(ev[0], h->stream);
     set_fx_mode(T, timed_fx_mode((r + nm) % nm, P.fx_lanes));
     for (int k = 0; k < (r < 0 ? 1 : burst) && e == cudaSuccess; ++k)

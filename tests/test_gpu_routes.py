@@ -145,18 +145,23 @@ def test_product_in_a_caller_capture(gpu_lib):
 
 
 @pytest.mark.parametrize("tune", [False, True])
+@pytest.mark.parametrize("copies", [1, 20, 160])
 @pytest.mark.parametrize("degree", [1, 2])
-def test_ensemble_tiles(gpu_lib, degree, tune):
-    """Instances of one cell, of one row, and just past a warp's width or a tile's height."""
+def test_ensemble_tiles(gpu_lib, degree, copies, tune):
+    """Instances of one cell, of one row, and just past a warp's width or a tile's height, as few as
+    run on one thread per point and as many as take either lane layout."""
     subs = [(1, 1), (31, 1), (1, 33), (32, 5), (33, 7), (29, 13), (3, 19)]
     h = 2.0
     meshes = [RectangularMesh(dim=2, degree=degree, size=(h * a, h * b, 1.0), subdivisions=(a, b, 1)) for a, b in subs]
     rng = np.random.default_rng(degree)
     ics = [rng.uniform(0.0, 1.0, size=int(np.prod(m.nodes))) for m in meshes]
-    mw, ka, dt, steps = [1.0] * len(subs), [2.0] * len(subs), 0.01, 5
-    ens = E.Ensemble(meshes, mw, ka, dt)
-    for i, ic in enumerate(ics):
-        ens.upload(i, ic)
+    dt, steps = 0.01, 5
+    # (a spare Q1 or Q2 instance, so that a launch holds both degrees)
+    other = RectangularMesh(dim=2, degree=3 - degree, size=(h * 9, h * 4, 1.0), subdivisions=(9, 4, 1))
+    ens = E.Ensemble(meshes * copies + [other], [1.0] * (len(subs) * copies + 1), [2.0] * (len(subs) * copies + 1), dt)
+    for i in range(len(subs) * copies):
+        ens.upload(i, ics[i % len(subs)])
+    ens.upload(len(subs) * copies, np.zeros(int(np.prod(other.nodes))))
     if tune:
         ens.autotune(steps=1)  # runs every tile shape and grid
     ens.run(steps, use_graph=True)
@@ -165,7 +170,25 @@ def test_ensemble_tiles(gpu_lib, degree, tune):
         wl.mesh, wl.initial = m, {0: ics[i]}
         o = po.Oracle(wl)
         assert o.run(steps) == 0
-        assert rel_l2(ens.download(i), o.get(0, 1)) < 1e-9, subs[i]
+        for j in (i, len(subs) * (copies - 1) + i):
+            assert rel_l2(ens.download(j), o.get(0, 1)) < 1e-9, (subs[i], j)
+    assert np.all(ens.download(len(subs) * copies) == 0.0)
+
+
+@pytest.mark.parametrize("runs", [(2,), (30, 5, 24), (7, 7, 7)])
+def test_ensemble_graphs(gpu_lib, runs):
+    """Runs from every phase of the accumulator rotation, shorter and longer than a captured graph."""
+    meshes, mw, ka, ics = E.allen_cahn_ensemble(n_instances=5, min_cells=8, max_cells=24, seed=3)
+    res = []
+    for use_graph in (False, True):
+        ens = E.Ensemble(meshes, mw, ka, 0.01)
+        for i, ic in enumerate(ics):
+            ens.upload(i, ic)
+        for n in runs:
+            ens.run(n, use_graph=use_graph)
+        res.append([ens.download(i) for i in range(len(meshes))])
+    for a, b in zip(*res):
+        assert rel_l2(b, a) < 1e-12
 
 
 def test_inclusions_ruled_out_by_distance(gpu_lib):
