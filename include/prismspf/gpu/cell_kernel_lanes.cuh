@@ -37,9 +37,9 @@
 // Accuracy: every derivative and every node's integral is one rounding of an exact sum of values
 // cut to 2^-59 (derivatives) or 2^-57 (integration, 2^-59 on Q1 cells) of the largest magnitude of their cell and row.
 //
-// What bounds it: instruction issue (58-61 % of the slots, the ALU pipe 50-57 % busy, the FP64 pipe
-// 31-55 %; DRAM 4 %). Cahn-Hilliard 64^3 Q2, per launch of the c and the mu block: 130 and 157 us at
-// 444 instructions a point, against 208 and 213 us at 690 with rounded instead of cut conversions,
+// What bounds it: instruction issue (53-61 % of the slots at 32 warps an SM, the ALU pipe 42-49 %, the
+// FP64 pipe 34-59 %; DRAM 3-5 %). Cahn-Hilliard 64^3 Q2, per launch of the c and the mu block: 130 and
+// 157 us at 460 instructions a point, against 208 and 213 us at 690 with rounded instead of cut conversions,
 // weights as 64-bit shifts and the terms through shared memory, and 243 and 293 us for cell_kernel.
 // Stretched cells (64 x 60 x 52): 105 and 128 us against 188 and 226 us for cell_kernel.
 #pragma once
