@@ -596,19 +596,7 @@ class FieldContainer {
         // a row declared without gradients has no fixed-point copy (exponent -1)
       }
     }
-    if constexpr (std::is_same<number, float>::value && degree <= 2) {
-      // the FP32 lane kernel: the own value (one load for all directions), then the others of the line
-      if (ctx.lean) {
-        const number* u = ctx.vals + row * ctx.stride + ctx.pe;
-        const number* Dr = ctx.tab->Dh[d][ctx.qi[d]];
-        const int st = ctx.step[d], i = ctx.qi[d];
-        if (n > 2 && i == 1) return fma(Dr[n - 1], u[st], fma(Dr[0], u[-st], Dr[1] * u[0]));
-        number s = fma(Dr[n > 2 ? 1 : 1 - i], u[st], Dr[i] * u[0]);
-        if (n > 2) s = fma(Dr[2 - i], u[2 * st], s);
-        return s;
-      }
-    }
-    // contraction over the nodal values
+    // FP64 contraction over the nodal values
     const int q0 = ctx.q - qd * stride_d;
     const number* Dr = ctx.tab->Dh[d][qd];
     if (ctx.cpt) {

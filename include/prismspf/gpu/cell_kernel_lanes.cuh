@@ -453,51 +453,35 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
 // FP32 operators (the smoothing levels of a mixed-precision V-cycle) on the same layout: 32 cells
 // a tile, a line of each cell per thread, plain FP32 contractions (derivatives from the nodal
 // values, integration with the tables' jdt weights), so a tile needs two barriers (nodal values;
-// submitted terms). Any cell shape. Shared-memory accesses bound it: the terms of the thread's
-// line stay in registers (only the others' along the first directions are read back), no row is
-// cleared, and a point's own value is loaded once, 36 accesses a point of a 3-component gradient
-// operator on Q2 3-D instead of 84.
+// submitted terms). Any cell shape. (Keeping the terms of a thread's line in registers, 36 instead of
+// 84 shared accesses a point, is no faster: 143 against 134 us for the 64^3 Q2 elasticity product.)
 template <int dim, int degree>
-__host__ __device__ constexpr size_t lane_f32_smem_bytes(int nrows_in, int nout) {
+__host__ __device__ constexpr size_t lane_f32_smem_bytes(int nrows_in, int nrows_out) {
   using S = LaneShape<dim, degree>;
-  return (size_t)S::nq * LANE_CPT * 4 * (size_t)(nrows_in + nout * (dim - 1));
+  return (size_t)S::nq * LANE_CPT * 4 * (size_t)(nrows_in + nrows_out);
 }
 
-// resident blocks of the FP32 kernel: its unrolled line holds n (1 + dim) terms a component,
-// 72 registers without a spill (64^3 Q2 elasticity, GMG-CG in mixed precision: 125 ms a solve, 137 ms
-// with the terms in shared memory, 144 ms at 96 registers)
-template <class PDE, int dim, int degree, int NC>
-constexpr int lane_f32_min_blocks() {
-  using S = LaneShape<dim, degree>;
-  constexpr int regs = CellLaneMinBlocks<PDE, S::threads>::value;
-  constexpr int line = 65536 / (S::threads * 72);
-  return NC == 1 || regs < line ? regs : (line > 0 ? line : 1);
-}
-
-template <class PDE, int dim, int degree, int NC, int MINB>
+template <class PDE, int dim, int degree, int MODE, int MINB>
 __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
     cell_kernel_lanes_f32(const __grid_constant__ CellLaunch P, const __grid_constant__ PDE pde,
                           const __grid_constant__ pg::CellTables<dim, degree, float> T,
                           const __grid_constant__ LaneRows R) {
-  static_assert(degree <= 2, "the FP32 lane kernel covers Q1/Q2 LHS launches");
+  static_assert(degree <= 2 && MODE == MODE_LHS, "the FP32 lane kernel covers Q1/Q2 LHS launches");
   using S = LaneShape<dim, degree>;
   using Tab = pg::CellTables<dim, degree, float>;
   constexpr int n = S::n, nq = S::nq, cols = S::cols, k = degree, CPT = LANE_CPT;
   constexpr int ROW = nq * CPT;
   constexpr int JS = cols * CPT;
-  constexpr int TC = 1 + dim;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Tab* tab = &T;
   float* vals = reinterpret_cast<float*>(smem_raw);  // [nin][q][cell]
-  float* outs = vals + R.nin * ROW;                  // gradient terms of the first directions [NC][dim - 1][q][cell]
+  float* outs = vals + R.nin * ROW;                  // [out rows][q][cell]
   const int t = threadIdx.x;
   const int lc = t & 31;
-  const int w = __shfl_sync(0xffffffffu, t >> 5, 0);
+  const int w = t >> 5;
   const int p0 = w * CPT + lc;
   const int qa = w % n;
   const int qb = dim > 2 ? w / n : 0;
-  const int step0 = qa == k ? -CPT : CPT;
-  const int step1 = qb == k ? -n * CPT : n * CPT;
   const unsigned int nn0 = (unsigned int)P.nn[0], nn1 = (unsigned int)P.nn[1];
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;
   const unsigned int ncells = (unsigned int)P.ncells;
@@ -522,8 +506,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
     }
     const unsigned int node0 = dim > 2 ? ((unsigned int)(k * cz) * nn1 + (unsigned int)(k * cy + qb)) * nn0 + (unsigned int)(k * cx + qa)
                                        : (unsigned int)(k * cy) * nn0 + (unsigned int)(k * cx + qa);
-    // every thread is past the previous tile's callbacks (it has passed their barrier), which were
-    // the last to read the nodal values
+    // the previous tile's integration read the submitted terms and values: done by all threads
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < LANE_MAX_IN; ++r) {
       if (r < R.nin) {
@@ -543,16 +527,22 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
         }
       }
     }
-    __syncthreads();  // nodal values visible; the previous tile's terms read by all
+#pragma unroll
+    for (int o = 0; o < LANE_MAX_OUT; ++o)
+      if (o < R.nout)
+#pragma unroll
+        for (int i = 0; i <= dim; ++i)
+#pragma unroll
+          for (int j = 0; j < n; ++j) outs[(R.out_row[o] + i) * ROW + p0 + j * JS] = 0.f;
+    __syncthreads();  // nodal values visible
 
     const SimulationTimer& timer = P.timer_dev ? *P.timer_dev : P.timer;
-    float term[n][NC * TC];
-#pragma unroll
+#pragma unroll 1
     for (int j = 0; j < n; ++j) {
       pg::CellCtx<dim, degree, float> ctx;
       ctx.tab = tab;
       ctx.vals = vals;
-      ctx.outs = nullptr;
+      ctx.outs = outs;
       ctx.stride = ROW;
       ctx.lc = lc;
       ctx.q = w + j * cols;
@@ -562,56 +552,33 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
       ctx.err = P.err;
       ctx.submitted = 0;
       ctx.cpt = CPT;
-      ctx.lean = 1;
-      ctx.qi[0] = qa;
-      ctx.qi[1] = dim > 2 ? qb : j;
-      ctx.qi[2] = dim > 2 ? j : 0;
-      ctx.pe = p0 + j * JS;
-      ctx.step[0] = step0;
-      ctx.step[1] = dim > 2 ? step1 : (j == k ? -JS : JS);
-      ctx.step[2] = dim > 2 ? (j == k ? -JS : JS) : 0;
-      ctx.nterm = NC;
-#pragma unroll
-      for (int i = 0; i < NC * TC; ++i) ctx.term[i] = 0.f;
       FieldContainer<dim, degree, float> fc(ctx);
       pde.compute_lhs(fc, timer, P.block_id);
-#pragma unroll
-      for (int i = 0; i < NC * TC; ++i) term[j][i] = ctx.term[i];
     }
-#pragma unroll
-    for (int o = 0; o < NC; ++o)
-#pragma unroll
-      for (int d = 0; d < dim - 1; ++d)
-#pragma unroll
-        for (int j = 0; j < n; ++j) outs[(o * (dim - 1) + d) * ROW + p0 + j * JS] = term[j][o * TC + 1 + d];
     __syncthreads();  // submitted terms visible
 
-    // integrate (the tables' jdt weights; the own terms from registers) and scatter
+    // integrate (the tables' jdt weights) and scatter
 #pragma unroll
-    for (int j = 0; j < n; ++j) {
-      const int q = w + j * cols;
+    for (int o = 0; o < LANE_MAX_OUT; ++o) {
+      if (o < R.nout) {
+        const int rv = R.out_row[o];
 #pragma unroll
-      for (int o = 0; o < NC; ++o) {
-        float r = term[j][o * TC] * tab->jxw[q];
+        for (int j = 0; j < n; ++j) {
+          const int q = w + j * cols;
+          const int qi[3] = {qa, dim > 2 ? qb : j, dim > 2 ? j : 0};
+          float r = outs[rv * ROW + p0 + j * JS];
 #pragma unroll
-        for (int d = 0; d < dim - 1; ++d) {
-          const float* g = outs + (o * (dim - 1) + d) * ROW + p0 + j * JS;
-          const float* wt = tab->jdt[d][q];
-          const int st = d == 0 ? step0 : step1, id = d == 0 ? qa : qb;
-          r = fmaf(wt[id], term[j][o * TC + 1 + d], r);
-          if (n > 2 && id == 1) {
-            r = fmaf(wt[0], g[-st], r);
-            r = fmaf(wt[n - 1], g[st], r);
-          } else {
-            r = fmaf(wt[n > 2 ? 1 : 1 - id], g[st], r);
-            if (n > 2) r = fmaf(wt[2 - id], g[2 * st], r);
+          for (int d = 0; d < dim; ++d) {
+            const int sd = d == 0 ? 1 : (d == 1 ? n : n * n);
+            const float* g = outs + (rv + 1 + d) * ROW + (q - qi[d] * sd) * CPT + lc;
+            const float* wt = tab->jdt[d][q];
+#pragma unroll
+            for (int m = 0; m < n; ++m) r = fmaf(wt[m], g[m * sd * CPT], r);
           }
+          const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
+          const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
+          if (active && target >= 0) atomicAdd(global_ptr(reinterpret_cast<float*>(R.out_acc[o]) + target), r);
         }
-#pragma unroll
-        for (int m = 0; m < n; ++m) r = fmaf(tab->jdt[dim - 1][q][m], term[m][o * TC + dim], r);
-        const unsigned int idx = node0 + (unsigned int)j * lstride + R.out_off[o];
-        const int target = R.out_cmap[o] ? __ldg(R.out_cmap[o] + idx) : (int)idx;
-        if (active && target >= 0) atomicAdd(global_ptr(reinterpret_cast<float*>(R.out_acc[o]) + target), r);
       }
     }
   }
@@ -689,11 +656,11 @@ cudaError_t launch_lanes(const CellLaunch& P, const LaneRows& R, const void* obj
                         *reinterpret_cast<const pg::CellTables<dim, degree, double>*>(P.tables_host), R);
 }
 
-template <class PDE, int dim, int degree, int NC>
+template <class PDE, int dim, int degree, int MINB>
 cudaError_t launch_lanes_f32(const CellLaunch& P, const LaneRows& R, const void* obj, cudaStream_t s) {
   using S = LaneShape<dim, degree>;
-  auto kern = cell_kernel_lanes_f32<PDE, dim, degree, NC, lane_f32_min_blocks<PDE, dim, degree, NC>()>;
-  const size_t smem = lane_f32_smem_bytes<dim, degree>(R.nin, NC);
+  auto kern = cell_kernel_lanes_f32<PDE, dim, degree, MODE_LHS, MINB>;
+  const size_t smem = lane_f32_smem_bytes<dim, degree>(R.nin, P.nrows_out);
   constexpr int MAX_DEVICES = 64;
   static size_t attr_smem_of[MAX_DEVICES] = {};
   static int occ_of[MAX_DEVICES] = {};
@@ -727,19 +694,11 @@ cudaError_t launch_lanes_f32(const CellLaunch& P, const LaneRows& R, const void*
 // the FP32 lane kernel for an FP32 Q1/Q2 left-hand side, or cudaErrorNotSupported
 template <class PDE, int dim, int degree>
 cudaError_t launch_cell_kernel_lanes_f32_impl(const CellLaunch& P, const void* obj, cudaStream_t s) {
+  constexpr int MINB = CellLaneMinBlocks<PDE, LaneShape<dim, degree>::threads>::value;
   LaneRows R;
   if (!P.tables_host || !lane_rows(P, dim, &R)) return cudaErrorNotSupported;
-  if (lane_f32_smem_bytes<dim, degree>(R.nin, R.nout) > 232448) return cudaErrorNotSupported;
-  constexpr unsigned int C = CellLaneComponents<PDE>::value;
-  if constexpr (C & 2u)
-    if (R.nout == 1) return launch_lanes_f32<PDE, dim, degree, 1>(P, R, obj, s);
-  if constexpr (C & 4u)
-    if (R.nout == 2) return launch_lanes_f32<PDE, dim, degree, 2>(P, R, obj, s);
-  if constexpr (C & 8u)
-    if (R.nout == 3) return launch_lanes_f32<PDE, dim, degree, 3>(P, R, obj, s);
-  if constexpr (C & 16u)
-    if (R.nout == 4) return launch_lanes_f32<PDE, dim, degree, 4>(P, R, obj, s);
-  return cudaErrorNotSupported;
+  if (lane_f32_smem_bytes<dim, degree>(R.nin, P.nrows_out) > 232448) return cudaErrorNotSupported;
+  return launch_lanes_f32<PDE, dim, degree, MINB>(P, R, obj, s);
 }
 
 // launches the lane kernel, or returns cudaErrorNotSupported when the launch's rows exceed its
