@@ -430,8 +430,8 @@ int ppf_tangent_linear(ppf_handle h, int block, int n_steps, const double* du0, 
 long long ppf_checkpoint_schedule_cost(int n_steps, int n_snapshots);
 
 /* Replay the explicit increment loop of ppf_run from a CUDA graph (on by default): one graph
- * holds as many increments as the age-rotation period, each followed by a device-side timer
- * advance. Used from increment 2 on when every block is Explicit or Constant, no PostProcess
+ * holds up to eight age-rotation periods of increments, which advance the device-side timer; fewer
+ * increments than it holds run as plain launches. Used from increment 2 on when every block is Explicit or Constant, no PostProcess
  * output is requested and kernel timing is off. */
 int ppf_set_use_graph(ppf_handle h, int on);
 
