@@ -415,7 +415,7 @@ int ppf_ensemble_set_stream(ppf_ensemble e, void* stream);
  *
  * ppf_adjoint_forward: runs n_steps explicit steps from the fields' current vectors (u_0),
  *   keeping n_snapshots checkpoint slots (u_0 included) placed by the binomial schedule; the
- *   fields' current vectors then hold u_K.
+ *   fields' current vectors then hold u_K and their old_1 vectors u_{K-1}, as after a run.
  * ppf_adjoint_backward: from dJ/du_K returns dJ/d(Mc, Kn) and dJ/du_0, recomputing the
  *   states it needs from the checkpoints; forward_steps reports the forward steps taken by the
  *   forward and backward calls together.

@@ -343,16 +343,20 @@ int ppf_adjoint_forward(ppf_handle h, int b, int n_steps, int n_snapshots) {
     a = m;
     --s;
   }
-  // u_K into the work slot and the fields' current vectors
-  const int src = slot_of_step(A, a);
+  // on to u_{K-1}, and the last step on the fields' own vectors: as after a run, old_1 holds u_{K-1}
+  // and the current vectors u_K
   double* work = A.slot[A.S];
-  PPF_CUDA(h, cudaMemcpyAsync(work, A.slot[src], sizeof(double) * 2 * A.N, cudaMemcpyDeviceToDevice, h->stream));
-  for (int k = a; k < n_steps; ++k) {
-    rc = forward_step(h, A, work, work);
+  double* u = A.slot[slot_of_step(A, a)];
+  for (int k = a; k + 1 < n_steps; ++k) {
+    rc = forward_step(h, A, u, work);
     if (rc) return rc;
+    u = work;
   }
-  PPF_CUDA(h, cudaMemcpyAsync(f.c->cur, work, sizeof(double) * A.N, cudaMemcpyDeviceToDevice, h->stream));
-  PPF_CUDA(h, cudaMemcpyAsync(f.n->cur, work + A.N, sizeof(double) * A.N, cudaMemcpyDeviceToDevice, h->stream));
+  PPF_CUDA(h, cudaMemcpyAsync(f.c->old[0], u, sizeof(double) * A.N, cudaMemcpyDeviceToDevice, h->stream));
+  PPF_CUDA(h, cudaMemcpyAsync(f.n->old[0], u + A.N, sizeof(double) * A.N, cudaMemcpyDeviceToDevice, h->stream));
+  rc = explicit_solve_entry(h, b);
+  if (rc) return rc;
+  A.forward_steps++;
   return check_err(h);
 }
 
