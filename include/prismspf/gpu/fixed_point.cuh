@@ -286,14 +286,15 @@ PPF_FX long long to_fixed_cut_scaled(double v, unsigned int Ehi, unsigned long l
 }
 
 // the general case of to_double_cut: any |x| = a < 2^63, exponents beyond the normal range (an
-// infinity or a NaN), a quiet NaN when `bad`
+// infinity), a quiet NaN when `bad`
 PPF_FX double to_double_any(unsigned long long a, unsigned int sign, int lsb, bool bad) {
   if (bad) return quiet_nan();
   if (a == 0) return 0.0;
   const int lz = clz64(a);  // at least 1
   const unsigned long long r = ((a << (lz - 1)) + 0x200ull) >> 10;
   const int be1 = 1085 + lsb - lz;
-  const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)(be1 < 2046 ? be1 : 2046) << 20);
+  if (be1 >= 2046) return double_of(join(0u, 0x7ff00000u | sign));
+  const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)be1 << 20);
   return double_of(join((unsigned int)r, hi | sign));
 }
 
