@@ -112,6 +112,8 @@ struct CellTables {
   // at a float's exponent position, EXP_BIAS more so that it is never negative
   unsigned int hadd;
   unsigned int radd[3];
+  // the least block exponents of the gradient rows and (EXP_BIAS more) of the terms, likewise
+  unsigned int floor_in, floor_out;
 };
 
 template <int dim, int degree, typename number = double>

@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   constexpr int TOPT = n == 2 ? fx::LANE_TOP_INTEGRAL_Q1 : fx::LANE_TOP_INTEGRAL;
   constexpr int TC = 1 + dim;     // terms of a component
   constexpr bool REGS = NC == 1;
-  constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20, FLOOR_OUT = (fx::EXP_FLOOR + fx::EXP_BIAS) << 20;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // the tables are a kernel parameter: read-only constant-bank loads, uniform where their index is
   const Tab* tab = &T;
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const int step1 = qb == k ? -n * CPT : n * CPT;
   const int hpow2 = tab->hpow2, hk = tab->hk;
   const unsigned long long hsig = tab->hsig;
-  for (int i = t; i < 2 * (R.ng + NC) * CPT; i += S::threads) ex_in[i] = i < 2 * R.ng * CPT ? FLOOR : FLOOR_OUT;
+  for (int i = t; i < 2 * (R.ng + NC) * CPT; i += S::threads) ex_in[i] = i < 2 * R.ng * CPT ? tab->floor_in : tab->floor_out;
   const unsigned int nn0 = (unsigned int)P.nn[0], nn1 = (unsigned int)P.nn[1];
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;  // lattice stride of the last direction
   const unsigned int ncells = (unsigned int)P.ncells;
@@ -276,8 +275,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
         for (int j = 0; j < n; ++j) x[j * JS] = fx::to_fixed_cut<fx::LANE_TOP_VALUES>(__longlong_as_double(x[j * JS]), E);
       }
     }
-    for (int g = w; g < R.ng; g += cols) exn[g * CPT + lc] = FLOOR;
-    for (int o = w; o < NC; o += cols) exon[o * CPT + lc] = FLOOR_OUT;
+    for (int g = w; g < R.ng; g += cols) exn[g * CPT + lc] = tab->floor_in;
+    for (int o = w; o < NC; o += cols) exon[o * CPT + lc] = tab->floor_out;
     __syncthreads();  // fixed-point copies visible
 
     // the user callback at each of the thread's points

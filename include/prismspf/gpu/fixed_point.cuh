@@ -214,10 +214,14 @@ PPF_FX double to_double_fast(long long x, int lsb, unsigned long long sig, bool 
 }
 
 // The conversions of the lane kernel's rows. They differ from to_fixed_fast / to_double_fast in what
-// their callers guarantee: block exponents are at least EXP_FLOOR (rows start their exponent there),
-// and the scales of an operator are within 2^+-MAX_SCALE (the tables leave the lane kernel off
-// otherwise), so that no result falls below the normal range and zeros need no test of their own.
-constexpr int EXP_FLOOR = 192;
+// their callers guarantee: block exponents are at least EXP_FLOOR (rows start their exponent there, or
+// where a scale asks for it: lane_floor), so that zeros, which get no test of their own, shift out and
+// results of more than 32 bits are normal numbers; and the scales of an operator are within
+// 2^+-MAX_SCALE (the tables leave the lane kernel off otherwise). A cell whose largest value lies below
+// 2^(EXP_FLOOR - 1023) = 5e-289 keeps the resolution of that one, 2^-1018 or 16 times the smallest
+// normal number. (Tests for zeros in place of the floor, in a branch for smaller cells, took 3 % more
+// for Cahn-Hilliard 64^3 Q2 and 4 % for the 48^3 elasticity product.)
+constexpr int EXP_FLOOR = 64;
 // fixed-point tops of the lane kernel: |3 u + 4 v + w| <= 8 * 2^60 keeps a derivative's line sum
 // below 2^63; so does |x + sum_d L_d|, a node's integral over its weight, which is at most
 // (1 + 3 * 2) 2^60 on Q1 cells and (1 + 3 * 8) 2^58 on Q2 cells
@@ -227,6 +231,9 @@ constexpr int LANE_TOP_INTEGRAL = 57;
 constexpr int MAX_SCALE = 60;
 constexpr int EXP_BIAS = 64;    // of the exponents of scaled terms
 constexpr int EXP_WIDE = 1900;  // block exponents from here on may give results beyond the range
+// the least block exponent of a row whose entries are scaled by 2^up at most before they are converted,
+// and whose sums, of fixed-point top 57 to 59, are by 2^down at least afterwards
+inline int lane_floor(int up, int down) { return std::max(EXP_FLOOR + std::max(up, 0), 32 - down); }
 
 // a >> r for any r >= 0 (zero from 64 up)
 PPF_FX unsigned long long shr64(unsigned long long a, unsigned int r) {
@@ -274,7 +281,7 @@ PPF_FX long long to_fixed_cut(double v, unsigned int Ehi) {
 PPF_FX unsigned int high_exponent(int E) { return ((unsigned int)E << 20) | 0xfffffu; }
 
 // v * sigma * 2^(k + 1023 + TOP - E) rounded towards zero, sigma = sig / 2^63 in [1, 2), for
-// exponent(v) + k + 1 <= E and E >= EXP_FLOOR
+// exponent(v) + k + 1 <= E and E >= EXP_FLOOR + k
 template <int TOP>
 PPF_FX long long to_fixed_cut_scaled(double v, unsigned int Ehi, unsigned long long sig, int k) {
   static_assert(TOP >= 52 && TOP <= 60, "fixed-point top out of range");
@@ -285,14 +292,15 @@ PPF_FX long long to_fixed_cut_scaled(double v, unsigned int Ehi, unsigned long l
   return with_sign(shr64(P, ((Ehi - ((unsigned int)k << 20) - (hi & 0x7fffffffu)) >> 20) + (62u - TOP)), hi);
 }
 
-// the general case of to_double_cut: any |x| = a < 2^63, exponents beyond the normal range (an
-// infinity), a quiet NaN when `bad`
+// the general case of to_double_cut: any |x| = a < 2^63, exponents above the normal range (an
+// infinity) or below it (a signed zero), a quiet NaN when `bad`
 PPF_FX double to_double_any(unsigned long long a, unsigned int sign, int lsb, bool bad) {
   if (bad) return quiet_nan();
   if (a == 0) return 0.0;
   const int lz = clz64(a);  // at least 1
   const unsigned long long r = ((a << (lz - 1)) + 0x200ull) >> 10;
   const int be1 = 1085 + lsb - lz;
+  if (be1 < 0) return double_of(join(0u, sign));
   if (be1 >= 2046) return double_of(join(0u, 0x7ff00000u | sign));
   const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)be1 << 20);
   return double_of(join((unsigned int)r, hi | sign));
@@ -300,8 +308,8 @@ PPF_FX double to_double_any(unsigned long long a, unsigned int sign, int lsb, bo
 
 // (+-x) * 2^lsb, or (+-x) * 2^lsb * sigma when `scaled` (from the product's floor to a multiple of
 // 2^(lsb + 1)), |x| < 2^63, rounded to nearest (ties away from zero), with x negated when `flip` is
-// the sign bit's mask (else 0); a quiet NaN when `bad`. The caller's E and scales keep the result
-// above the subnormal range, and below infinity unless `wide`. The common case (more than 32
+// the sign bit's mask (else 0); a quiet NaN when `bad`. The caller's E and scales keep a result of
+// more than 32 bits above the subnormal range, and below infinity unless `wide`. The common case (more than 32
 // significant bits) takes 32-bit shifts and adds only, the rest to_double_any: selects in place of
 // that branch measured slower (Cahn-Hilliard 64^3 Q2: 142 against 130 us a launch).
 PPF_FX double to_double_cut(long long x, int lsb, unsigned long long sig, bool scaled, bool wide, bool bad,

@@ -163,7 +163,7 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
   constexpr int n = S::n, nq = S::nq, cols = S::cols, k = degree, CPT = LANE_CPT, per = WARPS / cols;
   constexpr int ROW = nq * CPT, JS = cols * CPT;
   constexpr int TOPT = n == 2 ? fx::LANE_TOP_INTEGRAL_Q1 : fx::LANE_TOP_INTEGRAL;
-  constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20, FLOOR_OUT = (fx::EXP_FLOOR + fx::EXP_BIAS) << 20;
+  constexpr unsigned int FLOOR = fx::EXP_FLOOR << 20;
   const int lc = threadIdx.x & 31;
   const int wi = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
   const int sub = wi / cols, w = wi - sub * cols;  // tile of the block's group, point of the first direction
@@ -182,7 +182,8 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
       for (int b = 0; b < 4; ++b) __syncthreads();
     return;
   }
-  for (int i = w * 32 + lc; i < 4 * CPT; i += cols * 32) ex[i] = (i / CPT) & 1 ? FLOOR_OUT : FLOOR;
+  // (the terms' floor is the instance's, below)
+  for (int i = w * 32 + lc; i < 4 * CPT; i += cols * 32) ex[i] = (i / CPT) & 1 ? 0u : FLOOR;
   __syncthreads();
   int held = -1;  // the instance whose tables are in shared memory
   int par = 0;
@@ -231,7 +232,7 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
 #pragma unroll
       for (int j = 0; j < n; ++j) vfx[p0 + j * JS] = fx::to_fixed_cut<fx::LANE_TOP_VALUES>(vals[p0 + j * JS], E);
       if (w == 0) exn[lc] = FLOOR;
-      if (w == cols - 1) exn[CPT + lc] = FLOOR_OUT;
+      if (w == cols - 1) exn[CPT + lc] = 0u;
     }
     __syncthreads();  // fixed-point copies visible
     AllenCahn<2, degree, double> pde{I.m_well, I.kappa};
@@ -275,7 +276,7 @@ __device__ void ens_lane_tiles(const EnsLaunch& P, unsigned char* smem, long lon
     }
     {
       const unsigned int raw = max(max(em[0], em[1]), em[2]);
-      const unsigned int e = max(max(em[0] + tab->hadd, em[1] + tab->radd[0]), em[2] + tab->radd[1]);
+      const unsigned int e = max(max(em[0] + tab->hadd, em[1] + tab->radd[0]), max(em[2] + tab->radd[1], tab->floor_out));
       atomicMax(&exo[lc], raw >= 0x7ff00000u ? 0xfff00000u : e);
     }
     __syncthreads();  // the terms' block exponents complete
@@ -604,7 +605,8 @@ int ppf_ensemble_create(int n_instances, const ppf_mesh_desc* meshes, const doub
         return PPF_ERR_UNSUPPORTED;
       }
       I.tab_off = (long long)tables.size();
-      e->lanes = (i == 0 || e->lanes) && tables_lanes(tb, 2, I.degree) != 0;
+      // (the lane body's value rows start from the floor of cells up to 2^32, EXP_FLOOR)
+      e->lanes = (i == 0 || e->lanes) && tables_lanes(tb, 2, I.degree) != 0 && std::max(I.h[0], I.h[1]) <= 0x1p32;
       tables.insert(tables.end(), tb.begin(), tb.end());
       tables.resize((tables.size() + 15) / 16 * 16, 0);
     }

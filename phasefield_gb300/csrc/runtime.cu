@@ -222,6 +222,8 @@ static void fixed_point_tables(pg::CellTables<dim, degree, double>& t, const GLR
   }
   t.hadd = (unsigned int)(t.hk + (t.hpow2 ? 0 : 1) + pg::fx::EXP_BIAS) << 20;
   for (int d = 0; d < 3; ++d) t.radd[d] = (unsigned int)(t.rk[d] + (t.rpow2[d] ? 0 : 1) + pg::fx::EXP_BIAS) << 20;
+  t.floor_in = (unsigned int)pg::fx::lane_floor(0, std::min({0, t.dk[0], t.dk[1], t.dk[2]})) << 20;
+  t.floor_out = (unsigned int)(pg::fx::lane_floor(std::max({t.hk, t.rk[0], t.rk[1], t.rk[2]}), t.ik[0]) + pg::fx::EXP_BIAS) << 20;
   t.fx_lanes = in_range ? 1 : 0;
   t.fx = 1;
 }
