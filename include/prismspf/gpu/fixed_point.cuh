@@ -228,9 +228,14 @@ constexpr int EXP_FLOOR = 64;
 constexpr int LANE_TOP_VALUES = 59;
 constexpr int LANE_TOP_INTEGRAL_Q1 = 59;
 constexpr int LANE_TOP_INTEGRAL = 57;
-constexpr int MAX_SCALE = 60;
-constexpr int EXP_BIAS = 64;    // of the exponents of scaled terms
-constexpr int EXP_WIDE = 1900;  // block exponents from here on may give results beyond the range
+// The scales are 1/h_d, h_0, h_0 / h_d and the integral's detJ / (h_0 W^dim), W = 2 or 6 by degree, so
+// 2^+-MAX_SCALE is any box with edges of a cell between 2^-146 and 2^154 in 3-D (2^-290 and 2^300 in
+// 2-D) whose ratios are below 2^300. The bound keeps exponents of scaled terms within a high word's 12
+// bits above the mantissa (EXP_BIAS and the largest, 2046 + 301 + EXP_BIAS < 4095) and the results of
+// exponents below EXP_WIDE below 2^1023.
+constexpr int MAX_SCALE = 300;
+constexpr int EXP_BIAS = 320;   // of the exponents of scaled terms
+constexpr int EXP_WIDE = 1700;  // block exponents from here on may give results beyond the range
 // the least block exponent of a row whose entries are scaled by 2^up at most before they are converted,
 // and whose sums, of fixed-point top 57 to 59, are by 2^down at least afterwards
 inline int lane_floor(int up, int down) { return std::max(EXP_FLOOR + std::max(up, 0), 32 - down); }

@@ -80,3 +80,32 @@ def test_small_fields_in_an_ensemble(gpu_lib, degree, scale):
         o = po.Oracle(wl)
         assert o.run(3) == 0
         assert rel_l2(ens.download(i), o.get(0, 1), scale) < 1e-9, sub[i]
+
+
+@pytest.mark.parametrize("h", [1e-9, 3e-13, 1e-30, 2.0e25])
+@pytest.mark.parametrize("dim,degree,stretch,mode", [
+    (2, 1, 1.0, 4), (2, 2, 1.7, 5), (3, 1, 1.0, 4), (3, 1, 1.7, 5), (3, 2, 1.0, 4), (3, 2, 0.6, 5),
+])
+def test_cells_of_any_size(gpu_lib, monkeypatch, dim, degree, stretch, mode, h):
+    """A grid in nanometres given in metres, and farther out: the lane kernel is offered and is as exact."""
+    monkeypatch.setenv("PPF_CONTRACTION_MODE", str(mode))
+    sub = (5, 4, 3)[:dim] + (1,) * (3 - dim)
+    wl = W.cahn_hilliard_3d(refine=0, degree=degree, dim=dim, size=1.0, subdivisions=sub, dt=1e-2 * h * h)
+    wl.constants = [1.0, 1.5 * h * h, 4.0]
+    wl.mesh.size = tuple(n * h * stretch ** d for d, n in enumerate(sub))
+    p, o = wl.make_problem(), po.Oracle(wl)
+    rng = np.random.default_rng(9)
+    c, mu = rng.uniform(0.2, 0.8, p.n_nodes), rng.uniform(-1, 1, p.n_nodes)
+    for f, v, age in ((0, c, 0), (0, c, 1), (1, mu, 1)):
+        p.upload(f, v, age=age)
+        o.set(f, v, age=age)
+    for b in (0, 1):
+        assert rel_l2(p.apply(b, 0, None, scale=1), o.apply(b, 0, None, scale=1)) < 1e-12, b
+        assert p.contraction_mode(b, 0) == mode
+    wl = elasticity(dim, degree, tuple(h * stretch ** d for d in range(dim)))
+    p, o = wl.make_problem(), po.Oracle(wl)
+    u = rng.normal(size=p.field_length(0)) * h
+    for scale in (0, 2):
+        got, ref = p.apply(0, 1, u, scale=scale), o.apply(0, 1, u, scale=scale)
+        assert rel_l2(got, ref, np.abs(ref).max()) < 1e-12
+    assert p.contraction_mode(0, 1) == mode
