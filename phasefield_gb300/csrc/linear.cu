@@ -467,7 +467,9 @@ static unsigned dot_blocks(long long n) { return (unsigned)std::max<long long>(1
 
 static unsigned int* counters(LinearState& L) { return reinterpret_cast<unsigned int*>(L.partial + 2048); }
 
-// work space of the reductions and the Krylov scalars, on the device and in pinned host memory
+// work space of the reductions and the Krylov scalars, on the device and in pinned host memory (zeroed
+// on the handle's stream, ahead of the kernels that count on it: its own stream does not wait for the
+// default one)
 static int ensure_scalars(ppf_handle h, LinearState& L) {
   const size_t len = SC_EIG + 8 + 3 * (size_t)L.params.eig_cg_iterations;
   if (L.scal && len > L.scal_len) {  // (parameters set again before a block's first linear solve)
@@ -476,12 +478,12 @@ static int ensure_scalars(ppf_handle h, LinearState& L) {
   }
   if (!L.scal) {
     PPF_CUDA(h, cudaMalloc(&L.scal, sizeof(double) * len));
-    PPF_CUDA(h, cudaMemset(L.scal, 0, sizeof(double) * len));
+    PPF_CUDA(h, cudaMemsetAsync(L.scal, 0, sizeof(double) * len, h->stream));
     L.scal_len = len;
   }
   if (L.partial) return PPF_OK;
   PPF_CUDA(h, cudaMalloc(&L.partial, sizeof(double) * 2056));
-  PPF_CUDA(h, cudaMemset(L.partial, 0, sizeof(double) * 2056));
+  PPF_CUDA(h, cudaMemsetAsync(L.partial, 0, sizeof(double) * 2056, h->stream));
   PPF_CUDA(h, cudaMallocHost(&L.h_scal, sizeof(double) * 4));
   for (auto& ev : L.scal_ev) PPF_CUDA(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   return PPF_OK;
@@ -1672,7 +1674,7 @@ int newton_solve(ppf_handle h, int b) {
     cudaFree(L.newton_update);
     for (double*& p : L.kv) cudaFree(p);
     PPF_CUDA(h, cudaMalloc(&L.newton_update, sizeof(double) * n));
-    PPF_CUDA(h, cudaMemset(L.newton_update, 0, sizeof(double) * n));
+    PPF_CUDA(h, cudaMemsetAsync(L.newton_update, 0, sizeof(double) * n, h->stream));
     for (double*& p : L.kv) PPF_CUDA(h, cudaMalloc(&p, sizeof(double) * n));
     cudaFree(L.rhs);  // a Newton block's rhs vector holds its block residual
     PPF_CUDA(h, cudaMalloc(&L.rhs, sizeof(double) * n));
