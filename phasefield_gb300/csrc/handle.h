@@ -91,7 +91,8 @@ struct MGLevel {
   void* tables = nullptr;       // CellTables for the LHS (level precision)
   std::vector<unsigned char> h_tables;  // host copy (the lane kernel takes it as a kernel parameter)
   int fx_lanes = 0;             // the FP64 level's lane kernel mode (4, 5 or 0 for none)
-  void* acc = nullptr;          // accumulator of the next product, all zero
+  void* acc = nullptr;          // accumulator of the next product; acc_clean: all zero
+  bool acc_clean = false;
   void* acc2 = nullptr;         // the last product's: what reads one clears the other, and they swap
   void* x = nullptr;            // level solution
   void* b = nullptr;            // level defect (right-hand side)

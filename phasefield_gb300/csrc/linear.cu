@@ -717,6 +717,12 @@ static int online_mode_end(ppf_handle h, int& state, int& timed, cudaEvent_t* ev
   return PPF_OK;
 }
 
+// what follows a launch that read the level's accumulator and cleared the other one
+static void level_took(MGLevel& lv) {
+  std::swap(lv.acc, lv.acc2);
+  lv.acc_clean = true;
+}
+
 static int level_cell_launch(ppf_handle h, BlockState& B, MGLevel& lv, int mode, const void* src, bool plain_read) {
   const int f = B.desc.field_indices[0];
   FieldState& F = h->fields[f];
@@ -771,7 +777,10 @@ static int level_cell_launch(ppf_handle h, BlockState& B, MGLevel& lv, int mode,
   }
   const size_t smem = cell_smem(h->dim, h->k, lv.precision, P.nrows_in, P.nrows_out);
   const void* obj = lv.precision ? h->model_obj_f32.data() : h->model_obj.data();
-  // (the level's accumulator is all zero: the kernel that read the other one cleared it)
+  // the level's accumulator is all zero where the kernel that read the other one cleared it, that is
+  // unless a launch in between failed
+  if (!lv.acc_clean) PPF_CUDA(h, cudaMemsetAsync(lv.acc, 0, lv.len * esize(lv.precision), h->stream));
+  lv.acc_clean = false;
   const int rc = timed_cell_launch(h, lv.precision, mode, L, obj, smem);
   if (rc) return rc;
   return online_mode_end(h, lv.fx_mode, lv.fx_timed, lv.fx_ev, slot, lv.fx_lanes);
@@ -797,7 +806,7 @@ static int level_apply(ppf_handle h, BlockState& B, MGLevel& lv, const T* src, T
   if (out) grid.x = std::min(grid.x, 1024u / grid.y);
   PPF_CUDA(h, launch_chained(level_finalize_kernel<T>, grid, dim3(256), 0, h->stream, dst, (const T*)lv.acc, (T*)lv.acc2,
                              level_scale<T>(B.lin, lv), lv.N, src, B.lin.partial, counters(B.lin), out));
-  std::swap(lv.acc, lv.acc2);
+  level_took(lv);
   h->all_launches++;
   return PPF_OK;
 }
@@ -808,7 +817,7 @@ static int level_diagonal_t(ppf_handle h, BlockState& B, MGLevel& lv) {
   if (rc) return rc;
   PPF_CUDA(h, launch_chained(inv_diag_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.inv_diag,
                              (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), lv.N));
-  std::swap(lv.acc, lv.acc2);
+  level_took(lv);
   h->all_launches++;
   return PPF_OK;
 }
@@ -940,7 +949,7 @@ static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start, 
       PPF_CUDA(h, launch_chained(cheb_step_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, x, u, b,
                                  (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv),
                                  (const T*)lv.inv_diag, c1, c2, lv.N));
-      std::swap(lv.acc, lv.acc2);
+      level_took(lv);
     }
     h->all_launches++;
   }
@@ -984,7 +993,7 @@ static int vcycle_level(ppf_handle h, BlockState& B, int l, const T* b, T* x) {
   if (rc) return rc;
   PPF_CUDA(h, launch_chained(residual_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.r, b,
                              (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), lv.N));
-  std::swap(lv.acc, lv.acc2);
+  level_took(lv);
   auto restriction = h->k == 1 ? restrict_kernel<T, Tc, 1> : (h->k == 2 ? restrict_kernel<T, Tc, 2> : restrict_kernel<T, Tc, 3>);
   PPF_CUDA(h, launch_chained(restriction, level_grid(h, B, cl), dim3(256), 0, h->stream,
                              transfer<T>(h, cl, lv, false), (Tc*)cl.b, (const T*)lv.r, level_map(cl)));
@@ -1141,6 +1150,7 @@ static int init_linear(ppf_handle h, int b) {
       rc = alloc_real(h, p, lv.len, lv.precision);
       if (rc) return rc;
     }
+    lv.acc_clean = true;
     (void)is_fine;
   }
   // transfers between consecutive levels (stored on the coarse level; work buffers on the fine)
@@ -1242,14 +1252,21 @@ static int precondition_graphed(ppf_handle h, BlockState& B, const double* r, do
   }
   cudaGraph_t graph = nullptr;
   const cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
+  if (!rc && e != cudaSuccess) rc = fail(h, PPF_ERR_CUDA, std::string("preconditioner capture: ") + cudaGetErrorString(e));
+  if (!rc) {
+    const cudaError_t ie = cudaGraphInstantiate(&L.pc_graph, graph, 0);
+    if (ie != cudaSuccess) rc = fail(h, PPF_ERR_CUDA, std::string("preconditioner graph: ") + cudaGetErrorString(ie));
+  }
+  if (graph) cudaGraphDestroy(graph);
   if (rc) {
-    if (graph) cudaGraphDestroy(graph);
+    // nothing that was recorded has run
+    for (size_t l = 0; l < L.levels.size(); ++l) {
+      MGLevel& lv = L.levels[l];
+      if (lv.acc != acc0[l]) std::swap(lv.acc, lv.acc2);
+      lv.acc_clean = false;
+    }
     return rc;
   }
-  if (e != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("preconditioner capture: ") + cudaGetErrorString(e));
-  const cudaError_t ie = cudaGraphInstantiate(&L.pc_graph, graph, 0);
-  cudaGraphDestroy(graph);
-  if (ie != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("preconditioner graph: ") + cudaGetErrorString(ie));
   L.pc_in = r;
   L.pc_out = z;
   PPF_CUDA(h, cudaGraphLaunch(L.pc_graph, h->stream));
