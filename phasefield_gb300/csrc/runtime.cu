@@ -1623,7 +1623,15 @@ static int capture_graph(ppf_handle h, unsigned remaining) {
     if (rc) return rc;
     h->graph_acc.push_back(F.acc);
   }
-  cudaGraph_t g;
+  // the vectors as they stand, to return to should the capture fail
+  struct Vectors {
+    double* cur;
+    double* old[4];
+  };
+  std::vector<Vectors> before;
+  for (auto& F : h->fields) before.push_back({F.cur, {F.old[0], F.old[1], F.old[2], F.old[3]}});
+  const long long rot0 = h->rot_count;
+  cudaGraph_t g = nullptr;
   PPF_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   h->capturing = true;
   int rc = PPF_OK;
@@ -1637,11 +1645,23 @@ static int capture_graph(ppf_handle h, unsigned remaining) {
   h->capturing = false;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   h->timer = saved;
-  if (rc) return rc;
-  if (e != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-  e = cudaGraphInstantiate(&h->run_graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) return fail(h, PPF_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  if (!rc && e != cudaSuccess) rc = fail(h, PPF_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+  if (!rc && (e = cudaGraphInstantiate(&h->run_graph, g, 0)) != cudaSuccess)
+    rc = fail(h, PPF_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  if (g) cudaGraphDestroy(g);
+  if (rc) {
+    // nothing that was recorded has run
+    for (size_t f = 0; f < h->fields.size(); ++f) {
+      FieldState& F = h->fields[f];
+      F.cur = before[f].cur;
+      std::copy(before[f].old, before[f].old + 4, F.old);
+      if (F.acc != h->graph_acc[f]) std::swap(F.acc, F.acc2);
+      F.acc_clean = false;
+    }
+    h->rot_count = rot0;
+    h->all_launches = launches0;
+    return rc;
+  }
   h->graph_period = period;
   h->graph_phase = h->rot_count % base;
   h->graph_launches = h->all_launches - launches0;

@@ -46,6 +46,33 @@ def rel_l2(a, b):
     return np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
 
 
+@pytest.mark.parametrize("make,fields", [
+    (lambda: W.coupled_acch_2d(refine=3, degree=2, size=32.0, dt=1e-3, n_precip=3), (0, 1)),
+    (lambda: W.cahn_hilliard_3d(refine=2, degree=1, size=4.0, dt=1e-5), (0, 1)),
+])
+def test_explicit_run(gpu_lib, monkeypatch, make, fields):
+    monkeypatch.setenv("PPF_CONTRACTION_MODE", "1")  # (no timing launches)
+    n = 23
+    p = make().make_problem()
+    p.solve(n)
+    ref = [p.download_solution(f) for f in fields]
+    per = sum(b.solve_timing != 3 for b in make().blocks)  # cell launches an increment
+    p.close()
+    for fail_at in list(range(1, 8 * per)):
+        wl = make()
+        s = Stand_in(gpu_lib, wl.model)
+        wl.model = s.name
+        p = wl.make_problem()
+        s.fail_at = fail_at
+        with pytest.raises(capi.PPFError):
+            p.solve(n)
+        p.solve(n)
+        assert p.get_time()[0] == n + 1
+        for f, r in zip(fields, ref):
+            assert rel_l2(p.download_solution(f), r) < 1e-12, (fail_at, f)
+        p.close()
+
+
 @pytest.mark.parametrize("mixed", [0, 1])
 def test_multigrid_solve(gpu_lib, monkeypatch, mixed):
     monkeypatch.setenv("PPF_CONTRACTION_MODE", "1")
