@@ -429,10 +429,11 @@ int ppf_tangent_linear(ppf_handle h, int block, int n_steps, const double* du0, 
                        double* duK);
 long long ppf_checkpoint_schedule_cost(int n_steps, int n_snapshots);
 
-/* Replay the explicit increment loop of ppf_run from a CUDA graph (on by default): one graph
- * holds up to eight age-rotation periods of increments, which advance the device-side timer; fewer
- * increments than it holds run as plain launches. Used from increment 2 on when every block is Explicit or Constant, no PostProcess
- * output is requested and kernel timing is off. */
+/* Replay the explicit increment loop of ppf_run from CUDA graphs (on by default): one holds an
+ * age-rotation period of increments, and a second one, once that was replayed often enough, up to
+ * eight periods; they advance the device-side timer. What is left of a period runs as plain launches.
+ * Used from increment 2 on when every block is Explicit or Constant, no PostProcess output is
+ * requested and kernel timing is off. */
 int ppf_set_use_graph(ppf_handle h, int on);
 
 /* Device pointer of a field state (for zero-copy callers), valid until the next rotation or

@@ -690,10 +690,7 @@ int ppf_set_adaptivity(ppf_handle h, const ppf_adaptivity* a) {
     if ((rc = build_constraints(h, f))) return rc;
   }
   if ((rc = build_invm(h))) return rc;
-  if (h->run_graph) {
-    cudaGraphExecDestroy(h->run_graph);
-    h->run_graph = nullptr;
-  }
+  drop_graphs(h);
   cudaFree(h->d_scratch_src);
   cudaFree(h->d_scratch_dst);
   h->d_scratch_src = h->d_scratch_dst = nullptr;

@@ -176,6 +176,16 @@ struct BlockState {
 
 }  // namespace ppf
 
+// a captured run of increments
+struct IncrementGraph {
+  cudaGraphExec_t exec = nullptr;
+  int phase = 0;               // of the age rotation where it starts
+  int periods = 0;             // rotation periods it holds
+  long long launches = 0;
+  long long replayed = 0;      // periods replayed so far
+  std::vector<double*> acc;    // each field's accumulator at its start
+};
+
 struct ppf_handle_s {
   ppf_mesh_desc mesh;
   int dim = 2, k = 1, n = 2;
@@ -214,18 +224,14 @@ struct ppf_handle_s {
   ppf::AdjointState* adj = nullptr;  // adjoint / tangent-linear state (created on first use)
   ppf::AmrState* amr = nullptr;      // adaptive mesh (ppf_set_adaptivity), else null
   long long mesh_version = 0;
-  long long graph_mesh_version = -1;  // mesh the increment graph was captured on
   long long state_version = 0;        // bumped when a staged upload swaps a state buffer in
-  long long graph_state_version = -1; // state buffers the increment graph was captured on
-  // CUDA graph of the explicit increment loop
+  // CUDA graphs of the explicit increment loop
   prismspf::SimulationTimer* d_timer = nullptr;
-  std::vector<double*> graph_acc;  // each field's accumulator at the start of the graph
   bool advance_timer = false;      // (while capturing) the next finalize launch advances d_timer
-  cudaGraphExec_t run_graph = nullptr;
-  cudaStream_t graph_stream = nullptr;
-  int graph_period = 0;
-  long long graph_phase = 0;
-  long long graph_launches = 0;
+  std::vector<IncrementGraph> graphs;  // by phase of the age rotation: one of a period, one of several
+  cudaStream_t graph_stream = nullptr;  // the stream, mesh and state buffers they were captured on
+  long long graph_mesh_version = -1;
+  long long graph_state_version = -1;
   long long rot_count = 0;
   bool capturing = false;
   bool caller_captured = false;  // a caller has captured launches of this handle in a graph of its own
@@ -255,6 +261,8 @@ unsigned grid_for(long long n);
 int clear_acc(ppf_handle h, FieldState& F);
 int ensure_acc2(ppf_handle h, FieldState& F);
 void free_acc(FieldState& F);
+// destroys the captured increment graphs
+void drop_graphs(ppf_handle h);
 int check_err(ppf_handle h);
 double* state_ptr(ppf_handle h, int f, int age);
 // records a kernel launch for the statistics; brackets cell launches with events when timing

@@ -941,6 +941,11 @@ void free_acc(FieldState& F) {
   F.acc_clean = false;
 }
 
+void drop_graphs(ppf_handle h) {
+  for (auto& G : h->graphs) cudaGraphExecDestroy(G.exec);
+  h->graphs.clear();
+}
+
 static int explicit_solve(ppf_handle h, int b) {
   BlockState& B = h->blocks[b];
   bool alternate = true;
@@ -1405,7 +1410,7 @@ void ppf_destroy(ppf_handle h) {
   }
   free_adjoint(h->adj);
   free_amr(h->amr);
-  if (h->run_graph) cudaGraphExecDestroy(h->run_graph);
+  drop_graphs(h);
   cudaFree(h->d_timer);
   cudaFree(h->d_invm);
   cudaFree(h->d_invm_sqrt);
@@ -1566,10 +1571,10 @@ int ppf_solve_block(ppf_handle h, int b) {
   return check_err(h);
 }
 
-// The explicit increment loop can be replayed from a CUDA graph: one graph holds `period`
-// increments (the period of the age rotation, so the state pointers return to where they
-// were), each followed by a device-side timer advance; callbacks read the timer from device
-// memory during replays, so time-dependent operators see the right time.
+// The explicit increment loop can be replayed from CUDA graphs: one holds a number of periods of the
+// age rotation (so the state pointers return to where they were), and the last block's finalize
+// launch of each increment advances a timer on the device, which callbacks read during replays, so
+// time-dependent operators see the right time.
 static bool graph_eligible(ppf_handle h, int output_every) {
   // per-launch event timing needs plain launches; postprocess increments are not periodic
   // (adaptive meshes replay only between remeshing increments, see ppf_run); streamed outputs
@@ -1601,27 +1606,42 @@ static int rotation_period(ppf_handle h) {
   return p % 2 ? 2 * p : p;
 }
 
-// One graph holds up to GRAPH_PERIODS rotation periods, as many as the run has left: kernels of one
-// graph are chained, successive graphs are not (48^2 Q1: 1.4 us a graph launch).
+// Kernels of one graph are chained, successive graphs are not (48^2 Q1: 1.4 us a graph launch), but
+// recording and instantiating an increment costs about as much as launching it twice. So a phase of
+// the rotation first gets a graph of one period, which any run's length is made of, and once
+// GRAPH_WORTH periods are replayed or due on the same vectors one of up to GRAPH_PERIODS as well, as
+// many as the run has left. (A graph of whatever the first run had left made later, shorter runs and the
+// ends of runs plain launches: 100 increments of 128^2 Q1 Allen-Cahn 1.01 ms, 0.83 ms this way; and
+// where the vectors change before every run it recorded 16 increments to replay them once. With 64
+// periods for GRAPH_WORTH the first run of 100 increments on an adaptive mesh took 5 % longer.)
 constexpr int GRAPH_PERIODS = 8;
+constexpr int GRAPH_WORTH = 32;
+constexpr size_t MAX_GRAPHS = 16;
 
-static int capture_graph(ppf_handle h, unsigned remaining) {
-  if (h->run_graph) {
-    cudaGraphExecDestroy(h->run_graph);
-    h->run_graph = nullptr;
-  }
+// the graph of this phase with one period (several: with more than one), or null
+static IncrementGraph* held_graph(ppf_handle h, int phase, bool several) {
+  for (auto& G : h->graphs)
+    if (G.phase == phase && (G.periods > 1) == several) return &G;
+  return nullptr;
+}
+
+// captures `periods` periods as the graph of this phase, in place of one of its kind
+static int capture_graph(ppf_handle h, int periods) {
   if (!h->d_timer) PPF_CUDA(h, cudaMalloc(&h->d_timer, sizeof(prismspf::SimulationTimer)));
   const int base = rotation_period(h);
-  const int period = base * (int)std::max(1u, std::min((unsigned)GRAPH_PERIODS, remaining / (unsigned)base));
+  const int period = base * periods;
+  IncrementGraph G;
+  G.phase = (int)(h->rot_count % base);
+  G.periods = periods;
+  if (h->graphs.size() >= MAX_GRAPHS) drop_graphs(h);
   const prismspf::SimulationTimer saved = h->timer;
-  const long long launches0 = h->all_launches;
+  const long long launches0 = h->all_launches, cells0 = h->cell_launches;
   const int last = last_explicit_block(h);
-  h->graph_acc.clear();
   for (auto& F : h->fields) {
     int rc = ensure_acc2(h, F);
     if (!rc) rc = clear_acc(h, F);
     if (rc) return rc;
-    h->graph_acc.push_back(F.acc);
+    G.acc.push_back(F.acc);
   }
   // the vectors as they stand, to return to should the capture fail
   struct Vectors {
@@ -1645,8 +1665,9 @@ static int capture_graph(ppf_handle h, unsigned remaining) {
   h->capturing = false;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   h->timer = saved;
+  h->cell_launches = cells0;  // (recorded, not launched)
   if (!rc && e != cudaSuccess) rc = fail(h, PPF_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-  if (!rc && (e = cudaGraphInstantiate(&h->run_graph, g, 0)) != cudaSuccess)
+  if (!rc && (e = cudaGraphInstantiate(&G.exec, g, 0)) != cudaSuccess)
     rc = fail(h, PPF_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
   if (g) cudaGraphDestroy(g);
   if (rc) {
@@ -1655,20 +1676,66 @@ static int capture_graph(ppf_handle h, unsigned remaining) {
       FieldState& F = h->fields[f];
       F.cur = before[f].cur;
       std::copy(before[f].old, before[f].old + 4, F.old);
-      if (F.acc != h->graph_acc[f]) std::swap(F.acc, F.acc2);
+      if (F.acc != G.acc[f]) std::swap(F.acc, F.acc2);
       F.acc_clean = false;
     }
     h->rot_count = rot0;
     h->all_launches = launches0;
     return rc;
   }
-  h->graph_period = period;
-  h->graph_phase = h->rot_count % base;
-  h->graph_launches = h->all_launches - launches0;
+  G.launches = h->all_launches - launches0;
   h->all_launches = launches0;
-  h->graph_stream = h->stream;
-  h->graph_mesh_version = h->mesh_version;
-  h->graph_state_version = h->state_version;
+  if (IncrementGraph* old = held_graph(h, G.phase, periods > 1)) {
+    cudaGraphExecDestroy(old->exec);
+    *old = std::move(G);
+  } else {
+    h->graphs.push_back(std::move(G));
+  }
+  return PPF_OK;
+}
+
+// replays as much of the next `periods` rotation periods as one graph makes, captured here if need be
+static int replay_graph(ppf_handle h, int periods) {
+  if (h->graph_stream != h->stream || h->graph_mesh_version != h->mesh_version ||
+      h->graph_state_version != h->state_version) {
+    drop_graphs(h);
+    h->graph_stream = h->stream;
+    h->graph_mesh_version = h->mesh_version;
+    h->graph_state_version = h->state_version;
+  }
+  const int base = rotation_period(h), phase = (int)(h->rot_count % base);
+  const int most = std::min(periods, GRAPH_PERIODS);
+  IncrementGraph* one = held_graph(h, phase, false);
+  IncrementGraph* many = held_graph(h, phase, true);
+  const bool worth = (one ? one->replayed : 0) + periods >= GRAPH_WORTH;
+  if (most > 1 && worth && (!many || many->periods < most)) {
+    if (const int rc = capture_graph(h, most)) return rc;
+    many = held_graph(h, phase, true);
+  }
+  const bool several = many && many->periods <= periods;
+  if (!several && !one) {
+    if (const int rc = capture_graph(h, 1)) return rc;
+  }
+  IncrementGraph& G = *held_graph(h, phase, several);
+  PPF_CUDA(h, cudaMemcpyAsync(h->d_timer, &h->timer, sizeof(prismspf::SimulationTimer), cudaMemcpyHostToDevice,
+                              h->stream));
+  // the accumulators the graph starts from, all zero
+  for (size_t f = 0; f < h->fields.size(); ++f) {
+    FieldState& F = h->fields[f];
+    if (F.acc != G.acc[f]) {
+      std::swap(F.acc, F.acc2);
+      F.acc_clean = false;
+    }
+    const int rc = clear_acc(h, F);
+    if (rc) return rc;
+  }
+  const int reps = periods / G.periods;
+  for (int r = 0; r < reps; ++r) PPF_CUDA(h, cudaGraphLaunch(G.exec, h->stream));
+  const int increments = reps * G.periods * base;
+  for (int k = 0; k < increments; ++k) h->timer.increment(h->dt);
+  h->rot_count += increments;
+  h->all_launches += reps * G.launches;
+  G.replayed += (long long)reps * G.periods;
   return PPF_OK;
 }
 
@@ -1699,32 +1766,9 @@ static int run_increments(ppf_handle h, unsigned int n_increments, int output_ev
           else if (due - 1 < last) last = (unsigned)(due - 1);
         }
       const unsigned remaining = last >= inc ? last - inc + 1 : 0;
-      const bool valid = h->run_graph && h->graph_stream == h->stream && h->graph_phase == h->rot_count % period &&
-                         h->graph_mesh_version == h->mesh_version && h->graph_state_version == h->state_version;
-      // (fewer increments than a captured graph holds run as plain launches)
-      if (remaining >= (unsigned)(valid ? h->graph_period : period)) {
-        if (!valid) {
-          int rc = capture_graph(h, remaining);
-          if (rc) return rc;
-        }
-        PPF_CUDA(h, cudaMemcpyAsync(h->d_timer, &h->timer, sizeof(prismspf::SimulationTimer), cudaMemcpyHostToDevice,
-                                    h->stream));
-        // the accumulators the graph starts from, all zero
-        for (size_t f = 0; f < h->fields.size(); ++f) {
-          FieldState& F = h->fields[f];
-          if (F.acc != h->graph_acc[f]) {
-            std::swap(F.acc, F.acc2);
-            F.acc_clean = false;
-          }
-          const int rc = clear_acc(h, F);
-          if (rc) return rc;
-        }
-        const unsigned held = (unsigned)h->graph_period, reps = remaining / held;
-        for (unsigned r = 0; r < reps; ++r) PPF_CUDA(h, cudaGraphLaunch(h->run_graph, h->stream));
-        for (unsigned k = 0; k < reps * held; ++k) h->timer.increment(h->dt);
-        h->rot_count += (long long)reps * held;
-        h->all_launches += (long long)reps * h->graph_launches;
-        h->cell_launches += 0;
+      // (what is left of a period runs as plain launches)
+      if (remaining >= (unsigned)period) {
+        if (const int rc = replay_graph(h, (int)(remaining / (unsigned)period))) return rc;
         continue;
       }
     }

@@ -53,24 +53,26 @@ def rel_l2(a, b):
 def test_explicit_run(gpu_lib, monkeypatch, make, fields):
     monkeypatch.setenv("PPF_CONTRACTION_MODE", "1")  # (no timing launches)
     n = 23
-    p = make().make_problem()
-    p.solve(n)
-    ref = [p.download_solution(f) for f in fields]
-    per = sum(b.solve_timing != 3 for b in make().blocks)  # cell launches an increment
-    p.close()
-    for fail_at in list(range(1, 8 * per)):
+
+    def run(fail_at):
         wl = make()
         s = Stand_in(gpu_lib, wl.model)
         wl.model = s.name
         p = wl.make_problem()
         s.fail_at = fail_at
-        with pytest.raises(capi.PPFError):
-            p.solve(n)
+        if fail_at:
+            with pytest.raises(capi.PPFError):
+                p.solve(n)
         p.solve(n)
         assert p.get_time()[0] == n + 1
-        for f, r in zip(fields, ref):
-            assert rel_l2(p.download_solution(f), r) < 1e-12, (fail_at, f)
+        out = [p.download_solution(f) for f in fields]
         p.close()
+        return out, s.calls
+
+    ref, total = run(None)
+    for fail_at in range(1, total + 1):
+        for got, r, f in zip(run(fail_at)[0], ref, fields):
+            assert rel_l2(got, r) < 1e-12, (fail_at, f)
 
 
 @pytest.mark.parametrize("mixed", [0, 1])
