@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "../../include/ppf_gb300.h"
+#include "graph_lengths.h"
 #include "handle.h"
 #include "models.cuh"
 
@@ -435,9 +436,14 @@ struct ppf_ensemble_s {
   long long step = 0;  // accumulator rotation counter
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;
-  // the captured steps, by the accumulator rotation's phase they start from
-  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
-  int graph_shape[3] = {}, graph_grid[3] = {}, graph_steps[3] = {};
+  // the captured steps, by the accumulator rotation's phase they start from: one rotation, and several
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    int rotations = 0;
+    long long replayed = 0;  // rotations
+  };
+  StepGraph graph[3][2];
+  int graph_shape = -1, graph_grid = -1;  // what they were captured with
   std::string err;
   double gl_w[2][3];
   double gl_D[2][3][3];
@@ -449,10 +455,11 @@ namespace ppf {
 namespace {
 
 void drop_graphs(ppf_ensemble e) {
-  for (auto& g : e->graph) {
-    if (g) cudaGraphExecDestroy(g);
-    g = nullptr;
-  }
+  for (auto& phase : e->graph)
+    for (auto& g : phase) {
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g = {};
+    }
 }
 
 int efail(ppf_ensemble e, int code, const std::string& m) {
@@ -709,34 +716,51 @@ int ppf_ensemble_download(ppf_ensemble e, int i, double* host) {
   return PPF_OK;
 }
 
-// advance every instance by n_steps explicit steps: one launch per step; with use_graph the
-// steps are replayed from a captured graph of up to eight accumulator rotations (three steps each:
-// launches inside a graph overlap, successive graphs do not)
+namespace ppf {
+namespace {
+
+// captures `rotations` rotations of steps from the present phase into g
+int capture_steps(ppf_ensemble e, ppf_ensemble_s::StepGraph& g, int rotations) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  g = {};
+  cudaGraph_t graph = nullptr;
+  ENS_CUDA(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = PPF_OK;
+  for (int k = 0; k < 3 * rotations && !rc; ++k) rc = launch_step(e, e->step + k, e->stream);
+  const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
+  if (!rc && (end != cudaSuccess || cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess))
+    rc = efail(e, PPF_ERR_CUDA, "ensemble step capture failed");
+  if (graph) cudaGraphDestroy(graph);
+  g.rotations = rc ? 0 : rotations;
+  return rc;
+}
+
+}  // namespace
+}  // namespace ppf
+
+// advance every instance by n_steps explicit steps: one launch per step; with use_graph whole
+// accumulator rotations (three steps) are replayed from captured graphs, their lengths by
+// graph_lengths.h
 int ppf_ensemble_run(ppf_ensemble e, int n_steps, int use_graph) {
   if (!e || n_steps < 0) return PPF_ERR_ARG;
   int done = 0;
-  if (use_graph) {
-    const int phase = (int)(e->step % 3);
-    cudaGraphExec_t& exec = e->graph[phase];
-    if (!exec || e->graph_shape[phase] != e->shape || e->graph_grid[phase] != e->grid_mult) {
-      if (exec) cudaGraphExecDestroy(exec);
-      exec = nullptr;
-      const int held = 3 * std::max(1, std::min(8, n_steps / 3));
-      cudaGraph_t g;
-      ENS_CUDA(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < held; ++k) launch_step(e, e->step + k, e->stream);
-      ENS_CUDA(e, cudaStreamEndCapture(e->stream, &g));
-      ENS_CUDA(e, cudaGraphInstantiate(&exec, g, 0));
-      cudaGraphDestroy(g);
-      e->graph_shape[phase] = e->shape;
-      e->graph_grid[phase] = e->grid_mult;
-      e->graph_steps[phase] = held;
-    }
-    const int held = e->graph_steps[phase];
-    while (n_steps - done >= held) {
-      ENS_CUDA(e, cudaGraphLaunch(exec, e->stream));
-      done += held;
-      e->step += held;  // phase unchanged
+  if (use_graph && (e->graph_shape != e->shape || e->graph_grid != e->grid_mult)) {
+    drop_graphs(e);
+    e->graph_shape = e->shape;
+    e->graph_grid = e->grid_mult;
+  }
+  while (use_graph && n_steps - done >= 3) {
+    auto& held = e->graph[e->step % 3];
+    const int rotations = (n_steps - done) / 3;
+    const GraphChoice c = choose_graph(rotations, held[0].exec != nullptr, held[0].replayed, held[1].rotations);
+    auto& g = held[c.replay > 1];
+    if (c.capture)
+      if (const int rc = capture_steps(e, g, c.capture)) return rc;
+    for (int r = rotations / c.replay; r > 0; --r) {
+      ENS_CUDA(e, cudaGraphLaunch(g.exec, e->stream));
+      done += 3 * c.replay;
+      e->step += 3 * c.replay;  // phase unchanged
+      g.replayed += c.replay;
     }
   }
   for (; done < n_steps; ++done) {

@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "graph_lengths.h"
 #include "handle.h"
 
 namespace ppf {
@@ -1606,16 +1607,7 @@ static int rotation_period(ppf_handle h) {
   return p % 2 ? 2 * p : p;
 }
 
-// Kernels of one graph are chained, successive graphs are not (48^2 Q1: 1.4 us a graph launch), but
-// recording and instantiating an increment costs about as much as launching it twice. So a phase of
-// the rotation first gets a graph of one period, which any run's length is made of, and once
-// GRAPH_WORTH periods are replayed or due on the same vectors one of up to GRAPH_PERIODS as well, as
-// many as the run has left. (A graph of whatever the first run had left made later, shorter runs and the
-// ends of runs plain launches: 100 increments of 128^2 Q1 Allen-Cahn 1.01 ms, 0.83 ms this way; and
-// where the vectors change before every run it recorded 16 increments to replay them once. With 64
-// periods for GRAPH_WORTH the first run of 100 increments on an adaptive mesh took 5 % longer.)
-constexpr int GRAPH_PERIODS = 8;
-constexpr int GRAPH_WORTH = 32;
+// (lengths by graph_lengths.h)
 constexpr size_t MAX_GRAPHS = 16;
 
 // the graph of this phase with one period (several: with more than one), or null
@@ -1704,19 +1696,12 @@ static int replay_graph(ppf_handle h, int periods) {
     h->graph_state_version = h->state_version;
   }
   const int base = rotation_period(h), phase = (int)(h->rot_count % base);
-  const int most = std::min(periods, GRAPH_PERIODS);
-  IncrementGraph* one = held_graph(h, phase, false);
-  IncrementGraph* many = held_graph(h, phase, true);
-  const bool worth = (one ? one->replayed : 0) + periods >= GRAPH_WORTH;
-  if (most > 1 && worth && (!many || many->periods < most)) {
-    if (const int rc = capture_graph(h, most)) return rc;
-    many = held_graph(h, phase, true);
-  }
-  const bool several = many && many->periods <= periods;
-  if (!several && !one) {
-    if (const int rc = capture_graph(h, 1)) return rc;
-  }
-  IncrementGraph& G = *held_graph(h, phase, several);
+  const IncrementGraph* one = held_graph(h, phase, false);
+  const IncrementGraph* many = held_graph(h, phase, true);
+  const GraphChoice choice = choose_graph(periods, one != nullptr, one ? one->replayed : 0, many ? many->periods : 0);
+  if (choice.capture)
+    if (const int rc = capture_graph(h, choice.capture)) return rc;
+  IncrementGraph& G = *held_graph(h, phase, choice.replay > 1);
   PPF_CUDA(h, cudaMemcpyAsync(h->d_timer, &h->timer, sizeof(prismspf::SimulationTimer), cudaMemcpyHostToDevice,
                               h->stream));
   // the accumulators the graph starts from, all zero
