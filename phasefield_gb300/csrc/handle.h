@@ -183,7 +183,7 @@ struct IncrementGraph {
   int periods = 0;             // rotation periods it holds
   long long launches = 0;
   long long replayed = 0;      // periods replayed so far
-  std::vector<double*> acc;    // each field's accumulator at its start
+  std::vector<double*> acc;    // each field's accumulator at its start, null where the graph does not solve it
 };
 
 struct ppf_handle_s {

@@ -1129,13 +1129,16 @@ static void end_increment(ppf_handle h) {
   h->timer.increment(h->dt);
 }
 
+// whether an increment of the graph solves the block
+static bool solved_in_graph(const ppf_block_desc& d) {
+  return d.solve_type == PPF_EXPLICIT && d.solve_timing != PPF_POSTPROCESS && d.solve_timing != PPF_NUCLEATION_RATE;
+}
+
 // the block whose finalize launch ends an increment of the graph (-1: none does)
 static int last_explicit_block(ppf_handle h) {
   int last = -1;
-  for (int b = 0; b < (int)h->blocks.size(); ++b) {
-    const ppf_block_desc& d = h->blocks[b].desc;
-    if (d.solve_type == PPF_EXPLICIT && d.solve_timing != PPF_POSTPROCESS && d.solve_timing != PPF_NUCLEATION_RATE) last = b;
-  }
+  for (int b = 0; b < (int)h->blocks.size(); ++b)
+    if (solved_in_graph(h->blocks[b].desc)) last = b;
   return last;
 }
 
@@ -1586,7 +1589,6 @@ static bool graph_eligible(ppf_handle h, int output_every) {
   for (auto& B : h->blocks) {
     const int t = B.desc.solve_type;
     if (t != PPF_EXPLICIT && t != PPF_CONSTANT) return false;
-    if (B.desc.solve_timing == PPF_POSTPROCESS || B.desc.solve_timing == PPF_NUCLEATION_RATE) continue;
   }
   return true;
 }
@@ -1629,11 +1631,16 @@ static int capture_graph(ppf_handle h, int periods) {
   const prismspf::SimulationTimer saved = h->timer;
   const long long launches0 = h->all_launches, cells0 = h->cell_launches;
   const int last = last_explicit_block(h);
-  for (auto& F : h->fields) {
-    int rc = ensure_acc2(h, F);
-    if (!rc) rc = clear_acc(h, F);
-    if (rc) return rc;
-    G.acc.push_back(F.acc);
+  G.acc.assign(h->fields.size(), nullptr);
+  for (auto& B : h->blocks) {
+    if (!solved_in_graph(B.desc)) continue;
+    for (int i = 0; i < B.desc.n_fields; ++i) {
+      FieldState& F = h->fields[B.desc.field_indices[i]];
+      int rc = ensure_acc2(h, F);
+      if (!rc) rc = clear_acc(h, F);
+      if (rc) return rc;
+      G.acc[B.desc.field_indices[i]] = F.acc;
+    }
   }
   // the vectors as they stand, to return to should the capture fail
   struct Vectors {
@@ -1668,7 +1675,7 @@ static int capture_graph(ppf_handle h, int periods) {
       FieldState& F = h->fields[f];
       F.cur = before[f].cur;
       std::copy(before[f].old, before[f].old + 4, F.old);
-      if (F.acc != G.acc[f]) std::swap(F.acc, F.acc2);
+      if (G.acc[f] && F.acc != G.acc[f]) std::swap(F.acc, F.acc2);
       F.acc_clean = false;
     }
     h->rot_count = rot0;
@@ -1707,6 +1714,7 @@ static int replay_graph(ppf_handle h, int periods) {
   // the accumulators the graph starts from, all zero
   for (size_t f = 0; f < h->fields.size(); ++f) {
     FieldState& F = h->fields[f];
+    if (!G.acc[f]) continue;
     if (F.acc != G.acc[f]) {
       std::swap(F.acc, F.acc2);
       F.acc_clean = false;
