@@ -18,6 +18,7 @@
 #include <prismspf/dealii_shim.h>
 #include <prismspf/gpu/fixed_point.cuh>
 
+#include <cstddef>
 #include <type_traits>
 #include <utility>
 
@@ -83,15 +84,14 @@ struct CellTables {
   int dk[3];
   unsigned long long isig[3];     // c_d = detJ / (h_d W^dim), W = 2 (Q1) or 6 (Q2): isig / 2^63 * 2^ik
   int ik[3];
-  // the lane kernel (prismspf/gpu/cell_kernel_lanes.cuh, cubic cells): value terms are integrated
-  // in fixed point as h v next to the gradient terms, with the weight 2^vw_sh[q] = prod_e w_int(q_e)
-  // and h = hsig / 2^63 * 2^hk (hpow2: h is a power of two); dpow2[d]: 1/h_d is a power of two
+  // From here on the lane kernel's members (prismspf/gpu/cell_kernel_lanes.cuh), which the others do
+  // not stage (staged_table_bytes). Value terms are integrated in fixed point as h_0 v next to the
+  // gradient terms, h_0 = hsig / 2^63 * 2^hk (hpow2: a power of two); dpow2[d]: 1/h_d is a power of two
   int fx_lanes;
   int hpow2;
   int hk;
   int dpow2[3];
   unsigned long long hsig;
-  signed char vw_sh[nq];
   // the lane kernel keeps a double copy only of the value rows read as values or Hessians
   // (val_rows) and a fixed-point copy only of those read as gradients (fx_rows): slot of row r
   // in each, -1 without one (rows below LANE_ROW_SLOTS)
@@ -115,6 +115,18 @@ struct CellTables {
   // the least block exponents of the gradient rows and (EXP_BIAS more) of the terms, likewise
   unsigned int floor_in, floor_out;
 };
+
+// Bytes of the tables in the shared memory of a kernel that reads no lane member: what every adaptive
+// level's copy and every tile of rows has to share the 227 KB with
+template <int dim, int degree, typename number>
+PPF_HD constexpr size_t staged_table_bytes() {
+  using T = CellTables<dim, degree, number>;
+  return offsetof(T, fx_lanes);
+}
+template <int dim, int degree, typename number>
+PPF_HD constexpr size_t staged_table_room() {
+  return (staged_table_bytes<dim, degree, number>() + 15) / 16 * 16;
+}
 
 template <int dim, int degree, typename number = double>
 struct CellCtx {
@@ -458,8 +470,12 @@ class FieldContainer {
     return field_index < unsigned(gpu::MAX_FIELDS) && age >= 0 ? slots[field_index][age] : -1;
   }
 
-  // first output component of a block field in the lane kernel
+  // first output component of a block field
   PPF_HD int lane_component(unsigned int field_index) const {
+    if (!ctx.lean) {  // (the diagonal probe)
+      const int row = out_row(field_index);
+      return row < 0 ? -1 : row / (1 + int(dim));
+    }
     const int o = field_index < unsigned(gpu::MAX_FIELDS) ? ctx.tab->lane_out[field_index] : -1;
     if (o < 0) {
 #ifdef __CUDA_ARCH__

@@ -39,7 +39,7 @@ struct AmrCellLaunch {
 template <int dim, int degree, typename number>
 __host__ __device__ inline size_t amr_cell_smem_bytes(int nlev, int nrows_in, int nrows_out) {
   using S = CellShape<dim, degree>;
-  const size_t tab = (sizeof(pg::CellTables<dim, degree, number>) + 15) / 16 * 16;
+  const size_t tab = pg::staged_table_room<dim, degree, number>();
   size_t b = tab * (size_t)nlev + sizeof(number) * (size_t)(nrows_in + nrows_out) * S::threads + 16;
   // integer derivatives (FP64 Q1/Q2): fixed-point values and per-cell block exponents
   if (cell_fx_capable<dim, degree, number>())
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
   using S = CellShape<dim, degree>;
   using Tab = pg::CellTables<dim, degree, number>;
   constexpr int n = S::n, nq = S::nq, cpb = S::cpb;
-  constexpr size_t tab_stride = (sizeof(Tab) + 15) / 16 * 16;
+  constexpr size_t tab_stride = pg::staged_table_room<dim, degree, number>();
   const CellLaunch& P = A.base;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   number* vals = reinterpret_cast<number*>(smem_raw + tab_stride * A.nlev);
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, 1)
   }
 
   for (int l = 0; l < A.nlev; ++l) {
-    const int nwords = (int)(sizeof(Tab) / 4);
+    const int nwords = (int)(pg::staged_table_bytes<dim, degree, number>() / 4);
     const unsigned int* src =
         reinterpret_cast<const unsigned int*>(static_cast<const unsigned char*>(P.tables) + sizeof(Tab) * l);
     unsigned int* dst = reinterpret_cast<unsigned int*>(smem_raw + tab_stride * l);

@@ -26,7 +26,7 @@ namespace ppf {
 template <int dim, int degree, typename number>
 __host__ __device__ constexpr size_t cell_diagonal_smem_bytes(int nrows_in) {
   using S = CellShape<dim, degree>;
-  return (sizeof(pg::CellTables<dim, degree, number>) + 15) / 16 * 16 + sizeof(number) * (size_t)nrows_in * S::threads;
+  return pg::staged_table_room<dim, degree, number>() + sizeof(number) * (size_t)nrows_in * S::threads;
 }
 
 // NC: components of the block's one field
@@ -38,13 +38,13 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads)
   constexpr int n = S::n, nq = S::nq, cpb = S::cpb, k = degree, TC = 1 + dim;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Tab* tab = reinterpret_cast<Tab*>(smem_raw);
-  number* vals = reinterpret_cast<number*>(smem_raw + (sizeof(Tab) + 15) / 16 * 16);
+  number* vals = reinterpret_cast<number*>(smem_raw + pg::staged_table_room<dim, degree, number>());
   chain_wait();
   chain_release();
   {
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);
     unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
-    for (int i = threadIdx.x; i < (int)(sizeof(Tab) / 4); i += blockDim.x) dst[i] = src[i];
+    for (int i = threadIdx.x; i < (int)(pg::staged_table_bytes<dim, degree, number>() / 4); i += blockDim.x) dst[i] = src[i];
   }
   unsigned int probe_rows = 0;
   {

@@ -212,7 +212,7 @@ __host__ __device__ constexpr size_t warp_region_bytes(int nrows_in, int nrows_o
 template <int dim, int degree>
 __host__ __device__ constexpr size_t cell_warp_smem_bytes(int nrows_in, int nrows_out) {
   using W = WarpShape<dim, degree>;
-  return (sizeof(pg::CellTables<dim, degree, double>) + 15) / 16 * 16 +
+  return pg::staged_table_room<dim, degree, double>() +
          W::warps * warp_region_bytes<dim, degree>(nrows_in, nrows_out);
 }
 
@@ -221,7 +221,7 @@ __host__ __device__ constexpr size_t cell_warp_smem_bytes(int nrows_in, int nrow
 template <int dim, int degree, typename number>
 __host__ __device__ inline size_t cell_smem_bytes(int nrows_in, int nrows_out) {
   using S = CellShape<dim, degree>;
-  size_t tab = (sizeof(pg::CellTables<dim, degree, number>) + 15) / 16 * 16;
+  const size_t tab = pg::staged_table_room<dim, degree, number>();
   size_t b = tab + sizeof(number) * (size_t)(nrows_in + nrows_out) * S::threads + 16;
   if (cell_fx_capable<dim, degree, number>()) {
     b += sizeof(long long) * (size_t)nrows_in * S::threads + sizeof(int) * (size_t)(nrows_in + nrows_out) * S::cpb;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
   constexpr int n = S::n, nq = S::nq, cpb = S::cpb, k = degree;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Tab* tab = reinterpret_cast<Tab*>(smem_raw);
-  number* vals = reinterpret_cast<number*>(smem_raw + (sizeof(Tab) + 15) / 16 * 16);
+  number* vals = reinterpret_cast<number*>(smem_raw + pg::staged_table_room<dim, degree, number>());
   number* outs = vals + P.nrows_in * S::threads;
   __shared__ int sflags;
   // integer contractions: enabled by the launch's tables, and only with the shared memory for them
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(CellShape<dim, degree>::threads, CellMinBlocks
 
   // stage the tables once per resident block
   {
-    const int nwords = (int)(sizeof(Tab) / 4);
+    const int nwords = (int)(pg::staged_table_bytes<dim, degree, number>() / 4);
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);
     unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
     for (int i = threadIdx.x; i < nwords; i += blockDim.x) dst[i] = src[i];

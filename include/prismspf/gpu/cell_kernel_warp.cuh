@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
   chain_wait();
   chain_release();
   {
-    const int nwords = (int)(sizeof(Tab) / 4);
+    const int nwords = (int)(pg::staged_table_bytes<dim, degree, double>() / 4);
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables);
     unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
     for (int i = threadIdx.x; i < nwords; i += blockDim.x) dst[i] = src[i];
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(WarpShape<dim, degree>::threads, CellWarpMinBl
   const SimulationTimer timer = P.timer_dev ? *P.timer_dev : P.timer;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* wbase = smem_raw + (sizeof(Tab) + 15) / 16 * 16 +
+  unsigned char* wbase = smem_raw + pg::staged_table_room<dim, degree, double>() +
                          (size_t)warp * warp_region_bytes<dim, degree>(P.nrows_in, P.nrows_out);
   double* vals = reinterpret_cast<double*>(wbase);
   long long* vfx = reinterpret_cast<long long*>(vals + P.nrows_in * 32);

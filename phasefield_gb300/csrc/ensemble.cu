@@ -71,14 +71,14 @@ __device__ void ens_tile(const EnsLaunch& P, const EnsInstance& I, long long cel
   constexpr int n = degree + 1, nq = n * n;
   using Tab = pg::CellTables<2, degree, double>;
   Tab* tab = reinterpret_cast<Tab*>(smem);
-  double* vals = smem + (sizeof(Tab) + 7) / 8;
+  double* vals = smem + pg::staged_table_room<2, degree, double>() / 8;
   double* outs = vals + CPB * nq;
   const int t = threadIdx.x;
   // stage the instance's tables (built on the host for its mesh spacing)
   {
     const unsigned int* src = reinterpret_cast<const unsigned int*>(P.tables + I.tab_off);
     unsigned int* dst = reinterpret_cast<unsigned int*>(tab);
-    for (int k = t; k < (int)(sizeof(Tab) / 4); k += blockDim.x) dst[k] = src[k];
+    for (int k = t; k < (int)(pg::staged_table_bytes<2, degree, double>() / 4); k += blockDim.x) dst[k] = src[k];
   }
   const int lc = t / nq, q = t - lc * nq;
   const bool in_tile = lc < CPB;
@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(THREADS) ensemble_step_kernel(const EnsLaunch 
 template <int CPB1, int CPB2>
 size_t ens_smem_bytes() {
   // tables, values and three output rows
-  const size_t t1 = (sizeof(pg::CellTables<2, 1, double>) + 7) / 8 * 8 + 8 * 4 * CPB1 * 4;
-  const size_t t2 = (sizeof(pg::CellTables<2, 2, double>) + 7) / 8 * 8 + 8 * 4 * CPB2 * 9;
+  const size_t t1 = pg::staged_table_room<2, 1, double>() + 8 * 4 * CPB1 * 4;
+  const size_t t2 = pg::staged_table_room<2, 2, double>() + 8 * 4 * CPB2 * 9;
   return std::max(t1, t2) + 64;
 }
 

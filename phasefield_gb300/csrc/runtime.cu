@@ -197,14 +197,6 @@ static void fixed_point_tables(pg::CellTables<dim, degree, double>& t, const GLR
   t.fx_cubic = 1;
   for (int d = 1; d < dim; ++d)
     if (t.isig[d] != t.isig[0] || t.ik[d] != t.ik[0]) t.fx_cubic = 0;
-  for (int q = 0; q < nq; ++q) {
-    int sh = 0, r = q;
-    for (int e = 0; e < dim; ++e) {
-      sh += wsh[r % n];
-      r /= n;
-    }
-    t.vw_sh[q] = (signed char)sh;
-  }
   for (int d = 0; d < 3; ++d) t.dpow2[d] = t.dsig[d] == (1ull << 63) ? 1 : 0;
   const pg::fx::Scale hs = pg::fx::make_scale(h[0]);
   t.hsig = hs.sig;
@@ -311,7 +303,6 @@ static std::vector<unsigned char> tables_impl_f32(const double* lo, const double
   std::memcpy(t.slot_comp0, a.slot_comp0, sizeof(t.slot_comp0));
   std::memcpy(t.out_of, a.out_of, sizeof(t.out_of));
   std::memcpy(t.out_row0, a.out_row0, sizeof(t.out_row0));
-  std::memcpy(t.lane_out, a.lane_out, sizeof(t.lane_out));
   std::vector<unsigned char> out(sizeof(T32));
   std::memcpy(out.data(), &t, sizeof(T32));
   return out;
