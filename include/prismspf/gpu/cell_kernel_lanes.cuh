@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
   const int step1 = qb == k ? -n * CPT : n * CPT;
   const int hpow2 = tab->hpow2, hk = tab->hk;
   const unsigned long long hsig = tab->hsig;
-  for (int i = t; i < 2 * (R.ng + NC) * CPT; i += S::threads) ex_in[i] = i < 2 * R.ng * CPT ? tab->floor_in : tab->floor_out;
+  const unsigned int floor_in = tab->floor_in, floor_out = tab->floor_out;  // (read once: 1 % of a launch)
+  for (int i = t; i < 2 * (R.ng + NC) * CPT; i += S::threads) ex_in[i] = i < 2 * R.ng * CPT ? floor_in : floor_out;
   const unsigned int nn0 = (unsigned int)P.nn[0], nn1 = (unsigned int)P.nn[1];
   const unsigned int lstride = dim > 2 ? nn0 * nn1 : nn0;  // lattice stride of the last direction
   const unsigned int ncells = (unsigned int)P.ncells;
@@ -275,8 +276,8 @@ __global__ void __launch_bounds__(LaneShape<dim, degree>::threads, MINB)
         for (int j = 0; j < n; ++j) x[j * JS] = fx::to_fixed_cut<fx::LANE_TOP_VALUES>(__longlong_as_double(x[j * JS]), E);
       }
     }
-    for (int g = w; g < R.ng; g += cols) exn[g * CPT + lc] = tab->floor_in;
-    for (int o = w; o < NC; o += cols) exon[o * CPT + lc] = tab->floor_out;
+    for (int g = w; g < R.ng; g += cols) exn[g * CPT + lc] = floor_in;
+    for (int o = w; o < NC; o += cols) exon[o * CPT + lc] = floor_out;
     __syncthreads();  // fixed-point copies visible
 
     // the user callback at each of the thread's points

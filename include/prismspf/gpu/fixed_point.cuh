@@ -305,8 +305,7 @@ PPF_FX double to_double_any(unsigned long long a, unsigned int sign, int lsb, bo
   const int lz = clz64(a);  // at least 1
   const unsigned long long r = ((a << (lz - 1)) + 0x200ull) >> 10;
   const int be1 = 1085 + lsb - lz;
-  if (be1 < 0) return double_of(join(0u, sign));
-  if (be1 >= 2046) return double_of(join(0u, 0x7ff00000u | sign));
+  if ((unsigned int)be1 >= 2046u) return double_of(join(0u, (be1 < 0 ? 0u : 0x7ff00000u) | sign));
   const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)be1 << 20);
   return double_of(join((unsigned int)r, hi | sign));
 }
