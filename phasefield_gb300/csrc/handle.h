@@ -103,7 +103,7 @@ struct MGLevel {
   double lambda_min = 0.0;
   double pattern_mean = -1.0;   // mean of the eigenvalue estimate's start pattern over the free rows
   bool eig_done = false;
-  // separable transfer to the next finer level: per axis CSR of the 1-D prolongation
+  // separable transfer to the next finer level (degrees 3 and 4): per axis CSR of the 1-D prolongation
   // (fine index -> coarse entries) and of its transpose (coarse index -> fine entries)
   int* p_ptr[3] = {nullptr, nullptr, nullptr};
   int* p_col[3] = {nullptr, nullptr, nullptr};

@@ -5,14 +5,15 @@
 //   * operator: the LHS cell kernel (MODE_LHS) on each level, src read with the level's
 //     homogeneous constraints, output zero on constrained rows, scaled by invM^1/2 unless the
 //     tolerance type is AbsoluteResidual (MFOperator::compute_operator, mf_operator.cc:17-32);
-//   * diagonal: unit probes (MODE_DIAG), same scaling, zero entries set to one, inverted
+//   * diagonal: unit probes (prismspf/gpu/cell_diagonal.cuh), same scaling, zero entries set to one, inverted
 //     (MFOperator::compute_diagonal + eval_matrix_diagonal, mf_operator.cc:82-255);
 //   * Chebyshev smoother of the first kind on [lambda_max/range, lambda_max] with
 //     lambda_max = 1.2 x the largest eigenvalue of the Lanczos matrix of eig_cg_iterations
 //     CG steps (Jacobi-preconditioned) on the pattern (i mod 11) minus its mean;
-//   * transfers: the Gauss-Lobatto nodal interpolation from a level to the next finer one,
-//     applied axis by axis (prolongation) and its transpose (restriction); images of
-//     periodic nodes are condensed onto their masters and constrained rows zeroed;
+//   * transfers: the Gauss-Lobatto nodal interpolation from a level to the next finer one
+//     (prolongation; in one pass by closed forms for degrees 1 and 2, axis by axis for 3 and 4) and
+//     its transpose (restriction); images of periodic nodes are condensed onto their masters and
+//     constrained rows zeroed;
 //   * V-cycle: pre-smooth from zero (vmult), residual, restrict, recurse, prolongate-add,
 //     post-smooth (step); the coarsest level applies the smoother (MGCoarseGridApplySmoother);
 //   * mixed precision: all levels but the coarsest in FP32 (smoother, level operators,
@@ -136,44 +137,21 @@ __global__ void inv_diag_kernel(T* inv, const T* acc, T* clear, const T* __restr
   }
 }
 
-// One axis of a transfer between two levels as CSR rows (output index -> input entries)
-template <typename T>
-struct AxisRows {
-  const int* ptr;
-  const int* col;
-  const T* val;
-};
-template <typename T>
+// A transfer between two levels
 struct Transfer {
-  AxisRows<T> axis[3];
   int nout[3], nin[3];   // lattice extents of the output and the input level
   int periodic[3];
   int dim;
   long long Nout, Nin;
   pg::fx::FastDiv fd[2];  // multiply-high divisors of nout[0] and nout[1]
-  __device__ __forceinline__ unsigned div(unsigned v, int d) const { return fd[d].div(v); }
-};
-
-// the tensor product of one CSR row per axis applied to `in` (FP entries of type Ti)
-template <typename T, typename Ti>
-__device__ __forceinline__ T transfer_row(const Transfer<T>& A, const Ti* in, int i0, int i1, int i2) {
-  T s2 = T(0);
-  const int b2 = A.dim > 2 ? A.axis[2].ptr[i2] : 0, e2 = A.dim > 2 ? A.axis[2].ptr[i2 + 1] : 1;
-  const int b1 = A.axis[1].ptr[i1], e1 = A.axis[1].ptr[i1 + 1];
-  const int b0 = A.axis[0].ptr[i0], e0 = A.axis[0].ptr[i0 + 1];
-  for (int k2 = b2; k2 < e2; ++k2) {
-    const int c2 = A.dim > 2 ? A.axis[2].col[k2] : 0;
-    T s1 = T(0);
-    for (int k1 = b1; k1 < e1; ++k1) {
-      const Ti* row = in + ((long long)c2 * A.nin[1] + A.axis[1].col[k1]) * A.nin[0];
-      T s0 = T(0);
-      for (int k0 = b0; k0 < e0; ++k0) s0 += A.axis[0].val[k0] * T(row[A.axis[0].col[k0]]);
-      s1 += A.axis[1].val[k1] * s0;
-    }
-    s2 += A.dim > 2 ? A.axis[2].val[k2] * s1 : s1;
+  // the lattice indices of an output node
+  __device__ __forceinline__ void indices(unsigned node, int* i) const {
+    const unsigned r = fd[0].div(node), z = fd[1].div(r);
+    i[0] = (int)(node - r * (unsigned)nout[0]);
+    i[1] = (int)(r - z * (unsigned)nout[1]);
+    i[2] = (int)z;
   }
-  return s2;
-}
+};
 
 // Degrees 1 and 2, whose nodes nest, in closed form. A fine row of an axis is its coarse node, or
 // Q1 {1/2, 1/2}, Q2 {3/8, 3/4, -1/8} and its mirror image on the coarse cell's nodes; a coarse row
@@ -219,110 +197,163 @@ __device__ __forceinline__ float coarse_weight(int i, int o) {
 
 // the row (i0, i1, i2) of the prolongation applied to e
 template <typename T, typename Tc, int degree>
-__device__ __forceinline__ T prolong_row(const Transfer<T>& A, const Tc* e, int i0, int i1, int i2) {
-  if constexpr (degree > 2) {
-    return transfer_row<T, Tc>(A, e, i0, i1, i2);
-  } else {
-    const FineTaps t0 = fine_taps<degree>(i0), t1 = fine_taps<degree>(i1), t2 = fine_taps<degree>(i2);
-    T s2 = T(0);
-    for (int k2 = 0; k2 < t2.n; ++k2) {
-      T s1 = T(0);
-      for (int k1 = 0; k1 < t1.n; ++k1) {
-        const Tc* row = e + ((long long)(t2.c0 + k2) * A.nin[1] + (t1.c0 + k1)) * A.nin[0] + t0.c0;
-        T s0 = T(t0.w[0]) * T(row[0]);
-        if (t0.n > 1) s0 += T(t0.w[1]) * T(row[1]);
-        if (t0.n > 2) s0 += T(t0.w[2]) * T(row[2]);
-        s1 += T(k1 == 0 ? t1.w[0] : (k1 == 1 ? t1.w[1] : t1.w[2])) * s0;
-      }
-      s2 += T(k2 == 0 ? t2.w[0] : (k2 == 1 ? t2.w[1] : t2.w[2])) * s1;
+__device__ __forceinline__ T prolong_row(const Transfer& A, const Tc* e, int i0, int i1, int i2) {
+  const FineTaps t0 = fine_taps<degree>(i0), t1 = fine_taps<degree>(i1), t2 = fine_taps<degree>(i2);
+  T s2 = T(0);
+  for (int k2 = 0; k2 < t2.n; ++k2) {
+    T s1 = T(0);
+    for (int k1 = 0; k1 < t1.n; ++k1) {
+      const Tc* row = e + ((long long)(t2.c0 + k2) * A.nin[1] + (t1.c0 + k1)) * A.nin[0] + t0.c0;
+      T s0 = T(t0.w[0]) * T(row[0]);
+      if (t0.n > 1) s0 += T(t0.w[1]) * T(row[1]);
+      if (t0.n > 2) s0 += T(t0.w[2]) * T(row[2]);
+      s1 += T(k1 == 0 ? t1.w[0] : (k1 == 1 ? t1.w[1] : t1.w[2])) * s0;
     }
-    return s2;
+    s2 += T(k2 == 0 ? t2.w[0] : (k2 == 1 ? t2.w[1] : t2.w[2])) * s1;
   }
+  return s2;
 }
 
 // the coarse row (i0, i1, i2) of the restriction applied to r
 template <typename T, int degree>
-__device__ __forceinline__ T restrict_row(const Transfer<T>& A, const T* r, int i0, int i1, int i2) {
-  if constexpr (degree > 2) {
-    return transfer_row<T, T>(A, r, i0, i1, i2);
-  } else {
-    constexpr int H = degree == 1 ? 1 : 3;
-    const int h0 = degree == 2 && (i0 & 1) ? 1 : H, h1 = degree == 2 && (i1 & 1) ? 1 : H;
-    const int h2 = A.dim < 3 ? 0 : (degree == 2 && (i2 & 1) ? 1 : H);
-    T s2 = T(0);
-    for (int o2 = -h2; o2 <= h2; ++o2) {
-      const T w2 = T(coarse_weight<degree>(i2, o2));
-      const int f2 = 2 * i2 + o2;
-      if (w2 == T(0) || f2 < 0 || f2 >= A.nin[2]) continue;
-      T s1 = T(0);
-      for (int o1 = -h1; o1 <= h1; ++o1) {
-        const T w1 = T(coarse_weight<degree>(i1, o1));
-        const int f1 = 2 * i1 + o1;
-        if (w1 == T(0) || f1 < 0 || f1 >= A.nin[1]) continue;
-        const T* row = r + ((long long)f2 * A.nin[1] + f1) * A.nin[0] + 2 * i0;
-        T s0 = row[0];
-        const T e1 = T(coarse_weight<degree>(i0, 1));
-        if (i0 > 0) s0 += e1 * row[-1];
-        if (2 * i0 + 1 < A.nin[0]) s0 += e1 * row[1];
-        if (h0 == 3) {
-          const T e3 = T(coarse_weight<degree>(i0, 3));
-          if (i0 > 1) s0 += e3 * row[-3];
-          if (2 * i0 + 3 < A.nin[0]) s0 += e3 * row[3];
-        }
-        s1 += w1 * s0;
+__device__ __forceinline__ T restrict_row(const Transfer& A, const T* r, int i0, int i1, int i2) {
+  constexpr int H = degree == 1 ? 1 : 3;
+  const int h0 = degree == 2 && (i0 & 1) ? 1 : H, h1 = degree == 2 && (i1 & 1) ? 1 : H;
+  const int h2 = A.dim < 3 ? 0 : (degree == 2 && (i2 & 1) ? 1 : H);
+  T s2 = T(0);
+  for (int o2 = -h2; o2 <= h2; ++o2) {
+    const T w2 = T(coarse_weight<degree>(i2, o2));
+    const int f2 = 2 * i2 + o2;
+    if (w2 == T(0) || f2 < 0 || f2 >= A.nin[2]) continue;
+    T s1 = T(0);
+    for (int o1 = -h1; o1 <= h1; ++o1) {
+      const T w1 = T(coarse_weight<degree>(i1, o1));
+      const int f1 = 2 * i1 + o1;
+      if (w1 == T(0) || f1 < 0 || f1 >= A.nin[1]) continue;
+      const T* row = r + ((long long)f2 * A.nin[1] + f1) * A.nin[0] + 2 * i0;
+      T s0 = row[0];
+      const T e1 = T(coarse_weight<degree>(i0, 1));
+      if (i0 > 0) s0 += e1 * row[-1];
+      if (2 * i0 + 1 < A.nin[0]) s0 += e1 * row[1];
+      if (h0 == 3) {
+        const T e3 = T(coarse_weight<degree>(i0, 3));
+        if (i0 > 1) s0 += e3 * row[-3];
+        if (2 * i0 + 3 < A.nin[0]) s0 += e3 * row[3];
       }
-      s2 += w2 * s1;
+      s1 += w1 * s0;
     }
-    return s2;
+    s2 += w2 * s1;
+  }
+  return s2;
+}
+
+// Degrees 3 and 4 go axis by axis. A coarse row of degree 4 has up to 17 entries an axis, a fine one 5:
+// all axes in one pass are 4,913 and 125 multiplications a row where three passes take 51 and 15.
+// (V-cycle-preconditioned CG on 8^3 cells, three levels: degree 3 65 ms and degree 4 385 ms in one pass,
+// 57 and 276 ms with a launch per axis and component, 42 and 227 ms this way.)
+template <typename T>
+struct AxisPass {
+  const int* ptr;  // CSR rows of the axis: output index -> input entries
+  const int* col;
+  const T* val;
+  int axis, nin;   // and the input's extent along it; the others are the output's
+  Transfer g;      // the pass's output (nout, Nout, and the input's Nin)
+};
+
+template <typename T, typename Ti>
+__device__ __forceinline__ T axis_row(const AxisPass<T>& A, const Ti* in, const int* i) {
+  const int row = A.axis == 0 ? i[0] : (A.axis == 1 ? i[1] : i[2]);
+  const long long d0 = A.axis == 0 ? A.nin : A.g.nout[0], d1 = A.axis == 1 ? A.nin : A.g.nout[1];
+  const long long step = A.axis == 0 ? 1 : (A.axis == 1 ? d0 : d0 * d1);
+  const Ti* line = in + ((A.axis == 2 ? 0 : i[2]) * d1 + (A.axis == 1 ? 0 : i[1])) * d0 + (A.axis == 0 ? 0 : i[0]);
+  T s = T(0);
+  for (int k = A.ptr[row]; k < A.ptr[row + 1]; ++k) s += A.val[k] * T(line[A.col[k] * step]);
+  return s;
+}
+
+// one axis of a transfer before the last
+template <typename T, typename Ti>
+__global__ void __launch_bounds__(256) transfer_axis_kernel(const __grid_constant__ AxisPass<T> A, T* out, const Ti* in) {
+  chain_wait();
+  chain_release();
+  const long long N = A.g.Nout;
+  for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < N; n += (long long)gridDim.x * blockDim.x) {
+    int i[3];
+    A.g.indices((unsigned)n, i);
+    out[blockIdx.y * N + n] = axis_row<T, Ti>(A, in + blockIdx.y * A.g.Nin, i);
   }
 }
 
-// x += P e from the coarse correction e (type Tc): all axes in one pass (at most 27 entries a row,
-// 8 on average for Q2 3-D, read from L1/L2), where one launch per component and axis went through
-// fine-sized work vectors; images take their master's row, Dirichlet rows nothing
-template <typename T, typename Tc, int degree>
-__global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_constant__ Transfer<T> A, T* x, const Tc* e,
-                                                             const int* __restrict__ cmap) {
-  chain_wait();
-  chain_release();
+// x += P e: with `row` the prolongation's row at a lattice node; images take their master's row,
+// Dirichlet rows nothing
+template <typename T, class Row>
+__device__ __forceinline__ void prolongate_add(const Transfer& A, T* x, const int* __restrict__ cmap, Row&& row) {
   const long long base = blockIdx.y * A.Nout;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
     const int m = cmap ? cmap[base + i] : (int)(base + i);
     if (m < 0) continue;
-    const unsigned node = (unsigned)(m - base);
-    const unsigned r = A.div(node, 0);
-    const int i0 = (int)(node - r * (unsigned)A.nout[0]);
-    const int i2 = (int)A.div(r, 1);
-    const int i1 = (int)(r - (unsigned)i2 * (unsigned)A.nout[1]);
-    x[base + i] += prolong_row<T, Tc, degree>(A, e + blockIdx.y * A.Nin, i0, i1, i2);
+    int k[3];
+    A.indices((unsigned)(m - base), k);
+    x[base + i] += row(k);
   }
 }
 
-// b = P^T r on the coarse level (stored as Tc): all axes in one pass; a periodic node sums its
-// images' rows as well, constrained rows are zero
-template <typename T, typename Tc, int degree>
-__global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ Transfer<T> A, Tc* b, const T* r,
-                                                       const int* __restrict__ cmap) {
-  chain_wait();
-  chain_release();
+// b = P^T r on the coarse level: with `row` the restriction's row at a lattice node; a periodic node
+// sums its images' rows as well, constrained rows are zero
+template <typename T, typename Tc, class Row>
+__device__ __forceinline__ void restrict_to(const Transfer& A, Tc* b, const int* __restrict__ cmap, Row&& row) {
   const long long base = blockIdx.y * A.Nout;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < A.Nout; i += (long long)gridDim.x * blockDim.x) {
     T s = T(0);
     if (!cmap || cmap[base + i] == (int)(base + i)) {
-      const unsigned node = (unsigned)i;
-      const unsigned q = A.div(node, 0);
-      const int i0 = (int)(node - q * (unsigned)A.nout[0]);
-      const int i2 = (int)A.div(q, 1);
-      const int i1 = (int)(q - (unsigned)i2 * (unsigned)A.nout[1]);
-      const int m0 = A.periodic[0] && i0 == 0, m1 = A.periodic[1] && i1 == 0, m2 = A.periodic[2] && i2 == 0;
+      int k[3];
+      A.indices((unsigned)i, k);
+      const int m0 = A.periodic[0] && k[0] == 0, m1 = A.periodic[1] && k[1] == 0, m2 = A.periodic[2] && k[2] == 0;
       for (int e2 = 0; e2 <= m2; ++e2)
         for (int e1 = 0; e1 <= m1; ++e1)
-          for (int e0 = 0; e0 <= m0; ++e0)
-            s += restrict_row<T, degree>(A, r + blockIdx.y * A.Nin, e0 ? A.nout[0] - 1 : i0, e1 ? A.nout[1] - 1 : i1,
-                                         e2 ? A.nout[2] - 1 : i2);
+          for (int e0 = 0; e0 <= m0; ++e0) {
+            const int image[3] = {e0 ? A.nout[0] - 1 : k[0], e1 ? A.nout[1] - 1 : k[1], e2 ? A.nout[2] - 1 : k[2]};
+            s += row(image);
+          }
     }
     b[base + i] = Tc(s);
   }
+}
+
+// Degrees 1 and 2: all axes in one pass (at most 27 entries a row, 8 on average for Q2 3-D, read from
+// L1/L2), where one launch per component and axis went through fine-sized work vectors
+template <typename T, typename Tc, int degree>
+__global__ void __launch_bounds__(256) prolongate_add_kernel(const __grid_constant__ Transfer A, T* x, const Tc* e,
+                                                             const int* __restrict__ cmap) {
+  chain_wait();
+  chain_release();
+  const Tc* in = e + blockIdx.y * A.Nin;
+  prolongate_add(A, x, cmap, [&](const int* k) { return prolong_row<T, Tc, degree>(A, in, k[0], k[1], k[2]); });
+}
+template <typename T, typename Tc, int degree>
+__global__ void __launch_bounds__(256) restrict_kernel(const __grid_constant__ Transfer A, Tc* b, const T* r,
+                                                       const int* __restrict__ cmap) {
+  chain_wait();
+  chain_release();
+  const T* in = r + blockIdx.y * A.Nin;
+  restrict_to<T>(A, b, cmap, [&](const int* k) { return restrict_row<T, degree>(A, in, k[0], k[1], k[2]); });
+}
+// the last axis of the others
+template <typename T>
+__global__ void __launch_bounds__(256) prolongate_add_axis_kernel(const __grid_constant__ AxisPass<T> A, T* x, const T* e,
+                                                                  const int* __restrict__ cmap) {
+  chain_wait();
+  chain_release();
+  const T* in = e + blockIdx.y * A.g.Nin;
+  prolongate_add(A.g, x, cmap, [&](const int* k) { return axis_row<T, T>(A, in, k); });
+}
+template <typename T, typename Tc>
+__global__ void __launch_bounds__(256) restrict_axis_kernel(const __grid_constant__ AxisPass<T> A, Tc* b, const T* r,
+                                                            const int* __restrict__ cmap) {
+  chain_wait();
+  chain_release();
+  const T* in = r + blockIdx.y * A.g.Nin;
+  restrict_to<T>(A.g, b, cmap, [&](const int* k) { return axis_row<T, T>(A, in, k); });
 }
 
 // First Chebyshev step from x = 0: x = u = c2 P b
@@ -455,12 +486,6 @@ __global__ void lift_values_kernel(double* g, const int* __restrict__ cmap, cons
 // helpers
 // ------------------------------------------------------------------------------------------
 static size_t esize(int precision) { return precision ? sizeof(float) : sizeof(double); }
-
-template <typename F>
-static void by_precision(int precision, F&& f) {
-  if (precision) f(float(0));
-  else f(double(0));
-}
 
 // blocks of a reduction over n entries (at most 1024 partial sums)
 static unsigned dot_blocks(long long n) { return (unsigned)std::max<long long>(1, std::min<long long>(1024, (n + 255) / 256)); }
@@ -956,26 +981,82 @@ static int chebyshev(ppf_handle h, BlockState& B, MGLevel& lv, bool zero_start, 
   return PPF_OK;
 }
 
-// the transfer between level c and the next finer one f, output on f (prolongation) or on c
-template <typename T>
-static Transfer<T> transfer(ppf_handle h, const MGLevel& c, const MGLevel& f, bool prolongate) {
-  Transfer<T> A;
+// the transfer between lattices of extents nin and nout
+static Transfer transfer(ppf_handle h, const int* nout, const int* nin) {
+  Transfer A;
   std::memset(&A, 0, sizeof(A));
-  const MGLevel& out = prolongate ? f : c;
-  const MGLevel& in = prolongate ? c : f;
   A.dim = h->dim;
+  A.Nout = A.Nin = 1;
   for (int d = 0; d < 3; ++d) {
-    A.nout[d] = out.nn[d];
-    A.nin[d] = in.nn[d];
+    A.nout[d] = nout[d];
+    A.nin[d] = nin[d];
     A.periodic[d] = d < h->dim ? h->mesh.periodic[d] : 0;
-    A.axis[d].ptr = prolongate ? c.p_ptr[d] : c.r_ptr[d];
-    A.axis[d].col = prolongate ? c.p_col[d] : c.r_col[d];
-    A.axis[d].val = (const T*)(prolongate ? c.p_val[d] : c.r_val[d]);
+    A.Nout *= nout[d];
+    A.Nin *= nin[d];
   }
-  A.Nout = out.N;
-  A.Nin = in.N;
-  for (int d = 0; d < 2; ++d) A.fd[d].init((unsigned)out.nn[d]);
+  for (int d = 0; d < 2; ++d) A.fd[d].init((unsigned)nout[d]);
   return A;
+}
+
+// The passes of a transfer of degree 3 or 4 between level c and the next finer one f, the last axis
+// left to `last(pass, in)`; the levels' work vectors of a smoothing step hold what lies in between
+template <typename T, typename Ti, class Last>
+static int transfer_axes(ppf_handle h, const BlockState& B, const MGLevel& c, const MGLevel& f, bool prolongate,
+                         const Ti* in, Last&& last) {
+  const int ncomp = h->fields[B.desc.field_indices[0]].ncomp;
+  int n[3] = {1, 1, 1};
+  for (int d = 0; d < 3; ++d) n[d] = prolongate ? c.nn[d] : f.nn[d];
+  const T* from = nullptr;
+  for (int d = 0; d < h->dim; ++d) {
+    AxisPass<T> A;
+    A.ptr = prolongate ? c.p_ptr[d] : c.r_ptr[d];
+    A.col = prolongate ? c.p_col[d] : c.r_col[d];
+    A.val = (const T*)(prolongate ? c.p_val[d] : c.r_val[d]);
+    A.axis = d;
+    A.nin = n[d];
+    int out[3] = {n[0], n[1], n[2]};
+    out[d] = prolongate ? f.nn[d] : c.nn[d];
+    A.g = transfer(h, out, n);
+    if (d == h->dim - 1) return last(A, from);
+    T* to = (T*)(d == 0 ? f.w1 : f.w0);
+    const dim3 grid(grid_for(A.g.Nout), ncomp);
+    if (d == 0) PPF_CUDA(h, launch_chained(transfer_axis_kernel<T, Ti>, grid, dim3(256), 0, h->stream, A, to, in));
+    else PPF_CUDA(h, launch_chained(transfer_axis_kernel<T, T>, grid, dim3(256), 0, h->stream, A, to, from));
+    h->all_launches++;
+    from = to;
+    n[d] = out[d];
+  }
+  return PPF_OK;
+}
+
+// c.b = P^T f.r
+template <typename T, typename Tc>
+static int restrict_residual(ppf_handle h, const BlockState& B, MGLevel& c, const MGLevel& f) {
+  const dim3 grid = level_grid(h, B, c);
+  h->all_launches++;
+  if (h->k > 2)
+    return transfer_axes<T, T>(h, B, c, f, false, (const T*)f.r, [&](const AxisPass<T>& A, const T* in) -> int {
+      PPF_CUDA(h, launch_chained(restrict_axis_kernel<T, Tc>, grid, dim3(256), 0, h->stream, A, (Tc*)c.b, in, level_map(c)));
+      return PPF_OK;
+    });
+  PPF_CUDA(h, launch_chained(h->k == 1 ? restrict_kernel<T, Tc, 1> : restrict_kernel<T, Tc, 2>, grid, dim3(256), 0,
+                             h->stream, transfer(h, c.nn, f.nn), (Tc*)c.b, (const T*)f.r, level_map(c)));
+  return PPF_OK;
+}
+
+// x += P c.x on level f
+template <typename T, typename Tc>
+static int prolongate_correction(ppf_handle h, const BlockState& B, const MGLevel& c, const MGLevel& f, T* x) {
+  const dim3 grid = level_grid(h, B, f);
+  h->all_launches++;
+  if (h->k > 2)
+    return transfer_axes<T, Tc>(h, B, c, f, true, (const Tc*)c.x, [&](const AxisPass<T>& A, const T* in) -> int {
+      PPF_CUDA(h, launch_chained(prolongate_add_axis_kernel<T>, grid, dim3(256), 0, h->stream, A, x, in, level_map(f)));
+      return PPF_OK;
+    });
+  PPF_CUDA(h, launch_chained(h->k == 1 ? prolongate_add_kernel<T, Tc, 1> : prolongate_add_kernel<T, Tc, 2>, grid,
+                             dim3(256), 0, h->stream, transfer(h, f.nn, c.nn), x, (const Tc*)c.x, level_map(f)));
+  return PPF_OK;
 }
 
 static int vcycle(ppf_handle h, BlockState& B, int l, const void* b, void* x);
@@ -994,17 +1075,10 @@ static int vcycle_level(ppf_handle h, BlockState& B, int l, const T* b, T* x) {
   PPF_CUDA(h, launch_chained(residual_kernel<T>, level_grid(h, B, lv), dim3(256), 0, h->stream, (T*)lv.r, b,
                              (const T*)lv.acc, (T*)lv.acc2, level_scale<T>(B.lin, lv), lv.N));
   level_took(lv);
-  auto restriction = h->k == 1 ? restrict_kernel<T, Tc, 1> : (h->k == 2 ? restrict_kernel<T, Tc, 2> : restrict_kernel<T, Tc, 3>);
-  PPF_CUDA(h, launch_chained(restriction, level_grid(h, B, cl), dim3(256), 0, h->stream,
-                             transfer<T>(h, cl, lv, false), (Tc*)cl.b, (const T*)lv.r, level_map(cl)));
-  h->all_launches += 2;
-  rc = vcycle(h, B, l - 1, cl.b, cl.x);
-  if (rc) return rc;
-  auto prolongation = h->k == 1 ? prolongate_add_kernel<T, Tc, 1>
-                                : (h->k == 2 ? prolongate_add_kernel<T, Tc, 2> : prolongate_add_kernel<T, Tc, 3>);
-  PPF_CUDA(h, launch_chained(prolongation, level_grid(h, B, lv), dim3(256), 0, h->stream,
-                             transfer<T>(h, cl, lv, true), x, (const Tc*)cl.x, level_map(lv)));
   h->all_launches++;
+  if ((rc = restrict_residual<T, Tc>(h, B, cl, lv))) return rc;
+  if ((rc = vcycle(h, B, l - 1, cl.b, cl.x))) return rc;
+  if ((rc = prolongate_correction<T, Tc>(h, B, cl, lv, x))) return rc;
   return chebyshev<T>(h, B, lv, false, b, x);
 }
 
@@ -1153,8 +1227,9 @@ static int init_linear(ppf_handle h, int b) {
     lv.acc_clean = true;
     (void)is_fine;
   }
-  // transfers between consecutive levels (stored on the coarse level; work buffers on the fine)
-  for (int l = 0; l + 1 < depth; ++l) {
+  // transfers between consecutive levels as rows of each axis (stored on the coarse level; degrees 1
+  // and 2 have closed forms)
+  for (int l = 0; l + 1 < depth && h->k > 2; ++l) {
     MGLevel& cl = L.levels[l];
     MGLevel& fl = L.levels[l + 1];
     const int tp = fl.precision;  // transfers run in the fine level's precision
