@@ -135,8 +135,8 @@ struct CellLaunch {
   int fx_deriv;
   int fx_int;
   // the lane kernel (prismspf/gpu/cell_kernel_lanes.cuh): all-integer contractions of an FP64
-  // Q1/Q2 operator on cubic cells, when the tables allow it (fx_lanes); it takes the host copy
-  // of `tables` (tables_host) as a kernel parameter
+  // Q1/Q2 operator, when the tables allow it (fx_lanes); it takes the host copy of `tables`
+  // (tables_host) as a kernel parameter
   int fx_lanes;
   const void* tables_host;
   // cell index -> coordinates: multiply-high divisors of nc[0] and nc[1] (filled by the launchers: a

@@ -402,7 +402,8 @@ size_t cell_smem(int dim, int degree, int precision, int nrows_in, int nrows_out
 // accumulator of the field, which nothing reads any more) is zeroed for the next solve, and `timer`
 // (in a captured increment, after its last block) advanced: work that took a memset and a launch of
 // their own (128^2 Q1 Allen-Cahn: 12.9 us an increment before, with four launches).
-// Bound by memory: 36 bytes a node plus 8 for `clear`; four rows in flight a thread.
+// Bound by memory: 28 bytes a node (24 without constraints), 8 more for `clear` and 8 for u2; four rows
+// in flight a thread.
 __global__ void __launch_bounds__(256) finalize_explicit_kernel(double* u, const double* acc, double* clear,
                                                                 const double* __restrict__ invm,
                                                                 const int* __restrict__ cmap, const double* dvals,
